@@ -1,4 +1,4 @@
-// Plain attention over the paged cache: one warp per (token, query head).
+// Plain attention over the paged cache: one warp per (token, query head), or several where those are few.
 //
 // It is the float32 path's attention and the reference kernel that the faster
 // bfloat16 kernels are checked against.  It serves prompts, chunks of prompts and
@@ -46,90 +46,141 @@ struct AttnSimpleArgs {
     float softcap;            // 0: scores are not capped
 };
 
-#define ATTN_SIMPLE_WARPS 4
+#define ATTN_SIMPLE_WARPS 8
 #define ATTN_SIMPLE_MAX_HD 256
 
-template <typename T>
+// The keys of an item are walked 32 at a time.  A step of few (token, head) pairs leaves most of the machine idle with one warp an item
+// (24 items of 200 keys: 170 us, a chain of 7 blocks of keys whose loads wait on one another), so `wpi` warps of a CTA share
+// an item, every wpi-th block of keys each, and the first of them merges their maxima, denominators and sums in order.  Keys are
+// read 16 bytes at a time where a head's rows allow it (WIDE), values of four keys at a time, in the order of the keys.
+template <typename T, int NI, bool WIDE>
 __global__ void __launch_bounds__(ATTN_SIMPLE_WARPS * 32)
-attn_simple_kernel(AttnSimpleArgs a) {
+attn_simple_kernel(AttnSimpleArgs a, int wpi) {
     pdl_trigger();
     pdl_wait();
-    extern __shared__ float smem[];                  // [warps][hd] queries, [warps][32] probabilities
+    extern __shared__ __align__(16) float smem[];    // [warps][hd] queries, later sums; [warps][32] probabilities; [warps][2]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* qs = smem + warp * a.hd;
-    float* ps = smem + ATTN_SIMPLE_WARPS * a.hd + warp * 32;
-    const long long item = (long long)blockIdx.x * ATTN_SIMPLE_WARPS + warp;
-    if (item >= (long long)a.rows * a.nqh * a.value_heads) return;
-    const int row = (int)(item / (a.nqh * a.value_heads));
-    const int vhead = (int)(item - (long long)row * a.nqh * a.value_heads);       // head * value_heads + value head
+    const int hdp = (a.hd + 3) & ~3;
+    float* qs = smem + warp * hdp;
+    float* ps = smem + ATTN_SIMPLE_WARPS * hdp + warp * 32;
+    float* ml = smem + ATTN_SIMPLE_WARPS * (hdp + 32);
+    const int per = ATTN_SIMPLE_WARPS / wpi, slice = warp % wpi;
+    const long long item = (long long)blockIdx.x * per + warp / wpi;
+    const bool live = item < (long long)a.rows * a.nqh * a.value_heads;
+    const int row = live ? (int)(item / (a.nqh * a.value_heads)) : 0;
+    const int vhead = live ? (int)(item - (long long)row * a.nqh * a.value_heads) : 0;       // head * value_heads + value head
     const int head = vhead / a.value_heads;
     T* o = (T*)a.out + (size_t)row * a.out_row_stride + (size_t)vhead * a.hd;
-    const int seq = a.token_seq[row];
+    const int seq = live ? a.token_seq[row] : -1;
+    float m = -INFINITY, l = 0.f;
+    float acc[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) acc[i] = 0.f;
+    if (seq >= 0) {
+        const int pos = a.positions[row];
+        const int kvh = head / (a.nqh / a.nkh);
+        const int val_h = a.value_heads > 1 ? vhead - head * a.value_heads : kvh;
+        const float scale = a.head_scale ? a.scale * a.head_scale[head] : a.scale;
+        const float r1 = a.bias_slope ? a.bias_slope[head] : 0.f, r2 = a.bias_slope ? a.bias_rate[head] : 0.f;
+        const T* q = (const T*)a.q + (size_t)row * a.q_row_stride + (size_t)head * a.hd;
+        for (int d = lane; d < a.hd; d += 32) qs[d] = to_f32(q[d]);
+        __syncwarp();
+
+        const int lo = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
+        const int* table = a.page_table + (size_t)seq * a.table_cols;
+        const size_t head_stride = (size_t)a.page_size * a.hd;
+        int turn = 0;                                            // blocks of keys so far
+
+        const int kept = a.keep_first < lo ? a.keep_first : lo;      // kept first positions that the window has left
+        for (int part = kept > 0 ? 0 : 1; part < 2; ++part) {
+        const int end = part ? pos + 1 : kept;
+        for (int j0 = part ? lo : 0; j0 < end; j0 += 32, ++turn) {
+            if (turn % wpi != slice) continue;
+            const int j = j0 + lane;
+            float s = -INFINITY;
+            const T* vrow = nullptr;
+            if (j < end) {
+                const int block = j / a.page_size, off = j - block * a.page_size;
+                int page = (block < a.table_cols) ? table[block] : -1;
+                if (page < 0 || page >= a.num_pages) {      // never followed: flag it and read page 0 instead
+                    atomicExch(a.error_flag, 1);
+                    page = 0;
+                }
+                const T* kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
+                vrow = kbase + (size_t)(a.nkh + val_h - kvh) * head_stride;
+                float dot = 0.f;
+                if (WIDE) {
+                    constexpr int VW = 16 / sizeof(T);
+#pragma unroll 4
+                    for (int d = 0; d < a.hd; d += VW) {
+                        float kv[VW];
+                        load_run<T, VW>(kbase + d, kv);
+#pragma unroll
+                        for (int e = 0; e < VW; ++e) dot = fmaf(qs[d + e], kv[e], dot);
+                    }
+                } else {
+                    for (int d = 0; d < a.hd; ++d) dot = fmaf(qs[d], to_f32(kbase[d]), dot);
+                }
+                s = dot * scale;
+                if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+                if (a.bias_slope) s -= r1 * log1pf(r2 * (float)(pos - j));
+            }
+            const float cmax = warp_max(s);
+            const float m_new = fmaxf(m, cmax);
+            const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
+            const float p = (j < end) ? expf(s - m_new) : 0.f;
+            l = l * corr + warp_sum(p);
+            m = m_new;
+            ps[lane] = p;
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[i] *= corr;
+            const int n_valid = min(32, end - j0);
+            for (int jj = 0; jj < n_valid; jj += 4) {
+                float v[4][NI];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, jj + k);
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) v[k][i] = (jj + k < n_valid && lane + 32 * i < a.hd) ? to_f32(vr[lane + 32 * i]) : 0.f;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (jj + k < n_valid) {
+                        const float pj = ps[jj + k];
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, v[k][i], acc[i]);
+                    }
+            }
+            __syncwarp();
+        }
+        }
+    }
+    if (wpi > 1) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (lane + 32 * i < a.hd) qs[lane + 32 * i] = acc[i];
+        if (lane == 0) { ml[2 * warp] = m; ml[2 * warp + 1] = l; }
+        __syncthreads();
+        if (slice) return;
+        for (int w = 1; w < wpi; ++w) {
+            const float mw = ml[2 * (warp + w)], lw = ml[2 * (warp + w) + 1];
+            if (mw == -INFINITY) continue;                       // a warp without keys
+            const float m_new = fmaxf(m, mw);
+            const float mine = (m == -INFINITY) ? 0.f : expf(m - m_new), its = expf(mw - m_new);
+            l = l * mine + lw * its;
+            m = m_new;
+            const float* other = qs + w * hdp;
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+                if (lane + 32 * i < a.hd) acc[i] = acc[i] * mine + other[lane + 32 * i] * its;
+        }
+    }
+    if (!live) return;
     if (seq < 0) {
         for (int d = lane; d < a.hd; d += 32) o[d] = from_f32<T>(0.f);
         return;
-    }
-    const int pos = a.positions[row];
-    const int kvh = head / (a.nqh / a.nkh);
-    const int val_h = a.value_heads > 1 ? vhead - head * a.value_heads : kvh;
-    const float scale = a.head_scale ? a.scale * a.head_scale[head] : a.scale;
-    const float r1 = a.bias_slope ? a.bias_slope[head] : 0.f, r2 = a.bias_slope ? a.bias_rate[head] : 0.f;
-    const T* q = (const T*)a.q + (size_t)row * a.q_row_stride + (size_t)head * a.hd;
-    for (int d = lane; d < a.hd; d += 32) qs[d] = to_f32(q[d]);
-    __syncwarp();
-
-    const int lo = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
-    float m = -INFINITY, l = 0.f;
-    float acc[ATTN_SIMPLE_MAX_HD / 32];
-#pragma unroll
-    for (int i = 0; i < ATTN_SIMPLE_MAX_HD / 32; ++i) acc[i] = 0.f;
-    const int* table = a.page_table + (size_t)seq * a.table_cols;
-    const size_t head_stride = (size_t)a.page_size * a.hd;
-
-    const int kept = a.keep_first < lo ? a.keep_first : lo;      // kept first positions that the window has left
-    for (int part = kept > 0 ? 0 : 1; part < 2; ++part) {
-    const int end = part ? pos + 1 : kept;
-    for (int j0 = part ? lo : 0; j0 < end; j0 += 32) {
-        const int j = j0 + lane;
-        float s = -INFINITY;
-        const T* vrow = nullptr;
-        if (j < end) {
-            const int block = j / a.page_size, off = j - block * a.page_size;
-            int page = (block < a.table_cols) ? table[block] : -1;
-            if (page < 0 || page >= a.num_pages) {      // never followed: flag it and read page 0 instead
-                atomicExch(a.error_flag, 1);
-                page = 0;
-            }
-            const T* kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
-            vrow = kbase + (size_t)(a.nkh + val_h - kvh) * head_stride;
-            float dot = 0.f;
-            for (int d = 0; d < a.hd; ++d) dot = fmaf(qs[d], to_f32(kbase[d]), dot);
-            s = dot * scale;
-            if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
-            if (a.bias_slope) s -= r1 * log1pf(r2 * (float)(pos - j));
-        }
-        const float cmax = warp_max(s);
-        const float m_new = fmaxf(m, cmax);
-        const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-        const float p = (j < end) ? expf(s - m_new) : 0.f;
-        l = l * corr + warp_sum(p);
-        m = m_new;
-        ps[lane] = p;
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < ATTN_SIMPLE_MAX_HD / 32; ++i) acc[i] *= corr;
-        const int n_valid = min(32, end - j0);
-        for (int jj = 0; jj < n_valid; ++jj) {
-            const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, jj);
-            const float pj = ps[jj];
-#pragma unroll
-            for (int i = 0; i < ATTN_SIMPLE_MAX_HD / 32; ++i) {
-                const int d = lane + 32 * i;
-                if (d < a.hd) acc[i] = fmaf(pj, to_f32(vr[d]), acc[i]);
-            }
-        }
-        __syncwarp();
-    }
     }
     float corr_end = 1.f;
     if (a.has_sink) {                                // the sink joins as one more score, with no value
@@ -141,9 +192,32 @@ attn_simple_kernel(AttnSimpleArgs a) {
     float inv = corr_end * a.out_scale / l;
     if (a.head_gate) inv *= 1.f / (1.f + expf(-to_f32(((const T*)a.head_gate)[(size_t)row * a.gate_stride + head])));
 #pragma unroll
-    for (int i = 0; i < ATTN_SIMPLE_MAX_HD / 32; ++i) {
+    for (int i = 0; i < NI; ++i) {
         const int d = lane + 32 * i;
         if (d < a.hd) o[d] = from_f32<T>(acc[i] * inv);
+    }
+}
+
+template <typename T>
+static void attn_simple_launch(const AttnSimpleArgs& a, cudaStream_t s) {
+    const long long items = (long long)a.rows * a.nqh * a.value_heads;
+    // some 16 warps an SM, as long as a warp has a block of 32 keys of the longest context that the tables can hold
+    const long long span = a.window > 0 ? (long long)a.window + a.keep_first : (long long)a.table_cols * a.page_size;
+    int wpi = 1;
+    while (wpi < ATTN_SIMPLE_WARPS && items * wpi < 16 * 148 && 32LL * wpi < span) wpi *= 2;
+    const int per = ATTN_SIMPLE_WARPS / wpi;
+    const dim3 grid((unsigned)((items + per - 1) / per)), block(ATTN_SIMPLE_WARPS * 32);
+    const size_t smem = (size_t)ATTN_SIMPLE_WARPS * (((a.hd + 3) & ~3) + 32 + 2) * sizeof(float);
+    const bool wide = (a.hd * sizeof(T)) % 16 == 0 && ((uintptr_t)a.cache & 15) == 0;
+    if (a.hd <= 64) {
+        if (wide) braid_launch(attn_simple_kernel<T, 2, true>, grid, block, smem, s, a, wpi);
+        else braid_launch(attn_simple_kernel<T, 2, false>, grid, block, smem, s, a, wpi);
+    } else if (a.hd <= 128) {
+        if (wide) braid_launch(attn_simple_kernel<T, 4, true>, grid, block, smem, s, a, wpi);
+        else braid_launch(attn_simple_kernel<T, 4, false>, grid, block, smem, s, a, wpi);
+    } else {
+        if (wide) braid_launch(attn_simple_kernel<T, 8, true>, grid, block, smem, s, a, wpi);
+        else braid_launch(attn_simple_kernel<T, 8, false>, grid, block, smem, s, a, wpi);
     }
 }
 
@@ -170,12 +244,10 @@ extern "C" int braid_attn_simple(const void* q, void* out, int dtype, const void
                      rows, nqh, nkh, hd, page_size, table_cols, num_pages, window, scale, has_sink || head_sinks != nullptr, sink_score, out_scale, error_flag, head_sinks, head_gate, gate_stride,
                      keep_first, head_scale, value_heads, bias_slope, bias_rate, softcap};
     const long long items = (long long)rows * nqh * value_heads;
-    const long long blocks = (items + ATTN_SIMPLE_WARPS - 1) / ATTN_SIMPLE_WARPS;
-    if (blocks > 0x7fffffffLL) BRAID_REFUSE("attn_simple: %lld (token, head) pairs exceed one launch", items);
-    const size_t smem = (size_t)ATTN_SIMPLE_WARPS * (hd + 32) * sizeof(float);
+    if (items / ATTN_SIMPLE_WARPS >= 0x7fffffffLL) BRAID_REFUSE("attn_simple: %lld (token, head) pairs exceed one launch", items);
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == BRAID_F32) braid_launch(attn_simple_kernel<float>, dim3((int)blocks), dim3(ATTN_SIMPLE_WARPS * 32), smem, s, a);
-    else if (dtype == BRAID_BF16) braid_launch(attn_simple_kernel<__nv_bfloat16>, dim3((int)blocks), dim3(ATTN_SIMPLE_WARPS * 32), smem, s, a);
+    if (dtype == BRAID_F32) attn_simple_launch<float>(a, s);
+    else if (dtype == BRAID_BF16) attn_simple_launch<__nv_bfloat16>(a, s);
     else BRAID_REFUSE("attn_simple: unknown dtype code %d", dtype);
     BRAID_LAUNCH_CHECK();
 }
