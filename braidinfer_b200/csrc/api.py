@@ -11,7 +11,7 @@ import ctypes
 import os
 from ctypes import c_int, c_longlong, c_float, c_void_p, c_char_p
 from dataclasses import dataclass
-from typing import List, Optional, Tuple
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -65,6 +65,28 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.cat([g.view(blocks, 16, k), u.view(blocks, 16, k)], dim=1).reshape(blocks * 32, k).contiguous()
 
 
+def interleave_experts(gate: Sequence[torch.Tensor], up: Sequence[torch.Tensor]) -> torch.Tensor:
+    """[experts, 2 * (J rounded up to 16), K]: every expert's gate and up rows as `interleave_gate_up` lays them."""
+    (j, k), n = gate[0].shape, len(gate)
+    blocks = -(-j // 16)
+    w = gate[0].new_empty((n, blocks, 2, 16, k)) if j % 16 == 0 else gate[0].new_zeros((n, blocks, 2, 16, k))
+    whole = j // 16
+    for i, part in enumerate((gate, up)):
+        rows = torch.stack(tuple(part))
+        w[:, :whole, i] = rows[:, :16 * whole].reshape(n, whole, 16, k)
+        if j % 16:
+            w[:, whole, i, :j % 16] = rows[:, 16 * whole:]
+    return w.view(n, blocks * 32, k)
+
+
+def expert_halves(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Gate and up of `interleave_experts` as views [experts, J / 16, 16, K] (J rounded up)."""
+    e, n, k = w.shape
+    v = w.view(e, n // 32, 2, 16, k)
+    return v[:, :, 0], v[:, :, 1]
+
+
+MOE_TC_TILE = 32             # slots a tile of the plan that the experts' products on pairs of SMs walk
 PAIR_TOKEN_TILE = 256        # the token tile of the kernel that runs on pairs of SMs
 # Tokens a chunk of a long prompt's recurrence (csrc/scan.cu): 128 for sequences of 1,024 tokens and more, 64 below
 # (2,048 tokens, 8 heads of 128 x 256: 0.42 / 0.32 / 0.29 / 0.30 ms with chunks of 32 / 64 / 128 / 256); steps whose
@@ -703,15 +725,17 @@ class Kernels:
                          "braid_mlstm_out")
             elif name == "moe":
                 lib.braid_moe_route.argtypes = [c_void_p] * 3 + [c_int] * 5 + [c_float, c_int, c_int, c_void_p, c_void_p]
-                lib.braid_moe_plan.argtypes = [c_void_p] * 6 + [c_int] * 5 + [c_void_p]
+                lib.braid_moe_plan.argtypes = [c_void_p] * 7 + [c_int] * 6 + [c_void_p]
                 lib.braid_moe_gemm_simt.argtypes = [c_void_p] * 7 + [c_int, c_int, c_longlong, c_longlong] + [c_int] * 5 + \
-                                                   [c_void_p, c_void_p]
+                                                   [c_void_p, c_longlong, c_longlong, c_void_p]
                 lib.braid_moe_combine.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                                                   c_longlong, c_void_p]
                 lib.braid_moe_gemm_mma.argtypes = [c_void_p] * 7 + [c_int, c_longlong, c_longlong] + [c_int] * 5 + \
-                                                  [c_void_p, c_void_p]
-                lib.braid_moe_gemm_mma.restype = c_int
-                names = ("braid_moe_route", "braid_moe_plan", "braid_moe_gemm_simt", "braid_moe_combine")
+                                                  [c_void_p, c_longlong, c_longlong, c_void_p]
+                lib.braid_moe_gather.argtypes = [c_void_p] * 4 + [c_longlong] + [c_int] * 3 + [c_void_p]
+                lib.braid_moe_gemm_tc.argtypes = [c_void_p] * 7 + [c_int] * 5 + [c_longlong, c_int, c_int] + [c_void_p] * 3
+                names = ("braid_moe_gemm_mma", "braid_moe_gather", "braid_moe_gemm_tc",
+                         "braid_moe_route", "braid_moe_plan", "braid_moe_gemm_simt", "braid_moe_combine")
             elif name == "conv":
                 lib.braid_conv_heads.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_longlong] + \
                                                 [c_void_p] * 7 + [c_int] * 3 + [c_void_p, c_int, c_int, c_float, c_float] + \
@@ -875,33 +899,51 @@ class Kernels:
 
     def moe_plan(self, idx: torch.Tensor, token_seq: torch.Tensor, experts: int, tile: int):
         """Sort the (row, choice) pairs by expert, every expert's run padded to a multiple of `tile` slots.
-        Returns (slot_pair [max_tiles*tile], pair_slot [rows*top], tile_expert [max_tiles], meta [1], max_tiles)."""
+        Returns (slot_pair [max_tiles*tile], pair_slot [rows*top], tile_expert [max_tiles], meta [1], max_tiles); tiles of
+        `MOE_TC_TILE` slots come with the runs of tiles that `moe_gemm_tc` walks as a sixth."""
         lib = self.part_library("moe")
         rows, top = idx.shape
         max_tiles = self.moe_max_tiles(rows, top, experts, tile)
-        buf = torch.empty(max_tiles * tile + rows * top + max_tiles + 4, dtype=torch.int32, device=idx.device)
-        slot_pair = buf[:max_tiles * tile]
-        pair_slot = buf[max_tiles * tile:max_tiles * tile + rows * top]
-        tile_expert = buf[max_tiles * tile + rows * top:max_tiles * tile + rows * top + max_tiles]
-        meta = buf[max_tiles * tile + rows * top + max_tiles:]
+        max_wide = min(max_tiles, -(-max_tiles // 8) + experts) if tile == MOE_TC_TILE else 0
+        sizes = [4 * max_wide, max_tiles * tile, rows * top, max_tiles, 4]         # the runs first: they start on 16 bytes
+        buf = torch.empty(sum(sizes), dtype=torch.int32, device=idx.device)
+        wide, slot_pair, pair_slot, tile_expert, meta = buf.split(sizes)
         self.launches += 1
         self._check_lib(lib, lib.braid_moe_plan(idx.data_ptr(), token_seq.data_ptr(), slot_pair.data_ptr(),
-                                                pair_slot.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(), rows, top,
-                                                experts, tile, max_tiles, self._stream()), "moe_plan")
-        return slot_pair, pair_slot, tile_expert, meta, max_tiles
+                                                pair_slot.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(),
+                                                wide.data_ptr() if max_wide else None, rows, top, experts, tile, max_tiles,
+                                                max_wide, self._stream()), "moe_plan")
+        plan = (slot_pair, pair_slot, tile_expert, meta, max_tiles)
+        return plan + (wide,) if max_wide else plan
+
+    @staticmethod
+    def _moe_weights(w0: torch.Tensor, w1: Optional[torch.Tensor], j: int) -> Tuple[int, int, int]:
+        """(k, elements from expert to expert, elements from 16 rows to the next 16) of an expert stack: contiguous
+        [experts, J, K], or [experts, J / 16, 16, K], J rounded up, with room between the blocks of 16 rows (gate and up
+        of `interleave_experts`)."""
+        k = w0.shape[-1]
+        if w0.dim() == 3:
+            fits = w0.is_contiguous() and w0.shape[1] == j
+            strides = (j * k, 16 * k)
+        else:
+            fits = w0.dim() == 4 and w0.shape[2] == 16 and w0.shape[1] == -(-j // 16) and w0.stride()[2:] == (k, 1)
+            strides = (w0.stride(0), w0.stride(1))
+        if not fits or (w1 is not None and (w1.shape != w0.shape or w1.stride() != w0.stride() or w1.dtype != w0.dtype)):
+            raise KernelError("moe_gemm: expert weights must be contiguous [experts, J, K], or blocks of 16 such rows; gate and up alike")
+        return k, *strides
 
     def moe_gemm_simt(self, x: torch.Tensor, w0: torch.Tensor, w1: Optional[torch.Tensor], out: torch.Tensor, plan,
                       top: int, tile: int, relu2: bool = False, in_wgt: Optional[torch.Tensor] = None) -> None:
         """`in_wgt` (float32 [rows, top], with w1): a pair's weight multiplies the expert's input, that is gate and up
         before the activation.  The experts' products over a plan's slots, plain.  With w1: out[slot] = silu(w0[e] x[row]) * (w1[e] x[row]),
         x the step's rows; without: out[slot] = w0[e] x[slot], x a tensor of slots; with `relu2` (and no w1):
-        out[slot] = relu(w0[e] x[row])^2, x the step's rows (experts without a gate).  w0, w1 [experts, J, K]."""
+        out[slot] = relu(w0[e] x[row])^2, x the step's rows (experts without a gate).  w0, w1 [experts, J, K], or their blocks of
+        16 rows (`interleave_experts`)."""
         lib = self.part_library("moe")
-        slot_pair, _pair_slot, tile_expert, meta, max_tiles = plan
-        j, k = w0.shape[1], w0.shape[2]
-        if not w0.is_contiguous() or (w1 is not None and (not w1.is_contiguous() or w1.shape != w0.shape)):
-            raise KernelError("moe_gemm: expert weights must be contiguous [experts, J, K]")
-        if x.shape[1] != k or out.shape[1] != j or out.shape[0] != max_tiles * tile or x.stride(1) != 1 or out.stride(1) != 1:
+        slot_pair, _pair_slot, tile_expert, meta, max_tiles = plan[:5]
+        j = out.shape[1]
+        k, we, wb = self._moe_weights(w0, w1, j)
+        if x.shape[1] != k or out.shape[0] != max_tiles * tile or x.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("moe_gemm: shapes do not fit")
         if not (x.dtype == w0.dtype == out.dtype):
             raise KernelError("moe_gemm: every operand must have one element type")
@@ -909,7 +951,7 @@ class Kernels:
         self._check_lib(lib, lib.braid_moe_gemm_simt(
             x.data_ptr(), w0.data_ptr(), _ptr(w1), out.data_ptr(), slot_pair.data_ptr(), tile_expert.data_ptr(),
             meta.data_ptr(), dtype_code(x.dtype), self._moe_mode(w1, relu2), x.stride(0), out.stride(0), j, k, top, tile,
-            max_tiles, self._in_wgt(in_wgt, x, top, w1), self._stream()), "moe_gemm_simt")
+            max_tiles, self._in_wgt(in_wgt, x, top, w1), we, wb, self._stream()), "moe_gemm_simt")
 
     @staticmethod
     def _in_wgt(in_wgt, x, top: int, w1):
@@ -927,26 +969,58 @@ class Kernels:
 
     @staticmethod
     def moe_gemm_mma_eligible(x: torch.Tensor, w0: torch.Tensor, tile: int) -> bool:
-        return (x.dtype == torch.bfloat16 and w0.dtype == torch.bfloat16 and w0.shape[2] % 8 == 0 and x.stride(0) % 8 == 0
+        return (x.dtype == torch.bfloat16 and w0.dtype == torch.bfloat16 and w0.shape[-1] % 8 == 0 and x.stride(0) % 8 == 0
                 and x.data_ptr() % 16 == 0 and w0.data_ptr() % 16 == 0 and tile in (16, 64))
 
     def moe_gemm_mma(self, x: torch.Tensor, w0: torch.Tensor, w1: Optional[torch.Tensor], out: torch.Tensor, plan,
                      top: int, tile: int, relu2: bool = False, in_wgt: Optional[torch.Tensor] = None) -> None:
         """`moe_gemm_simt` in bfloat16 on the tensor cores; the plan's tile (16 or 64 slots) is the CTA's."""
         lib = self.part_library("moe")
-        slot_pair, _pair_slot, tile_expert, meta, max_tiles = plan
-        j, k = w0.shape[1], w0.shape[2]
-        if not self.moe_gemm_mma_eligible(x, w0, tile) or not w0.is_contiguous() or (w1 is not None and (
-                not w1.is_contiguous() or w1.shape != w0.shape or w1.dtype != w0.dtype or w1.data_ptr() % 16)):
+        slot_pair, _pair_slot, tile_expert, meta, max_tiles = plan[:5]
+        j = out.shape[1]
+        if not self.moe_gemm_mma_eligible(x, w0, tile) or (w1 is not None and w1.data_ptr() % 16):
             raise KernelError("moe_gemm_mma: bfloat16 operands, k and row strides in multiples of 8, starts on 16 bytes")
-        if x.shape[1] != k or out.shape[1] != j or out.shape[0] != max_tiles * tile or out.dtype != torch.bfloat16 \
+        k, we, wb = self._moe_weights(w0, w1, j)
+        if x.shape[1] != k or out.shape[0] != max_tiles * tile or out.dtype != torch.bfloat16 \
                 or x.stride(1) != 1 or out.stride(1) != 1 or out.data_ptr() % 4:
             raise KernelError("moe_gemm_mma: shapes do not fit")
         self.launches += 1
         self._check_lib(lib, lib.braid_moe_gemm_mma(
             x.data_ptr(), w0.data_ptr(), _ptr(w1), out.data_ptr(), slot_pair.data_ptr(), tile_expert.data_ptr(),
             meta.data_ptr(), self._moe_mode(w1, relu2), x.stride(0), out.stride(0), j, k, top, tile, max_tiles,
-            self._in_wgt(in_wgt, x, top, w1), self._stream()), "moe_gemm_mma")
+            self._in_wgt(in_wgt, x, top, w1), we, wb, self._stream()), "moe_gemm_mma")
+
+    def moe_gather(self, x: torch.Tensor, plan, top: int) -> torch.Tensor:
+        """The rows of a plan's slots (tiles of `MOE_TC_TILE`), [slots, k]: x's row of each slot's token, zeros for padding slots."""
+        lib = self.part_library("moe")
+        slot_pair, _pair_slot, _tile_expert, meta, max_tiles = plan[:5]
+        xs = torch.empty((max_tiles * MOE_TC_TILE, x.shape[1]), dtype=x.dtype, device=x.device)
+        if x.dtype != torch.bfloat16 or x.stride(1) != 1 or slot_pair.numel() != xs.shape[0]:
+            raise KernelError("moe_gather: bfloat16 rows and a plan of tiles of 32 slots")
+        self.launches += 1
+        self._check_lib(lib, lib.braid_moe_gather(x.data_ptr(), xs.data_ptr(), slot_pair.data_ptr(), meta.data_ptr(), x.stride(0),
+                                                  x.shape[1], top, max_tiles, self._stream()), "moe_gather")
+        return xs
+
+    def moe_gemm_tc(self, xs: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan, gated: bool = False, relu2: bool = False,
+                    in_wgt: Optional[torch.Tensor] = None) -> None:
+        """The experts' products over a plan of tiles of `MOE_TC_TILE` slots on pairs of SMs (tcgen05), bfloat16: xs [slots, k],
+        out [slots, J].  `gated`: w [experts, 2 * (J rounded up to 16), k] is `interleave_experts`' and out = silu(gate) * up,
+        times `in_wgt` (float32 [rows, top]) each first; else w [experts, J, k], out the product, or relu(.)^2 of it."""
+        lib = self.part_library("moe")
+        slot_pair, pair_slot, tile_expert, meta, max_tiles, wide = plan
+        experts, w_rows, k = w.shape
+        slots = max_tiles * MOE_TC_TILE
+        if not (xs.dtype == w.dtype == out.dtype == torch.bfloat16) or not w.is_contiguous() or not xs.is_contiguous() \
+                or tuple(xs.shape) != (slots, k) or out.shape[0] != slots or out.stride(1) != 1 or (gated and relu2):
+            raise KernelError("moe_gemm_tc: contiguous bfloat16 xs [slots, k] and w [experts, rows, k], out [slots, J]")
+        if in_wgt is not None and (in_wgt.dtype != torch.float32 or not in_wgt.is_contiguous() or in_wgt.numel() != pair_slot.numel()):
+            raise KernelError("moe_gemm_tc: the weights on the experts' input are float32, one a pair")
+        self.launches += 1
+        self._check_lib(lib, lib.braid_moe_gemm_tc(
+            xs.data_ptr(), w.data_ptr(), out.data_ptr(), slot_pair.data_ptr(), tile_expert.data_ptr(), wide.data_ptr(), meta.data_ptr(),
+            1 if gated else 2 if relu2 else 0, experts, w_rows, out.shape[1], k, out.stride(0), max_tiles, wide.numel() // 4,
+            _ptr(in_wgt), self._error_flag.data_ptr() + 4, self._stream()), "moe_gemm_tc")
 
     @staticmethod
     def attn_latent_mma_supports(rank: int, rot: int) -> bool:

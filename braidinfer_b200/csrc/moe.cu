@@ -133,62 +133,163 @@ extern "C" int braid_moe_route(const float* logits, int* idx, float* wgt, int ro
 }
 
 // ------------------------------------------------------------------ the plan
-// One block.  idx [rows * top] holds each pair's expert (-1: none); pairs of padding rows (token_seq < 0)
+// One cluster.  idx [rows * top] holds each pair's expert (-1: none); pairs of padding rows (token_seq < 0)
 // take no slot.  Outputs: slot_pair [cap] (pair of each slot, -1 for padding slots), pair_slot [rows * top]
-// (slot of each pair, -1 for none), tile_expert [max_tiles], meta[0] = tiles in use.
+// (slot of each pair, -1 for none), tile_expert [max_tiles], meta[0] = tiles in use.  With `wide` (tiles of 32 slots, moe_tc.cu):
+// an expert's tiles in runs of up to eight, shared out evenly: {first slot, tiles, the expert's first run, its runs} a run,
+// meta[1] = runs in use.
+// Bound by latency: two passes over the pairs (four loads in flight a thread, a shared-memory atomic a pair), shared by the CTAs of
+// one cluster, which read each other's counts, and two sums over the experts by shuffles.
 #define MOE_MAX_EXPERTS 1024
+#define MOE_PLAN_BATCH 4
+#define MOE_WIDE_TILES 8
+
+// the sums of a and b over the threads before this one; *total_* over all of them (1,024 threads)
+__device__ __forceinline__ void moe_scan2(int& a, int& b, int* total_a, int* total_b, int* warp_a, int* warp_b) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int ia = a, ib = b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int ta = __shfl_up_sync(0xffffffffu, ia, o), tb = __shfl_up_sync(0xffffffffu, ib, o);
+        if (lane >= o) { ia += ta; ib += tb; }
+    }
+    if (lane == 31) { warp_a[warp] = ia; warp_b[warp] = ib; }
+    __syncthreads();
+    int wa = warp_a[lane], wb = warp_b[lane];
+    const int own_a = wa, own_b = wb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int ta = __shfl_up_sync(0xffffffffu, wa, o), tb = __shfl_up_sync(0xffffffffu, wb, o);
+        if (lane >= o) { wa += ta; wb += tb; }
+    }
+    *total_a = __shfl_sync(0xffffffffu, wa, 31);
+    *total_b = __shfl_sync(0xffffffffu, wb, 31);
+    a = ia - a + __shfl_sync(0xffffffffu, wa - own_a, warp);
+    b = ib - b + __shfl_sync(0xffffffffu, wb - own_b, warp);
+}
+// the last e with start[e] <= t among those that own anything (start is not falling; start[experts] is the total)
+__device__ __forceinline__ int moe_owner(const int* start, int experts, int t) {
+    int lo = 0, hi = experts;                               // start[lo] <= t < start[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (start[mid] <= t) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+// the number at `p` (this CTA's shared memory) in CTA `rank` of the cluster
+__device__ __forceinline__ int moe_peer_load(const int* p, int rank) {
+    uint32_t at;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void moe_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ idx, const int* __restrict__ token_seq, int* __restrict__ slot_pair,
-                int* __restrict__ pair_slot, int* __restrict__ tile_expert, int* __restrict__ meta,
-                int rows, int top, int experts, int tile, int max_tiles) {
+                int* __restrict__ pair_slot, int* __restrict__ tile_expert, int* __restrict__ meta, int4* __restrict__ wide,
+                int rows, int top, int experts, int tile, int max_tiles, int max_wide) {
     pdl_trigger();
     pdl_wait();
-    __shared__ int count[MOE_MAX_EXPERTS];
-    __shared__ int start[MOE_MAX_EXPERTS];
-    const int pairs = rows * top;
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
-    for (int i = threadIdx.x; i < max_tiles * tile; i += blockDim.x) slot_pair[i] = -1;
+    __shared__ int count[MOE_MAX_EXPERTS], cursor[MOE_MAX_EXPERTS], start[MOE_MAX_EXPERTS + 1], start_w[MOE_MAX_EXPERTS + 1],
+        warp_a[32], warp_b[32];
+    const int pairs = rows * top, tid = threadIdx.x, ctas = gridDim.x, rank = blockIdx.x;      // the grid is one cluster
+    const int all = ctas * 1024, at = rank * 1024 + tid;
+    count[tid] = 0;
+    for (int i = at; i < max_tiles * tile; i += all) slot_pair[i] = -1;
     __syncthreads();
-    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-        const int e = (token_seq[i / top] >= 0) ? idx[i] : -1;
-        if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < experts; ++e) {
-            start[e] = run;
-            run += (count[e] + tile - 1) / tile;
+    auto fetch = [&](int base, int* e) {
+#pragma unroll
+        for (int j = 0; j < MOE_PLAN_BATCH; ++j) {
+            const int i = base + j * all + at;
+            e[j] = -1;
+            if (i < pairs) {
+                const int want = idx[i], seq = token_seq[i / top];
+                if (seq >= 0 && want >= 0 && want < experts) e[j] = want;
+            }
         }
-        meta[0] = run < max_tiles ? run : max_tiles;
+    };
+    for (int base = 0; base < pairs; base += MOE_PLAN_BATCH * all) {
+        int e[MOE_PLAN_BATCH];
+        fetch(base, e);
+#pragma unroll
+        for (int j = 0; j < MOE_PLAN_BATCH; ++j)
+            if (e[j] >= 0) atomicAdd(&count[e[j]], 1);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-        const int n = (count[e] + tile - 1) / tile;
-        for (int t = 0; t < n; ++t)
-            if (start[e] + t < max_tiles) tile_expert[start[e] + t] = e;
-        count[e] = 0;                       // from here on: the cursor within the expert's run
+    if (ctas > 1) moe_cluster_sync(); else __syncthreads();
+    // an expert's pairs over all CTAs, and those of the CTAs before this one
+    int total = 0, before = 0;
+    if (tid < experts) {
+        if (ctas == 1) total = count[tid];
+        else
+            for (int r = 0; r < ctas; ++r) {
+                const int n = moe_peer_load(&count[tid], r);
+                if (r < rank) before += n;
+                total += n;
+            }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-        const int e = (token_seq[i / top] >= 0) ? idx[i] : -1;
-        int slot = -1;
-        if (e >= 0 && e < experts) {
-            slot = start[e] * tile + atomicAdd(&count[e], 1);
-            if (slot < max_tiles * tile) slot_pair[slot] = i; else slot = -1;
+    cursor[tid] = before;
+    int tiles, wides, s = (total + tile - 1) / tile, w = (s + MOE_WIDE_TILES - 1) / MOE_WIDE_TILES;
+    moe_scan2(s, w, &tiles, &wides, warp_a, warp_b);
+    start[tid] = s;
+    start_w[tid] = w;
+    if (tid == 0) {
+        start[MOE_MAX_EXPERTS] = tiles;
+        start_w[MOE_MAX_EXPERTS] = wides;
+        if (rank == 0) {
+            meta[0] = tiles < max_tiles ? tiles : max_tiles;
+            if (wide) meta[1] = wides < max_wide ? wides : max_wide;
         }
-        pair_slot[i] = slot;
+    }
+    if (ctas > 1) moe_cluster_sync(); else __syncthreads();              // nobody leaves while its counts are read
+    for (int t = at; t < tiles && t < max_tiles; t += all) tile_expert[t] = moe_owner(start, experts, t);
+    if (wide)
+        for (int t = at; t < wides && t < max_wide; t += all) {
+            const int e = moe_owner(start_w, experts, t), first = start_w[e], runs = start_w[e + 1] - first, n = start[e + 1] - start[e];
+            const int lo = (t - first) * n / runs, hi = (t - first + 1) * n / runs;
+            wide[t] = make_int4((start[e] + lo) * tile, hi - lo, first, runs);
+        }
+    for (int base = 0; base < pairs; base += MOE_PLAN_BATCH * all) {
+        int e[MOE_PLAN_BATCH];
+        fetch(base, e);
+#pragma unroll
+        for (int j = 0; j < MOE_PLAN_BATCH; ++j) {
+            const int i = base + j * all + at;
+            if (i >= pairs) break;
+            int slot = e[j] >= 0 ? start[e[j]] * tile + atomicAdd(&cursor[e[j]], 1) : -1;
+            if (slot >= max_tiles * tile) slot = -1;
+            if (slot >= 0) slot_pair[slot] = i;
+            pair_slot[i] = slot;
+        }
     }
 }
 
 extern "C" int braid_moe_plan(const int* idx, const int* token_seq, int* slot_pair, int* pair_slot, int* tile_expert,
-                              int* meta, int rows, int top, int experts, int tile, int max_tiles, void* stream) {
+                              int* meta, int* wide, int rows, int top, int experts, int tile, int max_tiles, int max_wide, void* stream) {
     if (rows <= 0) return BRAID_OK;
     if (experts <= 0 || experts > MOE_MAX_EXPERTS) BRAID_REFUSE("moe_plan: %d experts (at most %d)", experts, MOE_MAX_EXPERTS);
     if (tile <= 0 || tile % 16) BRAID_REFUSE("moe_plan: the tile of %d slots must be a multiple of 16", tile);
-    braid_launch(moe_plan_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, idx, token_seq, slot_pair, pair_slot,
-                 tile_expert, meta, rows, top, experts, tile, max_tiles);
+    if (wide && ((uintptr_t)wide & 15)) BRAID_REFUSE("moe_plan: the runs of tiles must start on 16 bytes");
+    // one CTA for a decode step's pairs, up to a cluster of eight
+    const long long pairs = (long long)rows * top;
+    const int ctas = pairs <= 1024 ? 1 : pairs <= 2048 ? 2 : pairs <= 4096 ? 4 : 8;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(1024);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = braid_pdl_enabled();
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, moe_plan_kernel, idx, token_seq, slot_pair, pair_slot, tile_expert, meta, (int4*)wide, rows, top, experts,
+                       tile, max_tiles, max_wide);
     BRAID_LAUNCH_CHECK();
 }
 
@@ -211,7 +312,14 @@ struct MoeGemmArgs {
     long long ldx, ldo;
     int J, K, top, tile;
     const float* in_wgt;      // MODE 0: [rows * top] a weight a pair on the expert's input; or null
+    long long we, wb;         // elements from an expert's rows to the next one's, and from 16 of its rows to the next 16
 };
+
+// Row m of expert e: rows lie K apart in blocks of 16, the blocks `wb` apart (16 K where nothing lies between them).
+template <typename T>
+__device__ __forceinline__ const T* moe_weight_row(const MoeGemmArgs& a, const void* w, int e, int m) {
+    return (const T*)w + (size_t)e * a.we + (size_t)(m >> 4) * a.wb + (size_t)(m & 15) * a.K;
+}
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
@@ -231,8 +339,6 @@ moe_gemm_simt_kernel(MoeGemmArgs a) {
     const int my_pair = a.slot_pair[slot0 + ts];
     // the row this thread fetches for the x tile: thread (r = tid >> 4, c = tid & 15) loads x[slot r][k0 + c]
     const long long src_row = (MODE != 1) ? (my_pair >= 0 ? my_pair / a.top : -1) : (slot0 + ts);
-    const T* w0 = (const T*)a.w0 + (size_t)e * a.J * a.K;
-    const T* w1 = (MODE == 0) ? (const T*)a.w1 + (size_t)e * a.J * a.K : nullptr;
     float acc0[4] = {0.f, 0.f, 0.f, 0.f}, acc1[4] = {0.f, 0.f, 0.f, 0.f};
     for (int k0 = 0; k0 < a.K; k0 += 16) {
         {
@@ -245,8 +351,8 @@ moe_gemm_simt_kernel(MoeGemmArgs a) {
             const int r = el >> 4, c = el & 15;
             const int k = k0 + c, m = m0 + r;
             const bool ok = (m < a.J && k < a.K);
-            w0s[c][r] = ok ? to_f32(w0[(size_t)m * a.K + k]) : 0.f;
-            if (MODE == 0) w1s[c][r] = ok ? to_f32(w1[(size_t)m * a.K + k]) : 0.f;
+            w0s[c][r] = ok ? to_f32(moe_weight_row<T>(a, a.w0, e, m)[k]) : 0.f;
+            if (MODE == 0) w1s[c][r] = ok ? to_f32(moe_weight_row<T>(a, a.w1, e, m)[k]) : 0.f;
         }
         __syncthreads();
 #pragma unroll
@@ -281,12 +387,12 @@ moe_gemm_simt_kernel(MoeGemmArgs a) {
 extern "C" int braid_moe_gemm_simt(const void* x, const void* w0, const void* w1, void* out, const int* slot_pair,
                                    const int* tile_expert, const int* meta, int dtype, int mode, long long ldx,
                                    long long ldo, int J, int K, int top, int tile, int max_tiles, const float* in_wgt,
-                                   void* stream) {
+                                   long long w_expert, long long w_block, void* stream) {
     if (max_tiles <= 0 || J <= 0) return BRAID_OK;
     if (K <= 0) BRAID_REFUSE("moe_gemm: k=%d must be positive", K);
     if (tile <= 0 || tile % 16) BRAID_REFUSE("moe_gemm: the tile of %d slots must be a multiple of 16", tile);
     if (in_wgt && mode != 0) BRAID_REFUSE("moe_gemm: a weight on the expert's input goes with the gated first product (mode 0)");
-    MoeGemmArgs a{x, w0, w1, out, slot_pair, tile_expert, meta, ldx, ldo, J, K, top, tile, in_wgt};
+    MoeGemmArgs a{x, w0, w1, out, slot_pair, tile_expert, meta, ldx, ldo, J, K, top, tile, in_wgt, w_expert, w_block};
     const long long units = (long long)max_tiles * (tile / 16);
     if (units > 65535) BRAID_REFUSE("moe_gemm: %lld units of 16 slots exceed the grid limit", units);
     dim3 grid((J + 63) / 64, (unsigned)units);
@@ -339,8 +445,8 @@ moe_gemm_mma_kernel(MoeGemmArgs a) {
 #pragma unroll
     for (int i = 0; i < BCH; ++i) {
         const int m = m0 + ((tid + i * 128) >> 2);
-        b_rows[0][i] = m < a.J ? (const __nv_bfloat16*)a.w0 + ((size_t)e * a.J + m) * a.K : nullptr;
-        if (MODE == 0) b_rows[NB - 1][i] = m < a.J ? (const __nv_bfloat16*)a.w1 + ((size_t)e * a.J + m) * a.K : nullptr;
+        b_rows[0][i] = m < a.J ? moe_weight_row<__nv_bfloat16>(a, a.w0, e, m) : nullptr;
+        if (MODE == 0) b_rows[NB - 1][i] = m < a.J ? moe_weight_row<__nv_bfloat16>(a, a.w1, e, m) : nullptr;
     }
     float acc[NB][Tile::MI][Tile::NI][4];
     Tile::run(acc, (__nv_bfloat16*)moe_smem, a_rows, b_rows, a.K, a.w0);
@@ -387,14 +493,15 @@ moe_gemm_mma_kernel(MoeGemmArgs a) {
 
 extern "C" int braid_moe_gemm_mma(const void* x, const void* w0, const void* w1, void* out, const int* slot_pair,
                                   const int* tile_expert, const int* meta, int mode, long long ldx, long long ldo,
-                                  int J, int K, int top, int tile, int max_tiles, const float* in_wgt, void* stream) {
+                                  int J, int K, int top, int tile, int max_tiles, const float* in_wgt, long long w_expert,
+                                  long long w_block, void* stream) {
     if (max_tiles <= 0 || J <= 0) return BRAID_OK;
-    if (K <= 0 || K % 8 || ldx % 8) BRAID_REFUSE("moe_gemm_mma: k=%d and the row stride %lld must be multiples of 8", K, ldx);
+    if (K <= 0 || K % 8 || ldx % 8 || w_expert % 8 || w_block % 8) BRAID_REFUSE("moe_gemm_mma: k=%d, the row stride %lld and the weights' strides must be multiples of 8", K, ldx);
     if (((uintptr_t)x | (uintptr_t)w0 | (uintptr_t)w1) & 15) BRAID_REFUSE("moe_gemm_mma: operands must start on 16 bytes");
     if (tile != 16 && tile != 64) BRAID_REFUSE("moe_gemm_mma: the plan's tile must be 16 or 64 slots, not %d", tile);
     if (max_tiles > 65535) BRAID_REFUSE("moe_gemm_mma: %d tiles exceed the grid limit", max_tiles);
     if (in_wgt && mode != 0) BRAID_REFUSE("moe_gemm: a weight on the expert's input goes with the gated first product (mode 0)");
-    MoeGemmArgs a{x, w0, w1, out, slot_pair, tile_expert, meta, ldx, ldo, J, K, top, tile, in_wgt};
+    MoeGemmArgs a{x, w0, w1, out, slot_pair, tile_expert, meta, ldx, ldo, J, K, top, tile, in_wgt, w_expert, w_block};
     cudaStream_t s = (cudaStream_t)stream;
     // the down product over tiles of 64 slots takes 128 outputs a CTA (its rows are fetched half as often: 0.36 -> 0.29 ms
     // at 2,048 tokens of width 2048); gate+up with its two accumulators stays at 64 (at 128 it needs 237 registers and

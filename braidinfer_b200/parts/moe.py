@@ -85,7 +85,7 @@ class MixtureOfExperts(FeedForward):
         self.gate_names = [prefix + p.get("expert_gate", "mlp.e{e}.gate").format(e=e) for e in range(self.experts)]
         self.up_names = [prefix + p.get("expert_up", "mlp.e{e}.up").format(e=e) for e in range(self.experts)]
         self.down_names = [prefix + p.get("expert_down", "mlp.e{e}.down").format(e=e) for e in range(self.experts)]
-        self.w_gate = self.w_up = self.w_down = None
+        self.w_first = self.w_gate = self.w_up = self.w_down = None
 
     def tensor_specs(self) -> Dict[str, TensorSpec]:
         d = dict(self.router.tensor_specs())
@@ -106,14 +106,35 @@ class MixtureOfExperts(FeedForward):
             self.correction = tensors[self.correction_name].float().contiguous()     # routing is float32 in every run
         if self.shared is not None:
             self.shared.load(tensors)
-        if self.gated:
-            self.w_gate = torch.stack([tensors[n] for n in self.gate_names]).contiguous() # [experts, inter, hidden]
-        self.w_up = torch.stack([tensors[n] for n in self.up_names]).contiguous()
+        gate = [tensors[n] for n in self.gate_names] if self.gated else None
+        up = [tensors[n] for n in self.up_names]
+        if self.gated and self.rt.gemm_backend == "auto" and self.rt.act_dtype == torch.bfloat16 and gate[0].dtype == torch.bfloat16 \
+                and up[0].dtype == torch.bfloat16 and self.rt.kernels is not None:
+            # one stack for every kernel: the products on pairs of SMs want gate and up rows in turn, the others read views of it
+            from ..csrc.api import expert_halves, interleave_experts
+            self.w_first = interleave_experts(gate, up)               # [experts, 2 * (inter rounded up to 16), hidden]
+            self.w_gate, self.w_up = expert_halves(self.w_first)
+        else:
+            if self.gated:
+                self.w_gate = torch.stack(gate).contiguous()          # [experts, inter, hidden]
+            self.w_up = torch.stack(up).contiguous()
+            self.w_first = None if self.gated else self.w_up
         self.w_down = torch.stack([tensors[n] for n in self.down_names]).contiguous()     # [experts, hidden, inter]
 
-    def tile(self, rows: int) -> int:
-        """Slots a tile of the plan: 16 while an expert sees few rows, 64 beyond."""
-        return 16 if rows * self.top <= 16 * self.experts else 64
+    def on_pairs(self, x) -> bool:
+        """Whether the products can run on pairs of SMs (csrc/moe_tc.cu): bfloat16 whose rows, inputs and results alike, start on
+        16 bytes.  They are the fastest at every number of rows."""
+        return (self.rt.gemm_backend == "auto" and self.w_first is not None and self.w_first.dtype == torch.bfloat16
+                and self.w_down.dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0
+                and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+
+    def tile(self, x) -> int:
+        """Slots a tile of the plan: 32 for the products on pairs of SMs, which gather an expert's tiles themselves; for the
+        others 16 while an expert sees few rows, 64 beyond."""
+        from ..csrc.api import MOE_TC_TILE
+        if self.on_pairs(x):
+            return MOE_TC_TILE
+        return 16 if x.shape[0] * self.top <= 16 * self.experts else 64
 
     def forward(self, x, residual, ctx):
         y, plan, wgt, top = self._run(x, ctx)
@@ -139,7 +160,7 @@ class MixtureOfExperts(FeedForward):
         wgt = torch.empty((rows, self.top), dtype=torch.float32, device=x.device)
         K.moe_route(logits, idx, wgt, self.groups, self.keep, mult=self.out_mult, sigmoid=self.scoring == "sigmoid",
                     renorm=self.normalize, correction=self.correction)
-        tile = self.tile(rows)
+        tile = self.tile(x)
         plan = K.moe_plan(idx, ctx.token_seq, self.experts, tile)
         slots = plan[4] * tile
         act = self.rt.empty(slots, self.inter)
@@ -151,6 +172,11 @@ class MixtureOfExperts(FeedForward):
     def _experts(self, x, act, y, plan, tile, in_wgt=None) -> None:
         """bfloat16 rows that start on 16 bytes run on the tensor cores, everything else on the plain kernels."""
         K = self.rt.kernels
+        if len(plan) > 5:                                              # a plan of tiles of 32 slots
+            xs = K.moe_gather(x, plan, self.top)
+            K.moe_gemm_tc(xs, self.w_first, act, plan, gated=self.gated, relu2=not self.gated, in_wgt=in_wgt)
+            K.moe_gemm_tc(act, self.w_down, y, plan)
+            return
         tc = self.rt.gemm_backend == "auto"
         w0, w1 = (self.w_gate, self.w_up) if self.gated else (self.w_up, None)
         relu2 = not self.gated

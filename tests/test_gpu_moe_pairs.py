@@ -1,0 +1,122 @@
+"""The experts' products on pairs of SMs (csrc/moe_tc.cu) and the plan that they walk, at the edges of their tiles: experts
+without rows, with one, with a chunk of 32 slots more or less one, with more than a run of eight chunks."""
+import pytest
+import torch
+
+from braidinfer_b200.csrc.api import MOE_TC_TILE, expert_halves, get_kernels, interleave_experts
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# Rounding moves a number by at most half a step: 2^-24 of it in float32 (24 bits), 2^-8 in bfloat16 (8 bits); a sum that the
+# tensor cores cut off instead of rounding by a whole step, 2^-23.
+U = 2.0 ** -23
+
+
+@pytest.fixture(scope="module")
+def K():
+    return get_kernels(verbose=False)
+
+
+def choice(counts, top, seed):
+    """idx [rows, top]: expert e gets counts[e] pairs, in a shuffled order; -1 fills up the last row."""
+    flat = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)])
+    flat = flat[torch.randperm(flat.numel(), generator=torch.Generator().manual_seed(seed))]
+    pad = -flat.numel() % top
+    return torch.cat([flat, torch.full((pad,), -1)]).view(-1, top).to(torch.int32).to(DEV)
+
+
+COUNTS = [[0, 1, 31, 32, 33], [255, 0, 256, 257], [300, 520, 3], [1], [40] * 70, [3000, 1]]
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("tile", [16, 32, 64])
+def test_plan(K, counts, tile):
+    top = 3
+    idx = choice(counts, top, 1)
+    rows = idx.shape[0]
+    seq = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    seq[rows // 2] = -1                                              # a row of padding takes no slot
+    plan = [t.cpu() if torch.is_tensor(t) else t for t in K.moe_plan(idx, seq, len(counts), tile)]
+    slot_pair, pair_slot, tile_expert, meta, max_tiles = plan[:5]
+    live = idx.cpu().clone()
+    live[rows // 2] = -1
+    real = [int((live == e).sum()) for e in range(len(counts))]
+    assert meta[0] == sum(-(-n // tile) for n in real) <= max_tiles
+    for pair, (e, slot) in enumerate(zip(live.view(-1).tolist(), pair_slot.tolist())):
+        assert (slot < 0) == (e < 0)
+        if slot >= 0:
+            assert slot_pair[slot] == pair and tile_expert[slot // tile] == e
+    assert int((slot_pair >= 0).sum()) == sum(real)
+    if tile == MOE_TC_TILE:
+        wide = plan[5].view(-1, 4)[:meta[1]].tolist()
+        assert len(wide) == sum(-(-n // 256) for n in real)
+        at = 0
+        for w, (slot, chunks, first, runs) in enumerate(wide):       # every tile once, in order, an expert's runs alike
+            e = int(tile_expert[slot // tile])
+            assert slot == at and 1 <= chunks <= 8 and (tile_expert[slot // tile:slot // tile + chunks] == e).all()
+            assert first <= w < first + runs and runs == -(-real[e] // 256)
+            at += chunks * tile
+        assert at == meta[0] * tile
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("j, k", [(8, 8), (24, 40), (64, 64), (136, 72), (264, 200), (520, 520)])
+@pytest.mark.parametrize("mode", ["plain", "gated", "gated, weight on the input", "relu2"])
+def test_products(K, counts, j, k, mode):
+    top, experts = 2, len(counts)
+    g = torch.Generator(device=DEV).manual_seed(j + k + experts)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    idx = choice(counts, top, 2)
+    rows = idx.shape[0]
+    x = rnd(rows, k + 8).to(torch.bfloat16)[:, :k]                    # rows further apart than they are long
+    w0, w1 = [(rnd(experts, j, k) * k ** -0.5).to(torch.bfloat16) for _ in range(2)]
+    wgt = torch.rand(rows, top, device=DEV, generator=g)
+    plan = K.moe_plan(idx, torch.zeros(rows, dtype=torch.int32, device=DEV), experts, MOE_TC_TILE)
+    xs = K.moe_gather(x, plan, top)
+    out = torch.full((xs.shape[0], j), 3.0, device=DEV, dtype=torch.bfloat16)
+    gated = mode.startswith("gated")
+    in_wgt = wgt if "weight" in mode else None
+    K.moe_gemm_tc(xs, interleave_experts(w0, w1) if gated else w0, out, plan, gated=gated, relu2=mode == "relu2", in_wgt=in_wgt)
+    K.check_device_errors()
+    slot_pair = plan[0].long()
+    used = int(plan[3][0]) * MOE_TC_TILE
+    live = slot_pair >= 0
+    assert (xs[:used][~live[:used]] == 0).all() and torch.equal(xs[live], x[slot_pair[live] // top])
+    expert = idx.view(-1).long()[slot_pair[live]]
+    xd = xs[live].double()
+    prod = lambda w: torch.einsum("nk,njk->nj", xd, w[expert].double())
+    size = lambda w: torch.einsum("nk,njk->nj", xd.abs(), w[expert].double().abs())
+    e0, e1 = k * U * size(w0), k * U * size(w1)                      # float32 sums in any order, off by at most this
+    if gated:
+        s = wgt.view(-1)[slot_pair[live]].double()[:, None] if in_wgt is not None else 1.0
+        a, b, e0, e1 = prod(w0) * s, prod(w1) * s, e0 * s, e1 * s
+        want = a * torch.sigmoid(a) * b
+        slack = 1.1 * e0 * b.abs() + (a * torch.sigmoid(a)).abs() * e1 + 1.1 * e0 * e1
+    elif mode == "relu2":
+        want = prod(w0).clamp_min(0) ** 2
+        slack = 2 * e0 * prod(w0).abs() + e0 * e0
+    else:
+        want, slack = prod(w0), e0
+    # one rounding to bfloat16, and a part in 2^14 for the float32 activation
+    assert ((out[live].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -14) * want.abs() + 1.01 * slack + 1e-30).all()
+    if used < out.shape[0]:
+        assert (out[used:] == 3.0).all()                              # nothing is written past the plan's tiles
+
+
+def test_views_of_the_interleaved_stack_are_the_stack(K):
+    """The kernels of few rows read gate and up as blocks of 16 rows of the stack: the bits of separate tensors."""
+    g = torch.Generator(device=DEV).manual_seed(0)
+    experts, j, k, rows, top = 5, 40, 72, 33, 2
+    w0, w1 = [torch.randn(experts, j, k, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2)]
+    x = torch.randn(rows, k, device=DEV, generator=g).to(torch.bfloat16)
+    idx = torch.stack([torch.randperm(experts, generator=torch.Generator().manual_seed(r))[:top] for r in range(rows)]).int().to(DEV)
+    halves = expert_halves(interleave_experts(w0, w1))
+    for tile in (16, 64):
+        plan = K.moe_plan(idx, torch.zeros(rows, dtype=torch.int32, device=DEV), experts, tile)
+        for fn in (K.moe_gemm_mma, K.moe_gemm_simt):
+            res = []
+            for a, b in ((w0, w1), halves):
+                out = torch.zeros(plan[4] * tile, j, device=DEV, dtype=torch.bfloat16)
+                fn(x, a, b, out, plan, top, tile)
+                res.append(out)
+            assert torch.equal(*res)
