@@ -704,7 +704,13 @@ class Kernels:
                 lib.braid_gemm_heads_mma.restype = c_int
                 lib.braid_attn_latent_simple.argtypes = [c_void_p, c_void_p, c_int] + [c_void_p] * 4 + \
                                                         [c_longlong, c_longlong] + [c_int] * 8 + [c_float, c_void_p, c_void_p, c_void_p]
-                names = ("braid_latent_prep", "braid_gemm_heads", "braid_attn_latent_simple")
+                lib.braid_latent_expand_rows.argtypes = [c_void_p] * 5 + [c_int] * 8 + [c_void_p, c_void_p]
+                lib.braid_latent_attn_tc.argtypes = [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_int] + \
+                                                    [c_void_p] * 5 + [c_int] * 11 + [c_float, c_float, c_void_p, c_void_p, c_longlong,
+                                                                                      c_void_p, c_void_p]
+                lib.braid_latent_attn_tc_supported.argtypes = [c_int] * 4
+                names = ("braid_latent_prep", "braid_gemm_heads", "braid_attn_latent_simple", "braid_latent_expand_rows",
+                         "braid_latent_attn_tc", "braid_latent_attn_tc_supported")
             elif name == "scan":
                 lib.braid_causal_conv.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
                                                   c_void_p, c_longlong, c_longlong] + [c_void_p] * 4 + [c_int] * 5 + [c_void_p]
@@ -867,6 +873,63 @@ class Kernels:
             positions.data_ptr(), token_seq.data_ptr(), q_lat.stride(0), out.stride(0), rows, heads, d, rank,
             cache.shape[3], page_table.shape[1], cache.shape[0], int(window or 0), float(scale), _ptr(sinks),
             self._error_flag.data_ptr() + 16, self._stream()), "attn_latent_simple")
+
+    @staticmethod
+    def attn_latent_tc_supports(dim: int, rot: int, vdim: int, rank: int) -> bool:
+        """Head sizes that the prompt attention on expanded keys and values is built for (latent_attn_tc.cu)."""
+        return (dim, vdim) in ((128, 128), (64, 64)) and 0 < rot <= 64 and rot % 16 == 0 and rank % 8 == 0
+
+    @staticmethod
+    def latent_pages(q_len: Sequence[int], kv_before: Sequence[int], window: Optional[int]) -> List[int]:
+        """Pages of every sequence's context that a step's queries see: what `latent_expand_rows` lays out."""
+        page = build.page_size()
+        return [-(-(b + n) // page) - (max(0, b - window + 1) // page if window else 0) if n > 0 else 0
+                for n, b in zip(q_len, kv_before)]
+
+    def latent_expand_rows(self, cache: torch.Tensor, page_table: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, rank: int,
+                           window: Optional[int], pages: Sequence[int]) -> torch.Tensor:
+        """The latents of the step's context in neighbouring rows [sum(pages) * page_size, rank], sequence after sequence; rows past
+        a sequence's end are zero.  `pages` is `latent_pages` of what the device tables hold."""
+        lib = self.part_library("latent")
+        self._check_pages(cache)
+        n_seqs, total = len(pages), sum(pages)
+        d = cache.shape[4]
+        if cache.dtype != torch.bfloat16 or tuple(cache.shape[1:3]) != (1, 1) or not cache.is_contiguous() or n_seqs != page_table.shape[0]:
+            raise KernelError("latent_expand_rows: a bfloat16 cache [pages, 1, 1, page_size, D] and a table row a sequence")
+        rows = torch.empty((total * cache.shape[3], rank), dtype=cache.dtype, device=cache.device)
+        self.launches += 1
+        self._check_lib(lib, lib.braid_latent_expand_rows(
+            cache.data_ptr(), rows.data_ptr(), page_table.data_ptr(), q_len.data_ptr(), kv_before.data_ptr(), n_seqs, d, rank,
+            page_table.shape[1], cache.shape[0], int(window or 0), total, max(pages), self._error_flag.data_ptr() + 16, self._stream()),
+            "latent_expand_rows")
+        return rows
+
+    def attn_latent_tc(self, q_u: torch.Tensor, q_lat: torch.Tensor, kv: torch.Tensor, cache: torch.Tensor, out: torch.Tensor,
+                       page_table: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, n_seqs: int,
+                       max_q_len: int, vdim: int, rank: int, window: Optional[int], scale: float, out_scale: float = 1.0,
+                       sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> None:
+        """Attention of prompts over a latent cache on tcgen05, on keys and values expanded from the rows of `latent_expand_rows`:
+        q_u [rows, heads, dim] (a view), q_lat [rows, heads, rank + rot] whose last rot columns are the rotated query parts, kv
+        [rows of the context, heads * dim | heads * vdim], out [rows, heads * vdim].  `sinks`, `gate` ([rows, heads], a view is
+        fine) and `out_scale` as `head_sinks`, `head_gate` and `out_scale` of `attn_simple`.  Rows of padding are not written."""
+        lib = self.part_library("latent")
+        rows, heads, dim = q_u.shape
+        d = cache.shape[4]
+        self._check_pages(cache)
+        self._check_head_extras(sinks, gate, heads, out.dtype)
+        if not (q_u.dtype == q_lat.dtype == kv.dtype == cache.dtype == out.dtype == torch.bfloat16) or q_u.stride(2) != 1 \
+                or not q_lat.is_contiguous() or tuple(q_lat.shape) != (rows, heads, d) or not kv.is_contiguous() \
+                or kv.shape[1] != heads * (dim + vdim) or tuple(cache.shape[1:3]) != (1, 1) or not cache.is_contiguous() \
+                or tuple(out.shape) != (rows, heads * vdim) or out.stride(1) != 1 or page_table.shape[0] != n_seqs:
+            raise KernelError("attn_latent_tc: bfloat16 q_u [rows, heads, dim], q_lat [rows, heads, D], kv [context, heads * (dim + vdim)], "
+                              "cache [pages, 1, 1, page_size, D], out [rows, heads * vdim]")
+        self.launches += 1
+        self._check_lib(lib, lib.braid_latent_attn_tc(
+            q_u.data_ptr(), q_u.stride(1), q_u.stride(0), q_lat.data_ptr(), kv.data_ptr(), kv.shape[0], cache.data_ptr(), cache.shape[0],
+            out.data_ptr(), page_table.data_ptr(), q_start.data_ptr(), q_len.data_ptr(), kv_before.data_ptr(), rows, n_seqs, max_q_len,
+            heads, dim, d - rank, vdim, rank, page_table.shape[1], int(window or 0), out.stride(0), float(scale), float(out_scale),
+            _ptr(sinks), _ptr(gate), gate.stride(0) if gate is not None else 0, self._error_flag.data_ptr() + 12, self._stream()),
+            "attn_latent_tc")
 
     # ------------------------------------------------------------------ mixture of experts
     def moe_route(self, logits: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, groups: int, keep: int,

@@ -39,6 +39,10 @@ from .linear import Linear
 from .spec import CacheRequest, PartSpec, TensorSpec
 
 
+EXPAND_QUERIES = 16
+EXPAND_BYTES = 1 << 30
+
+
 @MIXERS.register("latent_attention")
 class LatentAttention(Mixer):
     """params: hidden_size, num_heads, dim (unrotated query/key numbers a head), rot_dim (rotated ones),
@@ -98,7 +102,7 @@ class LatentAttention(Mixer):
         self.uk_name = prefix + p.get("uk", "mix.uk")
         self.uv_name = prefix + p.get("uv", "mix.uv")
         self.o = Linear(runtime, [prefix + p.get("o", "mix.o")], [self.hidden], self.heads * self.vdim)
-        self.norm_w = self.uk_t = self.uv = None
+        self.norm_w = self.uk_t = self.uv = self.ukv = None
 
     def tensor_specs(self) -> Dict[str, TensorSpec]:
         d = dict(self.proj.tensor_specs())
@@ -140,7 +144,13 @@ class LatentAttention(Mixer):
         self.norm_w = tensors[self.norm_name] if not self.shared_kv else None
         # [heads, kv_rank, dim]: head h's matrix that carries q_u into the latent space, [out, in]
         self.uk_t = tensors[self.uk_name].view(self.heads, self.dim, self.rank).transpose(1, 2).contiguous()
-        self.uv = tensors[self.uv_name].view(self.heads, self.vdim, self.rank).contiguous()
+        uk, uv = tensors[self.uk_name], tensors[self.uv_name]
+        if (self.rt.gemm_backend == "auto" and self.rt.attention_backend == "auto" and self.rt.kernels is not None
+                and self.rt.act_dtype == uk.dtype == uv.dtype == torch.bfloat16
+                and self.rt.kernels.attn_latent_tc_supports(self.dim, self.rot, self.vdim, self.rank)):
+            self.ukv = torch.cat([uk, uv])                  # both as one weight: prompts expand keys and values with it
+            uv = self.ukv[uk.shape[0]:]
+        self.uv = uv.view(self.heads, self.vdim, self.rank).contiguous()
 
     def cache_request(self) -> Optional[CacheRequest]:
         return CacheRequest("window" if self.window else "full", 1, self.D, self.cache_window if self.window else None, planes=1)
@@ -171,6 +181,11 @@ class LatentAttention(Mixer):
                       self.heads, self.dim, self.rot, self.rank, self.pe.rope_dim, cache.page_size, self.eps,
                       adjacent=self.adjacent)
         q_u = queries[:, :self.q_cols].view(rows, self.heads, self.dim + self.rot)[:, :, :self.dim]
+        pages = self._expanded_pages(ctx)
+        if pages is not None:
+            gate = proj[:, self.gate_col:self.gate_col + self.heads] if self.gated else None
+            out = self._attend_expanded(q_u, q_lat, gate, pages, ctx, cache)
+            return self.o.forward(out, residual=residual, defer_to=ctx)
         tc = self.rt.gemm_backend == "auto"
         K.gemm_heads(q_u, self.uk_t, q_lat[:, :, :self.rank], tensor_cores=tc)
         o_lat = self.rt.empty(rows, self.heads, self.rank)
@@ -181,6 +196,36 @@ class LatentAttention(Mixer):
             raise RuntimeError("latent_attention: an output factor needs the gate's epilogue")
         K.gemm_heads(o_lat, self.uv, out.view(rows, self.heads, self.vdim), gate=gate, mult=self.out_mult, tensor_cores=tc)
         return self.o.forward(out, residual=residual, defer_to=ctx)
+
+    def _expanded_pages(self, ctx):
+        """The pages of every sequence's context if this step should expand keys and values from them
+        (csrc/latent_attn_tc.cu), else None.  Steps that a graph may hold (up to 256 tokens) never do: the context's extent is
+        read on the host.  Expanding costs a product of 2 kv_rank (dim + vdim) a row and head, attention saves
+        2 (2 kv_rank - dim - vdim) a query, row and head and a kernel that runs at a tenth of this one's rate: EXPAND_QUERIES
+        queries a row on average pay for it.  EXPAND_BYTES bounds the expanded rows a step holds."""
+        if self.ukv is None or ctx.n_tokens <= 256 or ctx.max_q_len <= 8 or not ctx.host_q_len:
+            return None
+        if self.gated is False and self.out_mult != 1.0:
+            return None
+        pages = self.rt.kernels.latent_pages(ctx.host_q_len, ctx.host_kv_before, self.window)
+        total = sum(pages)
+        if sum(n * p for n, p in zip(ctx.host_q_len, pages)) < EXPAND_QUERIES * total:
+            return None
+        if total * 64 * self.heads * (self.dim + self.vdim) * 2 > EXPAND_BYTES:
+            return None
+        return pages
+
+    def _attend_expanded(self, q_u, q_lat, gate, pages, ctx, cache):
+        K = self.rt.kernels
+        rows = K.latent_expand_rows(cache.storage, cache.page_table, ctx.q_len, ctx.kv_before, self.rank, self.window, pages)
+        kv = self.rt.empty(rows.shape[0], self.heads * (self.dim + self.vdim))
+        K.gemm_tc(rows, self.ukv, kv)
+        out = self.rt.empty(q_u.shape[0], self.heads * self.vdim)
+        if ctx.rows > ctx.n_tokens:
+            out.zero_()                                       # rows of padding are not written by the kernel
+        K.attn_latent_tc(q_u, q_lat, kv, cache.storage, out, cache.page_table, ctx.q_start, ctx.q_len, ctx.kv_before, ctx.n_seqs,
+                         ctx.max_q_len, self.vdim, self.rank, self.window, self.scale, out_scale=self.out_mult, sinks=self.sinks, gate=gate)
+        return out
 
     def _attend(self, q_lat, o_lat, ctx, cache) -> None:
         """bfloat16 runs use the tensor-core kernel where it is built for the latent's size (prompts and decoding

@@ -1,0 +1,140 @@
+"""Prompt attention over a latent cache on expanded keys and values (csrc/latent_attn_tc.cu) against float64, at the edges of its
+tiles of 128 queries and 64 keys, with contexts of earlier steps, windows, sinks and gates, and beside the latent form through
+the part that chooses between them."""
+import math
+
+import pytest
+import torch
+
+from braidinfer_b200.csrc.api import get_kernels
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF = torch.bfloat16
+
+
+@pytest.fixture(scope="module")
+def K():
+    return get_kernels(verbose=False)
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device=DEV)
+
+
+@pytest.mark.parametrize("dim, rot, vdim, rank", [(128, 64, 128, 512), (64, 32, 64, 256), (64, 64, 64, 40), (128, 16, 128, 72)])
+@pytest.mark.parametrize("seqs, window", [([(0, 1)], None), ([(0, 64), (0, 65)], None), ([(0, 127), (63, 129), (200, 3)], None),
+                                          ([(0, 300), (130, 257)], 70), ([(500, 130)], 64), ([(64, 128), (0, 0), (1, 64)], 1)])
+@pytest.mark.parametrize("extras", [False, True])
+def test_expanded_attention(K, dim, rot, vdim, rank, seqs, window, extras):
+    H, D = 3, rank + rot
+    g = torch.Generator(device=DEV).manual_seed(rank + len(seqs))
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    rows = sum(n for _, n in seqs)
+    q_start = [sum(n for _, n in seqs[:i]) for i in range(len(seqs))]
+    before, q_len = [b for b, _ in seqs], [n for _, n in seqs]
+    blocks = [-(-(b + n) // 64) for b, n in seqs]
+    cols = max(blocks) + 1
+    order = torch.randperm(sum(blocks) + 2, generator=torch.Generator().manual_seed(1)).tolist()
+    table = [[-1] * cols for _ in seqs]
+    at = 0
+    for i, n in enumerate(blocks):
+        first = max(0, before[i] - window + 1) // 64 if window else 0      # pages that the window has passed are gone
+        for b in range(first, n):
+            table[i][b] = order[at]
+            at += 1
+    cache = torch.full((sum(blocks) + 2, 1, 1, 64, D), float("nan"), device=DEV, dtype=BF)   # stale rows must not matter
+    ctx = []
+    for i, (b, n) in enumerate(seqs):
+        c = rnd(b + n, D).to(BF)
+        ctx.append(c)
+        for p in range(b + n):
+            if table[i][p // 64] >= 0:
+                cache[table[i][p // 64], 0, 0, p % 64] = c[p]
+    proj = rnd(rows, H * (dim + rot) + 8).to(BF)
+    q_u = proj[:, :H * (dim + rot)].view(rows, H, dim + rot)[:, :, :dim]
+    q_lat = torch.full((rows, H, D), float("nan"), device=DEV, dtype=BF)
+    q_lat[:, :, rank:] = rnd(rows, H, rot).to(BF)
+    uk, uv = (rnd(H * dim, rank) * rank ** -0.5).to(BF), (rnd(H * vdim, rank) * rank ** -0.5).to(BF)
+    sinks = rnd(H) if extras else None
+    gate = rnd(rows, H + 2).to(BF)[:, 1:H + 1] if extras else None
+    mult, scale = (0.7, (dim + rot) ** -0.5) if extras else (1.0, (dim + rot) ** -0.5)
+    pages = K.latent_pages(q_len, before, window)
+    t = i32(table)
+    rows_c = K.latent_expand_rows(cache, t, i32(q_len), i32(before), rank, window, pages)
+    at = 0
+    for i, (b, n) in enumerate(seqs):                                  # the context, page by page, zeros past its end
+        first = max(0, b - window + 1) // 64 * 64 if window else 0
+        if n == 0:
+            continue
+        got = rows_c[at:at + pages[i] * 64]
+        assert torch.equal(got[:b + n - first], ctx[i][first:, :rank]) and (got[b + n - first:] == 0).all()
+        at += pages[i] * 64
+    assert at == rows_c.shape[0]
+    kv = torch.empty(rows_c.shape[0], H * (dim + vdim), device=DEV, dtype=BF)
+    K.gemm_tc(rows_c, torch.cat([uk, uv]), kv)
+    out = torch.full((rows, H * vdim), 9.0, device=DEV, dtype=BF)
+    K.attn_latent_tc(q_u, q_lat, kv, cache, out, t, i32(q_start), i32(q_len), i32(before), len(seqs), max(q_len), vdim, rank, window,
+                     scale, out_scale=mult, sinks=sinks, gate=gate)
+    K.check_device_errors()
+    worst = 0.0
+    for i, (b, n) in enumerate(seqs):
+        if n == 0:
+            continue
+        c = ctx[i].double()
+        # keys and values as the kernel gets them: rounded to bfloat16 after the expansion
+        ku = (c[:, :rank] @ uk.double().T).to(BF).double().view(b + n, H, dim)
+        v = (c[:, :rank] @ uv.double().T).to(BF).double().view(b + n, H, vdim)
+        q = slice(q_start[i], q_start[i] + n)
+        s = torch.einsum("qhd,khd->hqk", q_u[q].double(), ku) + torch.einsum("qhr,kr->hqk", q_lat[q, :, rank:].double(), c[:, rank:])
+        s = s * scale
+        dist = torch.arange(b, b + n, device=DEV)[:, None] - torch.arange(b + n, device=DEV)[None]
+        hidden = (dist < 0) | ((dist >= window) if window else False)
+        s = s.masked_fill(hidden, -math.inf)
+        if sinks is not None:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(H, n, 1)], -1)
+        p = torch.softmax(s, -1)[..., :b + n]
+        want = torch.einsum("hqk,khd->qhd", p, v) * mult
+        if gate is not None:
+            want = want * torch.sigmoid(gate[q].double())[:, :, None]
+        err = (out[q].double().view(n, H, vdim) - want).abs()
+        # probabilities rounded to bfloat16 (2^-8 of each), keys that sit on a rounding edge (2^-8 of their score's terms), the
+        # result rounded once: a few parts in 2^8 of the values' size
+        size = torch.einsum("hqk,khd->qhd", p, v.abs()) * mult
+        worst = max(worst, float((err / (size + 0.05)).max()))
+    assert worst < 4 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("chunks", [[700], [300, 400], [40, 660], [690, 10]])
+def test_the_part_that_chooses(monkeypatch, chunks):
+    """A Bidinex model of one layer: prompts whole and in portions (the later ones expand the earlier ones' latents again), beside
+    the same engine with the latent form."""
+    from braidinfer_b200.engine import Engine
+    import braidinfer_b200.parts.latent_attention as LA
+    mixer = {"heads": 4, "dim": 64, "rot_dim": 32, "rot": {"base": 10000.0, "dims": 32}, "vdim": 64, "kv_rank": 256, "scale": 96 ** -0.5}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 4, "top": 2, "groups": {"count": 1, "keep": 1}}}
+    cfg = {"architecture": "Bidinex", "vocab": 256, "width": 128, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+           "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    eng = Engine.from_random(cfg, 3, max_tokens=2048, max_slots=2, verbose=False)
+    toks = torch.randint(0, 256, (sum(chunks),), generator=torch.Generator().manual_seed(2)).tolist()
+
+    def logits():
+        s, at, out = eng.open(), 0, []
+        for n in chunks:
+            out.append(eng.step([(s, toks[at:at + n])], want="all"))
+            at += n
+        eng.close(s)
+        eng.check()
+        return torch.cat(out).double()
+
+    calls = []
+    kernel = type(eng.kernels).attn_latent_tc
+    monkeypatch.setattr(type(eng.kernels), "attn_latent_tc", lambda self, *a, **kw: (calls.append(1), kernel(self, *a, **kw)))
+    got = logits()
+    assert len(calls) == sum(n > 256 for n in chunks)                  # steps of up to 256 tokens keep the latent form
+    monkeypatch.setattr(LA, "EXPAND_BYTES", 0)
+    calls.clear()
+    want = logits()
+    assert not calls
+    # both are bfloat16 of the same mechanism; the model's tests ask 1e-2 .. 2e-2 of either beside float64
+    assert float((got - want).norm() / want.norm()) < 1e-2
