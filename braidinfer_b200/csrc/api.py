@@ -86,6 +86,7 @@ def expert_halves(w: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     return v[:, :, 0], v[:, :, 1]
 
 
+FEW_MAX_ROWS = 16            # tokens that the product of a few tokens takes (gemm_few.cu)
 MOE_TC_TILE = 32             # slots a tile of the plan that the experts' products on pairs of SMs walk
 PAIR_TOKEN_TILE = 256        # the token tile of the kernel that runs on pairs of SMs
 # Tokens a chunk of a long prompt's recurrence (csrc/scan.cu): 128 for sequences of 1,024 tokens and more, 64 below
@@ -214,6 +215,7 @@ class Kernels:
         L.braid_gemm_tc.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int,
                                     c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int,
                                     c_void_p] + scale + [c_void_p, c_void_p, c_void_p]
+        L.braid_gemm_few.argtypes = [c_void_p] * 4 + [c_int] * 5 + [c_longlong] * 3 + scale + [c_void_p]
         L.braid_streamk_reduce_prep.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                 c_longlong, c_int, c_void_p]
         L.braid_gemm_tc2.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -238,7 +240,7 @@ class Kernels:
             getattr(L, name).restype = c_int
         for name in ("braid_embed", "braid_embed_pos", "braid_head_prep_kv", "braid_proj_prep_kv", "braid_head_gate", "braid_glu_clamp", "braid_rmsnorm", "braid_silu_mul", "braid_act_mul", "braid_head_norm_rope_kv",
                      "braid_act_mul_gather", "braid_rmsnorm_add", "braid_residual_add",
-                     "braid_rope_kv_write", "braid_cast", "braid_attn_simple", "braid_gemm_simt",
+                     "braid_rope_kv_write", "braid_cast", "braid_attn_simple", "braid_gemm_simt", "braid_gemm_few",
                      "braid_gemm_tc", "braid_gemm_tc2", "braid_argmax", "braid_sample", "braid_streamk_reduce",
                      "braid_streamk_reduce_norm", "braid_streamk_reduce_rope_kv", "braid_streamk_reduce_prep",
                      "braid_streamk_reduce_prep_cols"):
@@ -1488,6 +1490,25 @@ class Kernels:
         if need < 0:
             raise KernelError(f"gemm_tc: no stream-k plan for {n} rows x {w_rows} x {k} with token tile {block_n}")
         return self.tc_workspace(need)
+
+    def gemm_few(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
+                 swiglu: bool = False, in_scale: Optional[RowScale] = None, activation: str = "silu") -> None:
+        """`gemm_tc` for up to `FEW_MAX_ROWS` tokens in one kernel whose CTAs finish the sums of 16 weight rows (no partial sums)."""
+        n, k = x.shape
+        w_rows = w.shape[0]
+        m = out.shape[1] if swiglu else w_rows
+        if not self.gemm_tc_eligible(x, w) or w.shape[1] != k or out.stride(1) != 1 or out.shape != (n, m):
+            raise KernelError("gemm_few: bfloat16 x [n, k] and w [m, k] whose rows start on 16 bytes, out [n, m]")
+        if swiglu and w_rows != 2 * (-(-m // 16) * 16):
+            raise KernelError(f"the gated epilogue wants {2 * (-(-m // 16) * 16)} interleaved weight rows for "
+                              f"{m} outputs, got {w_rows} (see interleave_gate_up)")
+        if residual is not None and (residual.shape != out.shape or residual.stride() != out.stride()):
+            raise KernelError("gemm_few: the residual is laid out as the result")
+        mode = (2 | activation_code(activation) << 4) if swiglu else (1 if residual is not None else 0)
+        self.launches += 1
+        self._check(self.lib.braid_gemm_few(x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(residual), dtype_code(out.dtype), mode,
+                                            n, m, k, x.stride(0), w.stride(0), out.stride(0), *_scale_args(in_scale),
+                                            self._stream()), "gemm_few")
 
     def gemm_tc(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None,
                 swiglu: bool = False, block_n: int = 0, stream_k: bool = False,

@@ -43,6 +43,17 @@ def stream_k_pays(rows: int, w_rows: int, k_in: int, sms: Optional[int] = None) 
     return fill < (0.8 if rows <= 48 else 0.7)
 
 
+def few_rows_pay(rows: int, w_rows: int, k_in: int) -> bool:
+    """Whether the product of `rows` tokens with a [w_rows, k_in] bfloat16 weight should run as one kernel whose CTAs finish 16
+    weight rows each (csrc/gemm_few.cu) instead of as stream-k partial sums and their reduce kernel: where a second launch weighs
+    more than what is lost on an uneven spread of the CTAs, weights of up to 24 MB at up to 8 tokens and 7 MB at 9 to 16.  Whole turns
+    of 24 steps, ms, with the line at 0 / 7 / 24 / 51 MB: 8 sequences of a Loduzen model of width 1024 8.3 / 7.4 / 6.75 / 6.8, 2 of
+    width 2048 10.7 / 10.2 / 10.0 / 9.1, 4 of a Zisesun model of width 2048 7.65 / 7.3 / 7.2 / 7.55, 4 of the dense decoder of
+    width 4096 11.16 / 11.11 / 11.25 / 11.95; 12 of a Loduzen model of width 2048 12.8 / 12.6 / 13.1 / 12.8."""
+    from ..csrc.api import FEW_MAX_ROWS
+    return rows <= FEW_MAX_ROWS and w_rows * k_in * 2 <= (24 if rows <= 8 else 7) * 10 ** 6
+
+
 # Rows up to which a norm may leave its scale to the next product: beyond the token tiles of the
 # one-SM kernel the products run on pairs of SMs, which take no row scale.
 ROW_SCALE_MAX_ROWS = 128
@@ -127,6 +138,15 @@ class Linear:
             K.cast(y, y2)
             return y2
         use_tc = (self.rt.gemm_backend == "auto" and x.dtype == torch.bfloat16 and K.gemm_tc_eligible(x, w))
+        if use_tc and few_rows_pay(rows, w_rows, x.shape[1]):
+            if residual is not None:
+                K.gemm_few(x, w, residual, residual=residual)
+                return residual
+            if swiglu and not self.interleaved:
+                raise RuntimeError("a gated product on the tensor cores wants interleaved gate/up weights")
+            out = torch.empty((rows, self.out_features[0] if swiglu else w_rows), dtype=out_dtype or x.dtype, device=x.device)
+            K.gemm_few(x, w, out, swiglu=swiglu, in_scale=in_scale, activation=activation)
+            return out
         sk = use_tc and stream_k_pays(rows, w_rows, x.shape[1])
         can_defer = (defer_to is not None and sk and not swiglu
                      and self.rt.fuse_reduce and K.pending_partial is None)
