@@ -120,3 +120,23 @@ def test_views_of_the_interleaved_stack_are_the_stack(K):
                 fn(x, a, b, out, plan, top, tile)
                 res.append(out)
             assert torch.equal(*res)
+
+
+@pytest.mark.parametrize("rows, width, top, pad", [(1, 8, 1, 0), (3, 2048, 6, 0), (5, 520, 9, 8), (4, 1001, 3, 0), (2, 516, 17, 4), (700, 40, 2, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_weighted_sum(K, rows, width, top, pad, dtype, weighted):
+    """Widths and strides that allow 16-byte loads and ones that do not, more choices than are asked for at once, pairs without a slot."""
+    g = torch.Generator(device=DEV).manual_seed(rows + width)
+    slots = rows * top + 5
+    y = torch.randn(slots, width + pad, device=DEV, generator=g).to(dtype)[:, :width]
+    h = torch.randn(rows, width, device=DEV, generator=g)
+    wgt = torch.rand(rows, top, device=DEV, generator=g)
+    at = torch.randperm(slots, device=DEV, generator=g)[:rows * top].int()
+    at[::7] = -1
+    w = (wgt if weighted else torch.ones_like(wgt)).double() * (at.view(rows, top) >= 0)
+    terms = w[:, :, None] * y[at.clamp_min(0).long().view(rows, top)].double()
+    want = h.double() + terms.sum(1)
+    most = (top + 1) * U * (h.double().abs() + terms.abs().sum(1))
+    K.moe_combine(h, y, (None, at), wgt if weighted else None, top=top)
+    assert ((h.double() - want).abs() <= most).all()
