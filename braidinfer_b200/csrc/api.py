@@ -201,6 +201,8 @@ class Kernels:
         L.braid_cast.argtypes = [c_void_p, c_int, c_void_p, c_int, c_longlong, c_void_p]
         L.braid_gather_i32.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_void_p]
         L.braid_gather_i32.restype = c_int
+        L.braid_fetch_i32.argtypes = [c_void_p, c_void_p, c_int, c_void_p]
+        L.braid_fetch_i32.restype = c_int
         L.braid_attn_simple.argtypes = [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                         c_float, c_int, c_float, c_float, c_void_p, c_void_p, c_longlong, c_int, c_void_p,
@@ -453,6 +455,13 @@ class Kernels:
         self.launches += 1
         self._check(self.lib.braid_gather_i32(src.data_ptr(), index.data_ptr(), dst.data_ptr(), index.numel(),
                                               self._stream()), "gather_i32")
+
+    def fetch_i32(self, host: torch.Tensor, dst: torch.Tensor) -> None:
+        """dst <- host (pinned), int32, a multiple of four of them, read by a kernel.  What follows has to be launched without the
+        programmatic attribute (a graph is)."""
+        if not host.is_pinned() or host.dtype != torch.int32 or dst.dtype != torch.int32 or host.numel() != dst.numel():
+            raise KernelError("fetch_i32: pinned int32 to int32 of the same size")
+        self._check(self.lib.braid_fetch_i32(host.data_ptr(), dst.data_ptr(), dst.numel(), self._stream()), "fetch_i32")
 
     def rope_kv_write(self, qkv: torch.Tensor, inv_freq: torch.Tensor, positions: torch.Tensor,
                       token_seq: torch.Tensor, page_table: Optional[torch.Tensor], cache: Optional[torch.Tensor],

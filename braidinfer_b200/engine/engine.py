@@ -217,7 +217,7 @@ class Engine:
             raise ValueError("device_tokens needs a step of one token a sequence")
         ctx = self.packer.pack(slots, tokens, before, want_l, tables, bucket_tables=shaped,
                                token_source_rows=device_tokens[1] if device_tokens is not None else None,
-                               pad_rows_to=token_tile(sum(n_new)) if short_prompt else 0)
+                               pad_rows_to=token_tile(sum(n_new)) if short_prompt else 0, upload=False)
         ctx.kernels = self.kernels
         if shaped and ctx.page_tables:
             ctx.max_kv_len = max(t.shape[1] for t in ctx.page_tables) * PAGE_SIZE
@@ -225,6 +225,9 @@ class Engine:
             # no sequence brings more tokens than the step has rows; steps of a few tokens a sequence keep the
             # attention kernel that slices the context (it is chosen by this bound)
             ctx.max_q_len = FEW_TOKENS if max(n_new) <= FEW_TOKENS else ctx.rows
+        # a step that a graph will replay has its tables fetched by a kernel; one launched kernel by kernel, whose first kernels read
+        # the tables before they wait for their predecessors, by a copy
+        self.packer.upload(self.kernels if graphable and self._graph_ready(ctx) else None)
         if device_tokens is not None:
             self.kernels.gather_i32(device_tokens[0], self.packer.token_source_view, ctx.token_ids)
         try:
@@ -244,6 +247,15 @@ class Engine:
         self.steps_run += 1
         return logits
 
+    @staticmethod
+    def _graph_key(ctx: StepContext) -> tuple:
+        return (ctx.rows, ctx.n_seqs, ctx.n_want, ctx.max_q_len, tuple(tuple(t.shape) for t in ctx.page_tables))
+
+    def _graph_ready(self, ctx: StepContext) -> bool:
+        """Whether `_graph_step` will replay a graph that it has."""
+        return ((self.packer.generation, self.kernels.workspace_generation) == self._graph_generation
+                and self._graph_key(ctx) in self._graphs)
+
     def _graph_step(self, ctx: StepContext) -> Optional[torch.Tensor]:
         """Run a step of few tokens (one a sequence, or short prompts) through a CUDA graph.  The graph holds kernel
         launches only; the step's tables were copied to fixed device addresses before it.
@@ -254,7 +266,7 @@ class Engine:
             self._graphs.clear()
             self._graph_seen.clear()
             self._graph_generation = generation
-        key = (ctx.rows, ctx.n_seqs, ctx.n_want, ctx.max_q_len, tuple(tuple(t.shape) for t in ctx.page_tables))
+        key = self._graph_key(ctx)
         entry = self._graphs.get(key)
         if entry is None:
             seen = self._graph_seen.get(key, 0)

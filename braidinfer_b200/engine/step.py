@@ -110,36 +110,60 @@ class _Sized:                              # what `StepPacker._context` needs of
 
 
 class StepPacker:
-    """Builds a step's integer tables on the host and moves them to the device in one copy."""
+    """Builds a step's integer tables on the host and moves them to the device in one copy, or (`upload`) by one kernel.  The host
+    writes into pinned buffers in turn, so that it waits only for the use of a buffer three steps before."""
+
+    BUFFERS = 4
+    FETCH_MOST = 1 << 14         # ints that a kernel fetches; more go through a copy
 
     def __init__(self, device, row_multiple: int = 1) -> None:
         self.device = device
         self.row_multiple = max(1, int(row_multiple))
-        self._pinned: Optional[torch.Tensor] = None
+        self._pinned: List[list] = []        # [pinned int32, the same as numpy, event of its last use or None], used in turn
+        self._turn = 0
         self._dev: Optional[torch.Tensor] = None
-        self._copied: Optional[torch.cuda.Event] = None
+        self._pending: Optional[Tuple[list, int]] = None
         self.h2d_bytes_last = 0
         self.generation = 0          # grows when the device buffer moves (captured graphs are stale then)
 
-    def _buffers(self, n: int) -> Tuple[torch.Tensor, torch.Tensor]:
-        if self._pinned is None or self._pinned.numel() < n:
+    def _buffers(self, n: int) -> Tuple[list, torch.Tensor]:
+        if self._dev is None or self._dev.numel() < n:
             cap = max(1 << 18, 1 << (n - 1).bit_length())
-            if self._copied is not None:
-                self._copied.synchronize()
+            for st in self._pinned:
+                if st[2] is not None:
+                    st[2].synchronize()
             self.generation += 1
-            self._pinned = torch.empty(cap, dtype=torch.int32, pin_memory=True)
             self._dev = torch.empty(cap, dtype=torch.int32, device=self.device)
-        return self._pinned, self._dev
+            pinned = torch.empty((self.BUFFERS, cap), dtype=torch.int32, pin_memory=True)
+            self._pinned = [[b, b.numpy(), None] for b in pinned]
+        self._turn = (self._turn + 1) % self.BUFFERS
+        st = self._pinned[self._turn]
+        if st[2] is not None:
+            st[2].synchronize()             # the last copy out of this buffer is done
+        return st, self._dev
+
+    def upload(self, kernels=None) -> None:
+        """Move the tables of the last `pack(..., upload=False)` to the device: by a kernel of `kernels` that reads the pinned
+        buffer where that pays (what is launched next must wait for it to end, as a graph does), else by a copy."""
+        st, total = self._pending
+        self._pending = None
+        if kernels is not None and total <= self.FETCH_MOST:
+            kernels.fetch_i32(st[0][:total], self._dev[:total])
+        else:
+            self._dev[:total].copy_(st[0][:total], non_blocking=True)
+        if st[2] is None:
+            st[2] = torch.cuda.Event()
+        st[2].record()
 
     def pack(self, slots: Sequence[int], tokens: Sequence[Sequence[int]], kv_before: Sequence[int],
              want: Sequence[Sequence[int]], tables: Sequence[np.ndarray], bucket_tables: bool = False,
-             token_source_rows: Optional[Sequence[int]] = None, pad_rows_to: int = 0) -> StepContext:
-        """`bucket_tables` widens every page table to a power-of-two number of columns (at
+             token_source_rows: Optional[Sequence[int]] = None, pad_rows_to: int = 0, upload: bool = True) -> StepContext:
+        """`upload` False: the caller moves the tables to the device with `upload()`.  `bucket_tables` widens every page table to a power-of-two number of columns (at
         least 8), so that steps of the same shape lay their tables out identically.
         `pad_rows_to`: at least this many rows (the rows past the step's tokens are padding)."""
         n_seqs = len(slots)
         if bucket_tables and all(len(t) == 1 for t in tokens) and all(len(w) <= 1 for w in want):
-            return self._pack_one_token_each(slots, tokens, kv_before, want, tables, token_source_rows)
+            return self._pack_one_token_each(slots, tokens, kv_before, want, tables, token_source_rows, upload)
         if token_source_rows is not None:
             raise ValueError("tokens can be taken from the device only in steps of one token a sequence")
         if bucket_tables:
@@ -178,20 +202,21 @@ class StepPacker:
         for p in parts:
             offs.append(total)
             total += -(-p.size // 4) * 4
-        pinned, dev = self._buffers(max(total, 4))
-        if self._copied is not None:
-            self._copied.synchronize()          # the last copy out of the pinned buffer is done
-        pn = pinned.numpy()
+        st, dev = self._buffers(max(total, 4))
+        pn = st[1]
         for p, o in zip(parts, offs):
             pn[o:o + p.size] = p
-        dev[:total].copy_(pinned[:total], non_blocking=True)
-        self._copied = torch.cuda.Event()
-        self._copied.record()
-        self.h2d_bytes_last = total * 4
+        self._done(st, total, upload)
 
         return self._context(dev, parts, offs, tables, rows, n_tokens, n_seqs, q_len, kv_before, slots, want_rows)
 
-    def _pack_one_token_each(self, slots, tokens, kv_before, want, tables, token_source_rows=None) -> StepContext:
+    def _done(self, st, total: int, upload: bool) -> None:
+        self.h2d_bytes_last = total * 4
+        self._pending = (st, total)
+        if upload:
+            self.upload()
+
+    def _pack_one_token_each(self, slots, tokens, kv_before, want, tables, token_source_rows=None, upload=True) -> StepContext:
         """The same layout as `pack` for the common step of generation (one token a
         sequence, page tables widened to a power-of-two width), written straight into the
         pinned buffer."""
@@ -210,10 +235,8 @@ class StepPacker:
         for sz in sizes:
             offs.append(total)
             total += -(-sz // 4) * 4
-        pinned, dev = self._buffers(max(total, 4))
-        if self._copied is not None:
-            self._copied.synchronize()
-        pn = pinned.numpy()
+        st, dev = self._buffers(max(total, 4))
+        pn = st[1]
         ar = np.arange(n, dtype=np.int32)
         pn[offs[0]:offs[0] + rows] = 0
         pn[offs[0]:offs[0] + n] = [t[0] for t in tokens]
@@ -234,10 +257,7 @@ class StepPacker:
             shapes.append((n, cols))
         src_k = 8 + len(wide)                       # where each row's token lies in the sampler's output
         pn[offs[src_k]:offs[src_k] + n] = token_source_rows if token_source_rows is not None else ar
-        dev[:total].copy_(pinned[:total], non_blocking=True)
-        self._copied = torch.cuda.Event()
-        self._copied.record()
-        self.h2d_bytes_last = total * 4
+        self._done(st, total, upload)
         self.token_source_view = dev[offs[src_k]:offs[src_k] + n]
 
         parts = [_Sized(sz) for sz in sizes]
