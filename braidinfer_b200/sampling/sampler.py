@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from .params import SamplingParams
-from .rng import entropy_seed, uniform
+from .rng import entropy_seed, uniforms
 
 
 class Sampler:
@@ -62,49 +62,64 @@ class Sampler:
         `histories` is a list, or a function returning the list, of what the repetition
         penalty looks at for each row (prompt + generated); it is only asked for when some
         row has a penalty."""
+        return self._read(self._launch(logits, params, seeds, sequence_ids, steps, histories))
+
+    def _launch(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int], sequence_ids: Sequence[int],
+                steps: Sequence[int], histories=None, staged: bool = False) -> torch.Tensor:
+        """The choice on the device: every option of the step in one copy, the chain's kernel behind it.  `staged`: through the
+        sampler's pinned buffers and its work area, without waiting; else through memory of the call's own.  Returns the
+        tokens (int32, on the device)."""
         rows, vocab = logits.shape
         out = torch.empty(rows, dtype=torch.int32, device=self.device)
-        if all(p.is_plain_greedy for p in params):
+        one = params[0] if all(p is params[0] for p in params) else None       # one set of options for all rows
+        if one.is_plain_greedy if one is not None else all(p.is_plain_greedy for p in params):
             self.K.argmax(logits, out)
-            return self._read(out)
-        f = np.zeros((5, rows), dtype=np.float32)      # temperature, top_p, min_p, rep_penalty, uniform
-        k = np.zeros(rows, dtype=np.int32)
+            return out
+        distinct = params if one is None else (one,)
+        penalty = [p.repetition_penalty for p in distinct] * (rows if one is not None else 1)
+        penalised = any(p.repetition_penalty != 1.0 for p in distinct)
         if callable(histories):
-            histories = histories() if any(p.repetition_penalty != 1.0 for p in params) else None
-        hist_off, hist_tok, hist_cnt = [0], [], []
-        bias_off, bias_tok, bias_val = [0], [], []
-        for i, p in enumerate(params):
-            f[0, i], f[1, i], f[2, i], f[3, i] = p.temperature, p.top_p, p.min_p, p.repetition_penalty
-            f[4, i] = uniform(seeds[i], sequence_ids[i], steps[i])
-            k[i] = p.top_k
-            if p.repetition_penalty != 1.0 and histories is not None:
-                for tok, cnt in Counter(histories[i]).items():
-                    hist_tok.append(tok)
-                    hist_cnt.append(cnt)
-            hist_off.append(len(hist_tok))
-            if p.logit_bias:
-                for tok, delta in p.logit_bias:
+            histories = histories() if penalised else None
+        f = np.empty((5, rows), dtype=np.float32)      # temperature, top_p, min_p, rep_penalty, uniform
+        f[0] = [p.temperature for p in distinct]               # (one number fills the row)
+        f[1] = [p.top_p for p in distinct]
+        f[2] = [p.min_p for p in distinct]
+        f[3] = penalty
+        f[4] = uniforms(seeds, sequence_ids, steps)
+        k = np.empty(rows, dtype=np.int32)
+        k[:] = [p.top_k for p in distinct]
+        # what the penalty and the biases of each row name: offsets, tokens, numbers
+        hist_off, bias_off = np.zeros(rows + 1, np.int32), np.zeros(rows + 1, np.int32)
+        hist_tok, hist_cnt, bias_tok, bias_val = [], [], [], []
+        if penalised and histories is not None:
+            for i, v in enumerate(penalty):
+                if v != 1.0:
+                    for tok, cnt in Counter(histories[i]).items():
+                        hist_tok.append(tok)
+                        hist_cnt.append(cnt)
+                hist_off[i + 1] = len(hist_tok)
+        if any(p.logit_bias for p in distinct):
+            for i, p in enumerate(params):
+                for tok, delta in (p.logit_bias or ()):
                     bias_tok.append(tok)
                     bias_val.append(delta)
-            bias_off.append(len(bias_tok))
-        fd = torch.from_numpy(f).to(self.device)
-        ints = np.concatenate([k, np.asarray(hist_off, np.int32), np.asarray(bias_off, np.int32),
-                               np.asarray(hist_tok, np.int32), np.asarray(hist_cnt, np.int32),
-                               np.asarray(bias_tok, np.int32)]).astype(np.int32)
-        idev = torch.from_numpy(ints).to(self.device)
-        o = 0
-        kd = idev[o:o + rows]; o += rows
-        ho = idev[o:o + rows + 1]; o += rows + 1
-        bo = idev[o:o + rows + 1]; o += rows + 1
-        ht = idev[o:o + len(hist_tok)]; o += len(hist_tok)
-        hc = idev[o:o + len(hist_cnt)]; o += len(hist_cnt)
-        bt = idev[o:o + len(bias_tok)]
-        bv = torch.tensor(bias_val, dtype=torch.float32, device=self.device) if bias_val else None
-        work = torch.empty((rows, vocab), dtype=torch.float32, device=self.device)
-        self.K.sample(logits, work, out, fd[0], fd[4], top_k=kd, top_p=fd[1], min_p=fd[2], rep_penalty=fd[3],
-                      hist_off=ho, hist_tok=ht if hist_tok else None, hist_cnt=hc if hist_cnt else None,
-                      bias_off=bo, bias_tok=bt if bias_tok else None, bias_val=bv)
-        return self._read(out)
+                bias_off[i + 1] = len(bias_tok)
+        parts = [f.reshape(-1).view(np.int32), k, hist_off, bias_off, np.asarray(hist_tok, np.int32), np.asarray(hist_cnt, np.int32),
+                 np.asarray(bias_tok, np.int32), np.asarray(bias_val, np.float32).view(np.int32)]
+        sizes = [part.size for part in parts]
+        words = np.concatenate(parts)
+        if staged:
+            words, work = self._stage(words), self._work(rows, vocab)
+        else:
+            words = torch.from_numpy(words).to(self.device)
+            work = torch.empty((rows, vocab), dtype=torch.float32, device=self.device)
+        opts, kd, ho, bo, ht, hc, bt, bv = words[:sum(sizes)].split(sizes)
+        fd = opts.view(torch.float32).view(5, rows)
+        self.K.sample(logits, work, out, fd[0], fd[4], top_k=kd, top_p=fd[1], min_p=fd[2],
+                      rep_penalty=fd[3] if penalised else None, hist_off=ho if penalised else None,
+                      hist_tok=ht if hist_tok else None, hist_cnt=hc if hist_cnt else None,
+                      bias_off=bo, bias_tok=bt if bias_tok else None, bias_val=bv.view(torch.float32) if bias_tok else None)
+        return out
 
     def choose_async(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                      sequence_ids: Sequence[int], steps: Sequence[int]) -> "PendingTokens":
@@ -113,37 +128,8 @@ class Sampler:
         tokens stay on the device too (`PendingTokens.device`), where the next step can read them."""
         if any(p.repetition_penalty != 1.0 for p in params):
             raise ValueError("choose_async cannot apply a repetition penalty: it needs the tokens on the host")
-        rows, vocab = logits.shape
-        out = torch.empty(rows, dtype=torch.int32, device=self.device)
-        if all(p.is_plain_greedy for p in params):
-            self.K.argmax(logits, out)
-        else:
-            f = np.zeros((4, rows), dtype=np.float32)
-            k = np.zeros(rows, dtype=np.int32)
-            bias_off, bias_tok, bias_val = [0], [], []
-            for i, p in enumerate(params):
-                f[0, i], f[1, i], f[2, i] = p.temperature, p.top_p, p.min_p
-                f[3, i] = uniform(seeds[i], sequence_ids[i], steps[i])
-                k[i] = p.top_k
-                for tok, delta in (p.logit_bias or ()):
-                    bias_tok.append(tok)
-                    bias_val.append(delta)
-                bias_off.append(len(bias_tok))
-            # every option of the step in one pinned buffer and one copy that does not wait
-            nb = len(bias_tok)
-            words = np.concatenate([f.reshape(-1).view(np.int32), k, np.asarray(bias_off, np.int32),
-                                    np.asarray(bias_tok, np.int32), np.asarray(bias_val, np.float32).view(np.int32)])
-            dev = self._stage(words)
-            fd = dev[:4 * rows].view(torch.float32).view(4, rows)
-            o = 4 * rows
-            kd = dev[o:o + rows]; o += rows
-            bo = dev[o:o + rows + 1]; o += rows + 1
-            bt = dev[o:o + nb] if nb else None; o += nb
-            bv = dev[o:o + nb].view(torch.float32) if nb else None
-            work = self._work(rows, vocab)
-            self.K.sample(logits, work, out, fd[0], fd[3], top_k=kd, top_p=fd[1], min_p=fd[2],
-                          bias_off=bo, bias_tok=bt, bias_val=bv)
-        host = torch.empty(rows, dtype=torch.int32, pin_memory=True)
+        out = self._launch(logits, params, seeds, sequence_ids, steps, staged=True)
+        host = torch.empty(out.numel(), dtype=torch.int32, pin_memory=True)
         host.copy_(out, non_blocking=True)
         done = torch.cuda.Event()
         done.record()

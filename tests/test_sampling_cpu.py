@@ -29,3 +29,11 @@ def test_uniform_is_a_function_of_seed_sequence_and_step():
     assert abs(sum(xs) / len(xs) - 0.5) < 0.02
     import numpy as np
     assert all(float(np.float32(x)) == x for x in xs[:100])        # exact in float32
+
+
+def test_uniforms_of_a_batch_are_the_single_ones():
+    from braidinfer_b200.sampling.rng import uniforms
+    seeds = [0, 5, (1 << 64) - 1, 1 << 63, -7, (1 << 70) + 3] * 40
+    ids, steps = [i * 37 % 1009 for i in range(len(seeds))], [i * i for i in range(len(seeds))]
+    got = uniforms(seeds, ids, steps)
+    assert got.dtype.name == "float32" and [float(x) for x in got] == [uniform(*t) for t in zip(seeds, ids, steps)]
