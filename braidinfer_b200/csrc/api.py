@@ -735,6 +735,9 @@ class Kernels:
                                                 c_longlong, c_void_p] + [c_int] * 4 + [c_float, c_void_p]
                 lib.braid_scan_decay.argtypes = [c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_float, c_void_p]
                 lib.braid_linear_scan_work_floats.argtypes = [c_int] * 7
+                lib.braid_ssd_scan.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 4 + [c_longlong, c_void_p, c_longlong, c_longlong] + \
+                                              [c_void_p] * 3 + [c_int] * 5 + [c_float, c_void_p]
+                lib.braid_ssd_scan.restype = c_int
                 lib.braid_linear_scan_work_floats.restype = c_longlong
                 lib.braid_gated_norm.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong,
                                                  c_void_p] + [c_int] * 6 + [c_float, c_float, c_void_p]
@@ -1352,6 +1355,19 @@ class Kernels:
             y.data_ptr(), gate.data_ptr(), gate.stride(0), w.data_ptr(), w.numel(), out.data_ptr(), out.stride(0),
             token_seq.data_ptr(), dtype_code(out.dtype), rows, width, group, float(eps), self._stream()), "delta_gated_norm")
 
+    # Tokens of a step's longest sequence from which on a recurrence with a decay a head runs over chunks on the tensor cores
+    # (csrc/scan_mma.cu): a chunk of 64 takes what some 16 tokens take one by one.  Long sequences on fewer than 64 CTAs with keys of
+    # 64 stay with the walk, whose chunks run side by side (32 heads of 64 x 64, 2,048 tokens: 158 beside 204 us).
+    SSD_FROM = 17
+
+    def _ssd_fits(self, q, k, v, out, state, state_offset: int, ctx, heads: int, dk: int, dv: int, v_cols: int) -> bool:
+        if dk == 64 and int(ctx.max_q_len) >= 1024 and ctx.n_seqs * heads * (dv // 64) < 64:
+            return False
+        return (SCAN_CHUNK is None and q.dtype == torch.bfloat16 and int(ctx.max_q_len) >= self.SSD_FROM and dk in (64, 128)
+                and dv % 64 == 0 and v_cols == dv and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v))
+                and out.stride(0) % 2 == 0 and out.data_ptr() % 8 == 0
+                and (state.data_ptr() | int(state_offset) | state.stride(0)) % 8 == 0)
+
     def linear_scan(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, gate_bias: torch.Tensor,
                     out: torch.Tensor, state: torch.Tensor, state_offset: int, ctx, heads: int, groups: int, dk: int,
                     dv: int, mode: str, q_scale: float = 1.0, inv_tau: float = 1.0, a_log: Optional[torch.Tensor] = None,
@@ -1397,6 +1413,14 @@ class Kernels:
         vc = dv if v_cols is None else int(v_cols)
         if v.shape[1] < heads * vc or out.shape[1] < heads * dv:
             raise KernelError("linear_scan: v or out does not hold the heads' columns")
+        if chunk is None and mode == "head" and self._ssd_fits(q, k, v, out, state, state_offset, ctx, heads, dk, dv, vc):
+            self.launches += 1
+            self._check_lib(lib, lib.braid_ssd_scan(
+                q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(), gate.stride(0),
+                gate_bias.data_ptr(), a_log.data_ptr(), _ptr(skip), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
+                ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), ctx.n_seqs, heads, groups, dk, dv, float(q_scale),
+                self._stream()), "ssd_scan")
+            return
         if chunk is None:
             chunk = SCAN_CHUNK if SCAN_CHUNK is not None else (128 if int(ctx.max_q_len) >= 1024 else 64)
         chunk = int(chunk)
