@@ -71,7 +71,7 @@ class Sampler:
         tokens (int32, on the device)."""
         rows, vocab = logits.shape
         out = torch.empty(rows, dtype=torch.int32, device=self.device)
-        one = params[0] if all(p is params[0] for p in params) else None       # one set of options for all rows
+        one = params[0] if rows and all(p is params[0] for p in params) else None       # one set of options for all rows
         if one.is_plain_greedy if one is not None else all(p.is_plain_greedy for p in params):
             self.K.argmax(logits, out)
             return out
