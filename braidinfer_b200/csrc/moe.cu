@@ -535,8 +535,8 @@ extern "C" int braid_moe_gemm_mma(const void* x, const void* w0, const void* w1,
 // (wgt null: every weight is 1, for experts whose weight went into their input).
 // A thread owns V neighbouring columns of a row (16 bytes of y, or one number where sizes or starts do not allow that) and asks for
 // up to MOE_COMBINE_BATCH choices' outputs at once; a CTA of 64 threads a span of columns, so that a decode step's few rows
-// spread over the SMs.  12,288 outputs of 2,048 columns: 40 us with a CTA a row and 2-byte loads in a chain; a Bidinex
-// model's batch of 8, 25 steps of four such sums and more, 14.5 ms a turn so and 13.9 with these.
+// spread over the SMs.  12,288 outputs of 2,048 columns: 42 us with a CTA a row and 2-byte loads in a chain, 18 so; 8 rows of 6 choices
+// 15 and 2.7 us.
 #define MOE_COMBINE_THREADS 64
 #define MOE_COMBINE_BATCH 8
 template <typename T, int V>
