@@ -436,6 +436,8 @@ extern "C" int braid_latent_attn_tc(const void* q_u, long long qu_head, long lon
     if ((((uintptr_t)q_u | (uintptr_t)q_lat | (uintptr_t)kv | (uintptr_t)cache | (uintptr_t)out) & 15) || qu_head % 8 || qu_row % 8 || out_row_stride % 8)
         BRAID_REFUSE("latent_attn_tc: operands and their rows must start on 16 bytes");
     if (!error_flag) BRAID_REFUSE("latent_attn_tc: error_flag is required");
+    // the maximum is taken, and keys are masked, before the factor
+    if (!(scale > 0.f)) BRAID_REFUSE("latent_attn_tc: the factor on the scores must be positive, not %g", (double)scale);
     const int D = rank + rot;
     const cuuint64_t wide = (cuuint64_t)heads * (dim + vdim);
     CUtensorMap mqu, mqr, mkv, mkr;

@@ -207,6 +207,8 @@ class LatentAttention(Mixer):
             return None
         if self.gated is False and self.out_mult != 1.0:
             return None
+        if not self.scale > 0:                                # that kernel masks before the factor
+            return None
         pages = self.rt.kernels.latent_pages(ctx.host_q_len, ctx.host_kv_before, self.window)
         total = sum(pages)
         if sum(n * p for n, p in zip(ctx.host_q_len, pages)) < EXPAND_QUERIES * total:

@@ -6,7 +6,7 @@ import math
 import pytest
 import torch
 
-from braidinfer_b200.csrc.api import get_kernels
+from braidinfer_b200.csrc.api import KernelError, get_kernels
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -138,3 +138,31 @@ def test_the_part_that_chooses(monkeypatch, chunks):
     assert not calls
     # both are bfloat16 of the same mechanism; the model's tests ask 1e-2 .. 2e-2 of either beside float64
     assert float((got - want).norm() / want.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_score_factors_that_are_not_positive(K, monkeypatch, scale):
+    """The kernel masks before the factor, so it refuses such a factor and prompts keep the latent form."""
+    from braidinfer_b200.engine import Engine
+    import braidinfer_b200.parts.latent_attention as LA
+    mixer = {"heads": 4, "dim": 64, "rot_dim": 32, "rot": {"base": 10000.0, "dims": 32}, "vdim": 64, "kv_rank": 256, "scale": scale}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 4, "top": 2, "groups": {"count": 1, "keep": 1}}}
+    cfg = {"architecture": "Bidinex", "vocab": 256, "width": 128, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+           "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    eng = Engine.from_random(cfg, 3, max_tokens=512, max_slots=1, verbose=False)
+    toks = torch.randint(0, 256, (300,), generator=torch.Generator().manual_seed(2)).tolist()
+
+    def logits():
+        s = eng.open()
+        out = eng.step([(s, toks)], want="all")
+        eng.close(s)
+        eng.check()
+        return out
+
+    got = logits()
+    monkeypatch.setattr(LA, "EXPAND_BYTES", 0)
+    assert torch.isfinite(got).all() and torch.equal(got, logits())
+    z = lambda *s: torch.zeros(*s, device=DEV, dtype=BF)
+    with pytest.raises(KernelError, match="positive"):
+        K.attn_latent_tc(z(1, 1, 64), z(1, 1, 80), z(64, 128), z(1, 1, 1, 64, 80), z(1, 64), i32([[0]]), i32([0]), i32([1]), i32([0]), 1, 1,
+                         64, 64, None, scale)
