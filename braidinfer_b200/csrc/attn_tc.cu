@@ -418,6 +418,8 @@ extern "C" int braid_attn_tc(const void* q, void* out, const void* cache, long l
     if (!error_flag) BRAID_REFUSE("attn_tc: error_flag is required");
     if (!bias_slope != !bias_rate) BRAID_REFUSE("attn_tc: a distance bias has a slope and a rate a head");
     if (softcap > 0.f && bias_slope) BRAID_REFUSE("attn_tc: a cap on the scores and a distance bias are not combined");
+    // without a bias or a cap the maximum is taken, and keys are masked, before the factor
+    if (!(softcap > 0.f) && !bias_slope && !(scale > 0.f)) BRAID_REFUSE("attn_tc: the factor on plain scores must be positive, not %g", (double)scale);
     TcEncodeTiledFn fn = tc_encode_tiled_fn();
     if (!fn) BRAID_REFUSE("attn_tc: the driver does not export cuTensorMapEncodeTiled");
     const int g = nqh / nkh;

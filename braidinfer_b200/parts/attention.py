@@ -360,10 +360,12 @@ class GQAAttention(Mixer):
         runs use the tcgen05 kernel for prompts (head sizes 64 and 128; "mma" as the
         backend keeps them on the mma.sync kernel, which also serves every other head
         size), and the mma.sync kernel with the context sliced for steps of few tokens,
-        so that a handful of sequences still fills the machine."""
+        so that a handful of sequences still fills the machine.  A factor on plain scores that is not positive goes to the
+        mma.sync kernel too: the tcgen05 kernel masks before the factor."""
         K = self.rt.kernels
         plain = (self.rt.is_f32 or self.rt.attention_backend == "plain" or not K.attn_mma_supports(hd))
         extras = bool(self.keep_first) or self.head_scale is not None or value_heads > 1
+        scaled_late = self.distance_bias is None and not self.softcap and not self.scale > 0
         if plain:
             K.attn_simple(qkv, out, cache.storage, cache.page_table, ctx.positions, ctx.token_seq,
                           self.nqh, self.nkh, hd, cache.page_size, self.window, self.scale, sink=self.sink,
@@ -372,7 +374,7 @@ class GQAAttention(Mixer):
                           distance_bias=self.distance_bias, softcap=self.softcap)
             return
         few = ctx.max_q_len <= 8
-        if not few and self.rt.attention_backend == "auto" and K.attn_tc_supports(hd) and not extras:
+        if not few and self.rt.attention_backend == "auto" and K.attn_tc_supports(hd) and not extras and not scaled_late:
             K.attn_tc(qkv, out, cache.storage, cache.page_table, ctx.q_start, ctx.q_len, ctx.kv_before,
                       ctx.n_seqs, ctx.max_q_len, self.nqh, self.nkh, hd, self.window, self.scale, sink=self.sink,
                       head_sinks=self.head_sinks, head_gate=gate, out_scale=self.out_mult,

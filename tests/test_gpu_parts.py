@@ -187,3 +187,30 @@ def test_block_and_schedule_against_the_plain_model(tmp_path):
         eng.check()
         err = (torch.cat(got).double().cpu() - want).abs().max().item()
         assert err < (2e-5 if dtype == "float32" else 1.5e-2), err
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1, 0.1])
+def test_prompt_attention_with_any_factor_on_the_scores(scale):
+    """The tcgen05 kernel masks before the factor: one that is not positive goes to the mma.sync kernel."""
+    from braidinfer_b200.csrc.api import KernelError, get_kernels
+    from braidinfer_b200.engine import Engine
+    left = {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "scale": scale, "mask": {"size": 512},
+            "rot": {"base": 1e6, "dims": 32, "scaling": {"factor": 4.0, "original": 4096, "fast": 16.0, "slow": 2.0}}}
+    par = {"type": "parallel", "mlp": {"kind": "dense", "ff": 128},
+           "mixer": {"left": left, "right": {"heads": 2, "dim": 64, "vdim": 64, "tau": 8.0}, "left_scale": 1.0, "right_scale": 1.0}}
+    cfg = {"architecture": "Loduzen", "vocab": 256, "width": 128, "norm": {"eps": 1e-6}, "token_side": {"dim": 64}, "layers": [par]}
+    toks = torch.randint(0, 256, (300,), generator=torch.Generator().manual_seed(2)).tolist()
+    got = {}
+    for backend in ("auto", "mma"):
+        eng = Engine.from_random(cfg, 3, max_tokens=512, max_slots=1, verbose=False, attention_backend=backend)
+        got[backend] = eng.step([(eng.open(), toks)], want="all").double()
+        eng.check()
+    assert torch.isfinite(got["auto"]).all()
+    if scale > 0:
+        assert float((got["auto"] - got["mma"]).norm() / got["mma"].norm()) < 1e-2
+        return
+    assert torch.equal(got["auto"], got["mma"])
+    z = lambda *s: torch.zeros(*s, device=DEV, dtype=torch.bfloat16)
+    i = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    with pytest.raises(KernelError, match="positive"):
+        get_kernels().attn_tc(z(9, 192), z(9, 64), z(1, 2, 1, 64, 64), i(0)[None], i(0), i(9), i(0), 1, 9, 1, 1, 64, None, scale)
