@@ -127,8 +127,9 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
             }
             const float cmax = warp_max(s);
             const float m_new = fmaxf(m, cmax);
+            const float ref = m_new == -INFINITY ? 0.f : m_new;  // no finite score yet: every weight is 0, or NaN where a score is
             const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-            const float p = (j < end) ? expf(s - m_new) : 0.f;
+            const float p = (j < end) ? expf(s - ref) : 0.f;
             l = l * corr + warp_sum(p);
             m = m_new;
             ps[lane] = p;
@@ -165,10 +166,10 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
         __syncthreads();
         if (slice) return;
         for (int w = 1; w < wpi; ++w) {
+            // a warp without a finite score has weight 0, which leaves nothing of its zeros and all of a NaN
             const float mw = ml[2 * (warp + w)], lw = ml[2 * (warp + w) + 1];
-            if (mw == -INFINITY) continue;                       // a warp without keys
-            const float m_new = fmaxf(m, mw);
-            const float mine = (m == -INFINITY) ? 0.f : expf(m - m_new), its = expf(mw - m_new);
+            const float m_new = fmaxf(m, mw), ref = m_new == -INFINITY ? 0.f : m_new;
+            const float mine = expf(m - ref), its = expf(mw - ref);
             l = l * mine + lw * its;
             m = m_new;
             const float* other = qs + w * hdp;

@@ -45,3 +45,37 @@ def test_plain_attention_with_several_warps_an_item(K, hd, seqs, window, dtype):
     worst, out, _ = attention_case(K, "simple", dtype, hd, 4, 2, seqs, window)
     assert worst < (2e-5 if dtype == torch.float32 else 2e-2)       # as test_gpu_kernels.py asks of this kernel
     assert (out[-1] == 0).all()                                     # the row of padding
+
+
+def attend_one(K, dtype, spoil):
+    """One query of four heads over 700 keys, eight warps a (token, head): 22 blocks of 32 keys, every eighth a warp's."""
+    heads, kv_heads, hd, keys = 4, 2, 64, 700
+    k, v = rnd(keys, kv_heads, hd, dtype=dtype, seed=1), rnd(keys, kv_heads, hd, dtype=dtype, seed=2)
+    qkv = rnd(1, (heads + 2 * kv_heads) * hd, dtype=dtype, seed=3)
+    qkv[0, 0:heads * hd:hd] = 1.0
+    spoil(k)
+    cache = torch.zeros(11, 2, kv_heads, 64, hd, device=DEV, dtype=dtype)
+    for p in range(keys):
+        cache[p // 64, 0, :, p % 64], cache[p // 64, 1, :, p % 64] = k[p], v[p]
+    i = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    out = torch.empty(1, heads * hd, device=DEV, dtype=dtype)
+    K.attn_simple(qkv, out, cache, i(*range(11))[None], i(keys - 1), i(0), heads, kv_heads, hd, 64, None, 0.125)
+    q = qkv[0, :heads * hd].view(heads, hd).double()
+    s = torch.einsum("hd,khd->hk", q, k.double().repeat_interleave(2, 1)) * 0.125
+    return out.view(heads, hd), torch.einsum("hk,khd->hd", torch.softmax(s, -1), v.double().repeat_interleave(2, 1))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("blocks", [[0], [1], [5, 13, 21], [0, 1, 2, 3, 4, 5, 6, 7]])
+def test_blocks_of_keys_without_a_finite_score(K, dtype, blocks):
+    """A warp whose blocks, the first or all, hold no finite score: scores of -inf weigh nothing, a NaN is not lost."""
+    def spoil(value):
+        def f(k):
+            for b in blocks:
+                k[32 * b:32 * b + 32, :, 0] = value
+        return f
+
+    out, want = attend_one(K, dtype, spoil(float("-inf")))
+    assert (out.double() - want).abs().max() < (2e-5 if dtype == torch.float32 else 2e-2)
+    out, _ = attend_one(K, dtype, spoil(float("nan")))
+    assert torch.isnan(out).all()
