@@ -9,7 +9,8 @@
 // goes in as the sum of three bfloat16 numbers, 24 bits, in three products that add into one float32 accumulator: nothing is
 // rounded to fewer bits than the walk token by token keeps, only the order of the sums differs (the tests hold the error beside
 // float64 to the walk's own).  The decays are products of decays, never
-// differences of logarithms.
+// differences of logarithms.  A token's numbers never reach the tokens before it, be they infinite: the block on the diagonal
+// selects the later tokens away instead of multiplying them by zero.
 //
 // A CTA of four warps owns (head, sequence, 64 value columns) and walks the sequence's chunks, the state in its accumulator
 // registers (a warp a quarter of the key rows); a warp owns 16 tokens of a chunk's output, and its P goes from the accumulators of
@@ -19,6 +20,7 @@
 // 2,048 tokens 267 / 929.  32 heads of 64 x 64: 3 sequences 156 / 244, 300 tokens 38 / 68, one sequence of 2,048 tokens 204 / 158 (half a
 // CTA for every second SM, each on a chain of 32 chunks): that form stays with the walk in chunks.
 #include "common.cuh"
+#include <type_traits>
 
 #define SSD_C 64
 #define SSD_P 64
@@ -49,15 +51,24 @@ __device__ __forceinline__ void ssd_mma(float* c, const uint32_t* a, uint32_t b0
 __device__ __forceinline__ void ssd_copy16(void* dst, const void* src, bool in) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ssd_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
-// x = the sum of three bfloat16 numbers to float32's 24 bits; two x at once, packed
+// x = the sum of three bfloat16 numbers to float32's 24 bits; two x at once, packed.  The first two saturate, so that a number past the
+// largest bfloat16 one is still a sum of finite parts; an infinity is left over for the third.
 __device__ __forceinline__ void ssd_split2(float x0, float x1, uint32_t* w) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-        w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        x0 -= __low2float(h);
-        x1 -= __high2float(h);
+        if (i < 2) {
+            asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(x1), "f"(x0));
+        } else {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        x0 -= __uint_as_float(w[i] << 16);
+        x1 -= __uint_as_float(w[i] & 0xffff0000u);
     }
+}
+// two bfloat16 numbers, those that are not finite replaced by zero
+__device__ __forceinline__ uint32_t ssd_finite(uint32_t w) {
+    return ((w & 0x7f80u) == 0x7f80u ? 0u : w & 0xffffu) | ((w & 0x7f800000u) == 0x7f800000u ? 0u : w & 0xffff0000u);
 }
 // The byte offset of 16-byte run `c` of row `r` in a tile of rows of RUNS runs (8 or 16): runs are swapped within their group of eight
 // by the row's low bits, so that eight rows of one run lie in eight different banks' quads.
@@ -65,7 +76,7 @@ template <int RUNS>
 __device__ __forceinline__ uint32_t ssd_at(int r, int c) { return (uint32_t)(r * RUNS + (c ^ (r & 7))) * 16; }
 
 template <int DK> constexpr int ssd_smem() {
-    return SSD_C * DK * 2 * 2 + SSD_C * SSD_P * 2 + SSD_C * (SSD_C + 1) * 4 + 3 * DK * SSD_P * 2 + 4 * SSD_C * 4 + 16;
+    return SSD_C * DK * 2 * 2 + SSD_C * SSD_P * 2 + SSD_C * (SSD_C + 1) * 4 + 3 * DK * SSD_P * 2 + 4 * SSD_C * 4 + SSD_C / 16 * 4;
 }
 
 template <int DK>
@@ -83,6 +94,7 @@ ssd_chunk_kernel(SsdArgs a) {
     float* s_dt = s_a + C;
     float* s_d0 = s_dt + C;                                  // D(0, t)
     float* s_w = s_d0 + C;                                   // dt_t D(t, 64)
+    int* s_odd = (int*)(s_w + C);                            // [C / 16]
     uint8_t* sW = sQ;
     static_assert(3 * C * P * 2 <= C * DK * 2 + C * (C + 1) * 4, "the weighted values fit where q and the decays were");
     pdl_trigger();
@@ -164,6 +176,19 @@ ssd_chunk_kernel(SsdArgs a) {
                 run *= s_a[t];
                 s_d0[t] = run;
             }
+        } else if (warp == 3) {                              // meanwhile: which blocks of 16 tokens hold values that are not finite
+#pragma unroll
+            for (int b = 0; b < C / 16; ++b) {
+                uint32_t top = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(sV + (b * 128 + i * 32 + lane) * 16);
+                    top |= ((u.x & 0x7f807f80u) + 0x00800080u) | ((u.y & 0x7f807f80u) + 0x00800080u) |
+                           ((u.z & 0x7f807f80u) + 0x00800080u) | ((u.w & 0x7f807f80u) + 0x00800080u);
+                }
+                const bool any = __any_sync(0xffffffffu, top & 0x80008000u);
+                if (lane == 0) s_odd[b] = any;
+            }
         }
         // Q K^T, the warp's 16 tokens against the tokens up to them
         const int tw = warp * 16;
@@ -200,31 +225,66 @@ ssd_chunk_kernel(SsdArgs a) {
         const float d0 = s_d0[tw + g], d1 = s_d0[tw + g + 8];
 #pragma unroll
         for (int t = 0; t < 8; ++t) { o[t][0] *= d0; o[t][1] *= d0; o[t][2] *= d1; o[t][3] *= d1; }
+        // 16 tokens s against this warp's 16; `odd`: on the diagonal, with values that are not finite.  (A form of its own: looked at
+        // product by product it takes 13 % of the kernel.)
+        auto weigh = [&](int ks, auto odd) {
+            uint32_t pa[3][4];
+            float pw[2][4];
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)                       // 16 tokens s
-            if (ks <= warp) {
-                uint32_t pa[3][4];
+            for (int half = 0; half < 2; ++half) {
+                const int t = 2 * ks + half, s = t * 8 + q2;
+                const float *lo = sD + (tw + g) * (C + 1) + s, *hi = lo + 8 * (C + 1);
+                uint32_t w[3], x[3];
+                // tokens after this one are left out, whatever their products are: zero times an infinity is none
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int t = 2 * ks + half, s = t * 8 + q2;
-                    const float *lo = sD + (tw + g) * (C + 1) + s, *hi = lo + 8 * (C + 1);
-                    uint32_t w[3], x[3];
-                    ssd_split2(qk[t][0] * lo[0], qk[t][1] * lo[1], w);
-                    ssd_split2(qk[t][2] * hi[0], qk[t][3] * hi[1], x);
+                for (int e = 0; e < 4; ++e)
+                    pw[half][e] = s + (e & 1) <= tw + g + (e >> 1) * 8 ? qk[t][e] * (e < 2 ? lo : hi)[e & 1] : 0.f;
+                ssd_split2(pw[half][0], pw[half][1], w);
+                ssd_split2(pw[half][2], pw[half][3], x);
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) { pa[p][2 * half] = w[p]; pa[p][2 * half + 1] = x[p]; }
+                for (int p = 0; p < 3; ++p) { pa[p][2 * half] = w[p]; pa[p][2 * half + 1] = x[p]; }
+            }
+#pragma unroll
+            for (int pr = 0; pr < 4; ++pr) {
+                uint32_t vb[4];
+                ssd_ldm4t(vb, ssd_u32(sV) + ssd_at<8>(ks * 16 + (lm & 1) * 8 + lr, pr * 2 + (lm >> 1)));
+                if constexpr (odd.value) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) vb[i] = ssd_finite(vb[i]);
                 }
 #pragma unroll
-                for (int pr = 0; pr < 4; ++pr) {
-                    uint32_t vb[4];
-                    ssd_ldm4t(vb, ssd_u32(sV) + ssd_at<8>(ks * 16 + (lm & 1) * 8 + lr, pr * 2 + (lm >> 1)));
+                for (int p = 0; p < 3; ++p) {
+                    ssd_mma(o[2 * pr], pa[p], vb[0], vb[1]);
+                    ssd_mma(o[2 * pr + 1], pa[p], vb[2], vb[3]);
+                }
+            }
+            if constexpr (odd.value) {                       // the values left out, for their own and later tokens alone
+#pragma unroll 1
+                for (int s = 0; s < 16; ++s) {
+                    const int from = (lane & 28) | ((s & 7) >> 1);
+                    const float p0 = __shfl_sync(0xffffffffu, s & 8 ? (s & 1 ? pw[1][1] : pw[1][0]) : (s & 1 ? pw[0][1] : pw[0][0]), from);
+                    const float p1 = __shfl_sync(0xffffffffu, s & 8 ? (s & 1 ? pw[1][3] : pw[1][2]) : (s & 1 ? pw[0][3] : pw[0][2]), from);
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) {
-                        ssd_mma(o[2 * pr], pa[p], vb[0], vb[1]);
-                        ssd_mma(o[2 * pr + 1], pa[p], vb[2], vb[3]);
+                    for (int x = 0; x < 8; ++x) {
+                        const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(sV + ssd_at<8>(ks * 16 + s, x) + q2 * 2);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float v = e ? __high2float(vv) : __low2float(vv);
+                            if (isfinite(v)) continue;
+                            if (s <= g) o[x][e] = fmaf(p0, v, o[x][e]);
+                            if (s <= g + 8) o[x][2 + e] = fmaf(p1, v, o[x][2 + e]);
+                        }
                     }
                 }
             }
+        };
+        const bool odd = s_odd[warp];
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            if (ks > warp) continue;
+            if (odd && ks == warp) weigh(ks, std::true_type{});
+            else weigh(ks, std::false_type{});
+        }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int t = tw + g + e * 8;

@@ -77,6 +77,54 @@ def test_chunks(K, heads, groups, dk, dv, lens, decay, with_skip):
     assert max(errors[None]) < 1.5 * max(errors[0]) + 2.0 ** -22 and max(errors[None]) < 2.0 ** -19
 
 
+def scan(K, dk, tokens, spoil=None, chunk=None):
+    heads, groups, dv = 2, 1, 64
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v, gate = rnd(tokens, groups * dk).to(BF), rnd(tokens, groups * dk).to(BF), rnd(tokens, heads * dv).to(BF), rnd(tokens, heads).to(BF)
+    bias, a_log, S = rnd(heads).to(BF), (rnd(heads) * 0.3 - 6.0).to(BF), rnd(1, heads, dk, dv)
+    if spoil:
+        spoil({"q": q, "k": k, "v": v, "gate": gate, "state": S})
+    out = torch.empty(tokens, heads * dv, device=DEV)
+    K.linear_scan(q, k, v, gate, bias, out, S.view(1, -1).view(torch.uint8), 0, step([tokens], [0]), heads, groups, dk, dv, "head",
+                  a_log=a_log, chunk=chunk)
+    return out
+
+
+@pytest.mark.parametrize("dk", [64, 128])
+@pytest.mark.parametrize("at", [1, 9, 15, 16, 40, 79])
+@pytest.mark.parametrize("what", ["q", "k", "v", "gate"])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan"), 3e38])
+def test_a_token_leaves_the_tokens_before_it_alone(K, dk, at, what, bad):
+    """Numbers that are not finite, or whose products are not: the bits of earlier tokens stay, a value's other columns too, and the
+    results that are finite are those of the walk."""
+    def spoil(t):
+        t[what][at, 1] = bad
+
+    clean, got, walk = scan(K, dk, 80), scan(K, dk, 80, spoil), scan(K, dk, 80, spoil, chunk=0)
+    keep = torch.arange(80, device=DEV) != at if what == "q" else torch.arange(80, device=DEV) < at
+    assert torch.equal(got[keep], clean[keep])
+    if what == "v":
+        assert torch.equal(got[:, 2:], clean[:, 2:]) and torch.equal(got[:, :1], clean[:, :1])
+    if bad != 3e38 and not (what == "gate" and bad < 0):                # (a step that softplus makes zero: 0 times a number)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(walk))
+
+
+@pytest.mark.parametrize("dk", [64, 128])
+@pytest.mark.parametrize("big", [float("inf"), float("-inf"), 3.4e38])
+def test_the_largest_numbers_of_a_state(K, dk, big):
+    """3.4e38 is past the largest bfloat16 number: its three parts must be finite, and an infinity's must not be NaN."""
+    def spoil(t):
+        t["state"][0, 1, 5, 3] = big
+        t["q"] *= 2.0 ** -8
+
+    got, walk = (scan(K, dk, 40, spoil, chunk=c) for c in (None, 0))
+    for same in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(same(got), same(walk))
+    ok = torch.isfinite(walk)
+    assert float((got[ok].double() - walk[ok].double()).norm() / walk[ok].double().norm()) < 2.0 ** -18
+
+
 @pytest.mark.parametrize("rows, groups, group", [(90, 16, 256), (200, 8, 512), (160, 8, 520), (1190, 1, 136), (2, 16, 256)])
 @pytest.mark.parametrize("gate_type", [BF, torch.float32])
 @pytest.mark.parametrize("gate_first", [True, False])
