@@ -315,7 +315,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * sc;   // scale > 0 commutes with the maximum
             // raise m only when the tile towers over it; -inf + 8 = -inf, so the first finite maximum always does
             const bool raise = mx > m + FA_RAISE;
-            const float factor = raise ? fast_exp2(m - mx) : 1.f;                     // exp2(-inf) = 0: nothing was summed yet
+            const float factor = raise ? exp2f(m - mx) : 1.f;                     // exp2(-inf) = 0: nothing was summed yet
             if (raise) m = mx;
             // a row that is no query (past the tile's tokens) sums nothing: exp2(-inf) = 0
             const float ms = (!valid && all_visible) ? INFINITY : ((m == -INFINITY) ? 0.f : m);
@@ -323,8 +323,8 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
             uint32_t pk[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-                const float p0 = fast_exp2(fmaf(sv[2 * i], sc, -ms));
-                const float p1 = fast_exp2(fmaf(sv[2 * i + 1], sc, -ms));
+                const float p0 = exp2f(fmaf(sv[2 * i], sc, -ms));
+                const float p1 = exp2f(fmaf(sv[2 * i + 1], sc, -ms));
                 sum0 += p0;
                 sum1 += p1;
                 __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
@@ -361,7 +361,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
                 // the sink joins the sum where the row is finished: l counts in units of 2^m
                 float inv = a.out_scale / (a.head_sinks ? l + exp2f(a.head_sinks[head] * 1.4426950408889634f - m) : l);
                 const size_t row = (size_t)(q_start + tok0 + tl);
-                if (a.head_gate && valid) inv *= 1.f / (1.f + __expf(-__bfloat162float(a.head_gate[row * a.gate_stride + head])));
+                if (a.head_gate && valid) inv *= 1.f / (1.f + expf(-__bfloat162float(a.head_gate[row * a.gate_stride + head])));
                 __nv_bfloat16* dst = a.out + row * a.out_row_stride + (size_t)head * VDIM;
 #pragma unroll
                 for (int h = 0; h < VB; ++h) {

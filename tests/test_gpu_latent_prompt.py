@@ -166,3 +166,31 @@ def test_score_factors_that_are_not_positive(K, monkeypatch, scale):
     with pytest.raises(KernelError, match="positive"):
         K.attn_latent_tc(z(1, 1, 64), z(1, 1, 80), z(64, 128), z(1, 1, 1, 64, 80), z(1, 64), i32([[0]]), i32([0]), i32([1]), i32([0]), 1, 1,
                          64, 64, None, scale)
+
+
+def test_gate_is_float32(K):
+    """One visible key a query, so that the result is its value times the gate's sigmoid, rounded once to bfloat16 after float32 errors
+    of a few units (an exponential good to two, a division, the products)."""
+    H, dim, rot, vdim, rank, n = 64, 64, 16, 64, 64, 256
+    g = torch.Generator(device=DEV).manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(BF)
+    kv, gate = rnd(n, H * (dim + vdim)), -40 * torch.rand(n, H, device=DEV, generator=g).to(BF)
+    out = torch.empty(n, H * vdim, device=DEV, dtype=BF)
+    K.attn_latent_tc(rnd(n, H, dim), rnd(n, H, rank + rot), kv, rnd(4, 1, 1, 64, rank + rot), out, i32([[0, 1, 2, 3]]), i32([0]), i32([n]),
+                     i32([0]), 1, n, vdim, rank, 1, 0.1, gate=gate)
+    K.check_device_errors()
+    want = (kv[:, H * dim:].double().view(n, H, vdim) * torch.sigmoid(gate.double())[:, :, None]).view(n, -1)
+    half_step = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -126))) - 8)
+    assert ((out.double() - want).abs() <= half_step + 8 * 2.0 ** -24 * want.abs()).all()
+
+
+def test_small_probabilities(K):
+    """Two keys, one 2^-130 as likely as the other: bfloat16 holds that number, and its value of 2^125 shows it."""
+    dim, rot, vdim, rank = 64, 16, 64, 64
+    z = lambda *s: torch.zeros(*s, device=DEV, dtype=BF)
+    q_u, kv, out = z(2, 1, dim), z(64, dim + vdim), z(2, vdim)
+    q_u[1, 0, 0], kv[0, 0], kv[0, dim:] = 1.0, -130.0, 2.0 ** 125
+    K.attn_latent_tc(q_u, z(2, 1, rank + rot), kv, z(1, 1, 1, 64, rank + rot), out, i32([[0]]), i32([0]), i32([2]), i32([0]), 1, 2, vdim, rank,
+                     None, math.log(2.0))
+    K.check_device_errors()
+    assert ((out[1].double() - 2.0 ** -5).abs() <= 2.0 ** -5 * 2.0 ** -7).all()
