@@ -104,6 +104,19 @@ __device__ __forceinline__ float glu_act_fast(float g, int act) {
     return __fdividef(g, 1.f + __expf(e));
 }
 
+// silu for results that are rounded to bfloat16, in float32 to a few units of its last place like silu_f32, for kernels that the division's
+// special cases would slow down: z sigmoid(z) with sigmoid(z) = e / (1 + e) or 1 / (1 + e), e = exp(-|z|), so that the divisor lies
+// between 1 and 2 and a Newton step makes its approximate reciprocal whole.  (glu_act_fast loses bits with the size of z, and all of
+// them below -87.  The experts' gate and up of 2,048 tokens of six choices of 1,408: 155 us with that,
+// 176 with silu_f32, 158 so; 3,150 convolved rows of 6,144 channels: 32, 45 and 37 us.)
+__device__ __forceinline__ float silu_to_bf16(float z) {
+    const float e = expf(-fabsf(z)), d = 1.f + e;
+    float r = __fdividef(1.f, d);
+    r = fmaf(fmaf(-d, r, 1.f), r, r);
+    return z * ((z < 0.f ? e : 1.f) * r);
+}
+template <typename T> __device__ __forceinline__ float silu_as(float z) { return sizeof(T) == 2 ? silu_to_bf16(z) : silu_f32(z); }
+
 // V neighbouring numbers as float32, V = 1 or as many as 16 bytes hold (p on 16 bytes then).
 template <typename T, int V>
 __device__ __forceinline__ void load_run(const T* p, float* v) {

@@ -210,7 +210,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                         const float w2 = __shfl_sync(0xffffffffu, wi, 2 * p2 + (is_up ? 1 : 0));
                         const float g = (is_up ? from_gate : v[2 * p2]) * w2;
                         const float u = (is_up ? v[2 * p2 + 1] : from_up) * w2;
-                        dst[2 * p2 * 64] = __float2bfloat16_rn(glu_act_fast(g, BRAID_ACT_SILU) * u);
+                        dst[2 * p2 * 64] = __float2bfloat16_rn(silu_to_bf16(g) * u);
                     }
                 } else {
                     __nv_bfloat16* dst = (__nv_bfloat16*)tile + quarter * 32 + lane;

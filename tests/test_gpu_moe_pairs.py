@@ -103,6 +103,27 @@ def test_products(K, counts, j, k, mode):
         assert (out[used:] == 3.0).all()                              # nothing is written past the plan's tiles
 
 
+def test_activation_is_float32(K):
+    """Inputs that pick single weights, so that gate and up are exact: the result is silu(gate) * up rounded once to bfloat16 after
+    float32 errors of a few units (an exponential good to two, a division, two products), down to where silu is as small as
+    bfloat16's smallest normal numbers."""
+    gates = torch.cat([torch.linspace(-88.0, -60.0, 64), torch.linspace(-60.0, 8.0, 192)]).to(torch.bfloat16).to(DEV)
+    ups = torch.linspace(1.0, 2.0, 129)[:128].to(torch.bfloat16).to(DEV)
+    w0 = torch.zeros(1, gates.numel() * 128, 8, device=DEV, dtype=torch.bfloat16)
+    w1 = torch.zeros_like(w0)
+    w0[0, :, 0], w1[0, :, 1] = gates.repeat_interleave(128), ups.repeat(gates.numel())
+    x = torch.tensor([[1.0, 1.0] + [0.0] * 6], device=DEV, dtype=torch.bfloat16)
+    zero = torch.zeros(1, dtype=torch.int32, device=DEV)
+    plan = K.moe_plan(zero[None], zero, 1, MOE_TC_TILE)
+    xs = K.moe_gather(x, plan, 1)
+    out = torch.empty(xs.shape[0], w0.shape[1], device=DEV, dtype=torch.bfloat16)
+    K.moe_gemm_tc(xs, interleave_experts(w0, w1), out, plan, gated=True)
+    g, u = w0[0, :, 0].double(), w1[0, :, 1].double()
+    want = g * torch.sigmoid(g) * u
+    half_step = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -126))) - 8)
+    assert ((out[0].double() - want).abs() <= half_step + 8 * 2.0 ** -24 * want.abs()).all()
+
+
 def test_views_of_the_interleaved_stack_are_the_stack(K):
     """The kernels of few rows read gate and up as blocks of 16 rows of the stack: the bits of separate tensors."""
     g = torch.Generator(device=DEV).manual_seed(0)
