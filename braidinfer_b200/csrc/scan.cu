@@ -85,7 +85,7 @@ causal_conv_vec_kernel(ConvArgs a) {
         if (r >= 0 && r < a.rows) *reinterpret_cast<uint4*>(xin[u]) = *reinterpret_cast<const uint4*>((const T*)a.x + (size_t)r * a.x_stride + c0);
     }
     // a span inside one sequence, with every tap among the step's own rows: no look at the tables or the state, row by row
-    // (3,150 rows of 6,144 channels: 62 us row by row, 33 so)
+    // (3,150 rows of 6,144 channels: 62 us row by row, 37 so)
     const int last = min(row0 + RPT, a.rows) - 1, seq0 = a.token_seq[row0];
     if (seq0 >= 0 && seq0 == a.token_seq[last] && row0 - a.q_start[seq0] >= TAPS - 1) {
         float wf[VEC * TAPS], bf[VEC];
@@ -102,8 +102,7 @@ causal_conv_vec_kernel(ConvArgs a) {
                 float acc = bf[e];
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j) acc = fmaf(wf[e * TAPS + j], to_f32(xin[rr + j][e]), acc);
-                // (a bfloat16 result: the fast exponential and division are good to a few units of float32's last place)
-                out[e] = from_f32<T>(a.silu ? (sizeof(T) == 2 ? glu_act_fast(acc, BRAID_ACT_SILU) : silu_f32(acc)) : acc);
+                out[e] = from_f32<T>(a.silu ? silu_as<T>(acc) : acc);
             }
             *reinterpret_cast<uint4*>((T*)a.y + (size_t)(row0 + rr) * a.y_stride + c0) = *reinterpret_cast<const uint4*>(out);
         }
@@ -137,7 +136,7 @@ causal_conv_vec_kernel(ConvArgs a) {
         }
         T out[VEC];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) out[e] = from_f32<T>(a.silu ? (sizeof(T) == 2 ? glu_act_fast(acc[e], BRAID_ACT_SILU) : silu_f32(acc[e])) : acc[e]);
+        for (int e = 0; e < VEC; ++e) out[e] = from_f32<T>(a.silu ? silu_as<T>(acc[e]) : acc[e]);
         *reinterpret_cast<uint4*>((T*)a.y + (size_t)row * a.y_stride + c0) = *reinterpret_cast<const uint4*>(out);
     }
 }

@@ -75,3 +75,24 @@ def test_convolution(K, dtype, lens, taps, silu, bias):
         assert ((y[start[i]:start[i] + n].double() - want).abs() <= step * want.abs() + 1.01 * slack + 1e-30).all()
         assert torch.equal(state.view(torch.float32).view(before.shape)[i], full[n:].float())
     assert (y[rows:] == 9.0).all()
+
+
+@pytest.mark.parametrize("lens", [[600], [2, 3, 1, 3]])
+def test_activation_of_the_convolution_is_float32(K, lens):
+    """One tap alone, so that the sum is one product rounded to float32: the result is its silu rounded once to bfloat16 after float32
+    errors of a few units (an exponential good to two, a division, the product), down to silu's smallest normal numbers."""
+    gates = torch.cat([torch.linspace(-88.0, -60.0, 64), torch.linspace(-60.0, 8.0, 192)]).to(torch.bfloat16).to(DEV)
+    rows, ch, taps = sum(lens), gates.numel(), 4
+    x = torch.linspace(1.0, 2.0, rows + 1)[:rows].to(torch.bfloat16).to(DEV)[:, None].repeat(1, ch)
+    w = torch.zeros(ch, taps, device=DEV, dtype=torch.bfloat16)
+    w[:, taps - 1] = gates
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    state = torch.zeros(len(lens), (taps - 1) * ch * 4, dtype=torch.uint8, device=DEV)
+    ctx = types.SimpleNamespace(n_seqs=len(lens), token_seq=i32([i for i, n in enumerate(lens) for _ in range(n)]), q_len=i32(lens),
+                                q_start=i32([sum(lens[:i]) for i in range(len(lens))]), slot_ids=i32(list(range(len(lens)))))
+    y = torch.empty_like(x)
+    K.causal_conv(x, y, w, None, state, 0, ctx, silu=True)
+    z = (x.double() * gates.double()).float().double()
+    want = z * torch.sigmoid(z)
+    half_step = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -126))) - 8)
+    assert ((y.double() - want).abs() <= half_step + 8 * 2.0 ** -24 * want.abs()).all()
