@@ -219,6 +219,7 @@ class Engine:
                                token_source_rows=device_tokens[1] if device_tokens is not None else None,
                                pad_rows_to=token_tile(sum(n_new)) if short_prompt else 0, upload=False)
         ctx.kernels = self.kernels
+        ctx.may_be_captured = shaped
         if shaped and ctx.page_tables:
             ctx.max_kv_len = max(t.shape[1] for t in ctx.page_tables) * PAGE_SIZE
         if short_prompt:

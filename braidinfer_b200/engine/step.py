@@ -40,6 +40,10 @@ class StepContext:
     max_q_len: int
     max_kv_len: int
     all_decode: bool                  # every sequence brings exactly one token
+    # Whether a graph may hold the step's launches and replay them for other lengths of the same shape: a part may then
+    # look at the shape and its bounds only (rows, max_q_len, max_kv_len), never at the host copies below.  Only the engine
+    # knows that a step is none of these.
+    may_be_captured: bool = True
     # host copies, for parts written in Python (tests' toy parts) and for launch shaping
     host_q_len: Tuple[int, ...] = ()
     host_kv_before: Tuple[int, ...] = ()

@@ -199,11 +199,10 @@ class LatentAttention(Mixer):
 
     def _expanded_pages(self, ctx):
         """The pages of every sequence's context if this step should expand keys and values from them
-        (csrc/latent_attn_tc.cu), else None.  Steps that a graph may hold (up to 256 tokens) never do: the context's extent is
-        read on the host.  Expanding costs a product of 2 kv_rank (dim + vdim) a row and head, attention saves
+        (csrc/latent_attn_tc.cu), else None.  Steps that a graph may hold never do: the context's extent is read on the host.  Expanding costs a product of 2 kv_rank (dim + vdim) a row and head, attention saves
         2 (2 kv_rank - dim - vdim) a query, row and head and a kernel that runs at a tenth of this one's rate: EXPAND_QUERIES
         queries a row on average pay for it.  EXPAND_BYTES bounds the expanded rows a step holds."""
-        if self.ukv is None or ctx.n_tokens <= 256 or ctx.max_q_len <= 8 or not ctx.host_q_len:
+        if self.ukv is None or ctx.may_be_captured or ctx.max_q_len <= 8 or not ctx.host_q_len:
             return None
         if self.gated is False and self.out_mult != 1.0:
             return None

@@ -152,3 +152,17 @@ def test_plain_latent_attention_equals_attention_over_the_latent_itself():
         s = (q_lat @ row.T * 0.3).masked_fill(pos[None, :] > pos[:, None], -math.inf)
         out[:, hd] = (torch.softmax(s, -1) @ c) @ w["x.uv"][hd * 7:(hd + 1) * 7].T * torch.sigmoid(h @ w["x.g"].T)[:, hd:hd + 1]
     assert torch.allclose(out.reshape(T, 21) @ w["x.o"].T, want, atol=1e-10)
+
+
+def test_latents_are_expanded_only_where_no_graph_may_hold_the_step():
+    """The expanded context is laid out by lengths that the host reads, which a replay would not see change."""
+    import types
+    from braidinfer_b200.csrc.api import Kernels
+    from braidinfer_b200.parts.latent_attention import LatentAttention
+    part = object.__new__(LatentAttention)
+    part.ukv, part.gated, part.out_mult, part.scale, part.window, part.heads, part.dim, part.vdim = object(), True, 1.0, 0.1, None, 2, 64, 64
+    part.rt = types.SimpleNamespace(kernels=Kernels)
+    step = types.SimpleNamespace(n_tokens=300, max_q_len=300, host_q_len=(300,), host_kv_before=(70,), may_be_captured=True)
+    assert part._expanded_pages(step) is None
+    step.may_be_captured = False
+    assert part._expanded_pages(step) == [6]

@@ -194,3 +194,25 @@ def test_small_probabilities(K):
                      None, math.log(2.0))
     K.check_device_errors()
     assert ((out[1].double() - 2.0 ** -5).abs() <= 2.0 ** -5 * 2.0 ** -7).all()
+
+
+def test_steps_that_graphs_hold_keep_the_latent_form(monkeypatch):
+    """Whatever the engine's limit is: replays of a 300-token step behind other contexts give the bits of steps without graphs."""
+    import braidinfer_b200.engine.engine as E
+    mixer = {"heads": 4, "dim": 64, "rot_dim": 32, "rot": {"base": 10000.0, "dims": 32}, "vdim": 64, "kv_rank": 256, "scale": 96 ** -0.5}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 4, "top": 2, "groups": {"count": 1, "keep": 1}}}
+    cfg = {"architecture": "Bidinex", "vocab": 256, "width": 128, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+           "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    monkeypatch.setattr(E, "GRAPH_PROMPT_ROWS", 512)
+    toks = torch.randint(0, 256, (2000,), generator=torch.Generator().manual_seed(2)).tolist()
+    res = []
+    for graphs in (True, False):
+        eng = E.Engine.from_random(cfg, 3, max_tokens=2048, max_slots=1, use_graphs=graphs, verbose=False)
+        s, out, at = eng.open(), [], 0
+        for n in (300, 290, 300, 280, 300):
+            out.append(eng.step([(s, toks[at:at + n])]))
+            at += n
+        eng.check()
+        assert (eng.graph_replays > 0) == graphs
+        res.append(torch.cat(out))
+    assert torch.equal(*res)
