@@ -208,10 +208,13 @@ def test_steps_that_graphs_hold_keep_the_latent_form(monkeypatch):
     res = []
     for graphs in (True, False):
         eng = E.Engine.from_random(cfg, 3, max_tokens=2048, max_slots=1, use_graphs=graphs, verbose=False)
-        s, out, at = eng.open(), [], 0
-        for n in (300, 290, 300, 280, 300):
-            out.append(eng.step([(s, toks[at:at + n])]))
-            at += n
+        out = []
+        for n in (0, 100, 37, 140):
+            s = eng.open()
+            if n:
+                eng.step([(s, toks[:n])])
+            out.append(eng.step([(s, toks[n:n + 300])]))
+            eng.close(s)
         eng.check()
         assert (eng.graph_replays > 0) == graphs
         res.append(torch.cat(out))
