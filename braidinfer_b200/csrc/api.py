@@ -715,9 +715,9 @@ class Kernels:
                 lib.braid_gemm_heads_mma.restype = c_int
                 lib.braid_attn_latent_simple.argtypes = [c_void_p, c_void_p, c_int] + [c_void_p] * 4 + \
                                                         [c_longlong, c_longlong] + [c_int] * 8 + [c_float, c_void_p, c_void_p, c_void_p]
-                lib.braid_latent_expand_rows.argtypes = [c_void_p] * 5 + [c_int] * 8 + [c_void_p, c_void_p]
+                lib.braid_latent_expand_rows.argtypes = [c_void_p] * 5 + [c_int] * 9 + [c_void_p, c_void_p]
                 lib.braid_latent_attn_tc.argtypes = [c_void_p, c_longlong, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_int] + \
-                                                    [c_void_p] * 5 + [c_int] * 11 + [c_float, c_float, c_void_p, c_void_p, c_longlong,
+                                                    [c_void_p] * 5 + [c_int] * 12 + [c_float, c_float, c_void_p, c_void_p, c_longlong,
                                                                                       c_void_p, c_void_p]
                 lib.braid_latent_attn_tc_supported.argtypes = [c_int] * 4
                 names = ("braid_latent_prep", "braid_gemm_heads", "braid_attn_latent_simple", "braid_latent_expand_rows",
@@ -894,16 +894,17 @@ class Kernels:
         return (dim, vdim) in ((128, 128), (64, 64)) and 0 < rot <= 64 and rot % 16 == 0 and rank % 8 == 0
 
     @staticmethod
-    def latent_pages(q_len: Sequence[int], kv_before: Sequence[int], window: Optional[int]) -> List[int]:
-        """Pages of every sequence's context that a step's queries see: what `latent_expand_rows` lays out."""
+    def latent_pages(q_len: Sequence[int], kv_before: Sequence[int], window: Optional[int], min_q: int = 1) -> List[int]:
+        """Pages of every sequence's context that a step's queries see, for sequences that bring at least `min_q` tokens: what
+        `latent_expand_rows` lays out."""
         page = build.page_size()
-        return [-(-(b + n) // page) - (max(0, b - window + 1) // page if window else 0) if n > 0 else 0
+        return [-(-(b + n) // page) - (max(0, b - window + 1) // page if window else 0) if n >= max(1, min_q) else 0
                 for n, b in zip(q_len, kv_before)]
 
     def latent_expand_rows(self, cache: torch.Tensor, page_table: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, rank: int,
-                           window: Optional[int], pages: Sequence[int]) -> torch.Tensor:
+                           window: Optional[int], pages: Sequence[int], min_q: int = 1) -> torch.Tensor:
         """The latents of the step's context in neighbouring rows [sum(pages) * page_size, rank], sequence after sequence; rows past
-        a sequence's end are zero.  `pages` is `latent_pages` of what the device tables hold."""
+        a sequence's end are zero.  `pages` is `latent_pages` of what the device tables hold, and of `min_q`."""
         lib = self.part_library("latent")
         self._check_pages(cache)
         n_seqs, total = len(pages), sum(pages)
@@ -914,18 +915,19 @@ class Kernels:
         self.launches += 1
         self._check_lib(lib, lib.braid_latent_expand_rows(
             cache.data_ptr(), rows.data_ptr(), page_table.data_ptr(), q_len.data_ptr(), kv_before.data_ptr(), n_seqs, d, rank,
-            page_table.shape[1], cache.shape[0], int(window or 0), total, max(pages), self._error_flag.data_ptr() + 16, self._stream()),
+            page_table.shape[1], cache.shape[0], int(window or 0), int(min_q), total, max(pages), self._error_flag.data_ptr() + 16, self._stream()),
             "latent_expand_rows")
         return rows
 
     def attn_latent_tc(self, q_u: torch.Tensor, q_lat: torch.Tensor, kv: torch.Tensor, cache: torch.Tensor, out: torch.Tensor,
                        page_table: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, n_seqs: int,
                        max_q_len: int, vdim: int, rank: int, window: Optional[int], scale: float, out_scale: float = 1.0,
-                       sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> None:
+                       sinks: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, min_q: int = 1) -> None:
         """Attention of prompts over a latent cache on tcgen05, on keys and values expanded from the rows of `latent_expand_rows`:
         q_u [rows, heads, dim] (a view), q_lat [rows, heads, rank + rot] whose last rot columns are the rotated query parts, kv
         [rows of the context, heads * dim | heads * vdim], out [rows, heads * vdim].  `sinks`, `gate` ([rows, heads], a view is
-        fine) and `out_scale` as `head_sinks`, `head_gate` and `out_scale` of `attn_simple`.  Rows of padding are not written."""
+        fine) and `out_scale` as `head_sinks`, `head_gate` and `out_scale` of `attn_simple`.  Rows of padding, and of sequences that bring fewer than
+        `min_q` tokens, are not written."""
         lib = self.part_library("latent")
         rows, heads, dim = q_u.shape
         d = cache.shape[4]
@@ -941,7 +943,7 @@ class Kernels:
         self._check_lib(lib, lib.braid_latent_attn_tc(
             q_u.data_ptr(), q_u.stride(1), q_u.stride(0), q_lat.data_ptr(), kv.data_ptr(), kv.shape[0], cache.data_ptr(), cache.shape[0],
             out.data_ptr(), page_table.data_ptr(), q_start.data_ptr(), q_len.data_ptr(), kv_before.data_ptr(), rows, n_seqs, max_q_len,
-            heads, dim, d - rank, vdim, rank, page_table.shape[1], int(window or 0), out.stride(0), float(scale), float(out_scale),
+            heads, dim, d - rank, vdim, rank, page_table.shape[1], int(window or 0), int(min_q), out.stride(0), float(scale), float(out_scale),
             _ptr(sinks), _ptr(gate), gate.stride(0) if gate is not None else 0, self._error_flag.data_ptr() + 12, self._stream()),
             "attn_latent_tc")
 
@@ -1115,7 +1117,7 @@ class Kernels:
             lib = ctypes.CDLL(str(build.latent_attention_library(rank, rot, verbose=self._verbose)))
             lib.braid_last_error.restype = c_char_p
             lib.braid_latent_attn_mma.restype = c_int
-            lib.braid_latent_attn_mma.argtypes = [c_void_p] * 9 + [c_int] * 8 + [c_float, c_void_p, c_void_p, c_void_p]
+            lib.braid_latent_attn_mma.argtypes = [c_void_p] * 9 + [c_int] * 9 + [c_float, c_void_p, c_void_p, c_void_p]
             lib.braid_latent_attn_partial_floats.restype = c_longlong
             lib.braid_latent_attn_partial_floats.argtypes = [c_int, c_int, c_int]
             lib.vparts = lib.braid_latent_attn_vparts()
@@ -1137,8 +1139,9 @@ class Kernels:
     def attn_latent_mma(self, q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, page_table: torch.Tensor,
                         q_start: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, token_seq: torch.Tensor,
                         n_seqs: int, max_q_len: int, rank: int, window: Optional[int], scale: float,
-                        n_splits: int = 1, sinks: Optional[torch.Tensor] = None) -> None:
-        """`attn_latent_simple` in bfloat16 on the tensor cores.  Rows of padding are not written.  `n_splits` > 1
+                        n_splits: int = 1, sinks: Optional[torch.Tensor] = None, row0: int = 0) -> None:
+        """`attn_latent_simple` in bfloat16 on the tensor cores.  Rows of padding are not written.  `row0`: q_lat, out and
+        token_seq begin at that row of the step, the tables are of the sequences whose rows those are.  `n_splits` > 1
         slices the context (steps of few tokens) and merges the slices in a second kernel."""
         rows, heads, d = q_lat.shape
         lib = self.latent_attention_library(rank, d - rank)
@@ -1160,7 +1163,7 @@ class Kernels:
         self.launches += 1
         self._check_lib(lib, lib.braid_latent_attn_mma(
             q_lat.data_ptr(), out.data_ptr(), _ptr(partial), cache.data_ptr(), page_table.data_ptr(), q_start.data_ptr(),
-            q_len.data_ptr(), kv_before.data_ptr(), token_seq.data_ptr(), rows, n_seqs, max_q_len, heads,
+            q_len.data_ptr(), kv_before.data_ptr(), token_seq.data_ptr(), rows, int(row0), n_seqs, max_q_len, heads,
             page_table.shape[1], cache.shape[0], int(window or 0), n_splits, float(scale), _ptr(sinks),
             self._error_flag.data_ptr() + 16, self._stream()), "attn_latent_mma")
 

@@ -39,6 +39,7 @@ struct LatAttnArgs {
     const int* q_len;
     const int* kv_before;
     int heads, table_cols, num_pages, window, n_splits, total_pairs;
+    int row0;                      // row of the step that q, out and partial begin at
     float scale_log2;              // scale * log2(e)
     int* error_flag;
     const float* sinks;            // [heads] float32: a score a head that joins the denominator and has no value; or null
@@ -67,7 +68,7 @@ latent_attn_mma_kernel(LatAttnArgs a) {
     if (pair0 >= pairs) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int before = a.kv_before[seq];
-    const long long base_pair = (long long)a.q_start[seq] * a.heads + pair0;     // index of the tile's first pair in the step
+    const long long base_pair = (long long)(a.q_start[seq] - a.row0) * a.heads + pair0;     // index of the tile's first pair in the step
     const int n_here = min(BM, pairs - pair0);
 
     // keys this tile can see, and this CTA's slice of them (in tiles of BN keys)
@@ -267,7 +268,7 @@ latent_attn_few_kernel(LatAttnArgs a) {
     if (pair0 >= pairs) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int before = a.kv_before[seq];
-    const long long base_pair = (long long)a.q_start[seq] * a.heads + pair0;
+    const long long base_pair = (long long)(a.q_start[seq] - a.row0) * a.heads + pair0;
     const int n_here = min(FEW_ROWS, pairs - pair0);
     const int t_first = pair0 / a.heads, t_last = (pair0 + n_here - 1) / a.heads;
     const int hi = before + t_last;
@@ -501,11 +502,11 @@ extern "C" long long braid_latent_attn_partial_floats(int rows, int heads, int n
     return (long long)n_splits * rows * heads * (R + 4);
 }
 
-// rows: rows of the step (padding included); q [rows, heads, D], out [rows, heads, R]; rows that belong to no
-// sequence are not written.  max_q_len: an upper bound of q_len over the sequences (sizes the grid).
+// rows: rows of q [rows, heads, D] and out [rows, heads, R], those of the step (padding included) from row `row0` on (the
+// tables are of the sequences whose rows they are); rows that belong to no sequence are not written.  max_q_len: an upper bound of q_len over the sequences (sizes the grid).
 extern "C" int braid_latent_attn_mma(const void* q, void* out, float* partial, const void* cache, const int* page_table,
                                      const int* q_start, const int* q_len, const int* kv_before, const int* token_seq,
-                                     int rows, int n_seqs,
+                                     int rows, int row0, int n_seqs,
                                      int max_q_len, int heads, int table_cols, int num_pages, int window, int n_splits,
                                      float scale, const float* sinks, int* error_flag, void* stream) {
     if (rows <= 0 || n_seqs <= 0 || max_q_len <= 0) return BRAID_OK;
@@ -526,7 +527,7 @@ extern "C" int braid_latent_attn_mma(const void* q, void* out, float* partial, c
         attr_set = true;
     }
     LatAttnArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, n_splits > 1 ? partial : nullptr, (const __nv_bfloat16*)cache,
-                  page_table, q_start, q_len, kv_before, heads, table_cols, num_pages, window, n_splits, rows * heads,
+                  page_table, q_start, q_len, kv_before, heads, table_cols, num_pages, window, n_splits, rows * heads, row0,
                   scale * 1.4426950408889634f, error_flag, sinks};
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = few

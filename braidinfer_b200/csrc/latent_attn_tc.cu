@@ -38,12 +38,13 @@ static_assert(BRAID_PAGE_SIZE == LA_BN, "a key tile of this kernel is one page o
 #define LA_TMEM_COLS 256                         // S0 [0,64) S1 [64,128), O [128, 128 + VDIM)
 
 // Where a sequence's context lies among the step's expanded rows: its pages from the first that any of its queries sees,
-// sequence after sequence.  Called by whole warps.
+// sequence after sequence.  Sequences that bring fewer than min_q tokens have none: their queries stay with the latent form.
+// Called by whole warps.
 struct LaSpan { int page0, pages, base; };       // first page of the sequence, how many, and the expanded page of the first
-__device__ __forceinline__ LaSpan la_span(const int* q_len, const int* kv_before, int seq, int window) {
+__device__ __forceinline__ LaSpan la_span(const int* q_len, const int* kv_before, int seq, int window, int min_q) {
     const int lane = threadIdx.x & 31;
     auto first = [&](int s) { const int lo = window > 0 ? kv_before[s] - window + 1 : 0; return lo > 0 ? lo / LA_BN : 0; };
-    auto count = [&](int s) { return q_len[s] > 0 ? (kv_before[s] + q_len[s] + LA_BN - 1) / LA_BN - first(s) : 0; };
+    auto count = [&](int s) { return q_len[s] >= min_q ? (kv_before[s] + q_len[s] + LA_BN - 1) / LA_BN - first(s) : 0; };
     int n = 0;
     for (int s = lane; s < seq; s += 32) n += count(s);
 #pragma unroll
@@ -57,7 +58,7 @@ struct LaRowsArgs {
     uint4* rows;                 // [expanded pages * 64][rank]
     const int *page_table, *q_len, *kv_before;
     int d16, rank16;             // D and rank in runs of 16 bytes
-    int table_cols, num_pages, window, max_pages;
+    int table_cols, num_pages, window, min_q, max_pages;
     int* error_flag;
 };
 
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(256)
 latent_expand_rows_kernel(LaRowsArgs a) {
     pdl_trigger();
     const int seq = blockIdx.y, p = blockIdx.x;
-    const LaSpan at = la_span(a.q_len, a.kv_before, seq, a.window);
+    const LaSpan at = la_span(a.q_len, a.kv_before, seq, a.window, a.min_q);
     if (p >= at.pages || at.base + p >= a.max_pages) return;
     const int block = at.page0 + p;
     int page = block < a.table_cols ? a.page_table[(size_t)seq * a.table_cols + block] : -1;
@@ -86,13 +87,13 @@ latent_expand_rows_kernel(LaRowsArgs a) {
 
 // `max_pages`: expanded pages that `rows` holds; `max_seq_pages`: the most of one sequence.
 extern "C" int braid_latent_expand_rows(const void* cache, void* rows, const int* page_table, const int* q_len, const int* kv_before,
-                                        int n_seqs, int d, int rank, int table_cols, int num_pages, int window, int max_pages,
+                                        int n_seqs, int d, int rank, int table_cols, int num_pages, int window, int min_q, int max_pages,
                                         int max_seq_pages, int* error_flag, void* stream) {
     if (n_seqs <= 0 || max_pages <= 0 || max_seq_pages <= 0) return BRAID_OK;
     if (rank <= 0 || rank % 8 || d % 8 || d < rank || (((uintptr_t)cache | (uintptr_t)rows) & 15)) BRAID_REFUSE("latent_expand_rows: rows of %d numbers, %d of them latent, must be whole runs of 16 bytes", d, rank);
     if (num_pages <= 0 || table_cols <= 0 || n_seqs > 65535) BRAID_REFUSE("latent_expand_rows: %d pages, %d table columns, %d sequences", num_pages, table_cols, n_seqs);
     if (!error_flag) BRAID_REFUSE("latent_expand_rows: error_flag is required");
-    LaRowsArgs a{(const uint4*)cache, (uint4*)rows, page_table, q_len, kv_before, d / 8, rank / 8, table_cols, num_pages, window, max_pages, error_flag};
+    LaRowsArgs a{(const uint4*)cache, (uint4*)rows, page_table, q_len, kv_before, d / 8, rank / 8, table_cols, num_pages, window, min_q > 1 ? min_q : 1, max_pages, error_flag};
     braid_launch(latent_expand_rows_kernel, dim3(max_seq_pages, n_seqs), dim3(256), 0, (cudaStream_t)stream, a);
     BRAID_LAUNCH_CHECK();
 }
@@ -101,7 +102,7 @@ extern "C" int braid_latent_expand_rows(const void* cache, void* rows, const int
 struct LatentTcArgs {
     __nv_bfloat16* out;          // [rows, out_row_stride]: head h at column h * VDIM
     const int *page_table, *q_start, *q_len, *kv_before;
-    int out_row_stride, heads, table_cols, num_pages, window, rot, rank;
+    int out_row_stride, heads, table_cols, num_pages, window, min_q, rot, rank;
     float scale_log2, out_scale;
     const float* head_sinks;     // [heads] natural-log scores, or null
     const __nv_bfloat16* head_gate;
@@ -169,10 +170,10 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map_qu, const __grid_c
     const uint32_t tmem_o = tmem_base + 128;
     pdl_wait();
 
-    const LaSpan span = la_span(a.q_len, a.kv_before, seq, a.window);
+    const LaSpan span = la_span(a.q_len, a.kv_before, seq, a.window, a.min_q);
     const int q_len = a.q_len[seq];
     const int tok0 = tile * LA_BM;
-    const bool active = tok0 < q_len;             // uniform over the CTA
+    const bool active = tok0 < q_len && q_len >= a.min_q;      // uniform over the CTA
     const int q_start = a.q_start[seq], kv_before = a.kv_before[seq];
     const int n_tok = active ? min(LA_BM, q_len - tok0) : 0;
     const int pos_min = kv_before + tok0, pos_max = pos_min + n_tok - 1;
@@ -427,7 +428,7 @@ extern "C" int braid_latent_attn_tc_supported(int dim, int rot, int vdim, int ra
 extern "C" int braid_latent_attn_tc(const void* q_u, long long qu_head, long long qu_row, const void* q_lat, const void* kv, long long kv_rows,
                                     const void* cache, int num_pages, void* out, const int* page_table, const int* q_start,
                                     const int* q_len, const int* kv_before, int rows, int n_seqs, int max_q_len, int heads, int dim,
-                                    int rot, int vdim, int rank, int table_cols, int window, int out_row_stride, float scale,
+                                    int rot, int vdim, int rank, int table_cols, int window, int min_q, int out_row_stride, float scale,
                                     float out_scale, const float* head_sinks, const void* head_gate, long long gate_stride,
                                     int* error_flag, void* stream) {
     if (rows <= 0 || n_seqs <= 0 || max_q_len <= 0) return BRAID_OK;
@@ -460,7 +461,7 @@ extern "C" int braid_latent_attn_tc(const void* q_u, long long qu_head, long lon
     }
     const long long tiles = (max_q_len + LA_BM - 1) / LA_BM;
     if (tiles > 65535 || n_seqs > 65535) BRAID_REFUSE("latent_attn_tc: the step exceeds the grid limits (%lld token tiles, %d sequences)", tiles, n_seqs);
-    LatentTcArgs a{(__nv_bfloat16*)out, page_table, q_start, q_len, kv_before, out_row_stride, heads, table_cols, num_pages, window, rot, rank,
+    LatentTcArgs a{(__nv_bfloat16*)out, page_table, q_start, q_len, kv_before, out_row_stride, heads, table_cols, num_pages, window, min_q > 1 ? min_q : 1, rot, rank,
                    scale * 1.4426950408889634f, out_scale, head_sinks, (const __nv_bfloat16*)head_gate, gate_stride, error_flag};
     const dim3 grid(heads, n_seqs, (unsigned)tiles);
     cudaStream_t s = (cudaStream_t)stream;

@@ -41,6 +41,8 @@ from .spec import CacheRequest, PartSpec, TensorSpec
 
 EXPAND_QUERIES = 16
 EXPAND_BYTES = 1 << 30
+EXPAND_BESIDE_FLOPS = 6 * 10 ** 10       # what expanding the contexts of sequences of fewer queries may cost (see _expanded_pages)
+STEP_SEQUENCES = slice(None)             # all sequences of a step
 
 
 @MIXERS.register("latent_attention")
@@ -181,70 +183,105 @@ class LatentAttention(Mixer):
                       self.heads, self.dim, self.rot, self.rank, self.pe.rope_dim, cache.page_size, self.eps,
                       adjacent=self.adjacent)
         q_u = queries[:, :self.q_cols].view(rows, self.heads, self.dim + self.rot)[:, :, :self.dim]
-        pages = self._expanded_pages(ctx)
-        if pages is not None:
-            gate = proj[:, self.gate_col:self.gate_col + self.heads] if self.gated else None
-            out = self._attend_expanded(q_u, q_lat, gate, pages, ctx, cache)
-            return self.o.forward(out, residual=residual, defer_to=ctx)
-        tc = self.rt.gemm_backend == "auto"
-        K.gemm_heads(q_u, self.uk_t, q_lat[:, :, :self.rank], tensor_cores=tc)
-        o_lat = self.rt.empty(rows, self.heads, self.rank)
-        self._attend(q_lat, o_lat, ctx, cache)
-        out = self.rt.empty(rows, self.heads * self.vdim)
         gate = proj[:, self.gate_col:self.gate_col + self.heads] if self.gated else None
         if gate is None and self.out_mult != 1.0:
             raise RuntimeError("latent_attention: an output factor needs the gate's epilogue")
-        K.gemm_heads(o_lat, self.uv, out.view(rows, self.heads, self.vdim), gate=gate, mult=self.out_mult, tensor_cores=tc)
+        out = self.rt.empty(rows, self.heads * self.vdim)
+        pages, min_q = self._expanded_pages(ctx)
+        if pages is None:
+            self._attend_latents(q_u, q_lat, gate, out, ctx, cache)
+        else:
+            if ctx.rows > ctx.n_tokens:
+                out.zero_()                                   # rows of padding are not written by the kernels
+            for seqs in self._runs(pages):
+                self._attend_latents(q_u, q_lat, gate, out, ctx, cache, seqs)
+            self._attend_expanded(q_u, q_lat, gate, pages, min_q, out, ctx, cache)
         return self.o.forward(out, residual=residual, defer_to=ctx)
 
-    def _expanded_pages(self, ctx):
-        """The pages of every sequence's context if this step should expand keys and values from them
-        (csrc/latent_attn_tc.cu), else None.  Steps that a graph may hold never do: the context's extent is read on the host.  Expanding costs a product of 2 kv_rank (dim + vdim) a row and head, attention saves
-        2 (2 kv_rank - dim - vdim) a query, row and head and a kernel that runs at a tenth of this one's rate: EXPAND_QUERIES
-        queries a row on average pay for it.  EXPAND_BYTES bounds the expanded rows a step holds."""
-        if self.ukv is None or ctx.may_be_captured or ctx.max_q_len <= 8 or not ctx.host_q_len:
-            return None
-        if self.gated is False and self.out_mult != 1.0:
-            return None
-        if not self.scale > 0:                                # that kernel masks before the factor
-            return None
-        pages = self.rt.kernels.latent_pages(ctx.host_q_len, ctx.host_kv_before, self.window)
-        total = sum(pages)
-        if sum(n * p for n, p in zip(ctx.host_q_len, pages)) < EXPAND_QUERIES * total:
-            return None
-        if total * 64 * self.heads * (self.dim + self.vdim) * 2 > EXPAND_BYTES:
-            return None
-        return pages
+    @staticmethod
+    def _runs(pages):
+        """The neighbouring sequences without expanded pages, a slice a run."""
+        none = [i for i, p in enumerate(pages) if p == 0]
+        starts = [i for i in none if i == 0 or pages[i - 1]]
+        ends = [i + 1 for i in none if i + 1 == len(pages) or pages[i + 1]]
+        return [slice(a, b) for a, b in zip(starts, ends)]
 
-    def _attend_expanded(self, q_u, q_lat, gate, pages, ctx, cache):
+    def _expanded_pages(self, ctx):
+        """(the pages of every sequence's context that this step expands keys and values from (csrc/latent_attn_tc.cu), 0 for
+        sequences that keep the latent form, and the fewest tokens of a sequence that has pages), or (None, 0) if all keep it.
+        Steps that a graph may hold keep it: the context's extent is read on the host.
+
+        Expanding costs a product of 2 kv_rank (dim + vdim) a row and head, attention saves 2 (2 kv_rank - dim - vdim) a query, row
+        and head and a kernel that runs at a tenth of this one's rate: a sequence's rows pay for it where EXPAND_QUERIES of its
+        queries meet them.  Sequences that bring fewer (ones that decode beside a prompt) keep the latent form, in launches of
+        their own, unless all their rows cost no more than EXPAND_BESIDE_FLOPS, which is less than those launches do.  A step of
+        four layers, ms, all expanded / each by itself: 16 heads of 128, rank 512, a prompt of 2,048 tokens beside 12 contexts of
+        8,192 4.43 / 2.60, of 1,024 2.22 / 2.34, one of 512 beside 4 of 4,096 1.75 / 1.69; 8 heads of 64, rank 256, one of 300
+        beside 16 of 2,048 1.20 / 1.72.  EXPAND_BYTES bounds the expanded rows a step holds."""
+        if self.ukv is None or ctx.may_be_captured or ctx.max_q_len <= 8 or not ctx.host_q_len:
+            return None, 0
+        if self.gated is False and self.out_mult != 1.0:
+            return None, 0
+        if not self.scale > 0:                                # that kernel masks before the factor
+            return None, 0
+        if max(ctx.host_q_len) < EXPAND_QUERIES or (self.window and self.window < EXPAND_QUERIES):
+            return None, 0
+        numbers = 64 * self.heads * (self.dim + self.vdim)    # of a page, expanded
+        pages = {n: self.rt.kernels.latent_pages(ctx.host_q_len, ctx.host_kv_before, self.window, n) for n in (1, EXPAND_QUERIES)}
+        beside = sum(pages[1]) - sum(pages[EXPAND_QUERIES])
+        min_q = EXPAND_QUERIES
+        if beside * numbers * 2 * self.rank <= EXPAND_BESIDE_FLOPS and sum(pages[1]) * numbers * 2 <= EXPAND_BYTES:
+            min_q = 1
+        if sum(pages[min_q]) * numbers * 2 > EXPAND_BYTES:
+            return None, 0
+        return pages[min_q], min_q
+
+    def _attend_expanded(self, q_u, q_lat, gate, pages, min_q, out, ctx, cache) -> None:
         K = self.rt.kernels
-        rows = K.latent_expand_rows(cache.storage, cache.page_table, ctx.q_len, ctx.kv_before, self.rank, self.window, pages)
+        rows = K.latent_expand_rows(cache.storage, cache.page_table, ctx.q_len, ctx.kv_before, self.rank, self.window, pages,
+                                    min_q)
         kv = self.rt.empty(rows.shape[0], self.heads * (self.dim + self.vdim))
         K.gemm_tc(rows, self.ukv, kv)
-        out = self.rt.empty(q_u.shape[0], self.heads * self.vdim)
-        if ctx.rows > ctx.n_tokens:
-            out.zero_()                                       # rows of padding are not written by the kernel
         K.attn_latent_tc(q_u, q_lat, kv, cache.storage, out, cache.page_table, ctx.q_start, ctx.q_len, ctx.kv_before, ctx.n_seqs,
-                         ctx.max_q_len, self.vdim, self.rank, self.window, self.scale, out_scale=self.out_mult, sinks=self.sinks, gate=gate)
-        return out
+                         ctx.max_q_len, self.vdim, self.rank, self.window, self.scale, out_scale=self.out_mult, sinks=self.sinks, gate=gate,
+                         min_q=min_q)
 
-    def _attend(self, q_lat, o_lat, ctx, cache) -> None:
+    def _attend_latents(self, q_u, q_lat, gate, out, ctx, cache, seqs=STEP_SEQUENCES) -> None:
+        """Queries into the latent space, attention over the cached rows, values out of it, for the sequences `seqs` of the
+        step (with all of them: its rows of padding too)."""
+        K, tc = self.rt.kernels, self.rt.gemm_backend == "auto"
+        row0, rows = 0, ctx.rows
+        if seqs is not STEP_SEQUENCES:
+            row0, rows = sum(ctx.host_q_len[:seqs.start]), sum(ctx.host_q_len[seqs])
+        at = slice(row0, row0 + rows)
+        K.gemm_heads(q_u[at], self.uk_t, q_lat[at, :, :self.rank], tensor_cores=tc)
+        o_lat = self.rt.empty(rows, self.heads, self.rank)
+        self._attend(q_lat[at], o_lat, ctx, cache, seqs, row0)
+        K.gemm_heads(o_lat, self.uv, out[at].view(rows, self.heads, self.vdim), gate=gate[at] if gate is not None else None,
+                     mult=self.out_mult, tensor_cores=tc)
+
+    def _attend(self, q_lat, o_lat, ctx, cache, seqs, row0) -> None:
         """bfloat16 runs use the tensor-core kernel where it is built for the latent's size (prompts and decoding
         alike; steps of few tokens slice the context so that a handful of sequences still fills the machine);
         float32 runs, runs that ask for the plain kernels, and other sizes use one warp per (token, head)."""
         K = self.rt.kernels
+        rows = slice(row0, row0 + q_lat.shape[0])
         if self.rt.is_f32 or self.rt.attention_backend == "plain" or not K.attn_latent_mma_supports(self.rank, self.rot):
-            K.attn_latent_simple(q_lat, o_lat, cache.storage, cache.page_table, ctx.positions, ctx.token_seq,
+            K.attn_latent_simple(q_lat, o_lat, cache.storage, cache.page_table, ctx.positions[rows], ctx.token_seq[rows],
                                  self.rank, self.window, self.scale, sinks=self.sinks)
             return
-        if ctx.rows > ctx.n_tokens:
+        n_seqs, max_q_len, max_kv_len = ctx.n_seqs, ctx.max_q_len, ctx.max_kv_len
+        if seqs is not STEP_SEQUENCES:
+            n_seqs, max_q_len = seqs.stop - seqs.start, max(ctx.host_q_len[seqs])
+            max_kv_len = max(n + b for n, b in zip(ctx.host_q_len[seqs], ctx.host_kv_before[seqs]))
+        elif ctx.rows > ctx.n_tokens:
             o_lat.zero_()                                     # rows of padding are not written by the kernel
         n_splits = 1
-        if ctx.max_q_len <= 8:
-            ctas = K.attn_latent_ctas(self.rank, self.rot, ctx.n_seqs, ctx.max_q_len, self.heads)
-            span = min(ctx.max_kv_len, self.window) if self.window else ctx.max_kv_len
+        if max_q_len <= 8:
+            ctas = K.attn_latent_ctas(self.rank, self.rot, n_seqs, max_q_len, self.heads)
+            span = min(max_kv_len, self.window) if self.window else max_kv_len
             tiles = max(1, -(-span // 32))
             n_splits = max(1, min(296 // ctas, tiles // 4, 32))      # two CTAs an SM, at least four key tiles a slice
-        K.attn_latent_mma(q_lat, o_lat, cache.storage, cache.page_table, ctx.q_start, ctx.q_len, ctx.kv_before,
-                          ctx.token_seq, ctx.n_seqs, ctx.max_q_len, self.rank, self.window, self.scale, n_splits=n_splits,
-                          sinks=self.sinks)
+        K.attn_latent_mma(q_lat, o_lat, cache.storage, cache.page_table[seqs], ctx.q_start[seqs], ctx.q_len[seqs], ctx.kv_before[seqs],
+                          ctx.token_seq[rows], n_seqs, max_q_len, self.rank, self.window, self.scale, n_splits=n_splits,
+                          sinks=self.sinks, row0=row0)

@@ -160,9 +160,32 @@ def test_latents_are_expanded_only_where_no_graph_may_hold_the_step():
     from braidinfer_b200.csrc.api import Kernels
     from braidinfer_b200.parts.latent_attention import LatentAttention
     part = object.__new__(LatentAttention)
-    part.ukv, part.gated, part.out_mult, part.scale, part.window, part.heads, part.dim, part.vdim = object(), True, 1.0, 0.1, None, 2, 64, 64
+    part.ukv, part.gated, part.out_mult, part.scale, part.window, part.heads, part.dim, part.vdim, part.rank = \
+        object(), True, 1.0, 0.1, None, 2, 64, 64, 64
     part.rt = types.SimpleNamespace(kernels=Kernels)
     step = types.SimpleNamespace(n_tokens=300, max_q_len=300, host_q_len=(300,), host_kv_before=(70,), may_be_captured=True)
-    assert part._expanded_pages(step) is None
+    assert part._expanded_pages(step)[0] is None
     step.may_be_captured = False
-    assert part._expanded_pages(step) == [6]
+    assert part._expanded_pages(step)[0] == [6]
+
+
+def test_each_sequence_is_looked_at_by_itself(monkeypatch):
+    """One long prompt does not expand the long contexts of sequences that decode beside it: 2,048 tokens beside 12 contexts of 8,192."""
+    import types
+    from braidinfer_b200.csrc.api import Kernels
+    import braidinfer_b200.parts.latent_attention as LA
+    part = object.__new__(LA.LatentAttention)
+    part.ukv, part.gated, part.out_mult, part.scale, part.window, part.heads, part.dim, part.vdim, part.rank = \
+        object(), True, 1.0, 0.1, None, 16, 128, 128, 512
+    part.rt = types.SimpleNamespace(kernels=Kernels)
+    n, before = [1] * 6 + [2048] + [1] * 6, [8191] * 6 + [0] + [8191] * 6
+    step = types.SimpleNamespace(n_tokens=sum(n), max_q_len=2048, host_q_len=tuple(n), host_kv_before=tuple(before), may_be_captured=False)
+    pages, least = part._expanded_pages(step)
+    assert pages == [0] * 6 + [32] + [0] * 6 and least == LA.EXPAND_QUERIES
+    assert part._runs(pages) == [slice(0, 6), slice(7, 13)] and part._runs([1, 2]) == [] and part._runs([0, 0, 3, 0]) == [slice(0, 2), slice(3, 4)]
+    step.host_kv_before = tuple(b // 64 for b in before)                # short contexts go along: fewer launches
+    assert part._expanded_pages(step) == ([2] * 6 + [32] + [2] * 6, 1)
+    part.window = 8                                                      # no row meets enough queries
+    assert part._expanded_pages(step)[0] is None
+    part.window, step.host_q_len, step.max_q_len = None, (12,) * 13, 12
+    assert part._expanded_pages(step)[0] is None

@@ -219,3 +219,71 @@ def test_steps_that_graphs_hold_keep_the_latent_form(monkeypatch):
         assert (eng.graph_replays > 0) == graphs
         res.append(torch.cat(out))
     assert torch.equal(*res)
+
+
+def test_sequences_below_the_least_number_of_queries_are_left_out(K):
+    """Their pages are not laid out and their rows not written; the others' rows are those of a step without them."""
+    H, dim, rot, vdim, rank = 2, 64, 16, 64, 64
+    g = torch.Generator(device=DEV).manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).to(BF)
+    seqs = [(0, 3), (64, 70), (5, 1), (0, 129), (300, 4)]
+    cache, table = rnd(16, 1, 1, 64, rank + rot), [[3, 4, 5, 6, 7], [0, 1, 2, -1, -1], [8] + [-1] * 4, [9, 10, 11, -1, -1], [12, 13, 14, 15, 3]]
+    uk_uv = (rnd(H * (dim + vdim), rank).float() * rank ** -0.5).to(BF)
+    n = sum(q for _, q in seqs)
+    q_u, q_lat = rnd(n, H, dim), rnd(n, H, rank + rot)
+    start = [sum(q for _, q in seqs[:i]) for i in range(len(seqs))]
+
+    def run(pick, min_q):
+        q_len, before = [seqs[i][1] for i in pick], [seqs[i][0] for i in pick]
+        tables = i32([table[i] for i in pick]), i32(q_len), i32(before)
+        pages = K.latent_pages(q_len, before, None, min_q)
+        rows = K.latent_expand_rows(cache, *tables, rank, None, pages, min_q)
+        kv, out = torch.empty(rows.shape[0], H * (dim + vdim), device=DEV, dtype=BF), torch.full((n, H * vdim), 9.0, device=DEV, dtype=BF)
+        K.gemm_tc(rows, uk_uv, kv)
+        K.attn_latent_tc(q_u, q_lat, kv, cache, out, tables[0], i32([start[i] for i in pick]), *tables[1:], len(pick), max(q_len), vdim, rank,
+                         None, 0.1, min_q=min_q)
+        K.check_device_errors()
+        return pages, out
+
+    pages, got = run(range(5), 4)
+    assert pages == [0, 3, 0, 3, 5]
+    _, want = run([1, 3, 4], 1)
+    assert torch.equal(got, want) and (got[:3] == 9.0).all() and (got[73] == 9.0).all() and (got[74:] != 9.0).any()
+
+
+def test_a_prompt_beside_sequences_that_decode(monkeypatch):
+    """Every sequence is looked at by itself: long contexts that one query meets are not expanded because of the prompt beside them."""
+    from braidinfer_b200.engine import Engine
+    import braidinfer_b200.parts.latent_attention as LA
+    mixer = {"heads": 4, "dim": 64, "rot_dim": 32, "rot": {"base": 10000.0, "dims": 32}, "vdim": 64, "kv_rank": 256, "scale": 96 ** -0.5}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 4, "top": 2, "groups": {"count": 1, "keep": 1}}}
+    cfg = {"architecture": "Bidinex", "vocab": 256, "width": 128, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+           "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    eng = Engine.from_random(cfg, 3, max_tokens=64 * 64, max_slots=6, verbose=False)
+    toks = torch.randint(0, 256, (1000,), generator=torch.Generator().manual_seed(2)).tolist()
+    before, n = [600, 0, 700, 130, 0, 515], [1, 300, 1, 20, 10, 1]
+    seen = []
+    expand = type(eng.kernels).latent_expand_rows
+    monkeypatch.setattr(LA, "EXPAND_BESIDE_FLOPS", 0)                 # however little they cost here
+    monkeypatch.setattr(type(eng.kernels), "latent_expand_rows", lambda self, *a, **kw: (seen.append(list(a[6])), expand(self, *a, **kw))[1])
+
+    def logits():
+        slots = [eng.open() for _ in n]
+        for s, b in zip(slots, before):
+            if b:
+                eng.step([(s, toks[:b])])
+        seen.clear()
+        out = eng.step([(s, toks[b:b + q]) for s, b, q in zip(slots, before, n)], want="all").double()
+        for s in slots:
+            eng.close(s)
+        eng.check()
+        return out
+
+    got = logits()
+    assert seen == [[0, 5, 0, 3, 0, 0]]
+    monkeypatch.setattr(LA, "EXPAND_BYTES", 0)
+    want = logits()
+    assert not seen
+    at = [sum(n[:i]) for i in range(len(n) + 1)]
+    for a, b in zip(at, at[1:]):                                      # as test_the_part_that_chooses asks
+        assert float((got[a:b] - want[a:b]).norm() / want[a:b].norm()) < 1e-2
