@@ -46,6 +46,9 @@ class DecoderModel:
         self._keep_h0 = any(e.inject for e in spec.schedule)
         self.final_norm = NORMS.get(spec.final_norm.kind)(spec.final_norm.params, "", runtime)
         self.head = HEADS.get(spec.head.kind)(spec.head.params, "", runtime)
+        # whether what follows each schedule entry adds up a sum that is left on the stream (StepContext.sum_rides)
+        follows = [not e.inject and self.blocks[e.layer].takes_sum for e in spec.schedule[1:]]
+        self._takes_sum = follows + [self.final_norm.accepts_deferred]
 
     # ------------------------------------------------------------------ weights
     def all_parts(self):
@@ -107,6 +110,7 @@ class DecoderModel:
             view = cache.layer_view(e)
             if view is not None:
                 view.page_table = ctx.page_tables[view.group]
+            ctx.reader_takes_sum, ctx.sum_rides = self._takes_sum[e], False
             h = self.blocks[entry.layer].forward(h, ctx, view, cache.state_view(e))
             if tap is not None:
                 tap(e + 1, ctx.resolve(h) if self.streams is None else self.streams.total(h, ctx))

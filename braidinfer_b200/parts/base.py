@@ -178,6 +178,11 @@ class Block:
     h may arrive with a deferred sum pending (`ctx.deferred`): hand it only to a part with
     `accepts_deferred`, else call `ctx.resolve(h)` first."""
 
+    @property
+    def takes_sum(self) -> bool:
+        """Whether a kernel of the block's own adds up a sum that h arrives with."""
+        return False
+
     def __init__(self, mixer: Mixer, mixer_norm: Norm, feed_forward: Optional[FeedForward],
                  feed_forward_norm: Optional[Norm], layer_input: Optional[LayerInput] = None) -> None:
         self.mixer = mixer

@@ -43,15 +43,25 @@ def stream_k_pays(rows: int, w_rows: int, k_in: int, sms: Optional[int] = None) 
     return fill < (0.8 if rows <= 48 else 0.7)
 
 
-def few_rows_pay(rows: int, w_rows: int, k_in: int) -> bool:
+def few_rows_pay(rows: int, w_rows: int, k_in: int, rides: bool = False) -> bool:
     """Whether the product of `rows` tokens with a [w_rows, k_in] bfloat16 weight should run as one kernel whose CTAs finish 16
-    weight rows each (csrc/gemm_few.cu) instead of as stream-k partial sums and their reduce kernel: where a second launch weighs
-    more than what is lost on an uneven spread of the CTAs, weights of up to 24 MB at up to 8 tokens and 7 MB at 9 to 16.  Whole turns
-    of 24 steps, ms, with the line at 0 / 7 / 24 / 51 MB: 8 sequences of a Loduzen model of width 1024 8.3 / 7.4 / 6.75 / 6.8, 2 of
-    width 2048 10.7 / 10.2 / 10.0 / 9.1, 4 of a Zisesun model of width 2048 7.65 / 7.3 / 7.2 / 7.55, 4 of the dense decoder of
-    width 4096 11.16 / 11.11 / 11.25 / 11.95; 12 of a Loduzen model of width 2048 12.8 / 12.6 / 13.1 / 12.8."""
+    weight rows each (csrc/gemm_few.cu) instead of as stream-k partial sums.
+
+    Where the sums have a reduce kernel of their own, a second launch weighs more than an uneven spread of the CTAs up to 24 MB of
+    weights at up to 8 tokens and 7 MB at 9 to 16.  Whole turns of 24 steps, ms, with the line at 0 / 7 / 24 / 51 MB: 8 sequences of
+    a Loduzen model of width 1024 8.3 / 7.4 / 6.75 / 6.8, 2 of width 2048 10.7 / 10.2 / 10.0 / 9.1, 4 of a Zisesun model of width 2048
+    7.65 / 7.3 / 7.2 / 7.55, 4 of the dense decoder of width 4096 11.16 / 11.11 / 11.25 / 11.95; 12 of a Loduzen model of width 2048
+    12.8 / 12.6 / 13.1 / 12.8.
+
+    Where they ride in a kernel that runs anyway (`rides`: the next norm, the rotary encoding), no launch is saved, and the line lies
+    at 7 MB and 4.5: a step of four layers, us, with it at 0 / 7 / 9 / 13 / 24 MB, of the dense decoder of width 1024 (products of 1.6,
+    1.0 and 5.8 MB) 165 / 130 at 4 sequences, of width 2048 (12.6, 8.4 and 23.1 MB) 224 / 223 / 227 / 232 / 233 at 4 and 228 / 228 / 232 /
+    238 / 241 at 8; with it at 0 / 2.2 / 4.3 / 7 MB at 16 sequences of width 1024 168 / 166 / 167 / 172, at 12 of a Loduzen model of
+    width 1024 290 / 280 / 275 / 273.  (Products of 8.4 MB whose sums do not ride: 8 sequences of a Bidinex model of width 2048 507 ->
+    495 us, 5 of a Megerax model 234 -> 228.)"""
     from ..csrc.api import FEW_MAX_ROWS
-    return rows <= FEW_MAX_ROWS and w_rows * k_in * 2 <= (24 if rows <= 8 else 7) * 10 ** 6
+    most = (7 if rows <= 8 else 4.5) if rides else (24 if rows <= 8 else 7)
+    return rows <= FEW_MAX_ROWS and w_rows * k_in * 2 <= most * 10 ** 6
 
 
 # Rows up to which a norm may leave its scale to the next product: beyond the token tiles of the
@@ -106,14 +116,15 @@ class Linear:
 
     def forward(self, x: torch.Tensor, *, out_dtype: Optional[torch.dtype] = None,
                 residual: Optional[torch.Tensor] = None, swiglu: bool = False, defer_to=None,
-                in_scale=None, activation: str = "silu") -> torch.Tensor:
+                in_scale=None, activation: str = "silu", rides: Optional[bool] = None) -> torch.Tensor:
         """x [rows, in].  Plain: returns [rows, out] in `out_dtype` (default x's type).
         `residual` (float32 [rows, out]): returns residual + product, written in place.
         `swiglu`: the weight holds gate rows then up rows; returns act(gate) * up, act the
         `activation` ("silu", or "gelu_tanh" for the tanh form of gelu).
         `defer_to` (a StepContext): when the product runs in its stream-k form, leave the
         adding-up of its partial sums to whoever reads the result next
-        (`StepContext.deferred`); the returned tensor is complete only after that.
+        (`StepContext.deferred`); the returned tensor is complete only after that.  `rides`: whether that is a kernel
+        that runs anyway (default: what the block says, `StepContext.sum_rides`).
         `in_scale` (csrc.api.RowScale): x's rows still want this scale; the product applies it to
         its results (only where `takes_row_scale()`, and not with a residual)."""
         K = self.rt.kernels
@@ -138,7 +149,10 @@ class Linear:
             K.cast(y, y2)
             return y2
         use_tc = (self.rt.gemm_backend == "auto" and x.dtype == torch.bfloat16 and K.gemm_tc_eligible(x, w))
-        if use_tc and few_rows_pay(rows, w_rows, x.shape[1]):
+        sk = use_tc and stream_k_pays(rows, w_rows, x.shape[1])
+        can_defer = (defer_to is not None and sk and not swiglu
+                     and self.rt.fuse_reduce and K.pending_partial is None)
+        if use_tc and few_rows_pay(rows, w_rows, x.shape[1], can_defer and (defer_to.sum_rides if rides is None else rides)):
             if residual is not None:
                 K.gemm_few(x, w, residual, residual=residual)
                 return residual
@@ -147,9 +161,6 @@ class Linear:
             out = torch.empty((rows, self.out_features[0] if swiglu else w_rows), dtype=out_dtype or x.dtype, device=x.device)
             K.gemm_few(x, w, out, swiglu=swiglu, in_scale=in_scale, activation=activation)
             return out
-        sk = use_tc and stream_k_pays(rows, w_rows, x.shape[1])
-        can_defer = (defer_to is not None and sk and not swiglu
-                     and self.rt.fuse_reduce and K.pending_partial is None)
         if residual is not None:
             if can_defer:
                 defer_to.defer(residual, K.gemm_tc_partial(x, w), "residual")

@@ -58,8 +58,9 @@ class ParallelMixers(Mixer):
         return self._state_bytes
 
     def forward(self, x, residual, ctx, cache, state):
-        h = residual
+        h, rides = residual, ctx.sum_rides
         for c, off in zip(self.children, self.offsets):
+            ctx.sum_rides = rides and c is self.children[-1]
             # a sum that the mixer before left deferred lives in the products' workspace: completed first
             h = ctx.resolve(h)
             own = None

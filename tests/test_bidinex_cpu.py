@@ -189,3 +189,18 @@ def test_each_sequence_is_looked_at_by_itself(monkeypatch):
     assert part._expanded_pages(step)[0] is None
     part.window, step.host_q_len, step.max_q_len = None, (12,) * 13, 12
     assert part._expanded_pages(step)[0] is None
+
+
+def test_the_model_knows_which_sums_the_next_kernel_adds_up():
+    """Dynamic tanh needs finished rows, an RMS norm adds a deferred sum up itself, an injection between two layers does not."""
+    from braidinfer_b200.config import preset
+    from braidinfer_b200.models.decoder import DecoderModel
+    from braidinfer_b200.parts.linear import few_rows_pay
+    from braidinfer_b200.parts.runtime import Runtime
+    rt = Runtime(act_dtype=torch.bfloat16, device=torch.device("cpu"), kernels=None)
+    assert not any(DecoderModel(spec_of(BX_A), rt)._takes_sum)
+    dense = DecoderModel(spec_of(preset("tiny_b")), rt)
+    assert all(dense._takes_sum) and len(dense._takes_sum) == len(dense.spec.schedule)
+    assert few_rows_pay(8, 2048, 2048) and not few_rows_pay(8, 2048, 2048, rides=True)
+    assert few_rows_pay(8, 1024, 2816, rides=True) and not few_rows_pay(16, 1024, 2816, rides=True) and few_rows_pay(16, 1024, 2816)
+    assert not few_rows_pay(17, 8, 8) and few_rows_pay(16, 1024, 2048, rides=True)

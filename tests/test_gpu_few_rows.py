@@ -75,3 +75,39 @@ def test_refusals(K):
         K.gemm_few(x[:2], w.float(), out[:2])
     with pytest.raises(KernelError):
         K.gemm_few(x[:2], w[:, :8], out[:2])
+
+
+def products(monkeypatch, cfg, seqs):
+    """(weights whose products of one decode step go through `gemm_few`, through deferred partial sums), [rows, k] each."""
+    from braidinfer_b200.csrc.api import Kernels
+    from braidinfer_b200.engine import Engine
+    eng = Engine.from_random(cfg, 1, max_tokens=64 * seqs, max_slots=seqs, use_graphs=False, verbose=False)
+    slots = [eng.open() for _ in range(seqs)]
+    eng.step([(s, [1, 2, 3]) for s in slots])
+    few, deferred = [], []
+    run_few, run_partial = Kernels.gemm_few, Kernels.gemm_tc_partial
+    monkeypatch.setattr(Kernels, "gemm_few", lambda self, x, w, *a, **kw: (few.append(tuple(w.shape)), run_few(self, x, w, *a, **kw))[1])
+    monkeypatch.setattr(Kernels, "gemm_tc_partial", lambda self, x, w, *a, **kw: (deferred.append(tuple(w.shape)), run_partial(self, x, w, *a, **kw))[1])
+    logits = eng.step([(s, [4]) for s in slots])
+    eng.check()
+    monkeypatch.undo()
+    assert torch.isfinite(logits).all()
+    return few, deferred
+
+
+@pytest.mark.parametrize("seqs", [1, 8])
+def test_sums_that_ride_in_the_next_kernel_stay_deferred(monkeypatch, seqs):
+    """Products of 8.4 and 12.6 MB: with a norm and a rotary encoding that add the sums up they gain nothing from the other kernel;
+    where what follows needs finished rows (dynamic tanh), they do."""
+    dense = {"architectures": ["MistralForCausalLM"], "model_type": "mistral", "torch_dtype": "bfloat16", "num_hidden_layers": 1, "hidden_size": 2048,
+             "num_attention_heads": 16, "num_key_value_heads": 4, "head_dim": 128, "intermediate_size": 1024, "vocab_size": 512, "rope_theta": 1e6,
+             "rms_norm_eps": 1e-5, "sliding_window": None, "tie_word_embeddings": False, "max_position_embeddings": 4096}
+    few, deferred = products(monkeypatch, dense, seqs)
+    assert (2048, 2048) in deferred and (3072, 2048) in deferred
+    assert (2048, 1024) in few and (2048, 1024) not in deferred       # 4.2 MB: the lone kernel pays all the same
+    mixer = {"heads": 16, "dim": 128, "rot_dim": 64, "rot": {"base": 10000.0, "dims": 64}, "vdim": 128, "kv_rank": 512, "scale": 192 ** -0.5}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 4, "top": 2, "groups": {"count": 1, "keep": 1}}}
+    bidinex = {"architecture": "Bidinex", "vocab": 256, "width": 2048, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+               "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    few, deferred = products(monkeypatch, bidinex, seqs)
+    assert (2048, 2048) in few and (2048, 2048) not in deferred
