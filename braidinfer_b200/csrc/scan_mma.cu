@@ -17,8 +17,9 @@
 // Q K^T straight into the operands of P V.  Two CTAs an SM (108 KB of shared memory at dk 128).  The walk token by token in two
 // passes over chunks (scan.cu) is bound by shared-memory reads and shuffles.  Measured beside it, us, heads of 128 x 64:
 // 64 heads, 2,048 tokens 262 beside 478, 1,500 + 1,200 + 900 tokens 232 / 842, 8 x 64 tokens 36 / 97, 4 x 24 tokens 22 / 35; 128 heads,
-// 2,048 tokens 267 / 929.  32 heads of 64 x 64: 3 sequences 156 / 244, 300 tokens 38 / 68, one sequence of 2,048 tokens 204 / 158 (half a
-// CTA for every second SM, each on a chain of 32 chunks): that form stays with the walk in chunks.
+// 2,048 tokens 267 / 929.  32 heads of 64 x 64: 3 sequences 156 / 244, 300 tokens 38 / 68.  A long prompt on few CTAs is a
+// chain that leaves the machine idle (8 us a chunk; 8 heads of 128 x 64, 2,048 tokens: 259 us beside 129): such steps stay with
+// the walk whose chunks run side by side, by `ssd_pays` (api.py), which holds both forms' times.
 #include "common.cuh"
 #include <type_traits>
 

@@ -125,6 +125,19 @@ def test_the_largest_numbers_of_a_state(K, dk, big):
     assert float((got[ok].double() - walk[ok].double()).norm() / walk[ok].double().norm()) < 2.0 ** -18
 
 
+@pytest.mark.parametrize("heads, dk, tokens, serial", [(8, 128, 300, True), (8, 128, 2048, False), (16, 128, 2048, False), (64, 128, 2048, True),
+                                                       (32, 64, 700, True), (32, 64, 2048, False), (4, 64, 384, True), (4, 64, 385, False), (4, 128, 257, False)])
+def test_the_form_follows_ctas_and_length(K, heads, dk, tokens, serial):
+    """A long prompt on few CTAs keeps the walk whose chunks run side by side (three launches), whatever its keys' size."""
+    z = lambda *s: torch.zeros(*s, device=DEV, dtype=BF)
+    before = K.launches
+    K.linear_scan(z(tokens, dk), z(tokens, dk), z(tokens, heads * 64), z(tokens, heads), z(heads), torch.empty(tokens, heads * 64, device=DEV),
+                  torch.zeros(1, heads * dk * 64 * 4, dtype=torch.uint8, device=DEV), 0, step([tokens], [0]), heads, 1, dk, 64, "head", a_log=z(heads))
+    assert (K.launches - before == 1) == serial == K.ssd_pays(tokens, tokens, heads, dk, 64)
+    assert not K.ssd_pays(16, 16, 64, 128, 64)
+    assert not K.ssd_pays(2048 + 192, 2048, 16, 128, 64) and K.ssd_pays(4 * 2048, 2048, 16, 128, 64)    # beside short ones, or equals
+
+
 @pytest.mark.parametrize("rows, groups, group", [(90, 16, 256), (200, 8, 512), (160, 8, 520), (1190, 1, 136), (2, 16, 256)])
 @pytest.mark.parametrize("gate_type", [BF, torch.float32])
 @pytest.mark.parametrize("gate_first", [True, False])
