@@ -3,7 +3,7 @@ without rows, with one, with a chunk of 32 slots more or less one, with more tha
 import pytest
 import torch
 
-from braidinfer_b200.csrc.api import MOE_TC_TILE, expert_halves, get_kernels, interleave_experts
+from braidinfer_b200.csrc.api import MOE_TC_TILE, expert_halves, get_kernels, interleave_experts, interleave_gate_up
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -122,6 +122,20 @@ def test_activation_is_float32(K):
     want = g * torch.sigmoid(g) * u
     half_step = torch.exp2(torch.floor(torch.log2(want.abs().clamp_min(2.0 ** -126))) - 8)
     assert ((out[0].double() - want).abs() <= half_step + 8 * 2.0 ** -24 * want.abs()).all()
+
+
+@pytest.mark.parametrize("experts, j, k", [(1, 8, 8), (5, 24, 40), (7, 33, 9), (3, 16, 72), (40, 1040, 1024)])
+def test_laying_out_the_experts(experts, j, k):
+    """Every expert's rows as `interleave_gate_up` lays them, with no second copy of the weights on the way."""
+    g = torch.Generator(device=DEV).manual_seed(j)
+    gate, up = [[torch.randn(j, k, device=DEV, generator=g).to(torch.bfloat16) for _ in range(experts)] for _ in range(2)]
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    w = interleave_experts(gate, up)
+    assert torch.cuda.max_memory_allocated() - before <= w.numel() * 2 + (60 << 20)
+    for e in range(experts):
+        assert torch.equal(w[e], interleave_gate_up(gate[e], up[e]))
 
 
 def test_views_of_the_interleaved_stack_are_the_stack(K):
