@@ -1079,12 +1079,15 @@ class Kernels:
             meta.data_ptr(), self._moe_mode(w1, relu2), x.stride(0), out.stride(0), j, k, top, tile, max_tiles,
             self._in_wgt(in_wgt, x, top, w1), we, wb, self._stream()), "moe_gemm_mma")
 
-    def moe_gather(self, x: torch.Tensor, plan, top: int) -> torch.Tensor:
-        """The rows of a plan's slots (tiles of `MOE_TC_TILE`), [slots, k]: x's row of each slot's token, zeros for padding slots."""
+    def moe_gather(self, x: torch.Tensor, plan, top: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """The rows of a plan's slots (tiles of `MOE_TC_TILE`), [slots, k]: x's row of each slot's token, zeros for padding slots;
+        into `out` if it is given (contiguous, of x's type)."""
         lib = self.part_library("moe")
         slot_pair, _pair_slot, _tile_expert, meta, max_tiles = plan[:5]
-        xs = torch.empty((max_tiles * MOE_TC_TILE, x.shape[1]), dtype=x.dtype, device=x.device)
-        if x.dtype != torch.bfloat16 or x.stride(1) != 1 or slot_pair.numel() != xs.shape[0]:
+        shape = (max_tiles * MOE_TC_TILE, x.shape[1])
+        xs = torch.empty(shape, dtype=x.dtype, device=x.device) if out is None else out
+        if x.dtype != torch.bfloat16 or x.stride(1) != 1 or slot_pair.numel() != shape[0] or tuple(xs.shape) != shape \
+                or xs.dtype != x.dtype or not xs.is_contiguous():
             raise KernelError("moe_gather: bfloat16 rows and a plan of tiles of 32 slots")
         self.launches += 1
         self._check_lib(lib, lib.braid_moe_gather(x.data_ptr(), xs.data_ptr(), slot_pair.data_ptr(), meta.data_ptr(), x.stride(0),

@@ -173,7 +173,8 @@ class MixtureOfExperts(FeedForward):
         """bfloat16 rows that start on 16 bytes run on the tensor cores, everything else on the plain kernels."""
         K = self.rt.kernels
         if len(plan) > 5:                                              # a plan of tiles of 32 slots
-            xs = K.moe_gather(x, plan, self.top)
+            # the slots' inputs lie where their results will: the first product has read them when the second one writes there
+            xs = K.moe_gather(x, plan, self.top, out=y)
             K.moe_gemm_tc(xs, self.w_first, act, plan, gated=self.gated, relu2=not self.gated, in_wgt=in_wgt)
             K.moe_gemm_tc(act, self.w_down, y, plan)
             return

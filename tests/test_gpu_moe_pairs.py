@@ -175,3 +175,28 @@ def test_weighted_sum(K, rows, width, top, pad, dtype, weighted):
     most = (top + 1) * U * (h.double().abs() + terms.abs().sum(1))
     K.moe_combine(h, y, (None, at), wgt if weighted else None, top=top)
     assert ((h.double() - want).abs() <= most).all()
+
+
+def test_inputs_of_the_slots_take_no_memory_of_their_own(monkeypatch):
+    """A step's peak grows by the slots' results and inner rows, not by their gathered inputs too; twice the same bits."""
+    from braidinfer_b200.csrc.api import Kernels
+    from braidinfer_b200.engine import Engine
+    mixer = {"heads": 4, "dim": 64, "rot_dim": 32, "rot": {"base": 10000.0, "dims": 32}, "vdim": 64, "kv_rank": 256, "scale": 96 ** -0.5}
+    mlp = {"kind": "moe", "expert": {"ff": 64}, "router": {"experts": 8, "top": 4, "groups": {"count": 1, "keep": 1}}}
+    cfg = {"architecture": "Bidinex", "vocab": 256, "width": 256, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5}, "residual_mult": 1.0,
+           "logit_softcap": 30.0, "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": mlp}], "loop": None}
+    eng = Engine.from_random(cfg, 3, max_tokens=640, max_slots=1, verbose=False)
+    wrote = []
+    gather, product = Kernels.moe_gather, Kernels.moe_gemm_tc
+    monkeypatch.setattr(Kernels, "moe_gather", lambda self, *a, **kw: (wrote.append(gather(self, *a, **kw)), wrote[-1])[1])
+    monkeypatch.setattr(Kernels, "moe_gemm_tc", lambda self, xs, w, out, *a, **kw: (wrote.append(out), product(self, xs, w, out, *a, **kw))[1])
+    res = []
+    for _ in range(2):
+        s = eng.open()
+        wrote.clear()
+        res.append(eng.step([(s, [(7 * i) % 256 for i in range(600)])]))
+        inputs, inner, results = wrote
+        assert inputs.data_ptr() == results.data_ptr() != inner.data_ptr()
+        eng.close(s)
+    eng.check()
+    assert torch.equal(*res)
