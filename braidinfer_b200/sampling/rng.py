@@ -5,6 +5,7 @@ crates/braidinfer-runtime/src/sampling.rs:188-191; its generator is not reproduc
 from __future__ import annotations
 
 import os
+from operator import index
 from typing import Sequence
 
 import numpy as np
@@ -40,10 +41,11 @@ def _splitmix64_all(x: np.ndarray) -> np.ndarray:
 def uniforms(seeds: Sequence[int], sequences: Sequence[int], steps: Sequence[int]) -> np.ndarray:
     """`uniform` of every (seed, sequence, step), as float32, which holds each exactly."""
     def words(values, plus):
-        try:
-            return np.array(values, dtype=np.int64).view(np.uint64) + np.uint64(plus)
-        except OverflowError:                                  # numbers of more than 64 bits, or unsigned ones
-            return np.array([(v + plus) & _MASK for v in values], dtype=np.uint64)
+        a = np.asarray(values)
+        if a.dtype == np.int64:
+            return a.view(np.uint64) + np.uint64(plus)
+        # numbers of more than 64 bits, or unsigned ones; what is no whole number is refused, as `uniform` does
+        return np.array([(index(v) + plus) & _MASK for v in values], dtype=np.uint64)
 
     with np.errstate(over="ignore"):
         x = _splitmix64_all(words(seeds, 0))

@@ -71,10 +71,13 @@ class Sampler:
         tokens (int32, on the device)."""
         rows, vocab = logits.shape
         out = torch.empty(rows, dtype=torch.int32, device=self.device)
-        one = params[0] if rows and all(p is params[0] for p in params) else None       # one set of options for all rows
+        one = params[0] if rows and params and all(p is params[0] for p in params) else None       # one set of options for all rows
         if one.is_plain_greedy if one is not None else all(p.is_plain_greedy for p in params):
             self.K.argmax(logits, out)
             return out
+        if len(params) != rows or min(len(seeds), len(sequence_ids), len(steps)) < rows:
+            raise ValueError(f"{rows} rows of logits want as many options, seeds, sequences and steps, got {len(params)}, {len(seeds)}, "
+                             f"{len(sequence_ids)} and {len(steps)}")
         distinct = params if one is None else (one,)
         penalty = [p.repetition_penalty for p in distinct] * (rows if one is not None else 1)
         penalised = any(p.repetition_penalty != 1.0 for p in distinct)
@@ -85,7 +88,7 @@ class Sampler:
         f[1] = [p.top_p for p in distinct]
         f[2] = [p.min_p for p in distinct]
         f[3] = penalty
-        f[4] = uniforms(seeds, sequence_ids, steps)
+        f[4] = uniforms(seeds[:rows], sequence_ids[:rows], steps[:rows])
         k = np.empty(rows, dtype=np.int32)
         k[:] = [p.top_k for p in distinct]
         # what the penalty and the biases of each row name: offsets, tokens, numbers

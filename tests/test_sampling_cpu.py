@@ -37,3 +37,32 @@ def test_uniforms_of_a_batch_are_the_single_ones():
     ids, steps = [i * 37 % 1009 for i in range(len(seeds))], [i * i for i in range(len(seeds))]
     got = uniforms(seeds, ids, steps)
     assert got.dtype.name == "float32" and [float(x) for x in got] == [uniform(*t) for t in zip(seeds, ids, steps)]
+    with pytest.raises(TypeError):
+        uniforms([1.5], [0], [0])
+
+
+def test_rows_without_options_of_their_own_are_refused():
+    """As many options as rows of logits; more seeds than rows are fine, fewer are not (one seed is not every row's)."""
+    import torch
+    from braidinfer_b200.sampling.sampler import Sampler
+    seen = []
+
+    class Kernels:
+        def sample(self, logits, work, out, temperature, u, **kw):
+            seen.append(u.tolist())
+            out.zero_()
+
+        def argmax(self, logits, out):
+            out.zero_()
+
+        def check_device_errors(self):
+            pass
+
+    sampler, logits, p = Sampler(Kernels(), "cpu"), torch.zeros(3, 8), SamplingParams(top_k=5)
+    assert sampler.choose(logits, [p] * 3, [1, 2, 3, 4], [0, 1, 2, 3], [0] * 4) == [0, 0, 0]
+    assert seen == [[uniform(s, i, 0) for s, i in ((1, 0), (2, 1), (3, 2))]]
+    for params, seeds in (([p], [1, 2, 3]), ([p] * 2, [1, 2, 3]), ([p] * 4, [1, 2, 3, 4]), ([p] * 3, [1]), ([p] * 3, [1, 2])):
+        with pytest.raises(ValueError):
+            sampler.choose(logits, params, seeds, [0] * len(seeds), [0] * len(seeds))
+    for params in ([SamplingParams.greedy()] * 3, []):                  # nothing is drawn
+        assert sampler.choose(logits, params, [], [], []) == [0, 0, 0]
