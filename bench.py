@@ -788,7 +788,7 @@ def bidinex_kernels(z, T, B, C, timed, frac):
     peak its algorithmic FLOPs or bytes (whichever bounds it) reach."""
     import torch
     from braidinfer_b200.cache import PAGE_SIZE
-    from braidinfer_b200.csrc.api import get_kernels
+    from braidinfer_b200.csrc.api import MOE_TC_TILE, get_kernels, interleave_experts
     K = get_kernels(verbose=False)
     dev, bf = "cuda", torch.bfloat16
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
@@ -843,18 +843,19 @@ def bidinex_kernels(z, T, B, C, timed, frac):
         wg, wu = [torch.randn(E, ff, W, device=dev, dtype=bf) * 0.02 for _ in range(2)]
         wd = torch.randn(E, W, ff, device=dev, dtype=bf) * 0.02
         idx = torch.stack([torch.randperm(E, device=dev)[:top] for _ in range(rows)]).to(torch.int32)
-        tile = 16 if rows * top <= 16 * E else 64
+        tile = MOE_TC_TILE
         plan = K.moe_plan(idx, torch.zeros(rows, dtype=torch.int32, device=dev), E, tile)
         act = torch.empty(plan[4] * tile, ff, device=dev, dtype=bf)
         y = torch.empty(plan[4] * tile, W, device=dev, dtype=bf)
-        t1 = timed(lambda: K.moe_gemm_mma(x, wg, wu, act, plan, top, tile), graph=True)
-        t2 = timed(lambda: K.moe_gemm_mma(act, wd, None, y, plan, top, tile), graph=True)
+        w1 = interleave_experts(wg, wu)
+        t1 = timed(lambda: K.moe_gemm_tc(K.moe_gather(x, plan, top, out=y), w1, act, plan, gated=True), graph=True)
+        t2 = timed(lambda: K.moe_gemm_tc(act, wd, y, plan), graph=True)
         used = int(torch.unique(idx).numel())
         fl1, fl2 = 2 * rows * top * 2 * ff * W, 2 * rows * top * ff * W
         by1, by2 = used * 2 * ff * W * 2, used * ff * W * 2
         res[what] = {"gate_up_ms": round(t1 * 1e3, 4), "gate_up_frac": round(frac(t1, fl1, by1), 3),
                      "down_ms": round(t2 * 1e3, 4), "down_frac": round(frac(t2, fl2, by2), 3), "experts_used": used, "tile": tile}
-        del wg, wu, wd
+        del wg, wu, wd, w1
         I = top * ff
         from braidinfer_b200.csrc.api import interleave_gate_up
         from braidinfer_b200.parts.linear import stream_k_pays
@@ -1215,7 +1216,7 @@ def birepel_kernels(z, T, B, C, timed, frac):
     import torch
     from types import SimpleNamespace
     from braidinfer_b200.cache import PAGE_SIZE
-    from braidinfer_b200.csrc.api import get_kernels
+    from braidinfer_b200.csrc.api import MOE_TC_TILE, get_kernels, interleave_experts
     K = get_kernels(verbose=False)
     dev, bf = "cuda", torch.bfloat16
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
@@ -1372,11 +1373,12 @@ def birepel_kernels(z, T, B, C, timed, frac):
         idx = torch.empty(rows, top, dtype=torch.int32, device=dev)
         wgt = torch.empty(rows, top, device=dev)
         K.moe_route(lg, idx, wgt, 1, 1)
-        tile = 16 if rows * top <= 16 * E else 64
+        tile = MOE_TC_TILE
         plan = K.moe_plan(idx, stp.token_seq, E, tile)
         act = torch.empty(plan[4] * tile, J, device=dev, dtype=bf)
-        t1 = timed(lambda: K.moe_gemm_mma(x, wu, None, act, plan, top, tile, relu2=True), reps=5, graph=True)
-        t2 = timed(lambda: K.moe_gemm_mma(x, wg, wu, act, plan, top, tile), reps=5, graph=True)
+        xs, w1 = torch.empty(plan[4] * tile, Wd, device=dev, dtype=bf), interleave_experts(wg, wu)
+        t1 = timed(lambda: K.moe_gemm_tc(K.moe_gather(x, plan, top, out=xs), wu, act, plan, relu2=True), reps=5, graph=True)
+        t2 = timed(lambda: K.moe_gemm_tc(K.moe_gather(x, plan, top, out=xs), w1, act, plan, gated=True), reps=5, graph=True)
         used = min(E, rows * top)
         res[f"{what}_experts_first_product"] = {
             "birepel_ms": round(t1 * 1e3, 4), "birepel_frac": round(frac(t1, 2 * rows * top * J * Wd, used * J * Wd * 2), 3),
@@ -1491,7 +1493,7 @@ def ludazen_kernels(z, T, B, C, timed, frac):
     import torch
     from types import SimpleNamespace
     from braidinfer_b200.cache import PAGE_SIZE
-    from braidinfer_b200.csrc.api import get_kernels
+    from braidinfer_b200.csrc.api import MOE_TC_TILE, get_kernels, interleave_experts
     K = get_kernels(verbose=False)
     dev, bf = "cuda", torch.bfloat16
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)        # noqa: E731
@@ -1572,17 +1574,18 @@ def ludazen_kernels(z, T, B, C, timed, frac):
         wgt = torch.empty(rows, top, dtype=torch.float32, device=dev)
         tr1 = timed(lambda: K.moe_route(logits, idx, wgt, 1, 1, sigmoid=True), graph=True)
         tr2 = timed(lambda: K.moe_route(logits, idx, wgt, 1, 1), graph=True)
-        tile = 16 if rows * top <= 16 * E else 64
+        tile = MOE_TC_TILE
         plan = K.moe_plan(idx, torch.zeros(rows, dtype=torch.int32, device=dev), E, tile)
         act = torch.empty(plan[4] * tile, ff, device=dev, dtype=bf)
-        t1 = timed(lambda: K.moe_gemm_mma(x, wg, wu, act, plan, top, tile, in_wgt=wgt), graph=True)
-        t2 = timed(lambda: K.moe_gemm_mma(x, wg, wu, act, plan, top, tile), graph=True)
+        xs, w1 = torch.empty(plan[4] * tile, Wd, device=dev, dtype=bf), interleave_experts(wg, wu)
+        t1 = timed(lambda: K.moe_gemm_tc(K.moe_gather(x, plan, top, out=xs), w1, act, plan, gated=True, in_wgt=wgt), graph=True)
+        t2 = timed(lambda: K.moe_gemm_tc(K.moe_gather(x, plan, top, out=xs), w1, act, plan, gated=True), graph=True)
         used = int(torch.unique(idx).numel())
         fl1, by1 = 2 * rows * top * 2 * ff * Wd, used * 2 * ff * Wd * 2
         res[what] = {"weighted_input_ms": round(t1 * 1e3, 4), "weighted_input_frac": round(frac(t1, fl1, by1), 3),
                      "weighted_output_ms": round(t2 * 1e3, 4), "weighted_output_frac": round(frac(t2, fl1, by1), 3),
                      "route_sigmoid_ms": round(tr1 * 1e3, 4), "route_softmax_ms": round(tr2 * 1e3, 4), "experts_used": used, "tile": tile}
-        del wg, wu
+        del wg, wu, w1
     # ---- bias + two-piece activation (with the ones column) beside the gated unit's activation kernel
     I = top * ff
     for what, rows in (("prompt_activation", T), ("decode_activation", B)):
@@ -1702,7 +1705,7 @@ def zisesun_kernels(z, T, B, C, timed, frac):
     import torch
     from types import SimpleNamespace
     from braidinfer_b200.cache import PAGE_SIZE
-    from braidinfer_b200.csrc.api import get_kernels
+    from braidinfer_b200.csrc.api import MOE_TC_TILE, get_kernels, interleave_experts
     K = get_kernels(verbose=False)
     dev, bf = "cuda", torch.bfloat16
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)        # noqa: E731
@@ -1811,7 +1814,7 @@ def zisesun_kernels(z, T, B, C, timed, frac):
         t2 = timed(lambda: K.moe_route(lg, idx, wgt, 1, 1), reps=9, graph=True)
         t1 = timed(lambda: K.moe_route(lg, idx, wgt, 1, 1, renorm=False, correction=corr * 0.01), reps=9, graph=True)
         pair(f"{what}_routing", (t1, 0, rows * (E + 2 * top) * 4), (t2, 0, rows * (E + 2 * top) * 4))
-        tile = 16 if rows * top <= 16 * E else 64
+        tile = MOE_TC_TILE
         plan = K.moe_plan(idx, stp.token_seq, E, tile)
         ys = torch.randn(plan[4] * tile, Wd, device=dev, dtype=bf)
         t1 = timed(lambda: K.streams(x, x, n, y=(ys, plan, wgt, top), mix=mix, back=back, read=read, w=w1, eps=1e-6, out=xo), reps=9, graph=True)
@@ -1829,14 +1832,15 @@ def zisesun_kernels(z, T, B, C, timed, frac):
         w2 = torch.randn(E, J2, Wd, device=dev, dtype=bf) * 0.02
         act2 = torch.empty(plan[4] * tile, J2, device=dev, dtype=bf)
         used = int(torch.unique(idx).numel())
-        t1 = timed(lambda: K.moe_gemm_mma(xin, wg, wu, act, plan, top, tile), graph=True)
-        t2 = timed(lambda: K.moe_gemm_mma(xin, w2, None, act2, plan, top, tile, relu2=True), graph=True)
+        wi = interleave_experts(wg, wu)
+        t1 = timed(lambda: K.moe_gemm_tc(K.moe_gather(xin, plan, top, out=ys), wi, act, plan, gated=True), graph=True)
+        t2 = timed(lambda: K.moe_gemm_tc(K.moe_gather(xin, plan, top, out=ys), w2, act2, plan, relu2=True), graph=True)
         pair(f"{what}_experts_first_product", (t1, 4 * rows * top * J * Wd, 2 * used * J * Wd * 2), (t2, 2 * rows * top * J2 * Wd, used * J2 * Wd * 2))
         wd, wd2 = torch.randn(E, Wd, J, device=dev, dtype=bf) * 0.02, torch.randn(E, Wd, J2, device=dev, dtype=bf) * 0.02
-        t1 = timed(lambda: K.moe_gemm_mma(act, wd, None, ys, plan, top, tile), graph=True)
-        t2 = timed(lambda: K.moe_gemm_mma(act2, wd2, None, ys, plan, top, tile), graph=True)
+        t1 = timed(lambda: K.moe_gemm_tc(act, wd, ys, plan), graph=True)
+        t2 = timed(lambda: K.moe_gemm_tc(act2, wd2, ys, plan), graph=True)
         pair(f"{what}_experts_down_product", (t1, 2 * rows * top * J * Wd, used * J * Wd * 2), (t2, 2 * rows * top * J2 * Wd, used * J2 * Wd * 2))
-        del wg, wu, w2, wd, wd2
+        del wg, wu, wi, w2, wd, wd2
     K.check_device_errors()
     return res
 

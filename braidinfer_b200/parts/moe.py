@@ -130,7 +130,7 @@ class MixtureOfExperts(FeedForward):
 
     def tile(self, x) -> int:
         """Slots a tile of the plan: 32 for the products on pairs of SMs, which gather an expert's tiles themselves; for the
-        others 16 while an expert sees few rows, 64 beyond."""
+        plain ones 16 while an expert sees few rows, 64 beyond."""
         from ..csrc.api import MOE_TC_TILE
         if self.on_pairs(x):
             return MOE_TC_TILE
@@ -170,7 +170,7 @@ class MixtureOfExperts(FeedForward):
         return y, plan, None if on_input else wgt, self.top
 
     def _experts(self, x, act, y, plan, tile, in_wgt=None) -> None:
-        """bfloat16 rows that start on 16 bytes run on the tensor cores, everything else on the plain kernels."""
+        """bfloat16 rows that start on 16 bytes run on the tensor cores, everything else on the plain kernel."""
         K = self.rt.kernels
         if len(plan) > 5:                                              # a plan of tiles of 32 slots
             # the slots' inputs lie where their results will: the first product has read them when the second one writes there
@@ -178,12 +178,6 @@ class MixtureOfExperts(FeedForward):
             K.moe_gemm_tc(xs, self.w_first, act, plan, gated=self.gated, relu2=not self.gated, in_wgt=in_wgt)
             K.moe_gemm_tc(act, self.w_down, y, plan)
             return
-        tc = self.rt.gemm_backend == "auto"
         w0, w1 = (self.w_gate, self.w_up) if self.gated else (self.w_up, None)
-        relu2 = not self.gated
-        if tc and K.moe_gemm_mma_eligible(x, w0, tile) and K.moe_gemm_mma_eligible(act, self.w_down, tile):
-            K.moe_gemm_mma(x, w0, w1, act, plan, self.top, tile, relu2=relu2, in_wgt=in_wgt)
-            K.moe_gemm_mma(act, self.w_down, None, y, plan, self.top, tile)
-            return
-        K.moe_gemm_simt(x, w0, w1, act, plan, self.top, tile, relu2=relu2, in_wgt=in_wgt)
+        K.moe_gemm_simt(x, w0, w1, act, plan, self.top, tile, relu2=not self.gated, in_wgt=in_wgt)
         K.moe_gemm_simt(act, self.w_down, None, y, plan, self.top, tile)

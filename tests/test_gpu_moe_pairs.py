@@ -59,6 +59,41 @@ def test_plan(K, counts, tile):
         assert at == meta[0] * tile
 
 
+# pairs for a cluster of eight CTAs, with one turn of its loops and (past 32,768) with two; as many experts as there may be
+@pytest.mark.parametrize("counts", [[1400, 1400, 1399], [192] * 64, [5000, 0, 9000, 1, 11000, 8200], [e % 7 for e in range(1024)], [0] * 1023 + [40]])
+@pytest.mark.parametrize("tile", [16, 32])
+def test_plan_of_long_prompts(K, counts, tile):
+    top, experts = 3, len(counts)
+    idx = choice(counts, top, 4)
+    rows = idx.shape[0]
+    seq = torch.zeros(rows, dtype=torch.int32, device=DEV)
+    seq[rows // 2] = -1                                              # a row of padding takes no slot
+    plan = K.moe_plan(idx, seq, experts, tile)
+    slot_pair, pair_slot, tile_expert, meta, max_tiles = plan[:5]
+    live = idx.clone().long()
+    live[rows // 2] = -1
+    live = live.view(-1)
+    real = torch.bincount(live[live >= 0], minlength=experts)
+    tiles = -(-real // tile)
+    assert int(meta[0]) == int(tiles.sum()) <= max_tiles
+    assert torch.equal(tile_expert[:int(meta[0])].long(), torch.repeat_interleave(torch.arange(experts, device=DEV), tiles))
+    assert torch.equal(pair_slot >= 0, live >= 0)
+    pair = torch.nonzero(live >= 0).view(-1)
+    slot = pair_slot[pair].long()
+    assert torch.equal(slot_pair[slot].long(), pair) and torch.equal(tile_expert[slot // tile].long(), live[pair])
+    assert int((slot_pair >= 0).sum()) == pair.numel()
+    if tile == MOE_TC_TILE:
+        runs = -(-tiles // 8)
+        wide = plan[5].view(-1, 4)[:int(meta[1])].long()
+        assert wide.shape[0] == int(runs.sum())
+        owner = torch.repeat_interleave(torch.arange(experts, device=DEV), runs)
+        first = torch.cumsum(runs, 0) - runs
+        assert torch.equal(wide[:, 2], first[owner]) and torch.equal(wide[:, 3], runs[owner])
+        assert torch.equal(wide[:, 0], (torch.cumsum(wide[:, 1], 0) - wide[:, 1]) * tile) and int(wide[:, 1].sum()) == int(meta[0])
+        assert int(wide[:, 1].min()) >= 1 and int(wide[:, 1].max()) <= 8
+        assert torch.equal(tile_expert[wide[:, 0] // tile].long(), owner)
+
+
 @pytest.mark.parametrize("counts", COUNTS)
 @pytest.mark.parametrize("j, k", [(8, 8), (24, 40), (64, 64), (136, 72), (264, 200), (520, 520)])
 @pytest.mark.parametrize("mode", ["plain", "gated", "gated, weight on the input", "relu2"])
