@@ -56,10 +56,11 @@ class StepContext:
     # know about this calls `resolve(tensor)` first, or is handed a resolved tensor by the
     # block.  At most one sum is deferred at a time.
     deferred: dict = field(default_factory=dict)
-    # Whether the sum that the running sublayer would leave deferred is added up by a kernel that runs anyway (a norm that
-    # accepts it, the kernel of several streams) or by one of its own: set by the block, which knows the reader, for
-    # products that have another form (parts/linear.py).  `reader_takes_sum` is the model's word to the block on what follows it.
-    sum_rides: bool = False
+    # Whether the sum that the running sublayer would leave deferred is added up by a kernel that runs anyway, a norm that
+    # accepts it ("norm": of the same layer, "next": of the layer after it), or by one of its own (""): set by the block,
+    # which knows the reader, for products that have another form (parts/linear.py).  `reader_takes_sum` is the model's word
+    # to the block on what follows it.
+    sum_rides: str = ""
     reader_takes_sum: bool = False
     # Row scales.  In a step of few tokens a norm may leave its own scale (rsqrt(mean square + eps), one
     # number a row) to the product that reads its output, if the block says that this reader takes row

@@ -110,7 +110,7 @@ class DecoderModel:
             view = cache.layer_view(e)
             if view is not None:
                 view.page_table = ctx.page_tables[view.group]
-            ctx.reader_takes_sum, ctx.sum_rides = self._takes_sum[e], False
+            ctx.reader_takes_sum, ctx.sum_rides = self._takes_sum[e], ""
             h = self.blocks[entry.layer].forward(h, ctx, view, cache.state_view(e))
             if tap is not None:
                 tap(e + 1, ctx.resolve(h) if self.streams is None else self.streams.total(h, ctx))

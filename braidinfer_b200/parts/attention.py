@@ -272,7 +272,7 @@ class GQAAttention(Mixer):
         # the rotary encoding adds up a deferred sum in its own kernel, unless that kernel norms the heads or scales them too
         fused = (self.pe.accepts_deferred and not self.prep and not self.taps and not self.qk_norm and not self.value_from_key
                  and getattr(self.pe, "amplitude", 1.0) == 1.0)
-        qkv = self.qkv.forward(x, defer_to=ctx if fused else None, in_scale=ctx.take_row_scale(x), rides=fused)
+        qkv = self.qkv.forward(x, defer_to=ctx if fused else None, in_scale=ctx.take_row_scale(x), rides="rope")
         gate = qkv[:, self.gate_col:self.gate_col + self.nqh] if self.gate_col is not None else None
         if self.prep:
             return self._forward_padded(qkv, gate, residual, ctx, cache)

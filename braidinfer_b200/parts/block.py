@@ -30,8 +30,10 @@ class PreNormResidualBlock(Block):
         # h may still wait for a deferred sum (see StepContext.deferred); a norm that
         # accepts that adds it up in its own kernel, any other part gets h completed first
         x = self._norm(self.mixer_norm, h, ctx, self.mixer)
-        passed_on = ctx.reader_takes_sum and self.layer_input is None
-        ctx.sum_rides = self.feed_forward_norm.accepts_deferred if self.feed_forward is not None else passed_on
+        passed_on = "next" if ctx.reader_takes_sum and self.layer_input is None else ""
+        ctx.sum_rides = passed_on
+        if self.feed_forward is not None:
+            ctx.sum_rides = "norm" if self.feed_forward_norm.accepts_deferred else ""
         h = self.mixer.forward(x, h, ctx, cache, state)
         if self.feed_forward is not None:
             x = self._norm(self.feed_forward_norm, h, ctx, self.feed_forward)
@@ -58,7 +60,7 @@ class SublayerNormResidualBlock(Block):
 
     def forward(self, h, ctx, cache, state):
         h = ctx.resolve(h)
-        ctx.sum_rides = False
+        ctx.sum_rides = ""
         y = self._branch(self.mixer, h, ctx, lambda x, r: self.mixer.forward(x, r, ctx, cache, state))
         h = self.mixer_norm.add_into(y, h, ctx)
         if self.feed_forward is not None:
@@ -85,12 +87,8 @@ class HyperConnectedBlock(Block):
     outputs of a token's experts): the kernel that writes it back into the streams, which is the one that also reads
     them for the next sublayer and norms that, adds it up.  Mixer and feed-forward need `plain_output`."""
 
-    @property
-    def takes_sum(self) -> bool:
-        return True
-
     def forward(self, h, ctx, cache, state):
-        ctx.sum_rides = True
+        ctx.sum_rides = ""        # (the streams' kernel would add it up, but finished rows leave it as fast: see few_rows_pay)
         for p in (self.mixer, self.feed_forward):
             if p is not None and not p.plain_output:
                 raise RuntimeError(f"{type(p).__name__} cannot return its result alone, which hyper-connected layers need")

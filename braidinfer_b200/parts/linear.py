@@ -43,7 +43,12 @@ def stream_k_pays(rows: int, w_rows: int, k_in: int, sms: Optional[int] = None) 
     return fill < (0.8 if rows <= 48 else 0.7)
 
 
-def few_rows_pay(rows: int, w_rows: int, k_in: int, rides: bool = False) -> bool:
+# Weights, in MB, up to which the product of a few tokens runs as one kernel (few_rows_pay), at up to 8 tokens and at 9 to 16, by what adds
+# its partial sums up otherwise: a kernel of its own, the next layer's norm, the same layer's norm, the rotary encoding.
+FEW_MOST = {"": (24, 7), "next": (9, 4.5), "norm": (7, 4.5), "rope": (7, 4.5)}
+
+
+def few_rows_pay(rows: int, w_rows: int, k_in: int, rides: str = "") -> bool:
     """Whether the product of `rows` tokens with a [w_rows, k_in] bfloat16 weight should run as one kernel whose CTAs finish 16
     weight rows each (csrc/gemm_few.cu) instead of as stream-k partial sums.
 
@@ -51,17 +56,18 @@ def few_rows_pay(rows: int, w_rows: int, k_in: int, rides: bool = False) -> bool
     weights at up to 8 tokens and 7 MB at 9 to 16.  Whole turns of 24 steps, ms, with the line at 0 / 7 / 24 / 51 MB: 8 sequences of
     a Loduzen model of width 1024 8.3 / 7.4 / 6.75 / 6.8, 2 of width 2048 10.7 / 10.2 / 10.0 / 9.1, 4 of a Zisesun model of width 2048
     7.65 / 7.3 / 7.2 / 7.55, 4 of the dense decoder of width 4096 11.16 / 11.11 / 11.25 / 11.95; 12 of a Loduzen model of width 2048
-    12.8 / 12.6 / 13.1 / 12.8.
+    12.8 / 12.6 / 13.1 / 12.8.  (The streams' kernel adds sums up too, but there 8.4 MB pay as well: 4 sequences of that Zisesun model
+    445 / 442 us a step with the sums deferred / finished.)
 
-    Where they ride in a kernel that runs anyway (`rides`: the next norm, the rotary encoding), no launch is saved, and the line lies
-    at 7 MB and 4.5: a step of four layers, us, with it at 0 / 7 / 9 / 13 / 24 MB, of the dense decoder of width 1024 (products of 1.6,
-    1.0 and 5.8 MB) 165 / 130 at 4 sequences, of width 2048 (12.6, 8.4 and 23.1 MB) 224 / 223 / 227 / 232 / 233 at 4 and 228 / 228 / 232 /
-    238 / 241 at 8; with it at 0 / 2.2 / 4.3 / 7 MB at 16 sequences of width 1024 168 / 166 / 167 / 172, at 12 of a Loduzen model of
-    width 1024 290 / 280 / 275 / 273.  (Products of 8.4 MB whose sums do not ride: 8 sequences of a Bidinex model of width 2048 507 ->
-    495 us, 5 of a Megerax model 234 -> 228.)"""
+    Where they ride in a kernel that runs anyway (`rides`), no launch is saved, and the line lies lower.  A step of four layers, us:
+    the dense decoder of width 1024 (q/k/v 1.6 MB, output 1.0, down 5.8) with 4 sequences 165 with all of them deferred, 130
+    with none; of width 2048 (12.6, 8.4, 23.1) with 1 / 4 / 8 sequences 222 / 227 / 233 with all deferred, 223 / 230 / 236 with the output
+    finished, 237 / 244 / 250 with down finished, 228 / 231 / 237 with q/k/v finished; a Megerax model of width 2048, whose
+    recurrent layers' output (8.4) is read by the next layer's norm, with 1 / 5 / 8 sequences 219 / 240 / 252 with all deferred,
+    214 / 235 / 244 with those finished.  At 16 sequences of width 1024 168 with all deferred, 167 with products of up to 4.3 MB
+    finished, 172 of up to 7; at 12 of a Loduzen model of width 1024 290 / 275 / 273."""
     from ..csrc.api import FEW_MAX_ROWS
-    most = (7 if rows <= 8 else 4.5) if rides else (24 if rows <= 8 else 7)
-    return rows <= FEW_MAX_ROWS and w_rows * k_in * 2 <= most * 10 ** 6
+    return rows <= FEW_MAX_ROWS and w_rows * k_in * 2 <= FEW_MOST[rides][rows > 8] * 10 ** 6
 
 
 # Rows up to which a norm may leave its scale to the next product: beyond the token tiles of the
@@ -116,15 +122,15 @@ class Linear:
 
     def forward(self, x: torch.Tensor, *, out_dtype: Optional[torch.dtype] = None,
                 residual: Optional[torch.Tensor] = None, swiglu: bool = False, defer_to=None,
-                in_scale=None, activation: str = "silu", rides: Optional[bool] = None) -> torch.Tensor:
+                in_scale=None, activation: str = "silu", rides: Optional[str] = None) -> torch.Tensor:
         """x [rows, in].  Plain: returns [rows, out] in `out_dtype` (default x's type).
         `residual` (float32 [rows, out]): returns residual + product, written in place.
         `swiglu`: the weight holds gate rows then up rows; returns act(gate) * up, act the
         `activation` ("silu", or "gelu_tanh" for the tanh form of gelu).
         `defer_to` (a StepContext): when the product runs in its stream-k form, leave the
         adding-up of its partial sums to whoever reads the result next
-        (`StepContext.deferred`); the returned tensor is complete only after that.  `rides`: whether that is a kernel
-        that runs anyway (default: what the block says, `StepContext.sum_rides`).
+        (`StepContext.deferred`); the returned tensor is complete only after that.  `rides`: in which kernel
+        that runs anyway (see FEW_MOST; default: what the block says, `StepContext.sum_rides`).
         `in_scale` (csrc.api.RowScale): x's rows still want this scale; the product applies it to
         its results (only where `takes_row_scale()`, and not with a residual)."""
         K = self.rt.kernels
@@ -152,7 +158,8 @@ class Linear:
         sk = use_tc and stream_k_pays(rows, w_rows, x.shape[1])
         can_defer = (defer_to is not None and sk and not swiglu
                      and self.rt.fuse_reduce and K.pending_partial is None)
-        if use_tc and few_rows_pay(rows, w_rows, x.shape[1], can_defer and (defer_to.sum_rides if rides is None else rides)):
+        reader = "" if not can_defer else defer_to.sum_rides if rides is None else rides
+        if use_tc and few_rows_pay(rows, w_rows, x.shape[1], reader):
             if residual is not None:
                 K.gemm_few(x, w, residual, residual=residual)
                 return residual

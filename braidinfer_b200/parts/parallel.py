@@ -60,7 +60,7 @@ class ParallelMixers(Mixer):
     def forward(self, x, residual, ctx, cache, state):
         h, rides = residual, ctx.sum_rides
         for c, off in zip(self.children, self.offsets):
-            ctx.sum_rides = rides and c is self.children[-1]
+            ctx.sum_rides = rides if c is self.children[-1] else ""
             # a sum that the mixer before left deferred lives in the products' workspace: completed first
             h = ctx.resolve(h)
             own = None

@@ -201,6 +201,6 @@ def test_the_model_knows_which_sums_the_next_kernel_adds_up():
     assert not any(DecoderModel(spec_of(BX_A), rt)._takes_sum)
     dense = DecoderModel(spec_of(preset("tiny_b")), rt)
     assert all(dense._takes_sum) and len(dense._takes_sum) == len(dense.spec.schedule)
-    assert few_rows_pay(8, 2048, 2048) and not few_rows_pay(8, 2048, 2048, rides=True)
-    assert few_rows_pay(8, 1024, 2816, rides=True) and not few_rows_pay(16, 1024, 2816, rides=True) and few_rows_pay(16, 1024, 2816)
-    assert not few_rows_pay(17, 8, 8) and few_rows_pay(16, 1024, 2048, rides=True)
+    assert few_rows_pay(8, 2048, 2048) and not few_rows_pay(8, 2048, 2048, "norm") and few_rows_pay(8, 2048, 2048, "next")
+    assert few_rows_pay(8, 1024, 2816, "rope") and not few_rows_pay(16, 1024, 2816, "next") and few_rows_pay(16, 1024, 2816)
+    assert not few_rows_pay(17, 8, 8) and few_rows_pay(16, 1024, 2048, "norm")
