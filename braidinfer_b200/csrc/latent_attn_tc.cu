@@ -20,9 +20,9 @@
 // zeros beyond from TMA's fill).  The output gate, a factor and a sink a head are in the epilogue.
 //
 // Measured in microseconds (rank 512, heads of 128 + 64 | 128; gathered rows, product and attention together, beside queries into
-// the latent space, latent_attn_mma and values out of it): 16 heads, 2,048 tokens 94 beside 725; 512 tokens after 4,096 178
-// beside 940 (of which this kernel 107 beside 881); 16 sequences of 20 tokens after 1,024 130 beside 250.  32 heads, two
-// sequences of 1,777 and 1,244 tokens: this kernel 74 beside 1,390.
+// the latent space, latent_attn_mma and values out of it): 16 heads, 2,048 tokens 85 beside 725; 512 tokens after 4,096 152
+// beside 940 (of which this kernel 99 beside 881); 16 sequences of 20 tokens after 1,024 129 beside 250.  32 heads, two
+// sequences of 1,777 and 1,244 tokens: this kernel 85 beside 1,390.
 #include "common.cuh"
 #include "attn_tc.cuh"
 #include "page.h"

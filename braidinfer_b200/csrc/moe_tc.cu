@@ -15,10 +15,10 @@
 // Bound by the weights' bytes where an expert sees up to some 200 tokens, by the tensor cores and power beyond.  Measured in
 // microseconds, plan, gathered rows, gate+up and down together, beside the better of the mma.sync kernels of moe.cu (tiles of 16 or
 // 64 slots), L2 flushed; in brackets what the weights in use or the products take at 6.55 TB/s and 1.65 PFLOP/s:
-//   64 experts of 2048 x 1408, 6 a token: 8 tokens 138 beside 148 (100), 256 tokens 215 beside 279 (169), 2,048 tokens
-//   251 beside 865 (169), 4,096 tokens 472 beside 1,668 (258)
-//   8 experts of 4096 x 7168, 2 a token: 1 token 112 beside 185 (54), 8 tokens 277 beside 343 (215), 2,048 tokens 615 beside 2,830 (437)
-//   16 experts of 1024 x 1024, 2 a token: 1 token 31 beside 41, 2,048 tokens 67 beside 134 (16)
+//   64 experts of 2048 x 1408, 6 a token: 8 tokens 139 beside 157 (100), 256 tokens 213 beside 280 (169), 2,048 tokens
+//   255 beside 894 (169), 4,096 tokens 435 beside 1,668 (258)
+//   8 experts of 4096 x 7168, 2 a token: 1 token 111 beside 184 (54), 8 tokens 256 beside 293 (215), 2,048 tokens 642 beside 2,625 (437)
+//   16 experts of 1024 x 1024, 2 a token: 1 token 32 beside 39, 2,048 tokens 68 beside 133 (16)
 #include "common.cuh"
 #include "tcgen05_pair.cuh"
 

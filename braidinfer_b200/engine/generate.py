@@ -16,7 +16,8 @@ through those calls, so its decisions are tested on the CPU with stand-ins.
 `step=<k> tok=<token> logit_hash=<16 hex digits> seq=<request>` for every token chosen: k counts the
 request's tokens from 0, the hash is over the float32 logits the token was chosen from
 (`Engine.logit_hash`).  Two runs that should agree are compared by these files, and the first line that
-differs names the step to look at.  Tracing runs the loop unpipelined.
+differs names the step to look at.  The bits of a row's logits follow the sizes of the steps that it ran in, so runs of the same
+batches are compared, not a request alone with one among others.  Tracing runs the loop unpipelined.
 """
 from __future__ import annotations
 
