@@ -748,6 +748,12 @@ class Kernels:
                 lib.braid_ssd_scan.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 4 + [c_longlong, c_void_p, c_longlong, c_longlong] + \
                                               [c_void_p] * 3 + [c_int] * 5 + [c_float, c_void_p]
                 lib.braid_ssd_scan.restype = c_int
+                lib.braid_scan_chunk.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] + [c_void_p, c_longlong] * 2 + [c_longlong] + \
+                                                [c_void_p] * 3 + [c_int] * 7 + [c_float, c_float] + [c_int] * 3 + \
+                                                [c_void_p, c_longlong, c_void_p]
+                lib.braid_scan_chunk.restype = c_int
+                lib.braid_scan_chunk_work_floats.argtypes = [c_int] * 5
+                lib.braid_scan_chunk_work_floats.restype = c_longlong
                 lib.braid_linear_scan_work_floats.restype = c_longlong
                 lib.braid_gated_norm.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong,
                                                  c_void_p] + [c_int] * 6 + [c_float, c_float, c_void_p]
@@ -1400,6 +1406,20 @@ class Kernels:
                 and out.stride(0) % 2 == 0 and out.data_ptr() % 8 == 0
                 and (state.data_ptr() | int(state_offset) | state.stride(0)) % 8 == 0)
 
+    # Tokens of a step's longest sequence from which on a recurrence with a decay a key channel, or a constant one a head, runs over chunks
+    # on the tensor cores (csrc/scan_chunk.cu), for keys of 64 and of 128.  Beside the walk token by token, us: a decay a channel, 8 heads of
+    # 128 x 256 64 tokens 46 / 37, 96 46 / 79, 4 heads of 64 x 128 32 tokens 24 / 23, 64 24 / 37; constant decays 96 tokens 65 / 39, 128
+    # 65 / 69, and 64 28 / 31.
+    SCAN_CHUNK_FROM = {"channel": (48, 80), "constant": (64, 128)}
+
+    def scan_chunk_fits(self, q, k, v, out, state, state_offset: int, ctx, dk: int, dv: int, mode: str = "channel") -> bool:
+        """Whether `linear_scan` in mode "channel" or "constant" takes the form over chunks on the tensor cores, which works decays out of
+        their logits itself, once each."""
+        return (SCAN_CHUNK is None and q.dtype == torch.bfloat16 and dk in (64, 128) and dv % 64 == 0
+                and int(ctx.max_q_len) >= self.SCAN_CHUNK_FROM[mode][dk == 128]
+                and v.stride(0) % 8 == 0 and v.data_ptr() % 16 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 8 == 0
+                and (state.data_ptr() | int(state_offset) | state.stride(0)) % 16 == 0)
+
     def linear_scan(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, gate_bias: torch.Tensor,
                     out: torch.Tensor, state: torch.Tensor, state_offset: int, ctx, heads: int, groups: int, dk: int,
                     dv: int, mode: str, q_scale: float = 1.0, inv_tau: float = 1.0, a_log: Optional[torch.Tensor] = None,
@@ -1417,7 +1437,9 @@ class Kernels:
         `gate_bias` is then unused (pass any tensor of the rows' type).
         mode "constant": a = gate[head], float32 [heads], the same for every token, kappa = 1 (`gate_bias` is unused);
         with `act_silu` q, k and v are silu of what is given, computed in float32.
-        A step whose longest sequence brings at least two chunks of `chunk` tokens (default: see SCAN_CHUNK; 0: never)
+        bfloat16 rows of modes "channel" and "constant" run over chunks on the tensor cores where `scan_chunk_fits` and no `chunk`
+        is named, mode "head" where `ssd_pays`.  Else
+        a step whose longest sequence brings at least two chunks of `chunk` tokens (default: see SCAN_CHUNK; 0: never)
         walks its chunks side by side in three passes (see csrc/scan.cu); the results differ from the walk
         token by token by rounding only."""
         lib = self.part_library("scan")
@@ -1452,6 +1474,17 @@ class Kernels:
                 gate_bias.data_ptr(), a_log.data_ptr(), _ptr(skip), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
                 ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), ctx.n_seqs, heads, groups, dk, dv, float(q_scale),
                 self._stream()), "ssd_scan")
+            return
+        if chunk is None and mode in ("channel", "constant") and self.scan_chunk_fits(q, k, v, out, state, state_offset, ctx, dk, dv, mode):
+            need = lib.braid_scan_chunk_work_floats(q.shape[0], ctx.n_seqs, heads, dk, dv)
+            work = torch.empty(need, dtype=torch.float32, device=out.device)
+            self.launches += 3
+            self._check_lib(lib, lib.braid_scan_chunk(
+                q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(),
+                gate.stride(0), _ptr(gate_bias), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
+                ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), q.shape[0], ctx.n_seqs, int(ctx.max_q_len),
+                heads, groups, dk, dv, float(q_scale), float(inv_tau), int(mode == "constant"), int(gate_is_decay), int(act_silu),
+                work.data_ptr(), need, self._stream()), "scan_chunk")
             return
         if chunk is None:
             chunk = SCAN_CHUNK if SCAN_CHUNK is not None else (128 if int(ctx.max_q_len) >= 1024 else 64)

@@ -102,9 +102,9 @@ class GatedLinearAttention(Mixer):
             a1 = a1.contiguous()                                        # the tensor-core product wants aligned rows
         z = self.a2.forward(a1, out_dtype=torch.float32)                # the decay's logit, before its bias
         o = torch.empty((rows, H * dv), dtype=torch.float32, device=x.device)
-        # in a long step every decay is read by many CTAs of the recurrence: computed once, in place; a short
-        # step computes them where they are used and saves the launch
-        ready = rows > self.DECAY_IN_PLACE_ROWS
+        # in a long step every decay is read by many CTAs of the walk: computed once, in place; a short step, and the form over
+        # chunks on the tensor cores, compute them where they are used and save the launch
+        ready = rows > self.DECAY_IN_PLACE_ROWS and not K.scan_chunk_fits(q, k, v, o, state, 0, ctx, dk, dv)
         if ready:
             K.scan_decay(z, self.a2_bias, 1.0 / self.tau)
         K.linear_scan(q, k, v, z, self.a2_bias, o, state, 0, ctx, H, H, dk, dv, "channel",
