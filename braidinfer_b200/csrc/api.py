@@ -734,7 +734,7 @@ class Kernels:
                          "braid_latent_attn_tc", "braid_latent_attn_tc_supported")
             elif name == "scan":
                 lib.braid_causal_conv.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
-                                                  c_void_p, c_longlong, c_longlong] + [c_void_p] * 4 + [c_int] * 5 + [c_void_p]
+                                                  c_void_p, c_longlong, c_longlong] + [c_void_p] * 4 + [c_int] * 6 + [c_void_p]
                 lib.braid_linear_scan.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 3 + [c_void_p, c_longlong] + \
                                                  [c_void_p, c_longlong, c_longlong] + [c_void_p] * 3 + [c_int] * 7 + \
                                                  [c_float, c_float, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_int,
@@ -752,6 +752,10 @@ class Kernels:
                                                 [c_void_p] * 3 + [c_int] * 7 + [c_float, c_float] + [c_int] * 3 + \
                                                 [c_void_p, c_longlong, c_void_p]
                 lib.braid_scan_chunk.restype = c_int
+                lib.braid_scan_step.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 3 + [c_void_p, c_longlong] * 2 + [c_longlong] + \
+                                               [c_void_p] * 3 + [c_int] * 7 + [c_float, c_float, c_int, c_void_p, c_longlong, c_void_p,
+                                                                               c_void_p, c_longlong, c_int, c_float, c_float, c_void_p]
+                lib.braid_scan_step.restype = c_int
                 lib.braid_scan_chunk_work_floats.argtypes = [c_int] * 5
                 lib.braid_scan_chunk_work_floats.restype = c_longlong
                 lib.braid_linear_scan_work_floats.restype = c_longlong
@@ -778,6 +782,10 @@ class Kernels:
                                                 [c_int] * 5 + [c_void_p] * 5 + [c_int, c_void_p, c_void_p]
                 names = ("braid_conv_heads",)
             elif name == "delta":
+                lib.braid_delta_step.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p, c_void_p, c_void_p, c_longlong, c_int] + \
+                                                [c_void_p, c_longlong] * 2 + [c_longlong] + [c_void_p] * 3 + [c_int] * 5 + \
+                                                [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_float, c_void_p]
+                lib.braid_delta_step.restype = c_int
                 lib.braid_delta_rule.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p, c_void_p, c_void_p, c_longlong, c_int,
                                                  c_void_p, c_longlong, c_void_p, c_longlong, c_longlong] + [c_void_p] * 3 + \
                                                 [c_int] * 7 + [c_void_p, c_longlong, c_void_p]
@@ -1274,11 +1282,17 @@ class Kernels:
         if not (x.dtype == y.dtype == w.dtype) or (b is not None and b.dtype != x.dtype) or x.stride(1) != 1 \
                 or y.stride(1) != 1 or not w.is_contiguous() or w.shape[0] != channels or x.shape[1] != channels:
             raise KernelError("causal_conv: x, y, w, b of one element type; w contiguous [channels, taps]")
-        self.launches += 2 if taps > 1 else 1
+        vec = 16 // x.element_size()
+        # one token a sequence: convolution and the state's move in one kernel, where rows and state allow 16-byte moves
+        one = (getattr(ctx, "max_q_len", 0) == 1 and 2 <= taps <= 4 and all(n % vec == 0 for n in (channels, x.stride(0), y.stride(0)))
+               and all(p % 16 == 0 for p in (x.data_ptr(), y.data_ptr(), w.data_ptr(), b.data_ptr() if b is not None else 0))
+               and (state.data_ptr() | int(state_offset) | state.stride(0)) % 16 == 0)
+        self.launches += 2 if taps > 1 and not one else 1
         self._check_lib(lib, lib.braid_causal_conv(
             x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), w.data_ptr(), _ptr(b), dtype_code(x.dtype),
             *self._state_args(state, state_offset), ctx.token_seq.data_ptr(), ctx.q_start.data_ptr(),
-            ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), rows, ctx.n_seqs, channels, taps, int(silu), self._stream()),
+            ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), rows, ctx.n_seqs, channels, taps, int(silu), int(one),
+            self._stream()),
             "causal_conv")
 
     @staticmethod
@@ -1341,18 +1355,38 @@ class Kernels:
 
     def delta_rule(self, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, bias: torch.Tensor,
                    rate: torch.Tensor, b: torch.Tensor, out: torch.Tensor, state: torch.Tensor, state_offset: int, ctx,
-                   heads: int, groups: int, dk: int, dv: int, chunked: bool) -> None:
+                   heads: int, groups: int, dk: int, dv: int, chunked: bool, norm=None) -> None:
         """The gated delta rule along each sequence of the step (csrc/delta.cu): S <- diag(g) S; u = beta (v - S^T k);
         S <- S + k u^T; out = S^T q, with g = exp(-rate softplus(z + bias)) and beta = sigmoid(b); S float32 [heads, dk, dv] at
         `state_offset` bytes of each slot.  q, k [rows, groups * dk], v, out [rows, heads * dv], z [rows, heads * dk], bias
         [heads * dk], rate [heads]: float32; b [rows, heads] in the run's type.  `chunked`: 64 tokens at a time instead of one
-        (the results differ by rounding only)."""
+        (the results differ by rounding only).  Steps of one token a sequence have a kernel of their own where `scan_step_fits`; there
+        `norm` may be (gate's logits float32 [rows, heads * dv], w [dv], y [rows, heads * dv], eps): instead of `out`, which may
+        be None, y = o / rms(o) * w * sigmoid(gate) a head, as `delta_gated_norm` has it."""
         lib = self.part_library("delta")
-        if any(t.dtype != torch.float32 or t.stride(-1) != 1 for t in (q, k, v, z, bias, rate, out)) or b.stride(1) != 1:
+        if any(t.dtype != torch.float32 or t.stride(-1) != 1 for t in (q, k, v, z, bias, rate) + ((out,) if out is not None else ())) \
+                or b.stride(1) != 1:
             raise KernelError("delta_rule: float32 rows with contiguous elements")
         if q.shape[1] != groups * dk or k.shape[1] != groups * dk or v.shape[1] != heads * dv or z.shape[1] != heads * dk \
-                or bias.numel() != heads * dk or rate.numel() != heads or b.shape[1] < heads or out.shape[1] != heads * dv:
+                or bias.numel() != heads * dk or rate.numel() != heads or b.shape[1] < heads \
+                or (out.shape[1] != heads * dv if out is not None else norm is None):
             raise KernelError("delta_rule: the rows do not hold the heads")
+        step = not chunked and self.scan_step_fits(v, state, state_offset, ctx, dk, dv) \
+            and (out is None or (out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0))
+        gate, w, y, eps = norm if norm is not None else (None, None, None, 0.0)
+        if norm is not None and (not step or gate.dtype != torch.float32 or w.dtype != y.dtype or y.dtype != b.dtype or w.numel() != dv
+                                 or gate.shape[1] < heads * dv or y.shape[1] < heads * dv or not self.step_norm_fits(dv, gate, y)):
+            raise KernelError("delta_rule: the norm goes with one token a sequence, float32 gates, w and y of the run's type")
+        if step:
+            self.launches += 1
+            self._check_lib(lib, lib.braid_delta_step(
+                q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), z.data_ptr(), z.stride(0),
+                bias.data_ptr(), rate.data_ptr(), b.data_ptr(), b.stride(0), dtype_code(b.dtype), _ptr(out),
+                out.stride(0) if out is not None else 0, *self._state_args(state, state_offset), ctx.q_start.data_ptr(),
+                ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), ctx.n_seqs, heads, groups, dk, dv, _ptr(gate),
+                gate.stride(0) if gate is not None else 0, _ptr(w), _ptr(y), y.stride(0) if y is not None else 0, float(eps),
+                self._stream()), "delta_step")
+            return
         rows = out.shape[0]
         need = lib.braid_delta_work_floats(rows, ctx.n_seqs, heads, dk, dv) if chunked else 0
         work = torch.empty(need, dtype=torch.float32, device=out.device) if need > 0 else None
@@ -1406,6 +1440,39 @@ class Kernels:
                 and out.stride(0) % 2 == 0 and out.data_ptr() % 8 == 0
                 and (state.data_ptr() | int(state_offset) | state.stride(0)) % 8 == 0)
 
+    # Value columns a head whose gated norm the kernels of one token a sequence do themselves (csrc/scan_step.cu, csrc/delta.cu): a CTA
+    # holds them all.
+    STEP_NORM_COLS = (64, 128, 256)
+
+    @staticmethod
+    def scan_step_fits(v, state, state_offset: int, ctx, dk: int, dv: int) -> bool:
+        """Whether `linear_scan` and `delta_rule` take the kernels of one token a sequence: such a step, sizes and alignments of its moves of four
+        numbers."""
+        return (int(ctx.max_q_len) == 1 and dk in (64, 128) and dv % 64 == 0
+                and v.stride(0) % 4 == 0 and v.data_ptr() % (4 * v.element_size()) == 0
+                and (state.data_ptr() | int(state_offset) | state.stride(0)) % 16 == 0)
+
+    @classmethod
+    def step_norm_fits(cls, dv: int, *rows: torch.Tensor) -> bool:
+        """Whether the kernels of one token a sequence can also do the gated norm of a head's dv columns, gates and results in `rows`."""
+        return dv in cls.STEP_NORM_COLS and all(t.stride(-1) == 1 and t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0
+                                                for t in rows)
+
+    def _scan_step(self, lib, q, k, v, gate, gate_bias, out, state, state_offset, ctx, heads, groups, dk, dv, mode, q_scale, inv_tau,
+                   a_log, skip, act_silu, norm) -> None:
+        z, w, y, eps, out_scale = norm if norm is not None else (None, None, None, 0.0, 1.0)
+        if norm is not None and (not z.dtype == w.dtype == y.dtype == q.dtype or w.numel() != dv or z.shape[1] < heads * dv
+                                 or y.shape[1] < heads * dv or not self.step_norm_fits(dv, z, y)):
+            raise KernelError("linear_scan: gates, weights and results of the norm have the rows' element type and hold the heads' columns")
+        self.launches += 1
+        self._check_lib(lib, lib.braid_scan_step(
+            q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(), gate.stride(0),
+            _ptr(gate_bias), _ptr(a_log), _ptr(skip), _ptr(out), out.stride(0) if out is not None else 0,
+            *self._state_args(state, state_offset), ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(),
+            dtype_code(q.dtype), {"channel": 0, "head": 1, "constant": 3}[mode], ctx.n_seqs, heads, groups, dk, dv, float(q_scale),
+            float(inv_tau), int(act_silu), _ptr(z), z.stride(0) if z is not None else 0, _ptr(w), _ptr(y),
+            y.stride(0) if y is not None else 0, 0, float(eps), float(out_scale), self._stream()), "scan_step")
+
     # Tokens of a step's longest sequence from which on a recurrence with a decay a key channel, or a constant one a head, runs over chunks
     # on the tensor cores (csrc/scan_chunk.cu), for keys of 64 and of 128.  Beside the walk token by token, us: a decay a channel, 8 heads of
     # 128 x 256 64 tokens 46 / 37, 96 46 / 79, 4 heads of 64 x 128 32 tokens 24 / 23, 64 24 / 37; constant decays 96 tokens 65 / 39, 128
@@ -1424,7 +1491,7 @@ class Kernels:
                     out: torch.Tensor, state: torch.Tensor, state_offset: int, ctx, heads: int, groups: int, dk: int,
                     dv: int, mode: str, q_scale: float = 1.0, inv_tau: float = 1.0, a_log: Optional[torch.Tensor] = None,
                     skip: Optional[torch.Tensor] = None, chunk: Optional[int] = None, gate_is_decay: bool = False,
-                    kappa: Optional[torch.Tensor] = None, v_cols: Optional[int] = None, act_silu: bool = False) -> None:
+                    kappa: Optional[torch.Tensor] = None, v_cols: Optional[int] = None, act_silu: bool = False, norm=None) -> None:
         """The recurrence S <- diag(a) S + (kappa k) v^T, o = S^T (q_scale q) + skip v, token by token along each
         sequence of the step, S float32 [heads, dk, dv] at `state_offset` bytes of each slot.  mode "channel":
         a = sigmoid(gate + gate_bias)^inv_tau per key channel (gate float32 [rows, heads * dk]); mode "head":
@@ -1437,6 +1504,9 @@ class Kernels:
         `gate_bias` is then unused (pass any tensor of the rows' type).
         mode "constant": a = gate[head], float32 [heads], the same for every token, kappa = 1 (`gate_bias` is unused);
         with `act_silu` q, k and v are silu of what is given, computed in float32.
+        Steps of one token a sequence have a kernel of their own where `scan_step_fits`; there `norm` may be (gates [rows, heads * dv],
+        w [dv], y [rows, heads * dv], eps, out_scale), all of the run's type: instead of `out`, which may be None,
+        y = o / rms(o) * w * silu(gate) * out_scale a head, as `gated_norm` has it.
         bfloat16 rows of modes "channel" and "constant" run over chunks on the tensor cores where `scan_chunk_fits` and no `chunk`
         is named, mode "head" where `ssd_pays`.  Else
         a step whose longest sequence brings at least two chunks of `chunk` tokens (default: see SCAN_CHUNK; 0: never)
@@ -1444,8 +1514,9 @@ class Kernels:
         token by token by rounding only."""
         lib = self.part_library("scan")
         if not (q.dtype == k.dtype == v.dtype) or (gate_bias is not None and gate_bias.dtype != q.dtype) \
-                or (gate_bias is None and mode in ("channel", "head")) or out.dtype != torch.float32 \
-                or any(t.stride(-1) != 1 for t in (q, k, v, gate, out)):
+                or (gate_bias is None and mode in ("channel", "head")) or (out is None and norm is None) \
+                or (out is not None and (out.dtype != torch.float32 or out.stride(-1) != 1)) \
+                or any(t.stride(-1) != 1 for t in (q, k, v, gate)):
             raise KernelError("linear_scan: q, k, v and the gate's bias of one element type, out float32, rows contiguous")
         if mode == "channel":
             if gate.dtype != torch.float32 or gate.shape[1] != heads * dk or gate_bias.numel() != heads * dk:
@@ -1465,8 +1536,14 @@ class Kernels:
         else:
             raise KernelError(f"linear_scan: unknown decay mode {mode!r}")
         vc = dv if v_cols is None else int(v_cols)
-        if v.shape[1] < heads * vc or out.shape[1] < heads * dv:
+        if v.shape[1] < heads * vc or (out is not None and out.shape[1] < heads * dv):
             raise KernelError("linear_scan: v or out does not hold the heads' columns")
+        if chunk is None and mode != "given" and not gate_is_decay and self.scan_step_fits(v, state, state_offset, ctx, dk, dv) \
+                and (out is None or (out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0)):
+            return self._scan_step(lib, q, k, v, gate, gate_bias, out, state, state_offset, ctx, heads, groups, dk, dv, mode, q_scale,
+                                   inv_tau, a_log, skip, act_silu, norm)
+        if norm is not None:
+            raise KernelError("linear_scan: a norm goes with one token a sequence")
         if chunk is None and mode == "head" and self._ssd_fits(q, k, v, out, state, state_offset, ctx, heads, dk, dv, vc):
             self.launches += 1
             self._check_lib(lib, lib.braid_ssd_scan(

@@ -182,6 +182,102 @@ delta_walk_kernel(DeltaArgs a) {
         }
 }
 
+// ------------------------------------------------------------------ one token a sequence
+// Such a step is a read and a write of the state and otherwise latency.  A CTA owns (head, sequence, COLS value columns); eight row groups
+// of threads take every eighth key row, four neighbouring columns a thread, the state asked for all at once before the wait.  Where a
+// CTA holds all of a head's columns it goes on to the gated norm (y = o / rms(o) * w * sigmoid(gate)).  5 sequences of 8 heads of 128 x 256
+// between the kernels of a decode step: 12.5 us for the walk and the norm's kernel, 6.1 so.
+struct DeltaNorm {
+    const float* gate; long long gate_stride;    // [rows, heads * dv]: logits
+    const void* w;                               // [dv], run type
+    void* y; long long y_stride;                 // run type; null: o goes to `out`
+    float eps;
+};
+#define DELTA_RG 8
+template <typename T, int DK, int COLS>
+__global__ void __launch_bounds__(DELTA_RG * COLS / 4)
+delta_step_kernel(const __grid_constant__ DeltaArgs a, const __grid_constant__ DeltaNorm m) {
+    constexpr int CG = COLS / 4, NT = DELTA_RG * CG, R = DK / DELTA_RG;
+    __shared__ float sq[DK], sk[DK], sa[DK], skq[DELTA_RG], red[32];
+    __shared__ float4 pk[DELTA_RG][CG], pq[DELTA_RG][CG];
+    pdl_trigger();
+    const int h = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x, cg = tid % CG, rg = tid / CG, col = blockIdx.z * COLS + cg * 4;
+    if (a.q_len[seq] <= 0) return;
+    const size_t row = a.q_start[seq];
+    const int g = h / (a.heads / a.groups);
+    float4* S = (float4*)((float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + (size_t)rg * a.dv + col);
+    const size_t step = (size_t)DELTA_RG * a.dv / 4;
+    float4 s[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) s[j] = S[j * step];
+    const float rate = a.rate[h];
+    pdl_wait();
+    const float4 v = *reinterpret_cast<const float4*>(a.v + row * a.v_stride + (size_t)h * a.dv + col);
+    float4 gate = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (m.y && rg == 0) gate = *reinterpret_cast<const float4*>(m.gate + row * m.gate_stride + (size_t)h * a.dv + col);
+    const float beta = delta_sigmoid(to_f32(((const T*)a.b)[row * a.b_stride + h]));
+    for (int i = tid; i < DK; i += NT) {
+        sq[i] = a.q[row * a.q_stride + (size_t)g * DK + i];
+        sk[i] = a.k[row * a.k_stride + (size_t)g * DK + i];
+        sa[i] = delta_decay(a.z[row * a.z_stride + (size_t)h * DK + i] + a.bias[(size_t)h * DK + i], rate);
+    }
+    __syncthreads();
+    float4 tk = make_float4(0.f, 0.f, 0.f, 0.f), tq = tk;
+    float kq = 0.f;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const int i = rg + j * DELTA_RG;
+        const float av = sa[i], kk = sk[i], qq = sq[i];
+        s[j].x *= av; s[j].y *= av; s[j].z *= av; s[j].w *= av;
+        tk.x = fmaf(s[j].x, kk, tk.x); tk.y = fmaf(s[j].y, kk, tk.y); tk.z = fmaf(s[j].z, kk, tk.z); tk.w = fmaf(s[j].w, kk, tk.w);
+        tq.x = fmaf(s[j].x, qq, tq.x); tq.y = fmaf(s[j].y, qq, tq.y); tq.z = fmaf(s[j].z, qq, tq.z); tq.w = fmaf(s[j].w, qq, tq.w);
+        kq = fmaf(kk, qq, kq);
+    }
+    pk[rg][cg] = tk;
+    pq[rg][cg] = tq;
+    if (cg == 0) skq[rg] = kq;
+    __syncthreads();
+    float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < DELTA_RG; ++r) {
+        const float4 x = pk[r][cg];
+        u.x += x.x; u.y += x.y; u.z += x.z; u.w += x.w;
+    }
+    u = make_float4(beta * (v.x - u.x), beta * (v.y - u.y), beta * (v.z - u.z), beta * (v.w - u.w));
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        const float kk = sk[rg + j * DELTA_RG];
+        S[j * step] = make_float4(fmaf(kk, u.x, s[j].x), fmaf(kk, u.y, s[j].y), fmaf(kk, u.z, s[j].z), fmaf(kk, u.w, s[j].w));
+    }
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (rg == 0) {
+        kq = 0.f;
+#pragma unroll
+        for (int r = 0; r < DELTA_RG; ++r) {
+            const float4 x = pq[r][cg];
+            o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
+            kq += skq[r];
+        }
+        o = make_float4(fmaf(kq, u.x, o.x), fmaf(kq, u.y, o.y), fmaf(kq, u.z, o.z), fmaf(kq, u.w, o.w));
+        if (!m.y) *reinterpret_cast<float4*>(a.out + row * a.out_stride + (size_t)h * a.dv + col) = o;
+    }
+    if (!m.y) return;
+    const float r = 1.f / sqrtf(block_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w, red) / (float)COLS + m.eps);
+    if (rg > 0) return;
+    const float oo[4] = {o.x, o.y, o.z, o.w}, gg[4] = {gate.x, gate.y, gate.z, gate.w};
+    T* y = (T*)m.y + row * m.y_stride + (size_t)h * a.dv + col;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[e] = from_f32<T>(oo[e] * r * to_f32(((const T*)m.w)[cg * 4 + e]) * norm_gate(gg[e], 1));
+}
+
+template <typename T, int DK>
+static int launch_delta_step(const DeltaArgs& a, const DeltaNorm& m, int n_seqs, cudaStream_t s) {
+    if (!m.y || a.dv == 64) braid_launch(delta_step_kernel<T, DK, 64>, dim3(a.heads, n_seqs, a.dv / 64), dim3(DELTA_RG * 16), 0, s, a, m);
+    else if (a.dv == 128) braid_launch(delta_step_kernel<T, DK, 128>, dim3(a.heads, n_seqs), dim3(DELTA_RG * 32), 0, s, a, m);
+    else braid_launch(delta_step_kernel<T, DK, 256>, dim3(a.heads, n_seqs), dim3(DELTA_RG * 64), 0, s, a, m);
+    BRAID_LAUNCH_CHECK();
+}
+
 // ------------------------------------------------------------------ inside every chunk
 #define DELTA_INTRA_THREADS 256
 template <int DKP> constexpr int delta_intra_smem() { return (3 * DELTA_C * (DKP + 4) + DELTA_C + 3 * DKP) * 4; }
@@ -721,6 +817,32 @@ extern "C" int braid_delta_rule(const float* q, long long q_stride, const float*
     }
     if (dtype == BRAID_F32) return launch_delta<float>(a, n_seqs, work != nullptr, (cudaStream_t)stream);
     return launch_delta<__nv_bfloat16>(a, n_seqs, work != nullptr, (cudaStream_t)stream);
+}
+
+// One token a sequence (q_len 0 or 1).  dk 64 or 128, dv a multiple of 64; v, gate, state and results start on 16 bytes.  With y: out is not
+// written, y = the gated norm of every head's columns (gate's logits in float32, a sigmoid, w [dv]), dv 64, 128 or 256.
+extern "C" int braid_delta_step(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
+                                long long v_stride, const float* z, long long z_stride, const float* bias, const float* rate,
+                                const void* b, long long b_stride, int dtype, float* out, long long out_stride, void* state,
+                                long long state_stride, long long state_offset, const int* q_start, const int* q_len,
+                                const int* slot_ids, int n_seqs, int heads, int groups, int dk, int dv, const float* gate,
+                                long long gate_stride, const void* w, void* y, long long y_stride, float eps, void* stream) {
+    if (n_seqs <= 0) return BRAID_OK;
+    if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("delta_step: %d heads do not divide into %d groups", heads, groups);
+    if ((dk != 64 && dk != 128) || dv <= 0 || dv % 64) BRAID_REFUSE("delta_step: built for keys of 64 or 128 and values in multiples of 64, not %d x %d", dk, dv);
+    if (!state || (((uintptr_t)state | (uintptr_t)state_offset | (uintptr_t)state_stride) & 15)) BRAID_REFUSE("delta_step: the state must start on 16 bytes");
+    if (((uintptr_t)v & 15) || v_stride % 4) BRAID_REFUSE("delta_step: rows of v must start on 16 bytes");
+    if (!y && (!out || ((uintptr_t)out & 15) || out_stride % 4)) BRAID_REFUSE("delta_step: results must start on 16 bytes");
+    if (y && ((dv != 64 && dv != 128 && dv != 256) || !gate || !w || ((uintptr_t)gate & 15) || gate_stride % 4))
+        BRAID_REFUSE("delta_step: the norm is done for heads of 64, 128 or 256 columns with gates on 16 bytes, not %d", dv);
+    if (dtype != BRAID_F32 && dtype != BRAID_BF16) BRAID_REFUSE("delta_step: unknown dtype code %d", dtype);
+    if (n_seqs > 65535 || dv / 64 > 65535) BRAID_REFUSE("delta_step: the step exceeds the grid limits");
+    DeltaArgs a{q, q_stride, k, k_stride, v, v_stride, z, z_stride, bias, rate, b, b_stride, out, out_stride, (uint8_t*)state,
+                state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dk, dv};
+    const DeltaNorm m{gate, gate_stride, w, y, y_stride, eps};
+    cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == BRAID_F32) return dk == 64 ? launch_delta_step<float, 64>(a, m, n_seqs, s) : launch_delta_step<float, 128>(a, m, n_seqs, s);
+    return dk == 64 ? launch_delta_step<__nv_bfloat16, 64>(a, m, n_seqs, s) : launch_delta_step<__nv_bfloat16, 128>(a, m, n_seqs, s);
 }
 
 // The read-out's norm and gate (gated_norm.cuh), the gate's logits in float32.

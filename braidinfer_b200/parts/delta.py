@@ -125,13 +125,17 @@ class ChannelDelta(Mixer):
                      [K.conv_segment(G, dk, silu=True, norm="unit", factor=dk ** -0.5, out=q),
                       K.conv_segment(G, dk, silu=True, norm="unit", out=k), K.conv_segment(H, dv, silu=True, out=v)],
                      eps=self.unit_eps)
-        o = f32(H * dv)
         b = proj[:, low + self.channels:low + self.channels + H]
-        K.delta_rule(q, k, v, logits[:, :H * dk], self.dt_bias, self.rate, b, o, state, self.conv_state_bytes(), ctx, H, G, dk, dv,
-                     chunked=int(ctx.max_q_len) >= self.CHUNKED_FROM)
         padded = ctx.rows > ctx.n_tokens
         y = torch.zeros((rows, H * dv), dtype=x.dtype, device=x.device) if padded else self.rt.empty(rows, H * dv)
-        K.delta_gated_norm(o, logits[:, H * dk:], self.norm_w, y, ctx.token_seq, dv, self.eps)
+        gates = logits[:, H * dk:]
+        fused = K.scan_step_fits(v, state, self.conv_state_bytes(), ctx, dk, dv) and K.step_norm_fits(dv, gates, y)
+        o = None if fused else f32(H * dv)             # one token a sequence: rule and norm in one kernel
+        K.delta_rule(q, k, v, logits[:, :H * dk], self.dt_bias, self.rate, b, o, state, self.conv_state_bytes(), ctx, H, G, dk, dv,
+                     chunked=int(ctx.max_q_len) >= self.CHUNKED_FROM,
+                     norm=(gates, self.norm_w, y, self.eps) if fused else None)
+        if not fused:
+            K.delta_gated_norm(o, gates, self.norm_w, y, ctx.token_seq, dv, self.eps)
         if residual is None:
             return self.o.forward(y, out_dtype=torch.float32, defer_to=ctx)
         return self.o.forward(y, residual=residual, defer_to=ctx)

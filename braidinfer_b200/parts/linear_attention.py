@@ -101,6 +101,13 @@ class GatedLinearAttention(Mixer):
         if a1.data_ptr() % 16 or self.rank % 8:
             a1 = a1.contiguous()                                        # the tensor-core product wants aligned rows
         z = self.a2.forward(a1, out_dtype=torch.float32)                # the decay's logit, before its bias
+        padded = ctx.rows > ctx.n_tokens
+        y = torch.zeros((rows, H * dv), dtype=x.dtype, device=x.device) if padded else self.rt.empty(rows, H * dv)
+        if K.scan_step_fits(v, state, 0, ctx, dk, dv) and K.step_norm_fits(dv, g, y):
+            # one token a sequence: recurrence and norm in one kernel
+            K.linear_scan(q, k, v, z, self.a2_bias, None, state, 0, ctx, H, H, dk, dv, "channel", q_scale=dk ** -0.5,
+                          inv_tau=1.0 / self.tau, norm=(g, self.norm_w, y, self.eps, self.out_mult))
+            return self.o.forward(y, residual=residual, defer_to=ctx)
         o = torch.empty((rows, H * dv), dtype=torch.float32, device=x.device)
         # in a long step every decay is read by many CTAs of the walk: computed once, in place; a short step, and the form over
         # chunks on the tensor cores, compute them where they are used and save the launch
@@ -109,8 +116,6 @@ class GatedLinearAttention(Mixer):
             K.scan_decay(z, self.a2_bias, 1.0 / self.tau)
         K.linear_scan(q, k, v, z, self.a2_bias, o, state, 0, ctx, H, H, dk, dv, "channel",
                       q_scale=dk ** -0.5, inv_tau=1.0 / self.tau, gate_is_decay=ready)
-        padded = ctx.rows > ctx.n_tokens
-        y = torch.zeros((rows, H * dv), dtype=x.dtype, device=x.device) if padded else self.rt.empty(rows, H * dv)
         K.gated_norm(o, g, self.norm_w, y, ctx.token_seq, dv, False, self.eps, out_scale=self.out_mult)
         return self.o.forward(y, residual=residual, defer_to=ctx)
 
