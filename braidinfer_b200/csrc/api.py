@@ -1475,9 +1475,9 @@ class Kernels:
 
     # Tokens of a step's longest sequence from which on a recurrence with a decay a key channel, or a constant one a head, runs over chunks
     # on the tensor cores (csrc/scan_chunk.cu), for keys of 64 and of 128.  Beside the walk token by token, us: a decay a channel, 8 heads of
-    # 128 x 256 64 tokens 46 / 37, 96 46 / 79, 4 heads of 64 x 128 32 tokens 24 / 23, 64 24 / 37; constant decays 96 tokens 65 / 39, 128
-    # 65 / 69, and 64 28 / 31.
-    SCAN_CHUNK_FROM = {"channel": (48, 80), "constant": (64, 128)}
+    # 128 x 256 64 tokens 44 / 36, 96 44 / 49, 8 x 64 54 / 68; 4 heads of 64 x 128 32 tokens 22 / 23, 64 24 / 37; constant decays 96 tokens
+    # 62 / 39, 128 56 / 69 (which is the walk in chunks), and 64 28 / 31.
+    SCAN_CHUNK_FROM = {"channel": (32, 80), "constant": (64, 128)}
 
     def scan_chunk_fits(self, q, k, v, out, state, state_offset: int, ctx, dk: int, dv: int, mode: str = "channel") -> bool:
         """Whether `linear_scan` in mode "channel" or "constant" takes the form over chunks on the tensor cores, which works decays out of

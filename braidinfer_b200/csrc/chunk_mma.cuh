@@ -13,7 +13,10 @@
 #define CHK_C 64
 #define CHK_SUB 16
 #define CHK_THREADS 256
-#define CHK_SPREAD 8.6736174e-19f          // 2^-60
+// Inside a sub-chunk of 16 the decay from s to t is (start to t) (s to end) / (start to end).  The factors stay normal numbers, and what
+// is lost of the smallest is far below a sum's rounding, while a channel's decays over the sub-chunk multiply to 2^-100 or more; the
+// channels beyond are steep and multiplied up pair by pair.
+#define CHK_SPREAD 7.8886091e-31f          // 2^-100
 #define CHK_PPITCH (CHK_C + 8)
 
 __device__ __forceinline__ bool chk_not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
@@ -60,37 +63,165 @@ __device__ __forceinline__ void chk_store_split4(__nv_bfloat16* at, int part, fl
 // Operands of PA and PB parts: the pairs whose product is not below 2^-16 of the first parts'.
 #define CHK_PAIRS(PA, PB, pa, pb) _Pragma("unroll") for (int pa = 0; pa < PA; ++pa) _Pragma("unroll") for (int pb = 0; pb < PB; ++pb) if (pa + pb <= 2)
 
-// The outputs of 64 tokens x NB value columns by 256 threads: MW warps along the tokens, the others along the columns, 16 columns a warp.
-// The state's numbers go from memory straight into operand registers, each read by MW warps.  V has PV parts (1: bfloat16 numbers as they
-// are); `stage_v(dst, pitch, part)` brings its 64 rows to shared memory.  `store(token, column, x, y)` takes two neighbouring results.
-// With WALK, true for the whole CTA: a number of the state is not finite, or `odd`; nothing was stored.
-template <int DK, int PV, int NB> constexpr int chk_out_smem() {
-    return (3 * CHK_C * (DK + 8) + 3 * CHK_C * CHK_PPITCH + PV * CHK_C * (NB + 8)) * 2;
+// Four neighbouring numbers as float32, one by one where they do not start on 16 (8) bytes.
+__device__ __forceinline__ float4 chk_load4(const float* p, bool wide) {
+    return wide ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
 }
-template <int DK, int PV, int NB, bool WALK, typename StageV, typename Store>
-__device__ __forceinline__ bool chk_outputs(void* smem, const float* __restrict__ gq, const float* __restrict__ gp, const float* __restrict__ S,
-                                            int dv, int col0, bool odd, StageV stage_v, Store store) {
-    constexpr int C = CHK_C, NT = CHK_THREADS, QP = DK + 8, VP = NB + 8;
+// Eight neighbouring bfloat16 numbers as they lie.
+__device__ __forceinline__ uint4 chk_load8(const __nv_bfloat16* p, bool wide) {
+    if (wide) return *reinterpret_cast<const uint4*>(p);
+    const uint16_t* s = reinterpret_cast<const uint16_t*>(p);
+    return make_uint4(s[0] | (uint32_t)s[1] << 16, s[2] | (uint32_t)s[3] << 16, s[4] | (uint32_t)s[5] << 16, s[6] | (uint32_t)s[7] << 16);
+}
+
+// A channel's decays over a sub-chunk, by the thread that owns the two: `d` [16 rows of LD] holds the decays and gets the products from the
+// sub-chunk's start on; `k` is decayed to its end and, where asked for, `f` is k decayed from its start.  True: a steep channel.
+template <int LD, bool FORWARD>
+__device__ __forceinline__ bool chk_decays(float* d, float* k, float* f, float* total, float* inv) {
+    float dec[CHK_SUB], prod = 1.f, after = 1.f;
+#pragma unroll
+    for (int r = 0; r < CHK_SUB; ++r) dec[r] = d[r * LD];
+#pragma unroll
+    for (int r = 0; r < CHK_SUB; ++r) {
+        prod *= dec[r];
+        d[r * LD] = prod;
+        if (FORWARD) f[r * LD] = k[r * LD] * prod;
+    }
+#pragma unroll
+    for (int r = CHK_SUB - 1; r >= 0; --r) {
+        k[r * LD] *= after;
+        after *= dec[r];
+    }
+    const bool steep = !(prod >= CHK_SPREAD && prod <= 1.f / CHK_SPREAD);
+    *total = prod;
+    *inv = steep ? 0.f : 1.f / prod;
+    return steep;
+}
+
+// Products of a block of 16 rows (decayed from their sub-chunk's start) with the keys (decayed to their sub-chunk's end) of the same
+// sub-chunk J and the ones before it: acc[d] for sub-chunk J - d, TILES tiles of 8 keys from tile0 on, in mma.sync's layout; the products of
+// the first parts, and the small ones.  Between two sub-chunks lie the decays of those between; inside one, 1 / all of its decays.
+template <int DK, int LD, int TILES>
+__device__ __forceinline__ void chk_scores(const float* rows, const float* keys, const float* total, const float* inv, int J, int tile0,
+                                           float (*acc)[TILES][2][4]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q2 = (lane & 3) * 2;
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+#pragma unroll
+        for (int x = 0; x < TILES; ++x)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[d][x][e >> 2][e & 3] = 0.f;
+#pragma unroll 1
+    for (int c = q2; c < DK; c += 16) {                      // channels c, c + 1, c + 8, c + 9
+        uint32_t a[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 v = *reinterpret_cast<const float2*>(rows + (g + (e & 1) * 8) * LD + c + (e >> 1) * 8);
+            chk_split2(v.x, v.y, a[0][e], a[1][e], a[2][e]);
+        }
+        float2 f[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            if (d > J) continue;
+            const int I = J - d;
+            if (d > 1) {
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const float2 t = *reinterpret_cast<const float2*>(total + (I + 1) * DK + c + w * 8);
+                    f[w].x *= t.x;
+                    f[w].y *= t.y;
+                }
+            }
+            uint32_t b[TILES][3][2];
+#pragma unroll
+            for (int x = 0; x < TILES; ++x)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    float2 v = *reinterpret_cast<const float2*>(keys + (I * CHK_SUB + (tile0 + x) * 8 + g) * LD + c + w * 8);
+                    const float2 m = d == 0 ? *reinterpret_cast<const float2*>(inv + J * DK + c + w * 8) : f[w];
+                    chk_split2(v.x * m.x, v.y * m.y, b[x][0][w], b[x][1][w], b[x][2][w]);
+                }
+            CHK_PAIRS(3, 3, pa, pb) {
+#pragma unroll
+                for (int x = 0; x < TILES; ++x)
+                    if (pa + pb == 0) chk_mma_sum<true>(acc[d][x], a[pa], b[x][pb][0], b[x][pb][1]);
+                    else chk_mma_sum<false>(acc[d][x], a[pa], b[x][pb][0], b[x][pb][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+#pragma unroll
+        for (int x = 0; x < TILES; ++x)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[d][x][0][e] += acc[d][x][1][e];
+}
+
+// The steep channels' share of the blocks on the diagonal, pair by pair: for every sub-chunk J, `take(J, p, a)` after the sums of q_t k_s and
+// (BOTH) k_t k_s lie in p and a [16][17].  `inv` [4][DK] is 0 for a steep channel of a sub-chunk; `stage`: CHK_STEEP_FLOATS(DK) floats
+// that nobody else needs between the barriers around the call; q, k and decay of (token, channel) come from the caller.
+#define CHK_STEEP_FLOATS(DK) (3 * CHK_SUB * (DK) + 2 * CHK_SUB * 17)
+template <int DK, bool BOTH, typename Q, typename K, typename D, typename Take>
+__device__ __forceinline__ void chk_steep(float* stage, const float* inv, int n, Q q, K k, D decay, Take take) {
+    constexpr int SUB = CHK_SUB;
+    __shared__ uint32_t mask[DK / 32];
+    float *sG = stage, *sK = sG + SUB * DK, *sQ = sK + SUB * DK, *sP = sQ + SUB * DK, *sA = sP + SUB * 17;
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+#pragma unroll 1
+    for (int J = 0; J < 4; ++J) {
+        if (tid < DK) {
+            const uint32_t m = __ballot_sync(0xffffffffu, inv[J * DK + tid] == 0.f);
+            if ((tid & 31) == 0) mask[tid >> 5] = m;
+        }
+#pragma unroll 1
+        for (int idx = tid; idx < SUB * DK; idx += CHK_THREADS) {
+            const int r = idx / DK, i = idx % DK, t = J * SUB + r;
+            const bool in = t < n && inv[J * DK + i] == 0.f;
+            sG[idx] = in ? decay(t, i) : 1.f;
+            sK[idx] = in ? k(t, i) : 0.f;
+            sQ[idx] = in ? q(t, i) : 0.f;
+        }
+        __syncthreads();
+        float p = 0.f, a = 0.f;
+        if (tx <= ty)
+            for (int w = 0; w < DK / 32; ++w)
+                for (uint32_t m = mask[w]; m; m &= m - 1) {
+                    const int i = w * 32 + __ffs(m) - 1;
+                    float x = sK[tx * DK + i];
+                    for (int r = tx + 1; r <= ty; ++r) x *= sG[r * DK + i];
+                    p = fmaf(sQ[ty * DK + i], x, p);
+                    if (BOTH) a = fmaf(sK[ty * DK + i], x, a);
+                }
+        sP[ty * 17 + tx] = p;
+        if (BOTH) sA[ty * 17 + tx] = a;
+        __syncthreads();
+        take(J, sP, sA);
+    }
+    __syncthreads();
+}
+
+// The outputs of 64 tokens x NB value columns by 256 threads: MW warps along the tokens, the others along the columns, 16 columns a warp.
+// The state's numbers go from memory straight into operand registers, each read by MW warps: `fetch(x, ks)` brings, for keys
+// ks * 16 + lq, + 1, + 8, + 9, those of the warp's columns lg (x[0 ..]) and lg + 8 (x[4 ..]), lane = lg * 4 + lq / 2.  `stage(place)` brings
+// what the values need to shared memory, `values(b, ks, place)` their operands of 16 tokens in PV parts.  `store(token, column of the CTA, x, y)`
+// takes two neighbouring results.  With WALK, true for the whole CTA: a number of the state is not finite, or `odd`; nothing was stored.
+template <int DK, int STAGE> constexpr int chk_out_smem() { return (3 * CHK_C * (DK + 8) + 3 * CHK_C * CHK_PPITCH) * 2 + STAGE; }
+template <int NB> __device__ __forceinline__ int chk_out_col() { return (threadIdx.x >> 5) % (NB / 16) * 16; }      // the warp's first column
+template <int DK, int PV, int NB, bool WALK, typename Fetch, typename Stage, typename Values, typename Store>
+__device__ __forceinline__ bool chk_outputs(void* smem, const float* __restrict__ gq, const float* __restrict__ gp, bool odd, Fetch fetch, Stage stage,
+                                            Values values, Store store) {
+    constexpr int C = CHK_C, NT = CHK_THREADS, QP = DK + 8;
     constexpr int CW = NB / 16, MW = 8 / CW, MT = 4 / MW;    // warps along the columns, along the tokens; tiles of 16 tokens a warp
     __nv_bfloat16* sQ = (__nv_bfloat16*)smem;                // 3 x [C][QP]
     __nv_bfloat16* sP = sQ + 3 * C * QP;                     // 3 x [C][CHK_PPITCH]
-    __nv_bfloat16* sV = sP + 3 * C * CHK_PPITCH;             // PV x [C][VP]
+    __nv_bfloat16* place = sP + 3 * C * CHK_PPITCH;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 2, lq = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
     const int cw = warp % CW * 16, mw = warp / CW * MT;
-    const float* sp = S + (size_t)lq * dv + col0 + cw + lg;
     constexpr int AHEAD = 2;
     float sv[AHEAD][8];
-    auto fetch = [&](float* x, int ks) {                     // keys ks * 16 + lq, + 1, + 8, + 9; columns lg and lg + 8
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float* at = sp + (size_t)(ks * 16 + (e & 1) + (e >> 1) * 8) * dv;
-            x[e] = at[0];
-            x[4 + e] = at[8];
-        }
-    };
 #pragma unroll
     for (int ks = 0; ks < AHEAD; ++ks) fetch(sv[ks], ks);
-    stage_v(sV, VP, C * VP);
+    stage(place);
 #pragma unroll 4
     for (int idx = tid * 4; idx < C * DK; idx += NT * 4)
         chk_store_split4(sQ + idx / DK * QP + idx % DK, C * QP, *reinterpret_cast<const float4*>(gq + idx));
@@ -137,8 +268,7 @@ __device__ __forceinline__ bool chk_outputs(void* smem, const float* __restrict_
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
         uint32_t vb[PV][4];
-#pragma unroll
-        for (int p = 0; p < PV; ++p) chk_ldm4t(vb[p], chk_u32(sV + p * C * VP + (ks * 16 + (lm & 1) * 8 + lr) * VP + cw + (lm >> 1) * 8));
+        values(vb, ks, place);
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
             if (ks > mw + m) continue;
@@ -161,7 +291,7 @@ __device__ __forceinline__ bool chk_outputs(void* smem, const float* __restrict_
         for (int e = 0; e < 2; ++e)
 #pragma unroll
             for (int x = 0; x < 2; ++x)
-                store((mw + m) * 16 + lg + e * 8, col0 + cw + lq + x * 8, o[m][x][0][2 * e] + o[m][x][1][2 * e],
+                store((mw + m) * 16 + lg + e * 8, cw + lq + x * 8, o[m][x][0][2 * e] + o[m][x][1][2 * e],
                       o[m][x][0][2 * e + 1] + o[m][x][1][2 * e + 1]);
     return false;
 }

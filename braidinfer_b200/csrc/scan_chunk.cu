@@ -9,8 +9,7 @@
 //   scan_chunk_carry_kernel   the state that every chunk starts from, in U's place
 //   scan_chunk_out_kernel     O of every chunk
 // No logarithm is taken of a decay: what lies between two tokens is a product of decays, which rounds like the walk does.  Sub-chunks of
-// 16 tokens are related through the products at their edges.  Inside one the decay from s to t is (start to t) (s to end) / (start to
-// end) for the channels whose decays over the sub-chunk multiply to 2^-60 or more, and multiplied up pair by pair for the others.
+// 16 tokens are related through the products at their edges, the tokens inside one as chunk_mma.cuh has it.
 //
 // U and O are products on the tensor cores.  q, k and v as projected are bfloat16 numbers and exact there; what is float32 (decayed
 // q and k, P, S_0, anything that went through silu) goes in as the sum of three (chunk_mma.cuh).  A chunk with a number that is not finite
@@ -18,10 +17,10 @@
 //
 // The walk in two passes over chunks of 128 (scan.cu) is bound by shared-memory reads and shuffles: a state element costs a token five
 // instructions and a pass its own staging.  Measured beside it, with its kernel for the decays, L2 flushed, us: a decay a channel, 8 heads of
-// 128 x 256, 2,048 tokens 81 / 277, 1,500 + 1,200 + 900 tokens 153 / 500, 8 x 128 tokens 56 / 181; 16 heads 2,048 tokens 163 / 532; 4
-// heads of 64 x 128 32 / 155.  Constant decays behind silu, 8 heads of 128 x 256, 2,048 tokens 110 / 249; 4 heads of 64 x 128 34 / 91.  Of the
-// 153 the states of the chunks take 70, the carry 22, the outputs 59: float32 sums of P and splits in the first, products of six parts in
-// the last.
+// 128 x 256, 2,048 tokens 79 / 277, 1,500 + 1,200 + 900 tokens 146 / 500, 8 x 128 tokens 56 / 181; 4 heads of 64 x 128 2,048 tokens 32 / 155.
+// Constant decays behind silu, 8 heads of 128 x 256, 2,048 tokens 105 / 249; 4 heads of 64 x 128 34 / 91.  Of the 146 the states of the chunks
+// take 62, the carry 21, the outputs 60: mma.sync takes 8.2 cycles a scheduler, and the outputs 120 of them a warp for 48 KB of operands
+// that are split on the way.  (P by float32 sums, numbers loaded one by one and 32 decays a thread unrolled: 70 us for the states.)
 #include "chunk_mma.cuh"
 
 #define CHK_VB 64                          // value columns a turn of the state kernel
@@ -37,6 +36,7 @@ struct ChunkArgs {
     uint8_t* state; long long state_stride, state_offset;
     const int *q_start, *q_len, *slot_ids;
     int heads, groups, dv, constant, gate_is_decay;
+    int wide_qk, wide_gate;                // rows of q and k, of gate start on 16 bytes
     float q_scale, inv_tau;
     float *u, *qe, *p, *d;                 // blocks a (chunk, head): [dk][dv], [64][dk], [64][64], [dk]
     int* odd;                              // walked token by token
@@ -108,135 +108,121 @@ __device__ __noinline__ void chk_walk(const ChunkArgs& a, int dk, int h, int g, 
 }
 
 template <int DK, bool SILU> constexpr int chk_state_smem() {
-    return (2 * CHK_C * (DK + 4) + 8 * DK + CHK_SUB * (DK + 4)) * 4 + (SILU ? 3 : 2) * CHK_C * CHK_VPITCH * 2;
+    return (2 * CHK_C * (DK + 8) + 8 * DK) * 4 + (SILU ? 3 : 2) * CHK_C * CHK_VPITCH * 2;
 }
 
-// A CTA of eight warps owns a (chunk, head).  A thread takes a channel's decays over one or two sub-chunks; P is a 16 x 16 grid of threads,
-// each one row and column of every 16 x 16 block on or below the diagonal, so that a read of q or k serves up to four blocks; then a warp
-// owns 16 rows of U, its operand (k decayed to the chunk's end) stays in its registers for all value columns.
+// A CTA of eight warps owns a (chunk, head).  Everything is brought to shared memory 16 bytes a load, all loads in flight at once; a thread
+// works a channel's decays out over one or two sub-chunks; P's rows of 16 are shared by two warps each; then a warp owns 16 rows of U, its
+// operand (k decayed to the chunk's end) stays in its registers for all value columns.
 template <int DK, bool SILU>
 __global__ void __launch_bounds__(CHK_THREADS, 2)
 scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
-    constexpr int C = CHK_C, SUB = CHK_SUB, LD = DK + 4, NT = CHK_THREADS;
-    constexpr int SPT = 4 * DK / NT;                         // sub-chunks a thread
+    constexpr int C = CHK_C, SUB = CHK_SUB, LD = DK + 8, NT = CHK_THREADS;
     constexpr int PV = SILU ? 3 : 1;
-    static_assert(SPT == 1 || SPT == 2, "64 or 128 channels");
     extern __shared__ __align__(16) float chk_sm[];
-    float* sQ = chk_sm;                                      // [C][LD]: q decayed from its sub-chunk's start
-    float* sK = sQ + C * LD;                                 // [C][LD]: k decayed to its sub-chunk's end
+    float* sQ = chk_sm;                                      // [C][LD]: decays; then q decayed from its sub-chunk's start
+    float* sK = sQ + C * LD;                                 // [C][LD]: k, then decayed to its sub-chunk's end
     float* sT = sK + C * LD;                                 // [4][DK]: a sub-chunk's decays multiplied
     float* sI = sT + 4 * DK;                                 // [4][DK]: 1 / that, 0 for a steep channel
-    float* sG = sI + 4 * DK;                                 // [SUB][LD]: the decays of one sub-chunk
-    __nv_bfloat16* sV = (__nv_bfloat16*)(sG + SUB * LD);     // two buffers, or one of three parts
+    __nv_bfloat16* sV = (__nv_bfloat16*)(sI + 4 * DK);       // two buffers, or one of three parts
+    static_assert(CHK_STEEP_FLOATS(DK) <= C * LD, "the steep channels are staged where q was");
     const int h = blockIdx.x, seq = blockIdx.y, c = blockIdx.z, tid = threadIdx.x;
     const int n = min(C, a.q_len[seq] - c * C), r0 = a.q_start[seq] + c * C;
     if (n <= 0) return;
     const int g = h / (a.heads / a.groups), dv = a.dv;
     const size_t block = chk_block(a, seq, c, h);
+    const int warp = tid >> 5, lane = tid & 31, lg = lane >> 2, lq = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
     pdl_wait();
     bool bad = false;
-    uint4 vx[2];
+    uint4 vx[2], qx[C * DK / 8 / NT];
+    const int run = tid % (DK / 8) * 8, row8 = tid / (DK / 8);                   // this thread's channels of a row of q and k, its first row
+    const int ch4 = tid % (DK / 4) * 4, row4 = tid / (DK / 4);                   // of decays
+    constexpr int STEP8 = NT * 8 / DK, STEP4 = NT * 4 / DK;
+    {
+        uint4 kx[C * DK / 8 / NT];
+        float4 zx[C * DK / 4 / NT];
 #pragma unroll
-    for (int w = 0; w < 2; ++w) vx[w] = chk_load_v(a, h, r0, n, 0, tid + w * NT);
-    const int ch = tid % DK, j0 = tid / DK * SPT;
+        for (int w = 0; w < C * DK / 4 / NT; ++w) {
+            const int t = row4 + w * STEP4;
+            zx[w] = a.constant || t >= n ? make_float4(0.f, 0.f, 0.f, 0.f) : chk_load4(a.gate + (size_t)(r0 + t) * a.gate_stride + (size_t)h * DK + ch4, a.wide_gate);
+        }
+#pragma unroll
+        for (int w = 0; w < C * DK / 8 / NT; ++w) {
+            const int t = row8 + w * STEP8;
+            kx[w] = t < n ? chk_load8(a.k + (size_t)(r0 + t) * a.k_stride + (size_t)g * DK + run, a.wide_qk) : make_uint4(0, 0, 0, 0);
+            qx[w] = t < n ? chk_load8(a.q + (size_t)(r0 + t) * a.q_stride + (size_t)g * DK + run, a.wide_qk) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int w = 0; w < 2; ++w) vx[w] = chk_load_v(a, h, r0, n, 0, tid + w * NT);
+#pragma unroll
+        for (int w = 0; w < C * DK / 4 / NT; ++w) *reinterpret_cast<float4*>(sQ + (row4 + w * STEP4) * LD + ch4) = zx[w];
+#pragma unroll
+        for (int w = 0; w < C * DK / 8 / NT; ++w) *reinterpret_cast<uint4*>(sK + (row8 + w * STEP8) * LD + run) = kx[w];       // (widened below)
+    }
+    float bias[4] = {0.f, 0.f, 0.f, 0.f};
+    if (!a.constant && !a.gate_is_decay)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bias[e] = to_f32(a.gate_bias[(size_t)h * DK + ch4 + e]);
+#pragma unroll 2
+    for (int t = row4; t < C; t += STEP4) {                  // a loop: its body is the longest code of the kernel
+        float4* at = reinterpret_cast<float4*>(sQ + t * LD + ch4);
+        const float4 v = *at;
+        float d[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (a.constant) d[e] = a.gate[h];
+            else if (!a.gate_is_decay) d[e] = chk_decay_of_logit(d[e] + bias[e], a.inv_tau);
+            if (t >= n) d[e] = 1.f;
+            bad |= chk_not_finite(d[e]);
+        }
+        *at = make_float4(d[0], d[1], d[2], d[3]);
+    }
+    auto widen = [&](uint4 x, float* y) {
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            y[2 * e] = __uint_as_float(w[e] << 16);
+            y[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (SILU) y[e] = silu_f32(y[e]);
+            bad |= chk_not_finite(y[e]);
+        }
+    };
+#pragma unroll 1
+    for (int t = row8; t < C; t += STEP8) {
+        float* at = sK + t * LD + run;
+        float y[8];
+        widen(*reinterpret_cast<const uint4*>(at), y);
+        *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
+        *reinterpret_cast<float4*>(at + 4) = make_float4(y[4], y[5], y[6], y[7]);
+    }
+    __syncthreads();
     bool any_steep = false;
-#pragma unroll
-    for (int j = 0; j < SPT; ++j) {
-        float qq[SUB], kk[SUB], dec[SUB];
-#pragma unroll
-        for (int r = 0; r < SUB; ++r) {
-            const int t = (j0 + j) * SUB + r;
-            const size_t row = (size_t)(r0 + (t < n ? t : 0));
-            dec[r] = a.constant ? a.gate[h] : a.gate[row * a.gate_stride + (size_t)h * DK + ch];
-            qq[r] = to_f32(a.q[row * a.q_stride + (size_t)g * DK + ch]);
-            kk[r] = to_f32(a.k[row * a.k_stride + (size_t)g * DK + ch]);
-        }
-        const float bias = a.constant || a.gate_is_decay ? 0.f : to_f32(a.gate_bias[(size_t)h * DK + ch]);
-        float prod = 1.f;
-#pragma unroll
-        for (int r = 0; r < SUB; ++r) {
-            const int t = (j0 + j) * SUB + r;
-            if (t < n) {
-                if (!a.constant && !a.gate_is_decay) dec[r] = chk_decay_of_logit(dec[r] + bias, a.inv_tau);
-                if (SILU) { qq[r] = silu_f32(qq[r]); kk[r] = silu_f32(kk[r]); }
-                bad |= chk_not_finite(dec[r]) || chk_not_finite(qq[r]) || chk_not_finite(kk[r]);
-            } else {
-                dec[r] = 1.f;
-                qq[r] = kk[r] = 0.f;
-            }
-            prod *= dec[r];
-            sQ[t * LD + ch] = qq[r] * a.q_scale * prod;
-        }
-        const bool steep = !(prod >= CHK_SPREAD && prod <= 1.f / CHK_SPREAD);
-        sT[(j0 + j) * DK + ch] = prod;
-        sI[(j0 + j) * DK + ch] = steep ? 0.f : 1.f / prod;
-        any_steep |= steep;
-        float after = 1.f;
-#pragma unroll
-        for (int r = SUB - 1; r >= 0; --r) {
-            sK[((j0 + j) * SUB + r) * LD + ch] = kk[r] * after;
-            after *= dec[r];
-        }
+#pragma unroll 1
+    for (int w = tid; w < 4 * DK; w += NT) {                 // a (sub-chunk, channel)
+        float *d = sQ + w / DK * SUB * LD + w % DK, *k = sK + w / DK * SUB * LD + w % DK;
+        any_steep |= chk_decays<LD, false>(d, k, nullptr, sT + w, sI + w);
     }
     any_steep = __syncthreads_or(any_steep);
-    const int ty = tid >> 4, tx = tid & 15;
-    float P[4][4];
 #pragma unroll
-    for (int J = 0; J < 4; ++J)
+    for (int w = 0; w < C * DK / 8 / NT; ++w) {
+        float* at = sQ + (row8 + w * STEP8) * LD + run;
+        float y[8], e[8];
+        widen(qx[w], y);
+        *reinterpret_cast<float4*>(e) = *reinterpret_cast<const float4*>(at);
+        *reinterpret_cast<float4*>(e + 4) = *reinterpret_cast<const float4*>(at + 4);
 #pragma unroll
-        for (int I = 0; I < 4; ++I) P[J][I] = 0.f;
-#pragma unroll 2
-    for (int i = 0; i < DK; i += 4) {
-        float kb[4][4], t1[4], t2[4];
-#pragma unroll
-        for (int I = 0; I < 4; ++I) *reinterpret_cast<float4*>(kb[I]) = *reinterpret_cast<const float4*>(sK + (I * SUB + tx) * LD + i);
-        *reinterpret_cast<float4*>(t1) = *reinterpret_cast<const float4*>(sT + DK + i);
-        *reinterpret_cast<float4*>(t2) = *reinterpret_cast<const float4*>(sT + 2 * DK + i);
-#pragma unroll
-        for (int J = 0; J < 4; ++J) {
-            float qa[4], inv[4];
-            *reinterpret_cast<float4*>(qa) = *reinterpret_cast<const float4*>(sQ + (J * SUB + ty) * LD + i);
-            *reinterpret_cast<float4*>(inv) = *reinterpret_cast<const float4*>(sI + J * DK + i);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                P[J][J] = fmaf(qa[e] * inv[e], kb[J][e], P[J][J]);
-                float x = qa[e];
-#pragma unroll
-                for (int I = J - 1; I >= 0; --I) {           // through the sub-chunks between the two
-                    P[J][I] = fmaf(x, kb[I][e], P[J][I]);
-                    x *= I == 2 ? t2[e] : t1[e];
-                }
-            }
-        }
+        for (int x = 0; x < 8; ++x) y[x] *= a.q_scale * e[x];
+        *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
+        *reinterpret_cast<float4*>(at + 4) = make_float4(y[4], y[5], y[6], y[7]);
     }
-    if (any_steep) {                                       // the steep channels, pair by pair
-#pragma unroll 1
-        for (int J = 0; J < 4; ++J) {
-            __syncthreads();
-            for (int idx = tid; idx < SUB * DK; idx += NT) {
-                const int r = idx / DK, i = idx % DK;
-                sG[r * LD + i] = J * SUB + r < n ? chk_decay(a, DK, h, (size_t)(r0 + J * SUB + r), i) : 1.f;
-            }
-            __syncthreads();
-            const int t = J * SUB + ty, s = J * SUB + tx;
-            float acc = 0.f;
-            if (tx <= ty && t < n)
-                for (int i = 0; i < DK; ++i)
-                    if (sI[J * DK + i] == 0.f) {
-                        float x = chk_in<SILU>(a.k[(size_t)(r0 + s) * a.k_stride + (size_t)g * DK + i]);
-                        for (int r = tx + 1; r <= ty; ++r) x *= sG[r * LD + i];
-                        acc = fmaf(chk_in<SILU>(a.q[(size_t)(r0 + t) * a.q_stride + (size_t)g * DK + i]) * a.q_scale, x, acc);
-                    }
-#pragma unroll
-            for (int K = 0; K < 4; ++K)
-                if (K == J) P[K][K] += acc;
-        }
-    }
-    float* gP = a.p + block * (C * C);
-#pragma unroll
-    for (int J = 0; J < 4; ++J)
-#pragma unroll
-        for (int I = 0; I <= J; ++I) gP[(J * SUB + ty) * C + I * SUB + tx] = I < J || tx <= ty ? P[J][I] : 0.f;
+    __syncthreads();
+    // the rows of 16 by two warps each, 8 keys of every sub-chunk a warp; rows with more sub-chunks share a scheduler with ones of fewer
+    const int J = warp < 4 ? warp : 7 - warp, tile = warp >> 2;
+    float P[4][1][2][4];
+    chk_scores<DK, LD, 1>(sQ + J * SUB * LD, sK, sT, sI, J, tile, P);
     float* gQ = a.qe + block * (C * DK);
 #pragma unroll 4
     for (int idx = tid * 4; idx < C * DK; idx += NT * 4) {   // q decayed from the chunk's start
@@ -248,9 +234,30 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
             for (int e = 0; e < 4; ++e) x[e] *= sT[m * DK + i + e];
         *reinterpret_cast<float4*>(gQ + idx) = make_float4(x[0], x[1], x[2], x[3]);
     }
+    if (any_steep) {
+        __syncthreads();                                     // q has been used
+        chk_steep<DK, false>(sQ, sI, n, [&](int t, int i) { return chk_in<SILU>(a.q[(size_t)(r0 + t) * a.q_stride + (size_t)g * DK + i]) * a.q_scale; },
+                             [&](int t, int i) { return chk_in<SILU>(a.k[(size_t)(r0 + t) * a.k_stride + (size_t)g * DK + i]); },
+                             [&](int t, int i) { return chk_decay(a, DK, h, (size_t)(r0 + t), i); },
+                             [&](int sub, const float* p, const float*) {
+                                 if (sub == J)
+#pragma unroll
+                                     for (int e = 0; e < 4; ++e) P[0][0][0][e] += p[(lg + (e >> 1) * 8) * 17 + tile * 8 + lq + (e & 1)];
+                             });
+    }
+    float* gP = a.p + block * (C * C);
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+        if (d <= J)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int t = lg + e * 8, s = tile * 8 + lq;
+                float x = P[d][0][0][2 * e], y = P[d][0][0][2 * e + 1];
+                if (d == 0) { x = s <= t ? x : 0.f; y = s + 1 <= t ? y : 0.f; }      // later tokens are left out, whatever their products are
+                *reinterpret_cast<float2*>(gP + (J * SUB + t) * C + (J - d) * SUB + s) = make_float2(x, y);
+            }
     if (tid < DK) a.d[block * DK + tid] = sT[tid] * sT[DK + tid] * sT[2 * DK + tid] * sT[3 * DK + tid];
     // U: the warp's 16 rows, k decayed to the chunk's end in three parts
-    const int warp = tid >> 5, lane = tid & 31, lg = lane >> 2, lq = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
     constexpr int MT = DK / 16, NW = 8 / MT, TILES = CHK_VB / 8 / NW;      // warps that share 16 rows, tiles of 8 columns a warp
     const int m0 = warp % MT * 16, t0 = warp / MT * TILES;
     uint32_t ka[4][3][4];
@@ -371,17 +378,32 @@ scan_chunk_out_kernel(const __grid_constant__ ChunkArgs a) {
     const size_t block = chk_block(a, seq, c, h);
     pdl_wait();
     float* S = a.u + block * ((size_t)DK * a.dv);
+    constexpr int VP = NB + 8;
+    const int lane = tid & 31, lr = lane & 7, lm = lane >> 3, cw = chk_out_col<NB>();
+    const float* sp = S + (size_t)((lane & 3) * 2) * a.dv + col0 + cw + (lane >> 2);
     const bool odd = chk_outputs<DK, SILU ? 3 : 1, NB, true>(
-        chk_sm, a.qe + block * (C * DK), a.p + block * (C * C), S, a.dv, col0, a.odd[block] != 0,
-        [&](__nv_bfloat16* dst, int pitch, int part) {
+        chk_sm, a.qe + block * (C * DK), a.p + block * (C * C), a.odd[block] != 0,
+        [&](float* x, int ks) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* at = sp + (size_t)(ks * 16 + (e & 1) + (e >> 1) * 8) * a.dv;
+                x[e] = at[0];
+                x[4 + e] = at[8];
+            }
+        },
+        [&](__nv_bfloat16* v) {
 #pragma unroll
             for (int w = 0; w < NB / 32; ++w) {
                 const int idx = tid + (w & 1) * NT, b = (w >> 1) * 64;
-                chk_store_v<SILU>(dst + b, pitch, part, chk_load_v(a, h, r0, n, col0 + b, idx), idx);
+                chk_store_v<SILU>(v + b, VP, C * VP, chk_load_v(a, h, r0, n, col0 + b, idx), idx);
             }
         },
+        [&](uint32_t (*b)[4], int ks, const __nv_bfloat16* v) {
+#pragma unroll
+            for (int p = 0; p < (SILU ? 3 : 1); ++p) chk_ldm4t(b[p], chk_u32(v + p * C * VP + (ks * 16 + (lm & 1) * 8 + lr) * VP + cw + (lm >> 1) * 8));
+        },
         [&](int t, int col, float x, float y) {
-            if (t < n) *reinterpret_cast<float2*>(a.out + (size_t)(r0 + t) * a.out_stride + (size_t)h * a.dv + col) = make_float2(x, y);
+            if (t < n) *reinterpret_cast<float2*>(a.out + (size_t)(r0 + t) * a.out_stride + (size_t)h * a.dv + col0 + col) = make_float2(x, y);
         });
     if (odd) chk_walk<SILU, true>(a, DK, h, h / (a.heads / a.groups), r0, n, S, col0, NB);
 }
@@ -398,13 +420,13 @@ static int launch_scan_chunk(const ChunkArgs& a, int n_seqs, int chunks, cudaStr
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(scan_chunk_state_kernel<DK, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, chk_state_smem<DK, SILU>());
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(scan_chunk_out_kernel<DK, SILU, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (chk_out_smem<DK, SILU ? 3 : 1, NB>()));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(scan_chunk_out_kernel<DK, SILU, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (chk_out_smem<DK, (SILU ? 3 : 1) * CHK_C * (NB + 8) * 2>()));
         if (e != cudaSuccess) { braid_set_error("scan_chunk: cannot reserve shared memory: %s", cudaGetErrorString(e)); return (int)e; }
         configured = true;
     }
     braid_launch(scan_chunk_state_kernel<DK, SILU>, dim3(a.heads, n_seqs, chunks), dim3(CHK_THREADS), (size_t)chk_state_smem<DK, SILU>(), s, a);
     braid_launch(scan_chunk_carry_kernel<DK>, dim3((unsigned)(((long long)a.heads * DK * a.dv / 4 + 255) / 256), n_seqs), dim3(256), 0, s, a);
-    braid_launch(scan_chunk_out_kernel<DK, SILU, NB>, dim3(a.heads, n_seqs, chunks * (a.dv / NB)), dim3(CHK_THREADS), (size_t)(chk_out_smem<DK, SILU ? 3 : 1, NB>()), s, a);
+    braid_launch(scan_chunk_out_kernel<DK, SILU, NB>, dim3(a.heads, n_seqs, chunks * (a.dv / NB)), dim3(CHK_THREADS), (size_t)(chk_out_smem<DK, (SILU ? 3 : 1) * CHK_C * (NB + 8) * 2>()), s, a);
     BRAID_LAUNCH_CHECK();
 }
 
@@ -430,7 +452,8 @@ extern "C" int braid_scan_chunk(const void* q, long long q_stride, const void* k
     const long long blocks = chk_blocks(rows, n_seqs, heads);
     using B = const __nv_bfloat16*;
     ChunkArgs a{(B)q, (B)k, (B)v, q_stride, k_stride, v_stride, gate, gate_stride, (B)gate_bias, out, out_stride, (uint8_t*)state,
-                state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dv, constant, gate_is_decay, q_scale, inv_tau};
+                state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dv, constant, gate_is_decay,
+                (((uintptr_t)q | (uintptr_t)k) & 15) == 0 && q_stride % 8 == 0 && k_stride % 8 == 0, ((uintptr_t)gate & 15) == 0 && gate_stride % 4 == 0, q_scale, inv_tau};
     a.u = work;
     a.qe = a.u + blocks * dk * dv;
     a.p = a.qe + blocks * CHK_C * dk;
