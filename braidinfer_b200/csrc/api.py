@@ -1420,18 +1420,16 @@ class Kernels:
         """Whether a step of `rows` rows whose longest sequence brings `longest` should walk its chunks of 64 one after the other on
         the tensor cores, a CTA a (head, sequence, 64 value columns), instead of side by side on the FMA pipes (csrc/scan.cu).
 
-        The serial form takes 8 us a chunk with keys of 128, 6.3 with keys of 64, however few CTAs there are, up to two an SM; the
+        The serial form takes 7.6 us a chunk with keys of 128, 5.2 with keys of 64, however few CTAs there are, up to two an SM; the
         other one's time grows with the number of chunks of all heads.  So with CTAs for less than 64 heads' worth of the longest
-        sequence the line is a length that grows with them.  us, serial / side by side, keys of 128 x 64: 4 heads 256 tokens 41 / 44,
-        700 95 / 45; 8 heads 300 tokens 47 / 51, 700 95 / 57, 2,048 259 / 129; 16 heads 300 48 / 73, 700 95 / 91, 2,048 260 / 172;
-        32 heads 1,024 134 / 173, 2,048 260 / 256, 8,192 1,013 / 926; 64 heads 300 49 / 107, 2,048 262 / 477, 8,192 1,022 / 1,849.  Keys of
-        64 x 64: 8 heads 300 38 / 47, 700 75 / 48; 16 heads 300 38 / 53, 700 75 / 57; 32 heads 700 76 / 84, 1,023 106 / 89,
-        2,048 204 / 158; 64 heads 2,048 205 / 250, 8,192 793 / 856.  A prompt of 2,048 beside three of 64 counts as one of 2,048:
-        16 heads of 128 x 64 260 / 190, 64 heads 269 / 556."""
+        sequence the line is a length that grows with them.  us, serial / side by side, keys of 128 x 64: 8 heads 300 tokens 45 / 50,
+        700 90 / 56, 2,048 243 / 130; 16 heads 300 45 / 73, 700 90 / 91, 2,048 242 / 171; 64 heads 300 47 / 107, 2,048 256 / 478.  Keys of
+        64 x 64: 8 heads 300 33 / 48, 700 64 / 48, 2,048 166 / 85; 32 heads 300 33 / 69, 700 64 / 85, 2,048 170 / 157.  A prompt of 2,048
+        beside three of 64 counts as one of 2,048."""
         if longest < cls.SSD_FROM:
             return False
         ctas = heads * (dv // 64) * rows / longest
-        return ctas >= 64 or longest <= (max(256, 40 * ctas) if dk == 128 else max(384, 25 * ctas))
+        return ctas >= 64 or longest <= max(256 if dk == 128 else 384, 40 * ctas)
 
     def _ssd_fits(self, q, k, v, out, state, state_offset: int, ctx, heads: int, dk: int, dv: int, v_cols: int) -> bool:
         return (SCAN_CHUNK is None and q.dtype == torch.bfloat16 and dk in (64, 128) and dv % 64 == 0 and v_cols == dv

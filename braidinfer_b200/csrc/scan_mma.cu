@@ -12,16 +12,17 @@
 // differences of logarithms.  A token's numbers never reach the tokens before it, be they infinite: the block on the diagonal
 // selects the later tokens away instead of multiplying them by zero.
 //
-// A CTA of four warps owns (head, sequence, 64 value columns) and walks the sequence's chunks, the state in its accumulator
-// registers (a warp a quarter of the key rows); a warp owns 16 tokens of a chunk's output, and its P goes from the accumulators of
-// Q K^T straight into the operands of P V.  Two CTAs an SM (108 KB of shared memory at dk 128).  The walk token by token in two
-// passes over chunks (scan.cu) is bound by shared-memory reads and shuffles.  Measured beside it, us, heads of 128 x 64:
-// 64 heads, 2,048 tokens 262 beside 478, 1,500 + 1,200 + 900 tokens 232 / 842, 8 x 64 tokens 36 / 97, 4 x 24 tokens 22 / 35; 128 heads,
-// 2,048 tokens 267 / 929.  32 heads of 64 x 64: 3 sequences 156 / 244, 300 tokens 38 / 68.  A long prompt on few CTAs is a
-// chain that leaves the machine idle (8 us a chunk; 8 heads of 128 x 64, 2,048 tokens: 259 us beside 129): such steps stay with
+// A CTA of four warps owns (head, sequence, 64 value columns) and walks the sequence's chunks.  A warp owns 16 value columns and keeps their
+// transposed state in its accumulators, which are the operand of S^T Q^T as they are: the state never passes through shared memory.
+// P is worked out by rows of 16 tokens a warp and shared as three parts.  The next chunk is on its way while one is worked on (two
+// buffers); two CTAs an SM (112 KB of shared memory at dk 128).  Bound by mma.sync: some 500 a warp and chunk at 11 to 16 cycles each with one
+// warp a scheduler, 12,300 cycles a chunk with the splits between them.  us beside the form before, whose state went to shared memory in
+// parts for every chunk, / the walk token by token in two passes over chunks (scan.cu), heads of 128 x 64: 64 heads, 2,048 tokens
+// 256 / 262 / 478, 1,500 + 1,200 + 900 tokens 219 / 232 / 842, 64 tokens 16.5 / 22 / 31; 128 heads, 2,048 tokens 268 / 267 / 929.  32 heads of
+// 64 x 64: 3 sequences 135 / 156 / 244, 300 tokens 33 / 38 / 68.  A long prompt on few CTAs is a
+// chain that leaves the machine idle (8 heads of 128 x 64, 2,048 tokens: 243 us beside 130): such steps stay with
 // the walk whose chunks run side by side, by `ssd_pays` (api.py), which holds both forms' times.
-#include "common.cuh"
-#include <type_traits>
+#include "chunk_mma.cuh"
 
 #define SSD_C 64
 #define SSD_P 64
@@ -37,35 +38,9 @@ struct SsdArgs {
     float q_scale;
 };
 
-__device__ __forceinline__ uint32_t ssd_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ssd_ldm4(uint32_t* r, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ssd_ldm4t(uint32_t* r, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ssd_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // 16 bytes to shared memory, or zeros
-__device__ __forceinline__ void ssd_copy16(void* dst, const void* src, bool in) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ssd_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-// x = the sum of three bfloat16 numbers to float32's 24 bits; two x at once, packed.  The first two saturate, so that a number past the
-// largest bfloat16 one is still a sum of finite parts; an infinity is left over for the third.
-__device__ __forceinline__ void ssd_split2(float x0, float x1, uint32_t* w) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        if (i < 2) {
-            asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w[i]) : "f"(x1), "f"(x0));
-        } else {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        x0 -= __uint_as_float(w[i] << 16);
-        x1 -= __uint_as_float(w[i] & 0xffff0000u);
-    }
+__device__ __forceinline__ void ssd_copy16(uint32_t dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
 }
 // two bfloat16 numbers, those that are not finite replaced by zero
 __device__ __forceinline__ uint32_t ssd_finite(uint32_t w) {
@@ -76,114 +51,113 @@ __device__ __forceinline__ uint32_t ssd_finite(uint32_t w) {
 template <int RUNS>
 __device__ __forceinline__ uint32_t ssd_at(int r, int c) { return (uint32_t)(r * RUNS + (c ^ (r & 7))) * 16; }
 
+// A token's numbers of the chunk
+struct SsdToken {
+    float head;                  // its decay and those before it in its block of 16, multiplied
+    float tail;                  // those after it in its block, times its step
+    float start;                 // D(0, t) q_scale
+    float end;                   // dt_t D(t, 64)
+};
 template <int DK> constexpr int ssd_smem() {
-    return SSD_C * DK * 2 * 2 + SSD_C * SSD_P * 2 + SSD_C * (SSD_C + 1) * 4 + 3 * DK * SSD_P * 2 + 4 * SSD_C * 4 + SSD_C / 16 * 4;
+    return 2 * (2 * SSD_C * DK * 2 + SSD_C * SSD_P * 2) + 3 * SSD_C * SSD_C * 2 + SSD_C * 17 * 4 + SSD_C * 16 + 8 * 4;
 }
 
 template <int DK>
 __global__ void __launch_bounds__(SSD_THREADS, 2)
-ssd_chunk_kernel(SsdArgs a) {
-    constexpr int C = SSD_C, P = SSD_P, QR = DK / 8, MT = DK / 64;      // MT: 16-row tiles of the state a warp
-    extern __shared__ __align__(16) uint8_t ssd_sm[];
-    uint8_t* sQ = ssd_sm;                                    // [C][DK] bf16; from the state update on, with sD: the weighted values, 3 x [C][P]
-    uint8_t* sD_ = sQ + C * DK * 2;
-    float* sD = (float*)sD_;                                 // [t][s], rows of C + 1: dt_s D(s, t)
-    uint8_t* sK = sD_ + C * (C + 1) * 4;                     // [C][DK]
-    uint8_t* sV = sK + C * DK * 2;                           // [C][P]
-    uint8_t* sS = sV + C * P * 2;                            // 3 x [DK][P]: the state the chunk starts from
-    float* s_a = (float*)(sS + 3 * DK * P * 2);              // decays
-    float* s_dt = s_a + C;
-    float* s_d0 = s_dt + C;                                  // D(0, t)
-    float* s_w = s_d0 + C;                                   // dt_t D(t, 64)
-    int* s_odd = (int*)(s_w + C);                            // [C / 16]
-    uint8_t* sW = sQ;
-    static_assert(3 * C * P * 2 <= C * DK * 2 + C * (C + 1) * 4, "the weighted values fit where q and the decays were");
+ssd_chunk_kernel(const __grid_constant__ SsdArgs a) {
+    constexpr int C = SSD_C, P = SSD_P, QR = DK / 8, KT = DK / 8, QB = C * DK * 2, VB = C * P * 2, PB = C * C * 2;
+    extern __shared__ __align__(128) uint8_t ssd_sm[];
+    const uint32_t sQ = chk_u32(ssd_sm), sK = sQ + 2 * QB, sV = sK + 2 * QB, sP = sV + 2 * VB;      // q, k, v: two buffers; P: three parts
+    float* sD = (float*)(ssd_sm + 4 * QB + 2 * VB + 3 * PB);     // [t][17]: dt_s D(s, t), s in t's block of 16
+    SsdToken* tok = (SsdToken*)(sD + C * 17);                // [C]
+    float* s_block = (float*)(tok + C);                      // [4]: a block's decays multiplied
+    int* s_odd = (int*)(s_block + 4);                        // [4]: values that are not finite
     pdl_trigger();
     const int h = blockIdx.x, seq = blockIdx.y, j0 = blockIdx.z * P, tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q2 = (lane & 3) * 2;
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q2 = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
     const int n = a.q_len[seq], r0 = a.q_start[seq];
     if (n <= 0) return;
-    const int grp = h / (a.heads / a.groups);
+    const int grp = h / (a.heads / a.groups), cw = warp * 16;
     const float head_a = -expf(to_f32(a.a_log[h])), head_bias = to_f32(a.gate_bias[h]), skip = a.skip ? to_f32(a.skip[h]) : 0.f;
-    float* S_area = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + j0;
+    float* S_area = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + j0 + cw + g;
+    float S[KT][4];                                          // S^T: value columns cw + g (+ 8), keys x * 8 + q2 (+ 1)
+#pragma unroll
+    for (int x = 0; x < KT; ++x)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[x][e] = S_area[(size_t)(x * 8 + q2 + (e & 1)) * a.dv + (e >> 1) * 8];
     pdl_wait();
-    const int i0 = warp * (DK / 4);                          // this warp's rows of the state
-    float S[MT][8][4];
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float2 v = *reinterpret_cast<const float2*>(S_area + (size_t)(i0 + m * 16 + g + e * 8) * a.dv + t * 8 + q2);
-                S[m][t][2 * e] = v.x;
-                S[m][t][2 * e + 1] = v.y;
-            }
-    for (int t0 = 0; t0 < n; t0 += C) {
+    auto ask = [&](int t0, int buf) {                        // the tokens from t0 on, zeros past the sequence
         const int nt = min(C, n - t0);
-        // everything of the chunk asked for at once; it arrives under the split of the state
-#pragma unroll
+#pragma unroll 4
         for (int i = tid; i < C * QR; i += SSD_THREADS) {
             const int r = i / QR, c = i % QR;
             const bool in = r < nt;
             const size_t row = (size_t)(r0 + t0 + (in ? r : 0));
-            ssd_copy16(sQ + ssd_at<QR>(r, c), a.q + row * a.q_stride + (size_t)grp * DK + c * 8, in);
-            ssd_copy16(sK + ssd_at<QR>(r, c), a.k + row * a.k_stride + (size_t)grp * DK + c * 8, in);
+            ssd_copy16(sQ + buf * QB + ssd_at<QR>(r, c), a.q + row * a.q_stride + (size_t)grp * DK + c * 8, in);
+            ssd_copy16(sK + buf * QB + ssd_at<QR>(r, c), a.k + row * a.k_stride + (size_t)grp * DK + c * 8, in);
         }
 #pragma unroll
         for (int i = tid; i < C * 8; i += SSD_THREADS) {
             const int r = i / 8, c = i % 8;
             const bool in = r < nt;
-            ssd_copy16(sV + ssd_at<8>(r, c), a.v + (size_t)(r0 + t0 + (in ? r : 0)) * a.v_stride + (size_t)h * a.dv + j0 + c * 8, in);
+            ssd_copy16(sV + buf * VB + ssd_at<8>(r, c), a.v + (size_t)(r0 + t0 + (in ? r : 0)) * a.v_stride + (size_t)h * a.dv + j0 + c * 8, in);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (tid < C) {                                       // tokens past the end: no decay, no step
+    };
+    auto gate_of = [&](int t) { return tid < C && t < n ? to_f32(a.gate[(size_t)(r0 + t) * a.gate_stride + h]) : 0.f; };
+    ask(0, 0);
+    float z = gate_of(tid);
+    for (int t0 = 0, buf = 0; t0 < n; t0 += C, buf ^= 1) {
+        const int nt = min(C, n - t0);
+        const uint32_t q = sQ + buf * QB, k = sK + buf * QB, v = sV + buf * VB;
+        const uint8_t* v_bytes = ssd_sm + 4 * QB + buf * VB;
+        if (tid < C) {                                       // a thread a token; past the end: no decay, no step
             float dt = 0.f, dec = 1.f;
             if (tid < nt) {
-                const float x = to_f32(a.gate[(size_t)(r0 + t0 + tid) * a.gate_stride + h]) + head_bias;
+                const float x = z + head_bias;
                 dt = x > 20.f ? x : log1pf(expf(x));
                 dec = expf(head_a * dt);
             }
-            s_dt[tid] = dt;
-            s_a[tid] = dec;
-        }
-        // the state in three parts
+            const int l = lane & 15;
+            float run = dt, pre = dec, suf = dec;
+            sD[tid * 17 + l] = run;
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-            for (int t = 0; t < 8; ++t)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    uint32_t w[3];
-                    ssd_split2(S[m][t][2 * e], S[m][t][2 * e + 1], w);
-                    const int r = i0 + m * 16 + g + e * 8;
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(sS + p * DK * P * 2 + ssd_at<8>(r, t) + q2 * 2) = w[p];
+            for (int r = 1; r < 16; ++r) {                   // down the tokens of the block
+                const float d = __shfl_down_sync(0xffffffffu, dec, r, 16);
+                if (l + r < 16) {
+                    run *= d;
+                    sD[(tid + r) * 17 + l] = run;
                 }
+            }
+#pragma unroll
+            for (int r = 1; r < 16; r <<= 1) {
+                const float x = __shfl_up_sync(0xffffffffu, pre, r, 16), y = __shfl_down_sync(0xffffffffu, suf, r, 16);
+                if (l >= r) pre *= x;
+                if (l + r < 16) suf *= y;
+            }
+            const float after = __shfl_down_sync(0xffffffffu, suf, 1, 16);
+            tok[tid].head = pre;
+            tok[tid].tail = l < 15 ? dt * after : dt;
+            if (l == 15) s_block[tid >> 4] = pre;
+        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        if (tid < C) {                                       // a thread a column s: products down the tokens
-            float run = s_dt[tid];
-#pragma unroll 8
-            for (int t = 0; t < C; ++t) {
-                if (t > tid) run *= s_a[t];
-                sD[t * (C + 1) + tid] = t < tid ? 0.f : run;
-            }
-            s_w[tid] = run;
-        } else if (tid == C) {
-            float run = 1.f;
-#pragma unroll 8
-            for (int t = 0; t < C; ++t) {
-                run *= s_a[t];
-                s_d0[t] = run;
-            }
-        } else if (warp == 3) {                              // meanwhile: which blocks of 16 tokens hold values that are not finite
+        __syncthreads();                                     // the chunk is there; the one before has been read
+        if (t0 + C < n) {
+            ask(t0 + C, buf ^ 1);
+            z = gate_of(t0 + C + tid);
+        }
+        const float b0 = s_block[0], b1 = s_block[1], b2 = s_block[2], b3 = s_block[3], all = b0 * b1 * b2 * b3;
+        if (tid < C) {
+            const int b = tid >> 4;
+            tok[tid].start = tok[tid].head * (b == 0 ? 1.f : b == 1 ? b0 : b == 2 ? b0 * b1 : b0 * b1 * b2) * a.q_scale;
+            tok[tid].end = tok[tid].tail * (b == 3 ? 1.f : b == 2 ? b3 : b == 1 ? b2 * b3 : b1 * b2 * b3);
+        } else if (warp == 3) {                              // which blocks of 16 tokens hold values that are not finite
 #pragma unroll
             for (int b = 0; b < C / 16; ++b) {
                 uint32_t top = 0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint4 u = *reinterpret_cast<const uint4*>(sV + (b * 128 + i * 32 + lane) * 16);
+                    const uint4 u = *reinterpret_cast<const uint4*>(v_bytes + (b * 128 + i * 32 + lane) * 16);
                     top |= ((u.x & 0x7f807f80u) + 0x00800080u) | ((u.y & 0x7f807f80u) + 0x00800080u) |
                            ((u.z & 0x7f807f80u) + 0x00800080u) | ((u.w & 0x7f807f80u) + 0x00800080u);
                 }
@@ -191,160 +165,185 @@ ssd_chunk_kernel(SsdArgs a) {
                 if (lane == 0) s_odd[b] = any;
             }
         }
-        // Q K^T, the warp's 16 tokens against the tokens up to them
-        const int tw = warp * 16;
-        float o[8][4], qk[8][4];
+        {                                                    // P: the warp's 16 tokens against the tokens up to them
+            float qk[8][4];
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
+            for (int x = 0; x < 8; ++x)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { o[t][e] = 0.f; qk[t][e] = 0.f; }
-        const int lr = lane & 7, lm = lane >> 3;             // row and matrix of this lane's address in an ldmatrix of four
+                for (int e = 0; e < 4; ++e) qk[x][e] = 0.f;
 #pragma unroll
-        for (int ks = 0; ks < DK / 16; ++ks) {
-            uint32_t qa[4];
-            ssd_ldm4(qa, ssd_u32(sQ) + ssd_at<QR>(tw + (lm & 1) * 8 + lr, ks * 2 + (lm >> 1)));
+            for (int ks = 0; ks < DK / 16; ++ks) {
+                uint32_t qa[4];
+                chk_ldm4(qa, q + ssd_at<QR>(cw + (lm & 1) * 8 + lr, ks * 2 + (lm >> 1)));
 #pragma unroll
-            for (int pr = 0; pr < 4; ++pr)                   // 16 tokens s at a time
-                if (pr <= warp) {
-                    uint32_t kb[4];
-                    ssd_ldm4(kb, ssd_u32(sK) + ssd_at<QR>(pr * 16 + (lm >> 1) * 8 + lr, ks * 2 + (lm & 1)));
-                    ssd_mma(qk[2 * pr], qa, kb[0], kb[1]);
-                    ssd_mma(qk[2 * pr + 1], qa, kb[2], kb[3]);
+                for (int pr = 0; pr < 4; ++pr)
+                    if (pr <= warp) {
+                        uint32_t kb[4];
+                        chk_ldm4(kb, k + ssd_at<QR>(pr * 16 + (lm >> 1) * 8 + lr, ks * 2 + (lm & 1)));
+                        chk_mma(qk[2 * pr], qa, kb[0], kb[1]);
+                        chk_mma(qk[2 * pr + 1], qa, kb[2], kb[3]);
+                    }
+            }
+            const float h0 = tok[cw + g].head * a.q_scale, h1 = tok[cw + g + 8].head * a.q_scale;
+            float between = 1.f;
+#pragma unroll
+            for (int pr = 3; pr >= 0; --pr) {                // blocks of tokens s, from the warp's own back
+                if (pr > warp) continue;
+                if (pr < warp - 1) between *= pr == 0 ? b1 : b2;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int s = half * 8 + q2;
+                    float* x = qk[2 * pr + half];
+                    if (pr == warp) {                        // tokens after this one are left out, whatever their products are
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int t = g + (e >> 1) * 8;
+                            x[e] = s + (e & 1) <= t ? x[e] * (sD[(cw + t) * 17 + s + (e & 1)] * a.q_scale) : 0.f;
+                        }
+                    } else {
+                        const float f0 = tok[pr * 16 + s].tail * between, f1 = tok[pr * 16 + s + 1].tail * between;
+                        x[0] *= f0 * h0; x[1] *= f1 * h0; x[2] *= f0 * h1; x[3] *= f1 * h1;
+                    }
+                    uint32_t lo[3], hi[3];
+                    chk_split2(x[0], x[1], lo[0], lo[1], lo[2]);
+                    chk_split2(x[2], x[3], hi[0], hi[1], hi[2]);
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(sP + p * PB + ssd_at<8>(cw + g, pr * 2 + half) + q2 * 2), "r"(lo[p]) : "memory");
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(sP + p * PB + ssd_at<8>(cw + g + 8, pr * 2 + half) + q2 * 2), "r"(hi[p]) : "memory");
+                    }
                 }
-            // and Q S_0: the state's key rows ks * 16 ...
+            }
+        }
+        float o[8][2][4];                                    // O^T, value columns cw + g (+ 8), tokens x * 8 + q2 (+ 1)
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[x][e >> 2][e & 3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < DK / 16; ++ks) {               // S^T Q^T
+            uint32_t sa[3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float* s = S[2 * ks + (e >> 1)] + (e & 1) * 2;
+                chk_split2(s[0], s[1], sa[0][e], sa[1][e], sa[2][e]);
+            }
+            uint32_t qb[4][4];
+#pragma unroll
+            for (int pr = 0; pr < 4; ++pr) chk_ldm4(qb[pr], q + ssd_at<QR>(pr * 16 + (lm >> 1) * 8 + lr, ks * 2 + (lm & 1)));
 #pragma unroll
             for (int p = 0; p < 3; ++p)
 #pragma unroll
-                for (int pr = 0; pr < 4; ++pr) {
-                    uint32_t sb[4];
-                    ssd_ldm4t(sb, ssd_u32(sS) + p * DK * P * 2 + ssd_at<8>(ks * 16 + (lm & 1) * 8 + lr, pr * 2 + (lm >> 1)));
-                    ssd_mma(o[2 * pr], qa, sb[0], sb[1]);
-                    ssd_mma(o[2 * pr + 1], qa, sb[2], sb[3]);
+                for (int x = 0; x < 8; ++x) {
+                    const uint32_t* b = qb[x >> 1] + (x & 1) * 2;
+                    if (p == 0) chk_mma_sum<true>(o[x], sa[p], b[0], b[1]);
+                    else chk_mma_sum<false>(o[x], sa[p], b[0], b[1]);
                 }
         }
-        __syncthreads();                                     // the decays are there
-        const float d0 = s_d0[tw + g], d1 = s_d0[tw + g + 8];
+        __syncthreads();                                     // P and the tokens' numbers are there
 #pragma unroll
-        for (int t = 0; t < 8; ++t) { o[t][0] *= d0; o[t][1] *= d0; o[t][2] *= d1; o[t][3] *= d1; }
-        // 16 tokens s against this warp's 16; `odd`: on the diagonal, with values that are not finite.  (A form of its own: looked at
-        // product by product it takes 13 % of the kernel.)
-        auto weigh = [&](int ks, auto odd) {
-            uint32_t pa[3][4];
-            float pw[2][4];
+        for (int x = 0; x < 8; ++x) {
+            const float d0 = tok[x * 8 + q2].start, d1 = tok[x * 8 + q2 + 1].start;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int t = 2 * ks + half, s = t * 8 + q2;
-                const float *lo = sD + (tw + g) * (C + 1) + s, *hi = lo + 8 * (C + 1);
-                uint32_t w[3], x[3];
-                // tokens after this one are left out, whatever their products are: zero times an infinity is none
+            for (int w = 0; w < 2; ++w) { o[x][w][0] *= d0; o[x][w][1] *= d1; o[x][w][2] *= d0; o[x][w][3] *= d1; }
+        }
+        uint32_t wv[4][3][4];                                // (dt_t D(t, 64) v_t)^T in parts, for the state
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    pw[half][e] = s + (e & 1) <= tw + g + (e >> 1) * 8 ? qk[t][e] * (e < 2 ? lo : hi)[e & 1] : 0.f;
-                ssd_split2(pw[half][0], pw[half][1], w);
-                ssd_split2(pw[half][2], pw[half][3], x);
-#pragma unroll
-                for (int p = 0; p < 3; ++p) { pa[p][2 * half] = w[p]; pa[p][2 * half + 1] = x[p]; }
-            }
+        for (int ks = 0; ks < 4; ++ks) {                     // V^T P^T, 16 tokens s at a time
+            uint32_t va[4];
+            chk_ldm4t(va, v + ssd_at<8>(ks * 16 + (lm >> 1) * 8 + lr, cw / 8 + (lm & 1)));
+            const bool odd = s_odd[ks];
 #pragma unroll
             for (int pr = 0; pr < 4; ++pr) {
-                uint32_t vb[4];
-                ssd_ldm4t(vb, ssd_u32(sV) + ssd_at<8>(ks * 16 + (lm & 1) * 8 + lr, pr * 2 + (lm >> 1)));
-                if constexpr (odd.value) {
+                if (pr < ks) continue;
+                uint32_t pb[3][4], vf[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) vb[i] = ssd_finite(vb[i]);
-                }
+                for (int e = 0; e < 4; ++e) vf[e] = odd && pr == ks ? ssd_finite(va[e]) : va[e];
 #pragma unroll
-                for (int p = 0; p < 3; ++p) {
-                    ssd_mma(o[2 * pr], pa[p], vb[0], vb[1]);
-                    ssd_mma(o[2 * pr + 1], pa[p], vb[2], vb[3]);
-                }
+                for (int p = 0; p < 3; ++p) chk_ldm4(pb[p], sP + p * PB + ssd_at<8>(pr * 16 + (lm >> 1) * 8 + lr, ks * 2 + (lm & 1)));
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        if (p == 0) chk_mma_sum<true>(o[2 * pr + x], vf, pb[p][2 * x], pb[p][2 * x + 1]);
+                        else chk_mma_sum<false>(o[2 * pr + x], vf, pb[p][2 * x], pb[p][2 * x + 1]);
+                    }
             }
-            if constexpr (odd.value) {                       // the values left out, for their own and later tokens alone
+            if (odd) {                                       // the values left out on the diagonal, for their own and later tokens alone
 #pragma unroll 1
-                for (int s = 0; s < 16; ++s) {
-                    const int from = (lane & 28) | ((s & 7) >> 1);
-                    const float p0 = __shfl_sync(0xffffffffu, s & 8 ? (s & 1 ? pw[1][1] : pw[1][0]) : (s & 1 ? pw[0][1] : pw[0][0]), from);
-                    const float p1 = __shfl_sync(0xffffffffu, s & 8 ? (s & 1 ? pw[1][3] : pw[1][2]) : (s & 1 ? pw[0][3] : pw[0][2]), from);
+                for (int s = 0; s < 16; ++s)
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(sV + ssd_at<8>(ks * 16 + s, x) + q2 * 2);
+                    for (int e = 0; e < 2; ++e) {
+                        const int row = ks * 16 + s, col = cw + g + e * 8;
+                        const float y = to_f32(*reinterpret_cast<const __nv_bfloat16*>(v_bytes + ssd_at<8>(row, col >> 3) + (col & 7) * 2));
+                        if (isfinite(y)) continue;
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const float v = e ? __high2float(vv) : __low2float(vv);
-                            if (isfinite(v)) continue;
-                            if (s <= g) o[x][e] = fmaf(p0, v, o[x][e]);
-                            if (s <= g + 8) o[x][2 + e] = fmaf(p1, v, o[x][2 + e]);
+                        for (int x = 0; x < 4; ++x) {
+                            const int t = (x >> 1) * 8 + q2 + (x & 1);
+                            if (s > t) continue;
+                            float w = 0.f;
+#pragma unroll
+                            for (int p = 0; p < 3; ++p)
+                                w += to_f32(*reinterpret_cast<const __nv_bfloat16*>(ssd_sm + 4 * QB + 2 * VB + p * PB + ssd_at<8>(ks * 16 + t, row >> 3) + (row & 7) * 2));
+                            float* sum = &o[2 * ks + (x >> 1)][0][e * 2 + (x & 1)];
+                            *sum = fmaf(w, y, *sum);
                         }
                     }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                    // va[e]: column cw + g + (e & 1) * 8, tokens ks * 16 + (e >> 1) * 8 + q2 and the next
+                const int t = ks * 16 + (e >> 1) * 8 + q2;
+                const float v0 = __uint_as_float(va[e] << 16), v1 = __uint_as_float(va[e] & 0xffff0000u);
+                float* y = o[2 * ks + (e >> 1)][0] + (e & 1) * 2;
+                if (a.skip) {
+                    y[0] = fmaf(skip, v0, y[0]);
+                    y[1] = fmaf(skip, v1, y[1]);
                 }
-            }
-        };
-        const bool odd = s_odd[warp];
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            if (ks > warp) continue;
-            if (odd && ks == warp) weigh(ks, std::true_type{});
-            else weigh(ks, std::false_type{});
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int t = tw + g + e * 8;
-            if (t >= nt) continue;
-            float* orow = a.out + (size_t)(r0 + t0 + t) * a.out_stride + (size_t)h * a.dv + j0;
-#pragma unroll
-            for (int x = 0; x < 8; ++x) {
-                const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(sV + ssd_at<8>(t, x) + q2 * 2);
-                *reinterpret_cast<float2*>(orow + x * 8 + q2) =
-                    make_float2(fmaf(skip, __low2float(vv), o[x][2 * e] * a.q_scale), fmaf(skip, __high2float(vv), o[x][2 * e + 1] * a.q_scale));
+                chk_split2(v0 * tok[t].end, v1 * tok[t + 1].end, wv[ks][0][e], wv[ks][1][e], wv[ks][2][e]);
             }
         }
-        __syncthreads();                                     // q and the decays have been read
-#pragma unroll 4
-        for (int i = tid; i < C * P / 2; i += SSD_THREADS) { // the weighted values in three parts
-            const int t = i / (P / 2), c = i % (P / 2);
-            const uint32_t at = ssd_at<8>(t, c >> 2) + (c & 3) * 4;
-            const __nv_bfloat162 vv = *reinterpret_cast<const __nv_bfloat162*>(sV + at);
-            uint32_t w[3];
-            ssd_split2(__low2float(vv) * s_w[t], __high2float(vv) * s_w[t], w);
 #pragma unroll
-            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(sW + p * C * P * 2 + at) = w[p];
-        }
-        const float all = s_d0[C - 1];
-        __syncthreads();
+        for (int x = 0; x < 8; ++x)
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
+            for (int e = 0; e < 4; ++e) {
+                const int t = x * 8 + q2 + (e & 1);
+                if (t < nt) a.out[(size_t)(r0 + t0 + t) * a.out_stride + (size_t)h * a.dv + j0 + cw + g + (e >> 1) * 8] = o[x][0][e] + o[x][1][e];
+            }
 #pragma unroll
-            for (int t = 0; t < 8; ++t)
+        for (int x = 0; x < KT; ++x)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) S[m][t][e] *= all;
+            for (int e = 0; e < 4; ++e) S[x][e] *= all;
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {                     // 16 tokens
-            uint32_t ka[MT][4];
+        for (int part = 0; part < DK / 32; ++part) {         // the state, 32 keys at a time
+            float small[4][4];
 #pragma unroll
-            for (int m = 0; m < MT; ++m)                     // K^T: stored by token, transposed on the way
-                ssd_ldm4t(ka[m], ssd_u32(sK) + ssd_at<QR>(ks * 16 + (lm >> 1) * 8 + lr, (i0 + m * 16) / 8 + (lm & 1)));
+            for (int x = 0; x < 4; ++x)
 #pragma unroll
-            for (int p = 0; p < 3; ++p)
+                for (int e = 0; e < 4; ++e) small[x][e] = 0.f;
 #pragma unroll
-                for (int pr = 0; pr < 4; ++pr) {
-                    uint32_t wb[4];
-                    ssd_ldm4t(wb, ssd_u32(sW) + p * C * P * 2 + ssd_at<8>(ks * 16 + (lm & 1) * 8 + lr, pr * 2 + (lm >> 1)));
+            for (int ks = 0; ks < 4; ++ks) {
+                uint32_t kb[2][4];
 #pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        ssd_mma(S[m][2 * pr], ka[m], wb[0], wb[1]);
-                        ssd_mma(S[m][2 * pr + 1], ka[m], wb[2], wb[3]);
+                for (int pr = 0; pr < 2; ++pr) chk_ldm4t(kb[pr], k + ssd_at<QR>(ks * 16 + (lm & 1) * 8 + lr, part * 4 + pr * 2 + (lm >> 1)));
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const uint32_t* b = kb[x >> 1] + (x & 1) * 2;
+                        if (p == 0) chk_mma_sum<true>(S + part * 4 + x, wv[ks][p], b[0], b[1]);
+                        else chk_mma(small[x], wv[ks][p], b[0], b[1]);
                     }
-                }
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[part * 4 + x][e] += small[x][e];
         }
-        __syncthreads();                                     // k, v and the weighted values have been read
     }
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int x = 0; x < KT; ++x)
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                *reinterpret_cast<float2*>(S_area + (size_t)(i0 + m * 16 + g + e * 8) * a.dv + t * 8 + q2) = make_float2(S[m][t][2 * e], S[m][t][2 * e + 1]);
+        for (int e = 0; e < 4; ++e) S_area[(size_t)(x * 8 + q2 + (e & 1)) * a.dv + (e >> 1) * 8] = S[x][e];
 }
 
 template <int DK>
