@@ -18,52 +18,22 @@
 //     delta_intra_kernel   W, U0, P and the decayed q and k of every chunk
 //     delta_state_kernel   chunk after chunk, a tile of value columns a CTA: U, and the state every chunk starts from
 //     delta_out_kernel     O of every chunk
+// For keys of up to 128 delta_chunk.cu has all three with their products on the tensor cores.
 // No logarithm is taken: the decay between two tokens is a product of at most 16 decays at a time, which rounds like the walk
 // does.  Sub-chunks of 16 tokens are related through the products at their edges (never above one).  Inside a sub-chunk the
 // decay from s to t is taken as (edge to t) / (edge to s) for the channels whose decays over the sub-chunk multiply to 2^-60 or
 // more, and multiplied up pair by pair for the others.
-#include "common.cuh"
+#include "delta.cuh"
 #include "gated_norm.cuh"
 
 #define DELTA_MAX_DK 256
 #define DELTA_CV 4
 #define DELTA_WALK_THREADS 128
-#define DELTA_C 64                 // tokens a chunk
 #define DELTA_SUB 16               // tokens a sub-chunk
 #define DELTA_NSUB (DELTA_C / DELTA_SUB)
 #define DELTA_DVT 16               // value columns a CTA of the chunk-after-chunk kernel
 #define DELTA_OUT_COLS 64          // value columns a CTA of the output kernel
 #define DELTA_SPREAD 8.6736174e-19f      // 2^-60
-
-struct DeltaArgs {
-    const float* q; long long q_stride;          // [rows, groups * dk]
-    const float* k; long long k_stride;
-    const float* v; long long v_stride;          // [rows, heads * dv]
-    const float* z; long long z_stride;          // [rows, heads * dk]: decay logits
-    const float* bias;                           // [heads * dk]
-    const float* rate;                           // [heads], positive
-    const void* b; long long b_stride;           // [rows, heads], run type: the step sizes' logits
-    float* out; long long out_stride;            // [rows, heads * dv]
-    uint8_t* state; long long state_stride, state_offset;
-    const int *q_start, *q_len, *slot_ids;
-    int heads, groups, dk, dv;
-    // scratch of the chunked form: blocks a (chunk, head), see delta_block
-    float *w, *u, *qd, *kd, *p;                  // [64][LD], [tiles][64][16], [64][LD], [64][LD], [64][64]
-    float *gc, *sc;                              // [DKP], [tiles][DKP][16]
-    int tiles, max_chunks;                       // tiles of 16 value columns
-};
-
-// The place of chunk c of sequence seq among all chunks of the step: a sequence's chunks lie one after the other, and two
-// sequences' never meet (a sequence of n rows takes ceil(n / 64) places, the next one starts at least so many further on).
-__device__ __forceinline__ size_t delta_block(const DeltaArgs& a, int seq, int c, int h) {
-    return (size_t)(a.q_start[seq] / DELTA_C + seq + c) * a.heads + h;
-}
-
-// a decay from its logit: exp(-rate softplus(x))
-__device__ __forceinline__ float delta_decay(float x, float rate) {
-    return expf(-rate * (fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)))));
-}
-__device__ __forceinline__ float delta_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
 // ------------------------------------------------------------------ token by token
 // A CTA of 128 threads owns (head, sequence, a tile of value columns); a thread keeps R rows x 4 columns of S in registers,
@@ -737,12 +707,12 @@ delta_out_kernel(DeltaArgs a) {
 }
 
 // ------------------------------------------------------------------ host side
-static int delta_dkp(int dk) { return dk <= 64 ? 64 : dk <= 128 ? 128 : 256; }
 static long long delta_blocks(int rows, int n_seqs, int heads) { return ((long long)rows / DELTA_C + n_seqs + 1) * heads; }
 
 // Floats of scratch that the chunked form of a step needs.
 extern "C" long long braid_delta_work_floats(int rows, int n_seqs, int heads, int dk, int dv) {
-    const long long dkp = delta_dkp(dk), dvp = (dv + DELTA_DVT - 1) / DELTA_DVT * DELTA_DVT;
+    if (dk <= 128) return dlc_floats(delta_blocks(rows, n_seqs, heads), dk, dv);
+    const long long dkp = DELTA_MAX_DK, dvp = (dv + DELTA_DVT - 1) / DELTA_DVT * DELTA_DVT;
     return delta_blocks(rows, n_seqs, heads) * (3 * DELTA_C * (dkp + 4) + DELTA_C * dvp + DELTA_C * DELTA_C + dkp + dkp * dvp);
 }
 
@@ -770,11 +740,7 @@ static int launch_delta_chunks(const DeltaArgs& a, int n_seqs, cudaStream_t s) {
 
 template <typename T>
 static int launch_delta(const DeltaArgs& a, int n_seqs, bool chunked, cudaStream_t s) {
-    if (chunked) {
-        if (a.dk <= 64) return launch_delta_chunks<T, 64>(a, n_seqs, s);
-        if (a.dk <= 128) return launch_delta_chunks<T, 128>(a, n_seqs, s);
-        return launch_delta_chunks<T, 256>(a, n_seqs, s);
-    }
+    if (chunked) return launch_delta_chunks<T, DELTA_MAX_DK>(a, n_seqs, s);
     const int rg = a.dk <= 32 ? 4 : a.dk <= 64 ? 8 : 16;
     const int dvt = (DELTA_WALK_THREADS / rg) * DELTA_CV;
     const dim3 grid(a.heads, n_seqs, (a.dv + dvt - 1) / dvt), block(DELTA_WALK_THREADS);
@@ -799,14 +765,16 @@ extern "C" int braid_delta_rule(const float* q, long long q_stride, const float*
     if (dtype != BRAID_F32 && dtype != BRAID_BF16) BRAID_REFUSE("delta_rule: unknown dtype code %d", dtype);
     DeltaArgs a{q, q_stride, k, k_stride, v, v_stride, z, z_stride, bias, rate, b, b_stride, out, out_stride, (uint8_t*)state,
                 state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dk, dv,
-                nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, (dv + DELTA_DVT - 1) / DELTA_DVT,
+                (((uintptr_t)q | (uintptr_t)k) & 15) == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && dk % 4 == 0, ((uintptr_t)z & 15) == 0 && z_stride % 4 == 0 && dk % 4 == 0,
+                nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, (dv + DELTA_DVT - 1) / DELTA_DVT,
                 (max_q_len + DELTA_C - 1) / DELTA_C};
     const long long spans = (a.tiles * DELTA_DVT + DELTA_OUT_COLS - 1) / DELTA_OUT_COLS;
     if (n_seqs > 65535 || a.tiles > 65535 || (work && a.max_chunks * spans > 65535)) BRAID_REFUSE("delta_rule: the step exceeds the grid limits");
     if (work) {
         const long long need = braid_delta_work_floats(rows, n_seqs, heads, dk, dv);
         if (need > work_floats || ((uintptr_t)work & 15)) BRAID_REFUSE("delta_rule: the chunked form needs %lld floats of scratch on 16 bytes, it was given %lld", need, work_floats);
-        const long long blocks = delta_blocks(rows, n_seqs, heads), dkp = delta_dkp(dk), wide = blocks * DELTA_C * (dkp + 4);
+        const long long blocks = delta_blocks(rows, n_seqs, heads), dkp = DELTA_MAX_DK, wide = blocks * DELTA_C * (dkp + 4);
+        if (dk <= 128) return dlc_launch(a, dtype, n_seqs, blocks, work, (cudaStream_t)stream);
         a.w = work;
         a.qd = a.w + wide;
         a.kd = a.qd + wide;

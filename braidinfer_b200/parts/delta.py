@@ -36,7 +36,9 @@ class ChannelDelta(Mixer):
     a2, g1, g2, A_log, dt_bias, norm, o (under the prefix; the convolutions are stored under q, k, v with ".conv" added)."""
 
     plain_output = True
-    CHUNKED_FROM = 48          # steps whose longest sequence brings at least so many tokens take the form over chunks
+    # Steps whose longest sequence brings at least so many tokens take the form over chunks, keys of up to 64 and beyond.  Chunks / walk, us:
+    # 4 heads of 64 x 128 48 tokens 34 / 31, 8 x 64 36 / 39, 128 44 / 66; 8 heads of 128 x 256 64 tokens 91 / 47, 128 67 / 84, 8 x 64 99 / 111.
+    CHUNKED_FROM = (56, 96)
 
     def __init__(self, params, prefix, runtime) -> None:
         super().__init__(params, prefix, runtime)
@@ -132,7 +134,7 @@ class ChannelDelta(Mixer):
         fused = K.scan_step_fits(v, state, self.conv_state_bytes(), ctx, dk, dv) and K.step_norm_fits(dv, gates, y)
         o = None if fused else f32(H * dv)             # one token a sequence: rule and norm in one kernel
         K.delta_rule(q, k, v, logits[:, :H * dk], self.dt_bias, self.rate, b, o, state, self.conv_state_bytes(), ctx, H, G, dk, dv,
-                     chunked=int(ctx.max_q_len) >= self.CHUNKED_FROM,
+                     chunked=int(ctx.max_q_len) >= self.CHUNKED_FROM[dk > 64],
                      norm=(gates, self.norm_w, y, self.eps) if fused else None)
         if not fused:
             K.delta_gated_norm(o, gates, self.norm_w, y, ctx.token_seq, dv, self.eps)
