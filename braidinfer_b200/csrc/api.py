@@ -223,6 +223,8 @@ class Kernels:
                                       [c_void_p]
         L.braid_gemm_simt.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                       c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p]
+        L.braid_gemm_f32_tc.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_longlong] * 3 + [c_void_p, c_void_p]
+        L.braid_gemm_f32_tc.restype = c_int
         scale = [c_void_p, c_int, c_longlong, c_float, c_float]        # RowScale.args()
         L.braid_gemm_tc.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int,
                                     c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_int,
@@ -1637,6 +1639,12 @@ class Kernels:
             float(out_scale), self._stream()), "gated_norm")
 
     # ------------------------------------------------------------------ matrix products
+    @staticmethod
+    def f32_tc_pays(rows: int, m: int, k: int) -> bool:
+        """Whether a float32 product of `rows` tokens runs on the tensor cores (csrc/gemm_f32_tc.cu): beyond the rows that the kernel of few
+        rows takes, wherever it was measured (64 x 128 with 17 tokens 10 us beside 12, the other sizes there)."""
+        return rows > 16 and m >= 64 and k >= 128
+
     def gemm_simt(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None) -> None:
         n, k = x.shape
         m = w.shape[0]
@@ -1648,6 +1656,11 @@ class Kernels:
             raise KernelError(f"gemm_simt: shapes x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} do not fit")
         mode = 1 if residual is not None else 0
         self.launches += 1
+        if x.dtype == out.dtype == torch.float32 and self.f32_tc_pays(n, m, k) and k % 4 == 0 \
+                and x.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0:
+            self._check(self.lib.braid_gemm_f32_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(residual), n, m, k, x.stride(0),
+                                                   w.stride(0), out.stride(0), self._error_flag.data_ptr() + 4, self._stream()), "gemm_f32_tc")
+            return
         self._check(self.lib.braid_gemm_simt(x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(residual),
                                              dtype_code(x.dtype), dtype_code(out.dtype), mode, n, m, k,
                                              x.stride(0), w.stride(0), out.stride(0), self._stream()), "gemm_simt")

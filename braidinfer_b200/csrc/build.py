@@ -28,7 +28,7 @@ ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
 # Sources that do not depend on a model size.
-CORE_SOURCES = ["errors.cu", "elementwise.cu", "pointwise.cu", "attn_simple.cu", "gemm_simt.cu", "gemm_few.cu", "gemm_tc.cu", "gemm_tc2.cu",
+CORE_SOURCES = ["errors.cu", "elementwise.cu", "pointwise.cu", "attn_simple.cu", "gemm_simt.cu", "gemm_f32_tc.cu", "gemm_few.cu", "gemm_tc.cu", "gemm_tc2.cu",
                 "fused_reduce.cu", "sampling.cu"]
 # Kernels that only some models use: each a library of its own, compiled when a model that needs it is built.
 PART_SOURCES = {"latent": ["errors.cu", "latent.cu", "latent_attn_tc.cu"], "moe": ["errors.cu", "moe.cu", "moe_tc.cu"], "scan": ["errors.cu", "scan.cu", "scan_mma.cu", "scan_chunk.cu", "scan_step.cu"],

@@ -4,7 +4,8 @@
 // (kernels/megakernel_ops.hip:168-216 of the reference; oracle
 // crates/braidinfer-runtime/tests/linear_proj_test.rs:13-23).  Products and sums are
 // IEEE float32 FMA in a fixed order along k; no tensor cores and no reduced-precision
-// mode, which makes this the matrix product of the true 32-bit path.  With bfloat16
+// mode, which makes this the matrix product of the true 32-bit path (of more than 16 tokens where
+// gemm_f32_tc.cu does not pay).  With bfloat16
 // inputs it is the reference that the tensor-core kernel is checked against.
 //
 // Epilogues: 0 stores the product in `out_dtype`; 1 stores res + product as float32
