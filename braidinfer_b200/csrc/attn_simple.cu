@@ -53,7 +53,10 @@ struct AttnSimpleArgs {
 // (24 items of 200 keys: 170 us, a chain of 7 blocks of keys whose loads wait on one another), so `wpi` warps of a CTA share
 // an item, every wpi-th block of keys each, and the first of them merges their maxima, denominators and sums in order.  Keys are
 // read 16 bytes at a time where a head's rows allow it (WIDE), values of four keys at a time, in the order of the keys.
-template <typename T, int NI, bool WIDE>
+// DEEP: for steps whose CTAs do not fill the machine, which are a chain of trips to memory: a block's values (32 keys') and all 16-byte
+// loads of its keys are in flight together, whatever registers that takes.  The order of the sums is the same.  24 items of 200 keys of 64
+// numbers: 19.5 us with four of either in flight, 16.0 so.
+template <typename T, int NI, bool WIDE, bool DEEP = false>
 __global__ void __launch_bounds__(ATTN_SIMPLE_WARPS * 32)
 attn_simple_kernel(AttnSimpleArgs a, int wpi) {
     pdl_trigger();
@@ -98,7 +101,8 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
             if (turn % wpi != slice) continue;
             const int j = j0 + lane;
             float s = -INFINITY;
-            const T* vrow = nullptr;
+            const T *kbase = nullptr, *vrow = nullptr;
+            const int n_valid = min(32, end - j0);
             if (j < end) {
                 const int block = j / a.page_size, off = j - block * a.page_size;
                 int page = (block < a.table_cols) ? table[block] : -1;
@@ -106,12 +110,22 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
                     atomicExch(a.error_flag, 1);
                     page = 0;
                 }
-                const T* kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
+                kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
                 vrow = kbase + (size_t)(a.nkh + val_h - kvh) * head_stride;
+            }
+            T vs[DEEP ? 32 : 1][NI];
+            if (DEEP)
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, k);
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) vs[DEEP ? k : 0][i] = (k < n_valid && lane + 32 * i < a.hd) ? vr[lane + 32 * i] : from_f32<T>(0.f);
+                }
+            if (j < end) {
                 float dot = 0.f;
                 if (WIDE) {
                     constexpr int VW = 16 / sizeof(T);
-#pragma unroll 4
+#pragma unroll (DEEP ? 16 : 4)
                     for (int d = 0; d < a.hd; d += VW) {
                         float kv[VW];
                         load_run<T, VW>(kbase + d, kv);
@@ -136,8 +150,16 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < NI; ++i) acc[i] *= corr;
-            const int n_valid = min(32, end - j0);
-            for (int jj = 0; jj < n_valid; jj += 4) {
+            if (DEEP) {
+#pragma unroll
+                for (int k = 0; k < 32; ++k)
+                    if (k < n_valid) {
+                        const float pj = ps[k];
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, to_f32(vs[DEEP ? k : 0][i]), acc[i]);
+                    }
+            }
+            for (int jj = 0; jj < (DEEP ? 0 : n_valid); jj += 4) {
                 float v[4][NI];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -210,7 +232,10 @@ static void attn_simple_launch(const AttnSimpleArgs& a, cudaStream_t s) {
     const dim3 grid((unsigned)((items + per - 1) / per)), block(ATTN_SIMPLE_WARPS * 32);
     const size_t smem = (size_t)ATTN_SIMPLE_WARPS * (((a.hd + 3) & ~3) + 32 + 2) * sizeof(float);
     const bool wide = (a.hd * sizeof(T)) % 16 == 0 && ((uintptr_t)a.cache & 15) == 0;
-    if (a.hd <= 64) {
+    if (wide && grid.x <= 148 && a.hd <= 128) {
+        if (a.hd <= 64) braid_launch(attn_simple_kernel<T, 2, true, true>, grid, block, smem, s, a, wpi);
+        else braid_launch(attn_simple_kernel<T, 4, true, true>, grid, block, smem, s, a, wpi);
+    } else if (a.hd <= 64) {
         if (wide) braid_launch(attn_simple_kernel<T, 2, true>, grid, block, smem, s, a, wpi);
         else braid_launch(attn_simple_kernel<T, 2, false>, grid, block, smem, s, a, wpi);
     } else if (a.hd <= 128) {
