@@ -204,6 +204,12 @@ class Kernels:
         L.braid_act_mul_gather.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p,
                                            c_int, c_int, c_int, c_int, c_void_p]
         L.braid_rmsnorm_add.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_void_p]
+        L.braid_rmsnorm_add_norm.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_float, c_void_p, c_int,
+                                             c_void_p, c_int, c_int, c_void_p]
+        L.braid_rmsnorm_add_norm.restype = c_int
+        L.braid_gemm_few_table.argtypes = [c_void_p] * 3 + [c_int] * 3 + [c_longlong] * 3 + [c_void_p, c_longlong, c_void_p] + \
+                                          [c_int] * 3 + [c_void_p]
+        L.braid_gemm_few_table.restype = c_int
         L.braid_residual_add.argtypes = [c_void_p, c_void_p, c_int, c_longlong, c_void_p]
         L.braid_rope_kv_write.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -385,6 +391,37 @@ class Kernels:
         self.launches += 1
         self._check(self.lib.braid_rmsnorm_add(h.data_ptr(), y.data_ptr(), w.data_ptr(), dtype_code(w.dtype), h.shape[0],
                                                h.shape[1], float(eps), float(w_offset), self._stream()), "rmsnorm_add")
+
+    @staticmethod
+    def add_norm_fits(h: torch.Tensor, *rest: torch.Tensor) -> bool:
+        """Whether `rmsnorm_add_norm` takes rows of this width whose parts start so."""
+        return h.shape[1] % 4 == 0 and h.shape[1] <= 8192 and all(t.data_ptr() % 16 == 0 for t in (h,) + rest)
+
+    def rmsnorm_add_norm(self, h: torch.Tensor, y: torch.Tensor, w: torch.Tensor, eps: float, w2: torch.Tensor, out: torch.Tensor,
+                         eps2: float, row_index: Optional[torch.Tensor] = None) -> None:
+        """`rmsnorm_add`, and out = h / sqrt(mean(h^2) + eps2) * w2 of the sums in the same kernel.  With `row_index` out's rows are those
+        of the index and h is not written."""
+        if h.dtype != torch.float32 or y.dtype != torch.float32 or h.shape != y.shape or not h.is_contiguous() or not y.is_contiguous() \
+                or w.numel() != h.shape[1] or w2.numel() != h.shape[1] or out.shape[1] != h.shape[1] or not out.is_contiguous() \
+                or (row_index is None and out.shape[0] != h.shape[0]):
+            raise KernelError("rmsnorm_add_norm: h and y are contiguous float32 of one shape, w and w2 one number a column, out as wide")
+        self.launches += 1
+        self._check(self.lib.braid_rmsnorm_add_norm(h.data_ptr(), y.data_ptr(), w.data_ptr(), dtype_code(w.dtype), float(eps), w2.data_ptr(),
+                                                    dtype_code(w2.dtype), float(eps2), out.data_ptr(), dtype_code(out.dtype), _ptr(row_index),
+                                                    out.shape[0], h.shape[1], self._stream()), "rmsnorm_add_norm")
+
+    def gemm_few_table(self, x: torch.Tensor, w: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, col0: int, out: torch.Tensor,
+                       activation: str) -> None:
+        """out[r, j] = act((x w^T)[r, j]) * table[ids[r], col0 + j] for up to `FEW_MAX_ROWS` rows: x float32, rounded to bfloat16 as it is
+        read; w, table and out bfloat16."""
+        n, k = x.shape
+        if x.dtype != torch.float32 or not (w.dtype == table.dtype == out.dtype == torch.bfloat16) or w.shape[1] != k \
+                or tuple(out.shape) != (n, w.shape[0]) or any(t.stride(1) != 1 for t in (x, w, table, out)) or col0 + w.shape[0] > table.shape[1]:
+            raise KernelError("gemm_few_table: float32 rows; weights, table and results bfloat16; the table must hold the columns")
+        self.launches += 1
+        self._check(self.lib.braid_gemm_few_table(x.data_ptr(), w.data_ptr(), out.data_ptr(), n, w.shape[0], k, x.stride(0), w.stride(0),
+                                                  out.stride(0), table.data_ptr(), table.stride(0), ids.data_ptr(), table.shape[0], int(col0),
+                                                  activation_code(activation), self._stream()), "gemm_few_table")
 
     def head_prep_kv(self, src: torch.Tensor, q_out: torch.Tensor, positions: torch.Tensor, token_seq: torch.Tensor,
                      page_table: Optional[torch.Tensor], cache: Optional[torch.Tensor], nqh: int, nkh: int, dk: int, dv: int,

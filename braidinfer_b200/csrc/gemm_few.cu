@@ -10,7 +10,7 @@
 // barriers and tensor memory between a weight and its product).  U turns are in flight a warp, the first of them asked for before the
 // dependency wait: no kernel writes weights.  The warps' sums meet in shared memory in the order of the warps.
 //
-// Epilogues: 0 store, 1 float32 residual sum, 2 gated unit.  A gated tile is 8 gate rows and the 8 up rows that go with
+// Epilogues: 0 store, 1 float32 residual sum, 2 gated unit, 3 act(product) times a number of the row's token from a table.  A gated tile is 8 gate rows and the 8 up rows that go with
 // them (rows interleaved in blocks of 16, see gemm_tc.cu), so that both halves meet in one CTA.  A row scale that x still
 // wants (rowscale.cuh) multiplies the finished sums of 0 and 2.
 //
@@ -26,13 +26,18 @@
 #define FEW_MAX_ROWS 16
 
 struct GemmFewArgs {
-    const __nv_bfloat16 *x, *w;
+    const void* x;              // bfloat16, or float32 that is rounded as it is read (XF)
+    const __nv_bfloat16* w;
     void* out;                  // mode 0: bf16/f32; 1: f32; 2: bf16/f32
     const float* res;           // mode 1 (may be out)
     int n_rows, m_out, k8;      // m_out: outputs; k8: k / 8
     long long ldx, ldw, ldo;
     int out_f32, act;
     RowScaleArgs scale;
+    const __nv_bfloat16* table; // mode 3: [vocab, table_stride], output o of row n times table[ids[n], o]
+    long long table_stride;
+    const int* ids;
+    int vocab;
 };
 
 __device__ __forceinline__ uint4 few_load_weights(const uint4* p) {
@@ -45,8 +50,17 @@ __device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// eight numbers of a row, in bfloat16
+template <bool XF>
+__device__ __forceinline__ uint4 few_load_x(const void* x, size_t at) {
+    if (!XF) return *reinterpret_cast<const uint4*>((const __nv_bfloat16*)x + at);
+    const float4 a = *reinterpret_cast<const float4*>((const float*)x + at), b = *reinterpret_cast<const float4*>((const float*)x + at + 4);
+    const __nv_bfloat162 p[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
+    return *reinterpret_cast<const uint4*>(p);
+}
+
 // NT: blocks of 8 tokens.
-template <int MODE, int NT, int W, int U>
+template <int MODE, int NT, int W, int U, bool XF = false>
 __global__ void __launch_bounds__(W * 32)
 gemm_few_bf16_kernel(GemmFewArgs a) {
     __shared__ float part[W][NT][8][17];                     // [warp][token block][token][tile row]
@@ -77,12 +91,12 @@ gemm_few_bf16_kernel(GemmFewArgs a) {
     for (int u = 0; u < U; ++u) fetch(u, warp + u * W);
     pdl_wait();
     if (a.scale.shares && warp == W - 1 && lane < a.n_rows) rs[lane] = row_scale_of(a.scale, lane);
-    const uint4* xr[NT];
+    size_t xr[NT];
     bool live[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         live[n] = n * 8 + g < a.n_rows;
-        xr[n] = reinterpret_cast<const uint4*>(a.x + (size_t)(live[n] ? n * 8 + g : 0) * a.ldx);
+        xr[n] = (size_t)(live[n] ? n * 8 + g : 0) * a.ldx;
     }
     float acc[NT][4];
 #pragma unroll
@@ -99,7 +113,7 @@ gemm_few_bf16_kernel(GemmFewArgs a) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int c = turn * 8 + h * 4 + q;
-                    const uint4 xv = (live[n] && c < a.k8) ? xr[n][c] : zero;
+                    const uint4 xv = (live[n] && c < a.k8) ? few_load_x<XF>(a.x, xr[n] + c * 8) : zero;
                     few_mma(acc[n], wv[u][0][h].x, wv[u][1][h].x, wv[u][0][h].y, wv[u][1][h].y, xv.x, xv.y);
                     few_mma(acc[n], wv[u][0][h].z, wv[u][1][h].z, wv[u][0][h].w, wv[u][1][h].w, xv.z, xv.w);
                 }
@@ -130,6 +144,11 @@ gemm_few_bf16_kernel(GemmFewArgs a) {
         const size_t at = (size_t)n * a.ldo + m;
         if (MODE == 1) {
             ((float*)a.out)[at] = a.res[at] + v;
+            continue;
+        }
+        if (MODE == 3) {
+            const int id = min(max(a.ids[n], 0), a.vocab - 1);
+            ((__nv_bfloat16*)a.out)[at] = __float2bfloat16_rn(glu_act(v, a.act) * __bfloat162float(a.table[(size_t)id * a.table_stride + m]));
             continue;
         }
         const float s = a.scale.shares ? rs[n] : 1.f;
@@ -174,7 +193,7 @@ extern "C" int braid_gemm_few(const void* x, const void* w, void* out, const flo
     const RowScaleArgs rsa{shares, n_shares, share_stride, width, eps};
     if (const char* p = row_scale_problem(rsa, n_rows)) BRAID_REFUSE("gemm_few: row scale: %s", p);
     if (shares && mode == 1) BRAID_REFUSE("gemm_few: the residual sum applies no row scale");
-    GemmFewArgs a{(const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, res, n_rows, m_out, k_in / 8, ldx, ldw, ldo, out_dtype == BRAID_F32, act, rsa};
+    GemmFewArgs a{x, (const __nv_bfloat16*)w, out, res, n_rows, m_out, k_in / 8, ldx, ldw, ldo, out_dtype == BRAID_F32, act, rsa, nullptr, 0, nullptr, 0};
     const int tiles = mode == 2 ? (m_out + 7) / 8 : (m_out + 15) / 16;
     cudaStream_t s = (cudaStream_t)stream;
     if (n_rows <= 8) {
@@ -185,6 +204,31 @@ extern "C" int braid_gemm_few(const void* x, const void* w, void* out, const flo
         if (mode == 0) launch_few_bf16<0, 2>(a, tiles, s);
         else if (mode == 1) launch_few_bf16<1, 2>(a, tiles, s);
         else launch_few_bf16<2, 2>(a, tiles, s);
+    }
+    BRAID_LAUNCH_CHECK();
+}
+
+// x float32, rounded to bfloat16 as it is read: out[n, o] = act((x w^T)[n, o]) * table[ids[n], col0 + o] in bfloat16 (three kernels of 1.1, 2.0 and
+// 1.6 us between the others of a decode step of 8 rows, 128 x 1024: 3.2 in one).
+extern "C" int braid_gemm_few_table(const float* x, const void* w, void* out, int n_rows, int m_out, int k_in, long long ldx, long long ldw,
+                                    long long ldo, const void* table, long long table_stride, const int* ids, int vocab, int col0, int act,
+                                    void* stream) {
+    if (n_rows <= 0 || m_out <= 0) return BRAID_OK;
+    if (n_rows > FEW_MAX_ROWS) BRAID_REFUSE("gemm_few_table: %d rows (at most %d)", n_rows, FEW_MAX_ROWS);
+    if (k_in <= 0 || k_in % 8 || ldx % 4 || ldw % 8 || (((uintptr_t)x | (uintptr_t)w) & 15)) BRAID_REFUSE("gemm_few_table: k=%d must be a multiple of 8 and rows start on 16 bytes", k_in);
+    if (act < 0 || act >= BRAID_ACT_COUNT) BRAID_REFUSE("gemm_few_table: unknown activation %d", act);
+    if (!table || !ids || vocab <= 0 || col0 < 0) BRAID_REFUSE("gemm_few_table: vocab=%d, col0=%d", vocab, col0);
+    const GemmFewArgs a{x, (const __nv_bfloat16*)w, out, nullptr, n_rows, m_out, k_in / 8, ldx, ldw, ldo, 0, act, RowScaleArgs{},
+                        (const __nv_bfloat16*)table + col0, table_stride, ids, vocab};
+    const dim3 grid((m_out + 15) / 16);
+    cudaStream_t s = (cudaStream_t)stream;
+    // few CTAs: sixteen warps each, as k allows
+    if (n_rows <= 8) {
+        if (k_in >= 1024) braid_launch(gemm_few_bf16_kernel<3, 1, 16, 2, true>, grid, dim3(512), 0, s, a);
+        else braid_launch(gemm_few_bf16_kernel<3, 1, 4, 4, true>, grid, dim3(128), 0, s, a);
+    } else {
+        if (k_in >= 1024) braid_launch(gemm_few_bf16_kernel<3, 2, 16, 2, true>, grid, dim3(512), 0, s, a);
+        else braid_launch(gemm_few_bf16_kernel<3, 2, 4, 4, true>, grid, dim3(128), 0, s, a);
     }
     BRAID_LAUNCH_CHECK();
 }

@@ -52,7 +52,8 @@ class StepContext:
     # GEMM workspace and hand the adding-up to the part that reads the result next, which
     # fuses it with its own work (the next norm, the rotary encoding).  `deferred` maps the
     # tensor that is still to be completed (by its data pointer) to (handle, kind): kind
-    # "residual" means tensor += sum, "store" means tensor = sum.  A part that does not
+    # "residual" means tensor += sum, "store" means tensor = sum, "normed" means tensor += norm(y) * w with handle (y, w, eps),
+    # which needs no workspace.  A part that does not
     # know about this calls `resolve(tensor)` first, or is handed a resolved tensor by the
     # block.  At most one sum is deferred at a time.
     deferred: dict = field(default_factory=dict)
@@ -94,7 +95,9 @@ class StepContext:
             if self.kernels is None:
                 from ..csrc.api import get_kernels
                 self.kernels = get_kernels()
-            if kind == "residual":
+            if kind == "normed":
+                self.kernels.rmsnorm_add(tensor, *handle)
+            elif kind == "residual":
                 self.kernels.streamk_reduce(handle, tensor, residual=tensor)
             else:
                 self.kernels.streamk_reduce(handle, tensor)

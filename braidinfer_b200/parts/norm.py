@@ -73,6 +73,13 @@ class RMSNorm(Norm):
             self.rt.kernels.rmsnorm(x, self.weight, out, self.eps, row_index=row_index, w_offset=self.offset)
             return out
         d = ctx.take_deferred(x) if ctx is not None else None
+        if d is not None and d[1] == "normed":
+            y, w, eps = d[0]
+            if self.rt.kernels.add_norm_fits(x, y, w, self.weight, out):
+                self.rt.kernels.rmsnorm_add_norm(x, y, w, eps, self.weight, out, self.eps, row_index=row_index)
+                return out
+            self.rt.kernels.rmsnorm_add(x, y, w, eps)
+            d = None
         if (reader_takes_row_scale and self.rt.scaled_norm and ctx is not None and row_index is None and out.dtype == torch.bfloat16
                 and n <= ROW_SCALE_MAX_ROWS and self.width % 4 == 0 and self.rt.gemm_backend == "auto"):
             # a step of few tokens: x is completed, `out` = x * weight, and the scale is left to the reader.

@@ -13,7 +13,7 @@ from typing import Dict
 import torch
 
 from .base import LAYER_INPUTS, LayerInput
-from .linear import Linear
+from .linear import Linear, few_rows_pay
 from .spec import TensorSpec
 
 
@@ -59,13 +59,18 @@ class GatedTokenTable(LayerInput):
     def forward(self, h: torch.Tensor, ctx) -> torch.Tensor:
         K = self.rt.kernels
         rows = h.shape[0]
-        x = h
-        if not self.rt.is_f32:
-            x = self.rt.empty(rows, self.hidden)
-            K.cast(h, x)
-        gate = self.gate.forward(x)
         g = self.rt.empty(rows, self.dim)
-        K.act_mul_gather(gate, self.table, ctx.token_ids, self.index * self.dim, g, self.activation)
-        y = self.proj.forward(g, out_dtype=torch.float32)
-        K.rmsnorm_add(h, y, self.norm_w, self.eps)
+        w = self.gate.weight
+        if (not self.rt.is_f32 and self.rt.gemm_backend == "auto" and w.dtype == self.table.dtype == g.dtype == torch.bfloat16
+                and few_rows_pay(rows, self.dim, self.hidden) and self.hidden % 8 == 0 and w.stride(0) % 8 == 0
+                and h.stride(0) % 4 == 0 and (h.data_ptr() | w.data_ptr()) % 16 == 0):
+            K.gemm_few_table(h, w, self.table, ctx.token_ids, self.index * self.dim, g, self.activation)
+        else:
+            x = h
+            if not self.rt.is_f32:
+                x = self.rt.empty(rows, self.hidden)
+                K.cast(h, x)
+            K.act_mul_gather(self.gate.forward(x), self.table, ctx.token_ids, self.index * self.dim, g, self.activation)
+        # the norm that reads the stream next adds this one's result to it in its own kernel
+        ctx.defer(h, (self.proj.forward(g, out_dtype=torch.float32), self.norm_w, self.eps), "normed")
         return h
