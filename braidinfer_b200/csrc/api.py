@@ -813,6 +813,9 @@ class Kernels:
                                                   [c_void_p, c_longlong, c_longlong, c_void_p]
                 lib.braid_moe_gather.argtypes = [c_void_p] * 4 + [c_longlong] + [c_int] * 3 + [c_void_p]
                 lib.braid_moe_gemm_tc.argtypes = [c_void_p] * 7 + [c_int] * 5 + [c_longlong, c_int, c_int] + [c_void_p] * 3
+                lib.braid_moe_few.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong] + [c_void_p] * 3 + [c_int] * 7 + \
+                                             [c_void_p, c_void_p]
+                lib.braid_moe_few.restype = c_int
                 names = ("braid_moe_gemm_mma", "braid_moe_gather", "braid_moe_gemm_tc",
                          "braid_moe_route", "braid_moe_plan", "braid_moe_gemm_simt", "braid_moe_combine")
             elif name == "conv":
@@ -1166,6 +1169,24 @@ class Kernels:
             xs.data_ptr(), w.data_ptr(), out.data_ptr(), slot_pair.data_ptr(), tile_expert.data_ptr(), wide.data_ptr(), meta.data_ptr(),
             1 if gated else 2 if relu2 else 0, experts, w_rows, out.shape[1], k, out.stride(0), max_tiles, wide.numel() // 4,
             _ptr(in_wgt), self._error_flag.data_ptr() + 4, self._stream()), "moe_gemm_tc")
+
+    def moe_few(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan, rows: int, top: int = 0, gated: bool = False,
+                relu2: bool = False, in_wgt: Optional[torch.Tensor] = None) -> None:
+        """`moe_gemm_tc` for steps of up to 8 tokens, each of which chose different experts (csrc/moe_few.cu): with `top` x holds the
+        step's rows, which are read where they lie, else the slots'.  Rows of padding slots are not written."""
+        lib = self.part_library("moe")
+        slot_pair, pair_slot, tile_expert, meta, max_tiles = plan[:5]
+        experts, w_rows, k = w.shape
+        if not (x.dtype == w.dtype == out.dtype == torch.bfloat16) or not w.is_contiguous() or x.stride(1) != 1 or x.shape[1] != k \
+                or out.shape[0] != max_tiles * MOE_TC_TILE or out.stride(1) != 1 or (gated and relu2) \
+                or pair_slot.numel() % rows or x.shape[0] < (rows if top else out.shape[0]):
+            raise KernelError("moe_few: bfloat16 x, contiguous w [experts, rows, k], out [slots, J]")
+        if in_wgt is not None and (in_wgt.dtype != torch.float32 or not in_wgt.is_contiguous() or in_wgt.numel() != pair_slot.numel()):
+            raise KernelError("moe_few: the weights on the experts' input are float32, one a pair")
+        self.launches += 1
+        self._check_lib(lib, lib.braid_moe_few(
+            x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), slot_pair.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(),
+            1 if gated else 2 if relu2 else 0, rows, top, w_rows, out.shape[1], k, max_tiles, _ptr(in_wgt), self._stream()), "moe_few")
 
     @staticmethod
     def attn_latent_mma_supports(rank: int, rot: int) -> bool:

@@ -31,11 +31,11 @@ COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt
 CORE_SOURCES = ["errors.cu", "elementwise.cu", "pointwise.cu", "attn_simple.cu", "gemm_simt.cu", "gemm_f32_tc.cu", "gemm_few.cu", "gemm_tc.cu", "gemm_tc2.cu",
                 "fused_reduce.cu", "sampling.cu"]
 # Kernels that only some models use: each a library of its own, compiled when a model that needs it is built.
-PART_SOURCES = {"latent": ["errors.cu", "latent.cu", "latent_attn_tc.cu"], "moe": ["errors.cu", "moe.cu", "moe_tc.cu"], "scan": ["errors.cu", "scan.cu", "scan_mma.cu", "scan_chunk.cu", "scan_step.cu"],
+PART_SOURCES = {"latent": ["errors.cu", "latent.cu", "latent_attn_tc.cu"], "moe": ["errors.cu", "moe.cu", "moe_tc.cu", "moe_few.cu"], "scan": ["errors.cu", "scan.cu", "scan_mma.cu", "scan_chunk.cu", "scan_step.cu"],
                 "streams": ["errors.cu", "streams.cu"], "conv": ["errors.cu", "conv_heads.cu"],
                 "delta": ["errors.cu", "delta.cu", "delta_chunk.cu"]}
 HEADERS = ["common.cuh", "rowscale.cuh", "streamk.cuh", "tcgen05.cuh", "tcgen05_pair.cuh", "attn_tc.cuh", "attn_noalloc.h", "page.h", "trace.cuh",
-           "mma_tile.cuh", "softcap.cuh", "gated_norm.cuh", "chunk_mma.cuh", "delta.cuh"]
+           "mma_tile.cuh", "softcap.cuh", "gated_norm.cuh", "chunk_mma.cuh", "delta.cuh", "few.cuh"]
 
 
 class BuildError(RuntimeError):

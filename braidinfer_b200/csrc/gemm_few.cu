@@ -22,6 +22,7 @@
 // 4096 x 4096 and 4096 x 14336 so: 64.5 beside 51.6 ms a turn of one sequence): `few_rows_pay` (parts/linear.py) draws the line.
 #include "common.cuh"
 #include "rowscale.cuh"
+#include "few.cuh"
 
 #define FEW_MAX_ROWS 16
 
@@ -39,16 +40,6 @@ struct GemmFewArgs {
     const int* ids;
     int vocab;
 };
-
-__device__ __forceinline__ uint4 few_load_weights(const uint4* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // eight numbers of a row, in bfloat16
 template <bool XF>

@@ -37,6 +37,9 @@ from .linear import Linear
 from .spec import PartSpec, TensorSpec
 
 
+FEW_TOKENS = 8               # steps of up to so many tokens run the experts' products of few tokens (csrc/moe_few.cu has both sides' times)
+
+
 @FEED_FORWARDS.register("moe")
 class MixtureOfExperts(FeedForward):
     """params: hidden_size, intermediate_size (of one expert), experts, top, groups (default 1), keep
@@ -123,7 +126,7 @@ class MixtureOfExperts(FeedForward):
 
     def on_pairs(self, x) -> bool:
         """Whether the products can run on pairs of SMs (csrc/moe_tc.cu): bfloat16 whose rows, inputs and results alike, start on
-        16 bytes.  They are the fastest at every number of rows."""
+        16 bytes.  They are the fastest from 9 rows on, and few tokens' kernel wants the same of them."""
         return (self.rt.gemm_backend == "auto" and self.w_first is not None and self.w_first.dtype == torch.bfloat16
                 and self.w_down.dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.inter % 8 == 0
                 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
@@ -172,7 +175,11 @@ class MixtureOfExperts(FeedForward):
     def _experts(self, x, act, y, plan, tile, in_wgt=None) -> None:
         """bfloat16 rows that start on 16 bytes run on the tensor cores, everything else on the plain kernel."""
         K = self.rt.kernels
-        if len(plan) > 5:                                              # a plan of tiles of 32 slots
+        if len(plan) > 5 and x.shape[0] <= FEW_TOKENS:                 # a plan of tiles of 32 slots, of a step of few tokens
+            K.moe_few(x, self.w_first, act, plan, x.shape[0], self.top, gated=self.gated, relu2=not self.gated, in_wgt=in_wgt)
+            K.moe_few(act, self.w_down, y, plan, x.shape[0])
+            return
+        if len(plan) > 5:
             # the slots' inputs lie where their results will: the first product has read them when the second one writes there
             xs = K.moe_gather(x, plan, self.top, out=y)
             K.moe_gemm_tc(xs, self.w_first, act, plan, gated=self.gated, relu2=not self.gated, in_wgt=in_wgt)
