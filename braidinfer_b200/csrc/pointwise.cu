@@ -7,24 +7,48 @@
 // y[r, i] = tanh(alpha * (x[src(r), i] * in_scale)) * w[i] + b[i].  No mean and no variance: rows are
 // independent element by element.  alpha is one stored scalar.  `row_index` (may be null) picks the input
 // row of each output row; a negative index gives a row of zeros.  out may be x itself (TO = float).
-template <typename TW, typename TO>
+//
+// A thread has four numbers that lie side by side where VEC (else four that lie a block apart), a row as many CTAs as it takes, and the
+// weights are asked for before the wait: bound by one trip to memory.  A row a CTA whose threads walked it number by number, trip after
+// trip, took 5.6 us for 8 rows of 2,048 in the chain of a step; this takes 2.2.
+template <typename TW, typename TO, bool VEC>
 __global__ void dyt_kernel(const float* x, const TW* __restrict__ w, const TW* __restrict__ b,
                            const TW* __restrict__ alpha, TO* out, const int* __restrict__ row_index,
-                           int rows, int width, float in_scale) {
+                           int width, float in_scale) {
     pdl_trigger();
+    const int r = blockIdx.x, at = blockIdx.y * blockDim.x * 4 + threadIdx.x * (VEC ? 4 : 1), step = VEC ? 1 : blockDim.x;
+    float g[4], c[4], v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int i = at + e * step;
+        g[e] = i < width ? to_f32(w[i]) : 0.f;
+        c[e] = i < width ? to_f32(b[i]) : 0.f;
+    }
+    const float a = to_f32(alpha[0]);
     pdl_wait();
-    const int r = blockIdx.x;
-    if (r >= rows) return;
     const int src = row_index ? row_index[r] : r;
     TO* o = out + (size_t)r * width;
-    if (src < 0) {
-        for (int i = threadIdx.x; i < width; i += blockDim.x) o[i] = from_f32<TO>(0.f);
-        return;
+    const float* xr = x + (size_t)(src < 0 ? 0 : src) * width;
+    if (VEC) {
+        if (at >= width) return;
+        const float4 x4 = src < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(xr + at);
+        v[0] = x4.x; v[1] = x4.y; v[2] = x4.z; v[3] = x4.w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = (src >= 0 && at + e * step < width) ? xr[at + e * step] : 0.f;
     }
-    const float a = to_f32(alpha[0]) ;
-    const float* xr = x + (size_t)src * width;
-    for (int i = threadIdx.x; i < width; i += blockDim.x)
-        o[i] = from_f32<TO>(fmaf(tanhf(a * (xr[i] * in_scale)), to_f32(w[i]), to_f32(b[i])));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = src < 0 ? 0.f : fmaf(tanhf(a * (v[e] * in_scale)), g[e], c[e]);
+    if (VEC) {
+        struct alignas(4 * sizeof(TO)) { TO n[4]; } y;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y.n[e] = from_f32<TO>(v[e]);
+        *reinterpret_cast<decltype(y)*>(o + at) = y;
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (at + e * step < width) o[at + e * step] = from_f32<TO>(v[e]);
+    }
 }
 
 extern "C" int braid_dyt(const float* x, const void* w, const void* b, const void* alpha, int w_dtype,
@@ -33,8 +57,14 @@ extern "C" int braid_dyt(const float* x, const void* w, const void* b, const voi
     if (rows <= 0) return BRAID_OK;
     if (width <= 0) BRAID_REFUSE("dyt: width=%d must be positive", width);
     cudaStream_t s = (cudaStream_t)stream;
-    const int threads = width >= 1024 ? 256 : 128;
-#define BRAID_DYT(TW, TO) braid_launch(dyt_kernel<TW, TO>, dim3(rows), dim3(threads), 0, s, x, (const TW*)w, (const TW*)b, (const TW*)alpha, (TO*)out, row_index, rows, width, in_scale)
+    const int threads = 128;
+    const dim3 grid(rows, (width + threads * 4 - 1) / (threads * 4));
+    if (grid.y > 65535) BRAID_REFUSE("dyt: width=%d exceeds the grid limit", width);
+    const bool vec = width % 4 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
+#define BRAID_DYT(TW, TO) do { \
+        if (vec) braid_launch(dyt_kernel<TW, TO, true>, grid, dim3(threads), 0, s, x, (const TW*)w, (const TW*)b, (const TW*)alpha, (TO*)out, row_index, width, in_scale); \
+        else braid_launch(dyt_kernel<TW, TO, false>, grid, dim3(threads), 0, s, x, (const TW*)w, (const TW*)b, (const TW*)alpha, (TO*)out, row_index, width, in_scale); \
+    } while (0)
     if (w_dtype == BRAID_F32 && out_dtype == BRAID_F32) BRAID_DYT(float, float);
     else if (w_dtype == BRAID_F32 && out_dtype == BRAID_BF16) BRAID_DYT(float, __nv_bfloat16);
     else if (w_dtype == BRAID_BF16 && out_dtype == BRAID_F32) BRAID_DYT(__nv_bfloat16, float);
