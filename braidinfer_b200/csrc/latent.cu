@@ -14,6 +14,7 @@
 // Norm, angles, scores, softmax and accumulation are float32.
 #include "common.cuh"
 #include "mma_tile.cuh"
+#include "few.cuh"
 
 // ------------------------------------------------------------------ row preparation
 struct LatentPrepArgs {
@@ -260,25 +261,93 @@ extern "C" int braid_gemm_heads(const void* x, const void* w, void* out, const v
     BRAID_LAUNCH_CHECK();
 }
 
-// The same product in bfloat16 on the tensor cores (mma_tile.cuh): BM tokens x 64 outputs of one head a CTA.
-template <int BM>
+// The same product of up to 16 tokens in bfloat16: 16 weight rows of one head a CTA, whose warps share k, the weights asked for before the
+// wait and straight in the operand registers (as in gemm_few.cu).  Bound by latency: 2 MB of weights.  With 64 outputs a CTA (mma_tile.cuh),
+// whose steps of k follow one another, 8 tokens and 16 heads of 512 x 128 / 128 x 512 took 7.5 / 2.8 us in a step's chain; this 2.8 / 2.2.
+template <int NT, int W>
+__global__ void __launch_bounds__(W * 32)
+gemm_heads_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
+                      const __nv_bfloat16* __restrict__ gate, int n_rows, int J, int k8, long long ldx, long long hsx,
+                      long long ldo, long long hso, long long ldg, float mult) {
+    constexpr int U = 2;                                     // turns of 64 numbers of k in flight a warp
+    __shared__ float part[W][NT][8][17];                     // [warp][token block][token][output]
+    pdl_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int h = blockIdx.y, m0 = blockIdx.x * 16, turns = (k8 + 7) / 8;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const uint4* wr[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) wr[r] = reinterpret_cast<const uint4*>(w) + ((size_t)h * J + min(m0 + g + r * 8, J - 1)) * k8;
+    uint4 wv[U][2][2];
+    auto fetch = [&](int u, int turn) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = turn * 8 + e * 4 + q;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) wv[u][r][e] = c < k8 ? few_load_weights(wr[r] + c) : zero;
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < U; ++u) fetch(u, warp + u * W);
+    pdl_wait();
+    const uint4* xr[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) xr[n] = n * 8 + g < n_rows ? reinterpret_cast<const uint4*>(x + (size_t)(n * 8 + g) * ldx + (size_t)h * hsx) : nullptr;
+    float acc[NT][4] = {};
+    for (int t0 = warp; t0 < turns; t0 += U * W) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int turn = t0 + u * W;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int c = turn * 8 + e * 4 + q;
+                    const uint4 xv = (xr[n] && c < k8) ? xr[n][c] : zero;
+                    few_mma(acc[n], wv[u][0][e].x, wv[u][1][e].x, wv[u][0][e].y, wv[u][1][e].y, xv.x, xv.y);
+                    few_mma(acc[n], wv[u][0][e].z, wv[u][1][e].z, wv[u][0][e].w, wv[u][1][e].w, xv.z, xv.w);
+                }
+            if (turn + U * W < turns) fetch(u, turn + U * W);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        part[warp][n][2 * q][g] = acc[n][0];
+        part[warp][n][2 * q + 1][g] = acc[n][1];
+        part[warp][n][2 * q][g + 8] = acc[n][2];
+        part[warp][n][2 * q + 1][g + 8] = acc[n][3];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < NT * 8 * 16; i += W * 32) {
+        const int o = i & 15, n = i >> 4;
+        if (m0 + o >= J || n >= n_rows) continue;
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < W; ++k) v += part[k][n >> 3][n & 7][o];
+        if (gate) v *= mult / (1.f + expf(-__bfloat162float(gate[(size_t)n * ldg + h])));
+        out[(size_t)n * ldo + (size_t)h * hso + m0 + o] = __float2bfloat16_rn(v);
+    }
+}
+
+// The same product in bfloat16 on the tensor cores (mma_tile.cuh): 64 tokens x 64 outputs of one head a CTA.
 __global__ void __launch_bounds__(128)
 gemm_heads_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
                       const __nv_bfloat16* __restrict__ gate, int n_rows, int J, int K, long long ldx, long long hsx,
                       long long ldo, long long hso, long long ldg, float mult) {
-    using Tile = MmaTile<BM, 64, (BM >= 64 ? 2 : 1), (BM >= 64 ? 2 : 4), 1>;
+    constexpr int BM = 64;
+    using Tile = MmaTile<BM, 64, 2, 2, 1>;
     extern __shared__ __align__(16) unsigned char hg_smem[];
     pdl_trigger();
     pdl_wait();
     const int h = blockIdx.z, n0 = blockIdx.y * BM, m0 = blockIdx.x * 64;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int ACH = BM * 4 / 128 > 0 ? BM * 4 / 128 : 1;
+    constexpr int ACH = BM * 4 / 128;
     const __nv_bfloat16* a_rows[ACH];
     const __nv_bfloat16* b_rows[1][2];
 #pragma unroll
     for (int i = 0; i < ACH; ++i) {
         const int r = (tid + i * 128) >> 2;
-        a_rows[i] = (r < BM && n0 + r < n_rows) ? x + (size_t)(n0 + r) * ldx + (size_t)h * hsx : nullptr;
+        a_rows[i] = n0 + r < n_rows ? x + (size_t)(n0 + r) * ldx + (size_t)h * hsx : nullptr;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -287,7 +356,7 @@ gemm_heads_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* 
     }
     float acc[1][Tile::MI][Tile::NI][4];
     Tile::run(acc, (__nv_bfloat16*)hg_smem, a_rows, b_rows, K, w);
-    const int wm0 = (warp / (BM >= 64 ? 2 : 4)) * (BM / (BM >= 64 ? 2 : 1)), wn0 = (warp % (BM >= 64 ? 2 : 4)) * (64 / (BM >= 64 ? 2 : 4));
+    const int wm0 = (warp / 2) * (BM / 2), wn0 = (warp % 2) * 32;
     const bool pairs_ok = ((ldo | hso) & 1) == 0;
 #pragma unroll
     for (int mi = 0; mi < Tile::MI; ++mi)
@@ -319,17 +388,24 @@ extern "C" int braid_gemm_heads_mma(const void* x, const void* w, void* out, con
     if (((uintptr_t)x | (uintptr_t)w) & 15) BRAID_REFUSE("gemm_heads_mma: operands must start on 16 bytes");
     if (((uintptr_t)out & 3) != 0) BRAID_REFUSE("gemm_heads_mma: the output must start on 4 bytes");
     cudaStream_t s = (cudaStream_t)stream;
-    const int bm = n_rows <= 16 ? 16 : 64;
-    dim3 grid((J + 63) / 64, (n_rows + bm - 1) / bm, heads);
+    if (n_rows <= 16) {
+        const dim3 few((J + 15) / 16, heads);
+        if (few.y > 65535) BRAID_REFUSE("gemm_heads_mma: %d heads exceed the grid limit", heads);
+#define HEADS_FEW(NT, W) braid_launch(gemm_heads_few_kernel<NT, W>, few, dim3(W * 32), 0, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, \
+                                      (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, n_rows, J, K / 8, ldx, hsx, ldo, hso, ldg, mult)
+        // two warps where k is two turns of 64 numbers, else four
+        if (n_rows <= 8 && K <= 128) HEADS_FEW(1, 2);
+        else if (n_rows <= 8) HEADS_FEW(1, 4);
+        else if (K <= 128) HEADS_FEW(2, 2);
+        else HEADS_FEW(2, 4);
+#undef HEADS_FEW
+        BRAID_LAUNCH_CHECK();
+    }
+    dim3 grid((J + 63) / 64, (n_rows + 63) / 64, heads);
     if (grid.y > 65535 || grid.z > 65535) BRAID_REFUSE("gemm_heads_mma: %d rows x %d heads exceed the grid limit", n_rows, heads);
-    if (bm == 16)
-        braid_launch(gemm_heads_mma_kernel<16>, grid, dim3(128), (size_t)MmaTile<16, 64, 1, 4, 1>::SMEM_BYTES, s,
-                     (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, n_rows, J, K,
-                     ldx, hsx, ldo, hso, ldg, mult);
-    else
-        braid_launch(gemm_heads_mma_kernel<64>, grid, dim3(128), (size_t)MmaTile<64, 64, 2, 2, 1>::SMEM_BYTES, s,
-                     (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, n_rows, J, K,
-                     ldx, hsx, ldo, hso, ldg, mult);
+    braid_launch(gemm_heads_mma_kernel, grid, dim3(128), (size_t)MmaTile<64, 64, 2, 2, 1>::SMEM_BYTES, s,
+                 (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, (const __nv_bfloat16*)gate, n_rows, J, K,
+                 ldx, hsx, ldo, hso, ldg, mult);
     BRAID_LAUNCH_CHECK();
 }
 
