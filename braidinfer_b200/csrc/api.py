@@ -816,6 +816,8 @@ class Kernels:
                 lib.braid_moe_few.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong] + [c_void_p] * 3 + [c_int] * 7 + \
                                              [c_void_p, c_void_p]
                 lib.braid_moe_few.restype = c_int
+                lib.braid_moe_route_plan.argtypes = [c_void_p] * 3 + [c_int] * 5 + [c_float, c_int, c_int] + [c_void_p] * 7 + [c_int, c_int, c_void_p]
+                lib.braid_moe_route_plan.restype = c_int
                 names = ("braid_moe_gemm_mma", "braid_moe_gather", "braid_moe_gemm_tc",
                          "braid_moe_route", "braid_moe_plan", "braid_moe_gemm_simt", "braid_moe_combine")
             elif name == "conv":
@@ -1048,18 +1050,49 @@ class Kernels:
         `MOE_TC_TILE` slots come with the runs of tiles that `moe_gemm_tc` walks as a sixth."""
         lib = self.part_library("moe")
         rows, top = idx.shape
-        max_tiles = self.moe_max_tiles(rows, top, experts, tile)
-        max_wide = min(max_tiles, -(-max_tiles // 8) + experts) if tile == MOE_TC_TILE else 0
-        sizes = [4 * max_wide, max_tiles * tile, rows * top, max_tiles, 4]         # the runs first: they start on 16 bytes
-        buf = torch.empty(sum(sizes), dtype=torch.int32, device=idx.device)
-        wide, slot_pair, pair_slot, tile_expert, meta = buf.split(sizes)
+        max_tiles, max_wide, plan = self._moe_plan_buffers(rows, top, experts, tile, idx.device)
+        slot_pair, pair_slot, tile_expert, meta = plan[:4]
+        wide = plan[5] if max_wide else None
         self.launches += 1
         self._check_lib(lib, lib.braid_moe_plan(idx.data_ptr(), token_seq.data_ptr(), slot_pair.data_ptr(),
                                                 pair_slot.data_ptr(), tile_expert.data_ptr(), meta.data_ptr(),
-                                                wide.data_ptr() if max_wide else None, rows, top, experts, tile, max_tiles,
-                                                max_wide, self._stream()), "moe_plan")
+                                                _ptr(wide), rows, top, experts, tile, max_tiles, max_wide, self._stream()), "moe_plan")
+        return plan
+
+    def _moe_plan_buffers(self, rows: int, top: int, experts: int, tile: int, device):
+        """(max_tiles, max_wide, the plan's tensors) of `moe_plan`."""
+        max_tiles = self.moe_max_tiles(rows, top, experts, tile)
+        max_wide = min(max_tiles, -(-max_tiles // 8) + experts) if tile == MOE_TC_TILE else 0
+        sizes = [4 * max_wide, max_tiles * tile, rows * top, max_tiles, 4]         # the runs first: they start on 16 bytes
+        buf = torch.empty(sum(sizes), dtype=torch.int32, device=device)
+        wide, slot_pair, pair_slot, tile_expert, meta = buf.split(sizes)
         plan = (slot_pair, pair_slot, tile_expert, meta, max_tiles)
-        return plan + (wide,) if max_wide else plan
+        return max_tiles, max_wide, plan + (wide,) if max_wide else plan
+
+    @staticmethod
+    def moe_route_plan_fits(rows: int, experts: int, top: int, groups: int, tile: int) -> bool:
+        """Whether `moe_route_plan` takes a step: one CTA's tokens, registers and bits."""
+        return rows <= 8 and experts <= 256 and top <= 32 and groups <= 32 and tile == MOE_TC_TILE
+
+    def moe_route_plan(self, logits: torch.Tensor, token_seq: torch.Tensor, idx: torch.Tensor, wgt: torch.Tensor, groups: int, keep: int,
+                       mult: float = 1.0, sigmoid: bool = False, renorm: Optional[bool] = None, correction: Optional[torch.Tensor] = None):
+        """`moe_route` and `moe_plan` (tiles of `MOE_TC_TILE` slots) of a step of few tokens in one kernel; returns the plan."""
+        lib = self.part_library("moe")
+        rows, experts = logits.shape
+        top = idx.shape[1]
+        if logits.dtype != torch.float32 or not logits.is_contiguous() or idx.dtype != torch.int32 or wgt.dtype != torch.float32 \
+                or tuple(idx.shape) != (rows, top) or tuple(wgt.shape) != (rows, top) or not idx.is_contiguous() or not wgt.is_contiguous():
+            raise KernelError("moe_route_plan: logits float32 [rows, experts], idx int32 and wgt float32 [rows, top], contiguous")
+        if correction is not None and (correction.dtype != torch.float32 or correction.numel() != experts or not correction.is_contiguous()):
+            raise KernelError("moe_route_plan: the correction is float32, one number an expert")
+        max_tiles, max_wide, plan = self._moe_plan_buffers(rows, top, experts, MOE_TC_TILE, idx.device)
+        slot_pair, pair_slot, tile_expert, meta = plan[:4]
+        self.launches += 1
+        self._check_lib(lib, lib.braid_moe_route_plan(
+            logits.data_ptr(), idx.data_ptr(), wgt.data_ptr(), rows, experts, top, groups, keep, float(mult), int(sigmoid),
+            int(not sigmoid if renorm is None else renorm), _ptr(correction), token_seq.data_ptr(), slot_pair.data_ptr(), pair_slot.data_ptr(),
+            tile_expert.data_ptr(), meta.data_ptr(), plan[5].data_ptr(), max_tiles, max_wide, self._stream()), "moe_route_plan")
+        return plan
 
     @staticmethod
     def _moe_weights(w0: torch.Tensor, w1: Optional[torch.Tensor], j: int) -> Tuple[int, int, int]:

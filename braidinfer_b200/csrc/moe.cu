@@ -293,6 +293,160 @@ extern "C" int braid_moe_plan(const int* idx, const int* token_seq, int* slot_pa
     BRAID_LAUNCH_CHECK();
 }
 
+// ------------------------------------------------------------------ routing and plan of a few tokens
+// moe_route_kernel and moe_plan_kernel of a step of up to 8 tokens in one CTA: a warp routes a token, and with no expert above 8 pairs a
+// plan is bits: an expert's tile is the number of chosen experts below it, a pair's slot in it the number of earlier tokens that chose it.
+// Bound by latency (some hundred numbers): a lane holds its experts' scores in registers, and a choice is two warp-wide reductions, the
+// largest score's bits, then the lowest of the experts that have them, instead of ten shuffles.  The same numbers as the two kernels:
+// the sums are taken in their order.  8 tokens, 6 of 64 experts in 8 groups: 7.2 us and 3.8 in a step's chain, this 3.9
+// (4 tokens, 64 experts in one group: 4.1 and 3.5, this 3.2).  Larger steps keep the two kernels, whose CTAs share the tokens.
+#define MOE_RP_TOKENS 8
+#define MOE_RP_EXPERTS 256
+#define MOE_RP_TILE 32
+
+// A number's place among the floats, as an integer above 0; 0 for what can't be chosen (-inf, NaN).
+__device__ __forceinline__ uint32_t moe_key(float v) {
+    const uint32_t b = __float_as_uint(v + 0.f);             // (-0 and 0 are one)
+    return !(v > -INFINITY) ? 0u : (b & 0x80000000u) ? ~b : b | 0x80000000u;
+}
+
+template <int R>
+__global__ void __launch_bounds__(MOE_RP_TOKENS * 32)
+moe_route_plan_kernel(MoeRouteArgs a, const int* __restrict__ token_seq, int* __restrict__ slot_pair, int* __restrict__ pair_slot,
+                      int* __restrict__ tile_expert, int* __restrict__ meta, int4* __restrict__ wide, int max_tiles, int max_wide) {
+    pdl_trigger();
+    __shared__ uint32_t chosen[MOE_RP_EXPERTS / 32];         // a bit an expert
+    __shared__ uint32_t who[MOE_RP_EXPERTS];                 // an expert's tokens, a bit each
+    __shared__ float group_s[MOE_RP_TOKENS][MOE_RP_EXPERTS];
+    const int tid = threadIdx.x, row = tid >> 5, lane = tid & 31;
+    const bool live = row < a.rows;
+    who[tid] = 0;
+    if (tid < MOE_RP_EXPERTS / 32) chosen[tid] = 0;
+    const bool placed = live && token_seq[row] >= 0;         // the step's tables are there before its first kernel
+    pdl_wait();
+    for (int i = tid; i < max_tiles * MOE_RP_TILE; i += MOE_RP_TOKENS * 32) slot_pair[i] = -1;
+    __syncthreads();
+    int mine = -1;                                           // lane k: choice k
+    if (live) {
+        const float* z = a.logits + (size_t)row * a.experts;
+        float s[R];
+        uint32_t key[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) s[i] = lane + 32 * i < a.experts ? z[lane + 32 * i] : -INFINITY;
+        if (a.sigmoid) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) s[i] = 1.f / (1.f + expf(-s[i]));
+        } else {
+            float mx = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i) mx = fmaxf(mx, s[i]);
+            mx = warp_max(mx);
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (lane + 32 * i < a.experts) { s[i] = expf(s[i] - mx); sum += s[i]; }
+            const float inv = 1.f / warp_sum(sum);
+#pragma unroll
+            for (int i = 0; i < R; ++i) s[i] *= inv;
+        }
+        uint32_t kept = 0xffffffffu;                         // a bit a group
+        const int per = a.experts / a.groups;
+        if (a.keep < a.groups) {
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (lane + 32 * i < a.experts) group_s[row][lane + 32 * i] = s[i];
+            __syncwarp();
+            float m = -INFINITY;
+            if (lane < a.groups)
+                for (int i = 0; i < per; ++i) m = fmaxf(m, group_s[row][lane * per + i]);
+            // one above an expert's key: a group whose scores are no numbers is still a group
+            uint32_t gk = lane < a.groups ? moe_key(m) + 1u : 0u;
+            for (int k = 0; k < a.keep; ++k) {
+                const uint32_t best = __reduce_max_sync(0xffffffffu, gk);
+                const uint32_t who_best = __ballot_sync(0xffffffffu, gk == best);
+                if (lane == __ffs(who_best) - 1) gk = 0u;
+            }
+            kept = __ballot_sync(0xffffffffu, lane < a.groups && gk == 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int e = lane + 32 * i;
+            key[i] = 0u;
+            if (e < a.experts && (a.keep >= a.groups || (kept >> (e / per)) & 1u)) key[i] = moe_key(a.correction ? s[i] + a.correction[e] : s[i]);
+        }
+        float chosen_sum = 0.f, my_w = 0.f;
+        for (int k = 0; k < a.top; ++k) {
+            uint32_t bk = 0u;
+            int be = 0;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (key[i] > bk) { bk = key[i]; be = i; }    // an equal one further up waits
+            const uint32_t best = __reduce_max_sync(0xffffffffu, bk);
+            const int e = best ? (int)__reduce_min_sync(0xffffffffu, bk == best ? (uint32_t)(lane + 32 * be) : 0xffffffffu) : -1;
+            float w = 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                if (e == lane + 32 * i) { w = s[i]; key[i] = 0u; }
+            w = e >= 0 ? __shfl_sync(0xffffffffu, w, e & 31) : 0.f;
+            if (lane == k) { mine = e; my_w = w; }
+            chosen_sum += w;
+        }
+        const float norm = a.renorm ? a.mult / (chosen_sum + 1e-20f) : a.mult;
+        if (lane < a.top) {
+            a.idx[(size_t)row * a.top + lane] = mine;
+            a.wgt[(size_t)row * a.top + lane] = my_w * norm;
+        }
+        if (!placed) mine = -1;
+        if (mine >= 0) {
+            atomicOr(&who[mine], 1u << row);
+            atomicOr(&chosen[mine >> 5], 1u << (mine & 31));
+        }
+    }
+    __syncthreads();
+    auto below = [&](int e) {                                // chosen experts before e
+        int n = __popc(chosen[e >> 5] & ((1u << (e & 31)) - 1u));
+        for (int i = 0; i < (e >> 5); ++i) n += __popc(chosen[i]);
+        return n;
+    };
+    if (live && lane < a.top) {
+        const int pair = row * a.top + lane;
+        int slot = mine >= 0 ? below(mine) * MOE_RP_TILE + __popc(who[mine] & ((1u << row) - 1u)) : -1;
+        if (slot >= max_tiles * MOE_RP_TILE) slot = -1;
+        if (slot >= 0) slot_pair[slot] = pair;
+        pair_slot[pair] = slot;
+    }
+    if (who[tid]) {
+        const int t = below(tid);
+        if (t < max_tiles) tile_expert[t] = tid;
+        if (t < max_wide) wide[t] = make_int4(t * MOE_RP_TILE, 1, t, 1);
+    }
+    if (tid == 0) {
+        int n = 0;
+        for (int i = 0; i < MOE_RP_EXPERTS / 32; ++i) n += __popc(chosen[i]);
+        meta[0] = n < max_tiles ? n : max_tiles;
+        meta[1] = n < max_wide ? n : max_wide;
+    }
+}
+
+extern "C" int braid_moe_route_plan(const float* logits, int* idx, float* wgt, int rows, int experts, int top, int groups, int keep, float mult,
+                                    int sigmoid, int renorm, const float* correction, const int* token_seq, int* slot_pair, int* pair_slot,
+                                    int* tile_expert, int* meta, int* wide, int max_tiles, int max_wide, void* stream) {
+    if (rows <= 0) return BRAID_OK;
+    if (experts <= 0 || top <= 0 || top > experts) BRAID_REFUSE("moe_route_plan: top=%d of %d experts", top, experts);
+    if (groups <= 0 || experts % groups || keep <= 0 || keep > groups) BRAID_REFUSE("moe_route_plan: %d experts in %d groups, %d kept", experts, groups, keep);
+    if (correction && groups != 1) BRAID_REFUSE("moe_route_plan: a correction of the choice is built for experts in one group, not %d", groups);
+    if (rows > MOE_RP_TOKENS || experts > MOE_RP_EXPERTS || top > 32 || groups > 32)
+        BRAID_REFUSE("moe_route_plan: %d rows, %d choices of %d experts in %d groups are more than one CTA takes", rows, top, experts, groups);
+    if (!wide || ((uintptr_t)wide & 15)) BRAID_REFUSE("moe_route_plan: the runs of tiles must start on 16 bytes");
+    const MoeRouteArgs a{logits, idx, wgt, rows, experts, top, groups, keep, mult, sigmoid, renorm, correction};
+    cudaStream_t s = (cudaStream_t)stream;
+#define ROUTE_PLAN(R) braid_launch(moe_route_plan_kernel<R>, dim3(1), dim3(MOE_RP_TOKENS * 32), 0, s, a, token_seq, slot_pair, pair_slot, \
+                                   tile_expert, meta, (int4*)wide, max_tiles, max_wide)
+    if (experts <= 64) ROUTE_PLAN(2);
+    else ROUTE_PLAN(8);
+#undef ROUTE_PLAN
+    BRAID_LAUNCH_CHECK();
+}
+
 // ------------------------------------------------------------------ the experts' products, plain
 // Units of 16 slots x 64 outputs; 256 threads, each one slot and four outputs; float32 FMA in a fixed
 // order along k.  MODE 0: act[slot, j] = silu(x[token] . gate_e[j]) * (x[token] . up_e[j]), the input rows

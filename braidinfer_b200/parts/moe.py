@@ -161,10 +161,13 @@ class MixtureOfExperts(FeedForward):
         logits = self.router.forward(x, out_dtype=torch.float32)
         idx = torch.empty((rows, self.top), dtype=torch.int32, device=x.device)
         wgt = torch.empty((rows, self.top), dtype=torch.float32, device=x.device)
-        K.moe_route(logits, idx, wgt, self.groups, self.keep, mult=self.out_mult, sigmoid=self.scoring == "sigmoid",
-                    renorm=self.normalize, correction=self.correction)
         tile = self.tile(x)
-        plan = K.moe_plan(idx, ctx.token_seq, self.experts, tile)
+        how = dict(mult=self.out_mult, sigmoid=self.scoring == "sigmoid", renorm=self.normalize, correction=self.correction)
+        if K.moe_route_plan_fits(rows, self.experts, self.top, self.groups, tile):
+            plan = K.moe_route_plan(logits, ctx.token_seq, idx, wgt, self.groups, self.keep, **how)
+        else:
+            K.moe_route(logits, idx, wgt, self.groups, self.keep, **how)
+            plan = K.moe_plan(idx, ctx.token_seq, self.experts, tile)
         slots = plan[4] * tile
         act = self.rt.empty(slots, self.inter)
         y = self.rt.empty(slots, self.hidden)
