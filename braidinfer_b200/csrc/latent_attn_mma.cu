@@ -261,7 +261,7 @@ latent_attn_few_kernel(LatAttnArgs a) {
     __nv_bfloat16* Ks = Qs + FEW_ROWS * LDK;
     float* Sp = (float*)(Ks + 2 * BN * LDK);             // [2][4 warps][16][SP_LD]
     pdl_trigger();
-    pdl_wait();
+    // up to pdl_wait() only the step's tables and keys cached by earlier steps are read, which no kernel of this step writes
     const int seq = blockIdx.y, split = blockIdx.z;
     const int pairs = a.q_len[seq] * a.heads;
     const int pair0 = blockIdx.x * FEW_ROWS;
@@ -279,14 +279,6 @@ latent_attn_few_kernel(LatAttnArgs a) {
     const int my_lo = tile_lo + split * per;
     const int my_hi = min(tile_hi, my_lo + per - 1);
     constexpr int CH = D / 8;
-    {
-        const __nv_bfloat16* src = a.q + base_pair * D;
-        for (int c = tid; c < FEW_ROWS * CH; c += 128) {
-            const int r = c / CH, kc = (c - r * CH) * 8;
-            const bool ok = r < n_here;
-            mt_cp_async16(Qs + r * LDK + kc, ok ? src + (size_t)r * D + kc : a.q, ok ? 16 : 0);
-        }
-    }
     const int* table = a.page_table + (size_t)seq * a.table_cols;
     auto load_keys = [&](int tile, int stage) {
         const int j0 = tile * BN;
@@ -303,7 +295,20 @@ latent_attn_few_kernel(LatAttnArgs a) {
             mt_cp_async16(dst + r * LDK + kc, src + (size_t)r * D + kc, 16);
         }
     };
-    if (my_lo <= my_hi) load_keys(my_lo, 0);
+    auto cached = [&](int tile) { return tile <= my_hi && (tile + 1) * BN <= before; };
+    const bool early0 = cached(my_lo), early1 = cached(my_lo + 1);
+    if (early0) load_keys(my_lo, 0);
+    if (early1) load_keys(my_lo + 1, 1);
+    pdl_wait();
+    if (my_lo <= my_hi && !early0) load_keys(my_lo, 0);
+    {
+        const __nv_bfloat16* src = a.q + base_pair * D;
+        for (int c = tid; c < FEW_ROWS * CH; c += 128) {
+            const int r = c / CH, kc = (c - r * CH) * 8;
+            const bool ok = r < n_here;
+            mt_cp_async16(Qs + r * LDK + kc, ok ? src + (size_t)r * D + kc : a.q, ok ? 16 : 0);
+        }
+    }
     mt_commit();
     const int g = lane >> 2, qd = lane & 3;
     int pos_row[2];
@@ -323,7 +328,7 @@ latent_attn_few_kernel(LatAttnArgs a) {
     for (int tile = my_lo; tile <= my_hi; ++tile) {
         const int it = tile - my_lo, stage = it & 1;
         if (tile + 1 <= my_hi) {
-            load_keys(tile + 1, stage ^ 1);
+            if (it > 0 || !early1) load_keys(tile + 1, stage ^ 1);
             mt_commit();
             mt_wait<1>();
         } else {
@@ -444,13 +449,20 @@ __global__ void __launch_bounds__(128)
 latent_attn_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, const int* __restrict__ token_seq,
                          int heads, int total_pairs, int n_splits, const float* __restrict__ sinks) {
     pdl_trigger();
-    pdl_wait();
     __shared__ float wgt[LAT_MERGE_MAX_SPLITS];
     __shared__ float inv_s;
     const int pair = blockIdx.x;
-    if (token_seq[pair / heads] < 0) return;             // a padding row: nothing was computed for it
+    const bool padding = token_seq[pair / heads] < 0;    // the step's table: there before its first kernel
+    pdl_wait();
+    if (padding) return;                                 // nothing was computed for it
     const size_t stride = (size_t)total_pairs * (R + 4);
     const float* base = partial + (size_t)pair * (R + 4);
+    constexpr int B = 8;                                 // slices asked for together with the maxima and sums
+    const int c0 = threadIdx.x * 4;
+    float4 first[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i)
+        first[i] = i < n_splits && c0 < R ? *reinterpret_cast<const float4*>(base + i * stride + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (threadIdx.x < 32) {
         float m[2], l[2];
 #pragma unroll
@@ -472,10 +484,20 @@ latent_attn_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __res
     }
     __syncthreads();
     const float inv = inv_s;
-    for (int c = threadIdx.x * 4; c < R; c += 128 * 4) {
+    for (int c = c0; c < R; c += 128 * 4) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        int done = 0;
+        if (c == c0) {
+#pragma unroll
+            for (int i = 0; i < B; ++i) {
+                const float w = i < n_splits ? wgt[i] : 0.f;
+                acc.x = fmaf(w, first[i].x, acc.x); acc.y = fmaf(w, first[i].y, acc.y);
+                acc.z = fmaf(w, first[i].z, acc.z); acc.w = fmaf(w, first[i].w, acc.w);
+            }
+            done = B;
+        }
 #pragma unroll 8
-        for (int s_ = 0; s_ < n_splits; ++s_) {
+        for (int s_ = done; s_ < n_splits; ++s_) {
             const float4 v = *reinterpret_cast<const float4*>(base + s_ * stride + c);
             const float w = wgt[s_];
             acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y);
