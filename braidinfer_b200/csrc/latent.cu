@@ -41,7 +41,9 @@ struct LatentPrepArgs {
 
 // A CTA a row.  V neighbouring numbers a thread and turn (16 bytes, or one number where a size or stride does not allow it); the
 // first two runs of a thread stay in registers between the sums of squares and the results, and both norms' sums meet in one round.
-template <typename T, int V, int NT>
+// A few rows (SPLIT) have one CTA for the norms and others for the rotation, a pair a thread: bound by latency, the norms' weights and the
+// angles are there before the wait.  (In prompts the registers for those cost more than they give: 2,048 rows 15.5 us, without them 12.5.)
+template <typename T, int V, int NT, bool SPLIT>
 __global__ void __launch_bounds__(NT)
 latent_prep_kernel(LatentPrepArgs a) {
     pdl_trigger();
@@ -66,11 +68,29 @@ latent_prep_kernel(LatentPrepArgs a) {
     }
     // c = x / sqrt(mean(x^2) + eps) * w where there is a cache to write (a layer that reads another layer's latent has no c and
     // no kr in its rows), and the same for the queries' low-rank part where the rows have one: runs [0, nq) and [nq, nq + nc)
+    const bool norms = !SPLIT || blockIdx.y == 0, turns = !SPLIT || blockIdx.y > 0;
     const int nq = a.dq_out ? a.q_rank / V : 0, nc = a.cache ? a.rank / V : 0;
     constexpr int KEEP = 2;
-    float v[KEEP][V];
+    float v[KEEP][V], wk[SPLIT ? KEEP : 1][V];
+    auto weights = [&](int run, float* w) { load_run<T, V>(run < nq ? (const T*)a.dq_w + run * V : (const T*)a.norm_w + (run - nq) * V, w); };
+    // rotation: element i pairs with i + rot_dims/2 (or, `adjacent`, 2i with 2i + 1); vector 0 is the shared key
+    // part, 1.. are the heads' queries
+    const int half = a.rot_dims / 2;
+    const int per = half + (a.rot - a.rot_dims);           // work items a vector: pairs, then untouched elements
+    const int first = SPLIT && turns ? ((int)blockIdx.y - 1) * NT + tid : tid, stride = SPLIT ? ((int)gridDim.y - 1) * NT : NT;
+    const int last = turns ? (a.heads + 1) * per : 0;      // (0: nothing for the norms' CTA)
+    float sn = 0.f, cs = 1.f;
+    auto angle = [&](int e) {
+        const int p = e - e / per * per;
+        if (p < half) sincosf((float)pos * a.inv_freq[p], &sn, &cs);
+    };
+    if (SPLIT && first < last) angle(first);
+    if (SPLIT && norms)
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (tid + k * NT < nq + nc) weights(tid + k * NT, wk[SPLIT ? k : 0]);
     pdl_wait();
-    if (nq + nc > 0) {
+    if (norms && nq + nc > 0) {
         float2 ss = make_float2(0.f, 0.f);
         auto take = [&](int run, float* x) {
             load_run<T, V>(run < nq ? src + (size_t)run * V : cin + (size_t)(run - nq) * V, x);
@@ -95,40 +115,38 @@ latent_prep_kernel(LatentPrepArgs a) {
 #pragma unroll
         for (int w = 0; w < NT / 32; ++w) { sq += red[w].x; sc += red[w].y; }
         const float rq = 1.f / sqrtf(sq / (float)max(a.q_rank, 1) + a.eps), rc = 1.f / sqrtf(sc / (float)a.rank + a.eps);
-        auto give = [&](int run, const float* x) {
+        auto give = [&](int run, const float* x, const float* w) {
             const bool q = run < nq;
             const int i = (q ? run : run - nq) * V;
             T* out = q ? (T*)a.dq_out + (size_t)row * a.dq_ld : dst;
             if (!out) return;
-            float w[V], y[V];
-            load_run<T, V>((const T*)(q ? a.dq_w : a.norm_w) + i, w);
+            float y[V];
 #pragma unroll
             for (int e = 0; e < V; ++e) y[e] = x[e] * (q ? rq : rc) * w[e];
             store_run<T, V>(out + i, y);
         };
 #pragma unroll
         for (int k = 0; k < KEEP; ++k)
-            if (tid + k * NT < nq + nc) give(tid + k * NT, v[k]);
+            if (tid + k * NT < nq + nc) {
+                if (!SPLIT) weights(tid + k * NT, wk[0]);
+                give(tid + k * NT, v[k], wk[SPLIT ? k : 0]);
+            }
         for (int run = tid + KEEP * NT; run < nq + nc; run += NT) {
-            float x[V];
+            float x[V], w[V];
             load_run<T, V>(run < nq ? src + (size_t)run * V : cin + (size_t)(run - nq) * V, x);
-            give(run, x);
+            weights(run, w);
+            give(run, x, w);
         }
         if (a.dq_out)                                          // what the low-rank rows are padded with
             for (int i = a.q_rank + tid; i < a.dq_ld; i += NT) ((T*)a.dq_out)[(size_t)row * a.dq_ld + i] = from_f32<T>(0.f);
     }
-    // rotation: element i pairs with i + rot_dims/2 (or, `adjacent`, 2i with 2i + 1); vector 0 is the shared key
-    // part, 1.. are the heads' queries
-    const int half = a.rot_dims / 2;
-    const int per = half + (a.rot - a.rot_dims);           // work items a vector: pairs, then untouched elements
-    for (int e = threadIdx.x; e < (a.heads + 1) * per; e += blockDim.x) {
+    for (int e = first; e < last; e += stride) {
+        if (!SPLIT || e != first) angle(e);
         const int v = e / per, p = e - v * per;
         const T* in = (v == 0) ? kin : src + (size_t)(v - 1) * (a.dim + a.rot) + a.dim;
         T* out = (v == 0) ? (dst ? dst + a.rank : nullptr) : (T*)a.q_lat + ((size_t)row * a.heads + (v - 1)) * D + a.rank;
         if (!out) continue;
         if (p < half) {
-            float sn, cs;
-            sincosf((float)pos * a.inv_freq[p], &sn, &cs);
             const int i0 = a.adjacent ? 2 * p : p, i1 = a.adjacent ? 2 * p + 1 : p + half;
             const float x0 = to_f32(in[i0]), x1 = to_f32(in[i1]);
             out[i0] = from_f32<T>(x0 * cs - x1 * sn);
@@ -160,10 +178,15 @@ extern "C" int braid_latent_prep(const void* proj, long long ld, int q_cols, con
                       (((uintptr_t)proj | (uintptr_t)norm_w | (uintptr_t)cache | (uintptr_t)dq_out | (uintptr_t)dq_w) & 15) == 0;
     // 256 threads a row where the norms have that much to do, or where rows are few and a row's way is what counts
     const bool big = rows <= 64 || (dq_out ? q_rank : 0) + rank > 128 * vec;
+    // up to 64 rows the rotation has CTAs of its own: 8 rows of 16 heads, 512 latent and 64 rotated numbers 4.5 -> 3.0 us in a step's chain;
+    // with more rows the machine is full without
+    const long long items = (long long)(heads + 1) * (rot_dims / 2 + rot - rot_dims);
+    const int parts = rows <= 64 && items > 0 ? 1 + (int)((items + 255) / 256 < 8 ? (items + 255) / 256 : 8) : 1;
 #define LP_LAUNCH(T, V)                                                                                     \
     do {                                                                                                    \
-        if (big) braid_launch(latent_prep_kernel<T, V, 256>, dim3(rows), dim3(256), 0, s, a);               \
-        else braid_launch(latent_prep_kernel<T, V, 128>, dim3(rows), dim3(128), 0, s, a);                   \
+        if (parts > 1) braid_launch(latent_prep_kernel<T, V, 256, true>, dim3(rows, parts), dim3(256), 0, s, a); \
+        else if (big) braid_launch(latent_prep_kernel<T, V, 256, false>, dim3(rows), dim3(256), 0, s, a);   \
+        else braid_launch(latent_prep_kernel<T, V, 128, false>, dim3(rows), dim3(128), 0, s, a);            \
     } while (0)
     if (dtype == BRAID_F32 && wide) LP_LAUNCH(float, 4);
     else if (dtype == BRAID_F32) LP_LAUNCH(float, 1);
