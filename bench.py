@@ -825,7 +825,7 @@ def bidinex_kernels(z, T, B, C, timed, frac):
     o = torch.empty(B, H, R, device=dev, dtype=bf)
     seqs = torch.arange(B, dtype=torch.int32, device=dev)
     ones, befores, starts = i32([1] * B), i32([C - 1] * B), i32(list(range(B)))
-    n_splits = max(1, min(296 // K.attn_latent_ctas(R, rot, B, 1, H), (C // 32) // 4, 32))
+    n_splits = max(1, min(296 // K.attn_latent_ctas(R, rot, B, 1, H), (C // 32) // 2, 32))
     t = timed(lambda: K.attn_latent_mma(q, o, cache, table, starts, ones, befores, seqs, B, 1, R, None, 0.1, n_splits=n_splits), reps=9, graph=True)
     res["decode_attention"] = {"latent_mma_ms": round(t * 1e3, 4), "latent_frac": round(frac(t, 0, B * C * D * 2), 3), "slices": n_splits}
     dcache, dtable = paged(B, C, 2, nkh, hd)
@@ -1559,7 +1559,7 @@ def ludazen_kernels(z, T, B, C, timed, frac):
             span = min(before + each, w) if w else before + each
             sp = 1
             if each <= 8:
-                sp = max(1, min(296 // K.attn_latent_ctas(R, rot, n_seqs, each, H), (span // 32) // 4, 32))
+                sp = max(1, min(296 // K.attn_latent_ctas(R, rot, n_seqs, each, H), (span // 32) // 2, 32))
             t = timed(lambda: K.attn_latent_mma(q, o, cache, table, st.q_start, st.q_len, st.kv_before, st.token_seq, n_seqs, each, R, w,
                                                 0.1, n_splits=sp), graph=True)
             seen = sum(min(p + 1, w) if w else p + 1 for p in range(before, before + each)) * n_seqs
@@ -2070,7 +2070,7 @@ def megerax_kernels(name, T, B, C, timed, frac):
         D = R + rot
         cache, table = paged(n_seqs, length, 1, 1, D)
         ql, ol, sinks = rnd(rows, LH, D) * 0.3, torch.empty(rows, LH, R, device=dev, dtype=bf), torch.randn(LH, device=dev)
-        sp = max(1, min(296 // K.attn_latent_ctas(R, rot, n_seqs, each, LH), (length // 32) // 4, 32)) if few else 1
+        sp = max(1, min(296 // K.attn_latent_ctas(R, rot, n_seqs, each, LH), (length // 32) // 2, 32)) if few else 1
         fl, by = 2 * LH * (D + R) * sum(range(length - each + 1, length + 1)) * n_seqs, n_seqs * length * D * 2
         lat = lambda **kw: timed(lambda: K.attn_latent_mma(ql, ol, cache, table, stp.q_start, stp.q_len, stp.kv_before, stp.token_seq, n_seqs, each,     # noqa: E731
                                                            R, None, 0.1, n_splits=sp, **kw), reps=7, graph=True)
