@@ -1626,6 +1626,11 @@ class Kernels:
                 raise KernelError("linear_scan: constant decays are float32, one number a head")
         else:
             raise KernelError(f"linear_scan: unknown decay mode {mode!r}")
+        # (before any route is taken: the kernels of the routes below know neither)
+        if act_silu and mode != "constant":
+            raise KernelError("linear_scan: silu on what is given goes with a constant decay a head")
+        if v_cols is not None and 0 < v_cols < dv and mode != "given":
+            raise KernelError("linear_scan: value columns that read as 1 need given decays")
         vc = dv if v_cols is None else int(v_cols)
         if v.shape[1] < heads * vc or (out is not None and out.shape[1] < heads * dv):
             raise KernelError("linear_scan: v or out does not hold the heads' columns")

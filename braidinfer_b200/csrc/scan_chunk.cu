@@ -445,6 +445,7 @@ extern "C" int braid_scan_chunk(const void* q, long long q_stride, const void* k
     if (((uintptr_t)out & 7) || out_stride % 2 || !state || (((uintptr_t)state | (uintptr_t)state_offset | (uintptr_t)state_stride) & 15))
         BRAID_REFUSE("scan_chunk: results must start on 8 bytes and the state on 16");
     if (!gate || (!constant && !gate_is_decay && !gate_bias)) BRAID_REFUSE("scan_chunk: the decays are missing");
+    if (act_silu && !constant) BRAID_REFUSE("scan_chunk: silu on what is given goes with a constant decay a head");
     const long long need = braid_scan_chunk_work_floats(rows, n_seqs, heads, dk, dv);
     if (!work || need > work_floats || ((uintptr_t)work & 15)) BRAID_REFUSE("scan_chunk: needs %lld floats of scratch on 16 bytes, it was given %lld", need, work_floats);
     const int chunks = (max_q_len + CHK_C - 1) / CHK_C;

@@ -164,6 +164,7 @@ extern "C" int braid_scan_step(const void* q, long long q_stride, const void* k,
     if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("scan_step: %d heads do not divide into %d groups", heads, groups);
     if ((dk != 64 && dk != 128) || dv <= 0 || dv % 64) BRAID_REFUSE("scan_step: built for keys of 64 or 128 and values in multiples of 64, not %d x %d", dk, dv);
     if (mode != STEP_CHANNEL && mode != STEP_HEAD && mode != STEP_CONST) BRAID_REFUSE("scan_step: unknown decay mode %d", mode);
+    if (act_silu && mode != STEP_CONST) BRAID_REFUSE("scan_step: silu on what is given goes with a constant decay a head");
     if (dtype != BRAID_F32 && dtype != BRAID_BF16) BRAID_REFUSE("scan_step: unknown dtype code %d", dtype);
     if (!state || (((uintptr_t)state | (uintptr_t)state_offset | (uintptr_t)state_stride) & 15)) BRAID_REFUSE("scan_step: the state must start on 16 bytes");
     const uintptr_t rows = dtype == BRAID_F32 ? 15 : 7;

@@ -1,0 +1,64 @@
+"""Which kernels a call of the recurrences reaches (csrc/api.py), on the CPU: a library that notes the entry points it is asked for and
+launches nothing."""
+import types
+
+import pytest
+import torch
+
+from braidinfer_b200.csrc.api import KernelError, Kernels
+
+BF = torch.bfloat16
+
+
+class Entries:
+    """Every entry point, returning 0 and noting its name and arguments."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *args: self.calls.append((name, args)) or 0
+
+    def names(self):
+        return [n for n, _ in self.calls]
+
+
+@pytest.fixture
+def K(monkeypatch):
+    k = object.__new__(Kernels)
+    k.launches, k.entries = 0, Entries()
+    monkeypatch.setattr(k, "part_library", lambda name: k.entries, raising=False)
+    monkeypatch.setattr(k, "_stream", lambda: 0, raising=False)
+    return k
+
+
+def step(lens):
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32)
+    return types.SimpleNamespace(n_seqs=len(lens), max_q_len=max(lens), q_start=i32([sum(lens[:i]) for i in range(len(lens))]),
+                                 q_len=i32(lens), slot_ids=i32(list(range(len(lens)))))
+
+
+def scan(K, mode, lens, heads=2, dk=128, dv=64, dtype=BF, v_cols=None, **how):
+    rows = sum(lens)
+    vc = dv if v_cols is None else v_cols
+    q, k, v = (torch.zeros(rows, n, dtype=dtype) for n in (heads * dk, heads * dk, heads * vc))
+    gate = {"channel": torch.zeros(rows, heads * dk), "head": torch.zeros(rows, heads, dtype=dtype), "constant": torch.zeros(heads)}[mode]
+    bias = torch.zeros(heads * dk if mode == "channel" else heads, dtype=dtype)
+    state = torch.zeros(len(lens), heads * dk * dv * 4, dtype=torch.uint8)
+    K.linear_scan(q, k, v, gate, None if mode == "constant" else bias, torch.zeros(rows, heads * dv), state, 0, step(lens), heads, heads, dk, dv,
+                  mode, a_log=torch.zeros(heads, dtype=dtype) if mode == "head" else None, v_cols=v_cols, **how)
+    return [n for n in K.entries.names() if not n.endswith("_floats")]
+
+
+# one token a sequence, a short prompt, a prompt over chunks
+@pytest.mark.parametrize("lens", [[1, 1], [20], [300]])
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+@pytest.mark.parametrize("mode", ["channel", "head", "constant"])
+def test_options_of_another_mode_are_refused_on_every_route(K, mode, dtype, lens):
+    scan(K, mode, lens, dtype=dtype)
+    if mode != "constant":
+        with pytest.raises(KernelError):
+            scan(K, mode, lens, dtype=dtype, act_silu=True)
+    with pytest.raises(KernelError):
+        scan(K, mode, lens, dtype=dtype, v_cols=48)
+    assert len([n for n in K.entries.names() if not n.endswith("_floats")]) == 1            # the refused calls reached no kernel
