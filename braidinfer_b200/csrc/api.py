@@ -1544,16 +1544,17 @@ class Kernels:
                 and (state.data_ptr() | int(state_offset) | state.stride(0)) % 16 == 0)
 
     @classmethod
-    def step_norm_fits(cls, dv: int, *rows: torch.Tensor) -> bool:
-        """Whether the kernels of one token a sequence can also do the gated norm of a head's dv columns, gates and results in `rows`."""
-        return dv in cls.STEP_NORM_COLS and all(t.stride(-1) == 1 and t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0
-                                                for t in rows)
+    def step_norm_fits(cls, dv: int, *rows: torch.Tensor, w: Optional[torch.Tensor] = None) -> bool:
+        """Whether the kernels of one token a sequence can also do the gated norm of a head's dv columns, gates and results in `rows`; `w`: the
+        norm's weights where the kernel moves four of them at a time (`linear_scan`; `delta_rule` takes them wherever they start)."""
+        return dv in cls.STEP_NORM_COLS and (w is None or w.data_ptr() % (4 * w.element_size()) == 0) \
+            and all(t.stride(-1) == 1 and t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0 for t in rows)
 
     def _scan_step(self, lib, q, k, v, gate, gate_bias, out, state, state_offset, ctx, heads, groups, dk, dv, mode, q_scale, inv_tau,
                    a_log, skip, act_silu, norm) -> None:
         z, w, y, eps, out_scale = norm if norm is not None else (None, None, None, 0.0, 1.0)
         if norm is not None and (not z.dtype == w.dtype == y.dtype == q.dtype or w.numel() != dv or z.shape[1] < heads * dv
-                                 or y.shape[1] < heads * dv or not self.step_norm_fits(dv, z, y)):
+                                 or y.shape[1] < heads * dv or not self.step_norm_fits(dv, z, y, w=w)):
             raise KernelError("linear_scan: gates, weights and results of the norm have the rows' element type and hold the heads' columns")
         self.launches += 1
         self._check_lib(lib, lib.braid_scan_step(

@@ -103,7 +103,7 @@ class GatedLinearAttention(Mixer):
         z = self.a2.forward(a1, out_dtype=torch.float32)                # the decay's logit, before its bias
         padded = ctx.rows > ctx.n_tokens
         y = torch.zeros((rows, H * dv), dtype=x.dtype, device=x.device) if padded else self.rt.empty(rows, H * dv)
-        if K.scan_step_fits(v, state, 0, ctx, dk, dv) and K.step_norm_fits(dv, g, y):
+        if K.scan_step_fits(v, state, 0, ctx, dk, dv) and K.step_norm_fits(dv, g, y, w=self.norm_w):
             # one token a sequence: recurrence and norm in one kernel
             K.linear_scan(q, k, v, z, self.a2_bias, None, state, 0, ctx, H, H, dk, dv, "channel", q_scale=dk ** -0.5,
                           inv_tau=1.0 / self.tau, norm=(g, self.norm_w, y, self.eps, self.out_mult))

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from braidinfer_b200.csrc.api import KernelError, Kernels
+from braidinfer_b200.parts.linear_attention import GatedLinearAttention
 
 BF = torch.bfloat16
 
@@ -62,3 +63,21 @@ def test_options_of_another_mode_are_refused_on_every_route(K, mode, dtype, lens
     with pytest.raises(KernelError):
         scan(K, mode, lens, dtype=dtype, v_cols=48)
     assert len([n for n in K.entries.names() if not n.endswith("_floats")]) == 1            # the refused calls reached no kernel
+
+
+# a view into a packed buffer may start anywhere: the kernel that also does the norm moves four of its weights at a time
+@pytest.mark.parametrize("dtype", [BF, torch.float32])
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+def test_norm_weights_that_start_anywhere(K, dtype, off):
+    H, dk, dv, rank = 2, 64, 128, 8
+    part = object.__new__(GatedLinearAttention)
+    rows = lambda n, dt=dtype: types.SimpleNamespace(forward=lambda x, **how: torch.zeros(x.shape[0], n, dtype=how.get("out_dtype", dt)))
+    part.rt = types.SimpleNamespace(kernels=K, empty=lambda *s: torch.empty(*s, dtype=dtype))
+    part.heads, part.dk, part.dv, part.rank, part.tau, part.eps, part.out_mult = H, dk, dv, rank, 16.0, 1e-6, 1.0
+    part.cols = [H * dk, H * dk, H * dv, H * dv, rank]
+    part.proj, part.a2, part.o = rows(sum(part.cols)), rows(H * dk), rows(64)
+    part.a2_bias, part.norm_w = torch.zeros(H * dk, dtype=dtype), torch.zeros(dv + off, dtype=dtype)[off:]
+    ctx = step([1, 1, 1])
+    ctx.rows, ctx.n_tokens, ctx.token_seq = 3, 3, torch.arange(3, dtype=torch.int32)
+    part.forward(torch.zeros(3, 64, dtype=dtype), torch.zeros(3, 64), ctx, None, torch.zeros(3, part.state_bytes(), dtype=torch.uint8))
+    assert K.entries.names() == (["braid_scan_step"] if off % 4 == 0 else ["braid_scan_step", "braid_gated_norm"])
