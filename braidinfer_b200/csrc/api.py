@@ -773,7 +773,7 @@ class Kernels:
                          "braid_latent_attn_tc", "braid_latent_attn_tc_supported")
             elif name == "scan":
                 lib.braid_causal_conv.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
-                                                  c_void_p, c_longlong, c_longlong] + [c_void_p] * 4 + [c_int] * 6 + [c_void_p]
+                                                  c_void_p, c_longlong, c_longlong] + [c_void_p] * 4 + [c_int] * 7 + [c_void_p]
                 lib.braid_linear_scan.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 3 + [c_void_p, c_longlong] + \
                                                  [c_void_p, c_longlong, c_longlong] + [c_void_p] * 3 + [c_int] * 7 + \
                                                  [c_float, c_float, c_int, c_int, c_void_p, c_longlong, c_int, c_void_p, c_int,
@@ -785,7 +785,7 @@ class Kernels:
                 lib.braid_scan_decay.argtypes = [c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_float, c_void_p]
                 lib.braid_linear_scan_work_floats.argtypes = [c_int] * 7
                 lib.braid_ssd_scan.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 4 + [c_longlong, c_void_p, c_longlong, c_longlong] + \
-                                              [c_void_p] * 3 + [c_int] * 5 + [c_float, c_void_p]
+                                              [c_void_p] * 3 + [c_int] * 5 + [c_float, c_int, c_void_p]
                 lib.braid_ssd_scan.restype = c_int
                 lib.braid_scan_chunk.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] + [c_void_p, c_longlong] * 2 + [c_longlong] + \
                                                 [c_void_p] * 3 + [c_int] * 7 + [c_float, c_float] + [c_int] * 3 + \
@@ -793,7 +793,7 @@ class Kernels:
                 lib.braid_scan_chunk.restype = c_int
                 lib.braid_scan_step.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p] * 3 + [c_void_p, c_longlong] * 2 + [c_longlong] + \
                                                [c_void_p] * 3 + [c_int] * 7 + [c_float, c_float, c_int, c_void_p, c_longlong, c_void_p,
-                                                                               c_void_p, c_longlong, c_int, c_float, c_float, c_void_p]
+                                                                               c_void_p, c_longlong, c_int, c_float, c_float, c_int, c_void_p]
                 lib.braid_scan_step.restype = c_int
                 lib.braid_scan_chunk_work_floats.argtypes = [c_int] * 5
                 lib.braid_scan_chunk_work_floats.restype = c_longlong
@@ -828,11 +828,11 @@ class Kernels:
             elif name == "delta":
                 lib.braid_delta_step.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p, c_void_p, c_void_p, c_longlong, c_int] + \
                                                 [c_void_p, c_longlong] * 2 + [c_longlong] + [c_void_p] * 3 + [c_int] * 5 + \
-                                                [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_float, c_void_p]
+                                                [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_float, c_int, c_void_p]
                 lib.braid_delta_step.restype = c_int
                 lib.braid_delta_rule.argtypes = [c_void_p, c_longlong] * 4 + [c_void_p, c_void_p, c_void_p, c_longlong, c_int,
                                                  c_void_p, c_longlong, c_void_p, c_longlong, c_longlong] + [c_void_p] * 3 + \
-                                                [c_int] * 7 + [c_void_p, c_longlong, c_void_p]
+                                                [c_int] * 7 + [c_void_p, c_longlong, c_int, c_void_p]
                 lib.braid_delta_gated_norm.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_longlong,
                                                        c_void_p] + [c_int] * 4 + [c_float, c_void_p]
                 lib.braid_delta_work_floats.argtypes = [c_int] * 5
@@ -1237,7 +1237,7 @@ class Kernels:
             lib = ctypes.CDLL(str(build.latent_attention_library(rank, rot, verbose=self._verbose)))
             lib.braid_last_error.restype = c_char_p
             lib.braid_latent_attn_mma.restype = c_int
-            lib.braid_latent_attn_mma.argtypes = [c_void_p] * 9 + [c_int] * 9 + [c_float, c_void_p, c_void_p, c_void_p]
+            lib.braid_latent_attn_mma.argtypes = [c_void_p] * 9 + [c_int] * 9 + [c_float, c_void_p, c_int, c_void_p, c_void_p]
             lib.braid_latent_attn_partial_floats.restype = c_longlong
             lib.braid_latent_attn_partial_floats.argtypes = [c_int, c_int, c_int]
             lib.vparts = lib.braid_latent_attn_vparts()
@@ -1259,10 +1259,11 @@ class Kernels:
     def attn_latent_mma(self, q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, page_table: torch.Tensor,
                         q_start: torch.Tensor, q_len: torch.Tensor, kv_before: torch.Tensor, token_seq: torch.Tensor,
                         n_seqs: int, max_q_len: int, rank: int, window: Optional[int], scale: float,
-                        n_splits: int = 1, sinks: Optional[torch.Tensor] = None, row0: int = 0) -> None:
+                        n_splits: int = 1, sinks: Optional[torch.Tensor] = None, row0: int = 0, settled: bool = False) -> None:
         """`attn_latent_simple` in bfloat16 on the tensor cores.  Rows of padding are not written.  `row0`: q_lat, out and
         token_seq begin at that row of the step, the tables are of the sequences whose rows those are.  `n_splits` > 1
-        slices the context (steps of few tokens) and merges the slices in a second kernel."""
+        slices the context (steps of few tokens) and merges the slices in a second kernel.  `settled`: the keys of
+        earlier steps are in memory whatever kernels still run (`StepContext.settled`)."""
         rows, heads, d = q_lat.shape
         lib = self.latent_attention_library(rank, d - rank)
         self._check_pages(cache)
@@ -1284,7 +1285,7 @@ class Kernels:
         self._check_lib(lib, lib.braid_latent_attn_mma(
             q_lat.data_ptr(), out.data_ptr(), _ptr(partial), cache.data_ptr(), page_table.data_ptr(), q_start.data_ptr(),
             q_len.data_ptr(), kv_before.data_ptr(), token_seq.data_ptr(), rows, int(row0), n_seqs, max_q_len, heads,
-            page_table.shape[1], cache.shape[0], int(window or 0), n_splits, float(scale), _ptr(sinks),
+            page_table.shape[1], cache.shape[0], int(window or 0), n_splits, float(scale), _ptr(sinks), int(settled),
             self._error_flag.data_ptr() + 16, self._stream()), "attn_latent_mma")
 
     def moe_combine(self, h: torch.Tensor, y: torch.Tensor, plan, wgt: Optional[torch.Tensor], top: Optional[int] = None) -> None:
@@ -1364,6 +1365,12 @@ class Kernels:
             raise KernelError("a state area is a uint8 tensor [slots, bytes]")
         return state.data_ptr(), state.stride(0), int(offset)
 
+    @staticmethod
+    def _settled(ctx) -> int:
+        """Whether a kernel may read its state before the kernels ahead of it in the stream have ended (`StepContext.settled`): not
+        unless the step says so."""
+        return int(getattr(ctx, "settled", False))
+
     def causal_conv(self, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], state: torch.Tensor,
                     state_offset: int, ctx, silu: bool = True) -> None:
         """y[t, c] = act(b[c] + sum_j w[c, j] x[t - (taps - 1 - j), c]) along each sequence of the step (x, y
@@ -1385,7 +1392,7 @@ class Kernels:
             x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), w.data_ptr(), _ptr(b), dtype_code(x.dtype),
             *self._state_args(state, state_offset), ctx.token_seq.data_ptr(), ctx.q_start.data_ptr(),
             ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), rows, ctx.n_seqs, channels, taps, int(silu), int(one),
-            self._stream()),
+            self._settled(ctx), self._stream()),
             "causal_conv")
 
     @staticmethod
@@ -1478,7 +1485,7 @@ class Kernels:
                 out.stride(0) if out is not None else 0, *self._state_args(state, state_offset), ctx.q_start.data_ptr(),
                 ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), ctx.n_seqs, heads, groups, dk, dv, _ptr(gate),
                 gate.stride(0) if gate is not None else 0, _ptr(w), _ptr(y), y.stride(0) if y is not None else 0, float(eps),
-                self._stream()), "delta_step")
+                self._settled(ctx), self._stream()), "delta_step")
             return
         rows = out.shape[0]
         need = lib.braid_delta_work_floats(rows, ctx.n_seqs, heads, dk, dv) if chunked else 0
@@ -1488,7 +1495,7 @@ class Kernels:
             q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), z.data_ptr(), z.stride(0),
             bias.data_ptr(), rate.data_ptr(), b.data_ptr(), b.stride(0), dtype_code(b.dtype), out.data_ptr(), out.stride(0),
             *self._state_args(state, state_offset), ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), rows,
-            ctx.n_seqs, int(ctx.max_q_len), heads, groups, dk, dv, _ptr(work), need, self._stream()), "delta_rule")
+            ctx.n_seqs, int(ctx.max_q_len), heads, groups, dk, dv, _ptr(work), need, self._settled(ctx), self._stream()), "delta_rule")
 
     def delta_gated_norm(self, y: torch.Tensor, gate: torch.Tensor, w: torch.Tensor, out: torch.Tensor, token_seq: torch.Tensor,
                          group: int, eps: float) -> None:
@@ -1563,7 +1570,7 @@ class Kernels:
             *self._state_args(state, state_offset), ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(),
             dtype_code(q.dtype), {"channel": 0, "head": 1, "constant": 3}[mode], ctx.n_seqs, heads, groups, dk, dv, float(q_scale),
             float(inv_tau), int(act_silu), _ptr(z), z.stride(0) if z is not None else 0, _ptr(w), _ptr(y),
-            y.stride(0) if y is not None else 0, 0, float(eps), float(out_scale), self._stream()), "scan_step")
+            y.stride(0) if y is not None else 0, 0, float(eps), float(out_scale), self._settled(ctx), self._stream()), "scan_step")
 
     # Tokens of a step's longest sequence from which on a recurrence with a decay a key channel, or a constant one a head, runs over chunks
     # on the tensor cores (csrc/scan_chunk.cu), for keys of 64 and of 128.  Beside the walk token by token, us: a decay a channel, 8 heads of
@@ -1647,7 +1654,7 @@ class Kernels:
                 q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(), gate.stride(0),
                 gate_bias.data_ptr(), a_log.data_ptr(), _ptr(skip), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
                 ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), ctx.n_seqs, heads, groups, dk, dv, float(q_scale),
-                self._stream()), "ssd_scan")
+                self._settled(ctx), self._stream()), "ssd_scan")
             return
         if chunk is None and mode in ("channel", "constant") and self.scan_chunk_fits(q, k, v, out, state, state_offset, ctx, dk, dv, mode):
             need = lib.braid_scan_chunk_work_floats(q.shape[0], ctx.n_seqs, heads, dk, dv)

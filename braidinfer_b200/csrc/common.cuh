@@ -46,9 +46,17 @@ void braid_set_error(const char* fmt, ...);
 // attribute that lets it begin while its predecessor in the stream drains, calls
 // pdl_trigger() at its top (so that its own successor may be scheduled early; later where a kernel says why) and
 // pdl_wait() before its first access to memory that an earlier kernel may have written
-// (or may still read).  What comes before pdl_wait() must touch only weights and the
-// kernel's own shared or tensor memory.  BRAIDINFER_PDL=0 in the environment turns the
-// attribute off; the two instructions are then no-ops.
+// (or may still read).  What comes before pdl_wait() must touch only weights, tables that
+// something other than these kernels wrote (a copy, torch's kernels: full dependencies) and the
+// kernel's own shared or tensor memory.  States and cached keys are written by kernels of earlier
+// steps, so a kernel may read them before pdl_wait() only where its caller says, with an argument
+// `settled`, that everything earlier steps wrote is in memory: the engine's steps open with a copy
+// of their tables or a graph's launch, which wait for all kernels before them to end, and no
+// kernel of a step writes a state, or a key from before the step, that another of its kernels
+// reads.  Anyone else may call the same entry twice on one state with nothing in between.  So a
+// kernel that wants its state early begins with `if (!settled) pdl_wait();` (a second wait returns
+// at once).  BRAIDINFER_PDL=0 in the environment turns the attribute off; the two instructions are
+// then no-ops.
 int braid_pdl_enabled(void);
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

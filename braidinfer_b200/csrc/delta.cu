@@ -39,7 +39,7 @@
 // A CTA of 128 threads owns (head, sequence, a tile of value columns); a thread keeps R rows x 4 columns of S in registers,
 // the RG row groups of a column lie in one warp.  The read-out of the new state is taken from the decayed one,
 // S_new^T q = (g S)^T q + (k . q) u, so that a token costs one round of sums.  The state is asked for before the wait for
-// the kernel's predecessor: no other kernel of a step touches it.
+// the kernel's predecessor where that is safe (`settled`).
 template <typename T, int RG, int R>
 __global__ void __launch_bounds__(DELTA_WALK_THREADS)
 delta_walk_kernel(DeltaArgs a) {
@@ -56,6 +56,7 @@ delta_walk_kernel(DeltaArgs a) {
     if (n <= 0) return;
     const int dk = a.dk, dv = a.dv, g = h / (a.heads / a.groups);
     float* S_area = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * dk * dv;
+    if (!a.settled) pdl_wait();
     float s[R][CV];
 #pragma unroll
     for (int e = 0; e < R; ++e)
@@ -154,7 +155,7 @@ delta_walk_kernel(DeltaArgs a) {
 
 // ------------------------------------------------------------------ one token a sequence
 // Such a step is a read and a write of the state and otherwise latency.  A CTA owns (head, sequence, COLS value columns); eight row groups
-// of threads take every eighth key row, four neighbouring columns a thread, the state asked for all at once before the wait.  Where a
+// of threads take every eighth key row, four neighbouring columns a thread, the state asked for all at once, before the wait where that is safe.  Where a
 // CTA holds all of a head's columns it goes on to the gated norm (y = o / rms(o) * w * sigmoid(gate)).  5 sequences of 8 heads of 128 x 256
 // between the kernels of a decode step: 12.5 us for the walk and the norm's kernel, 6.1 so.
 struct DeltaNorm {
@@ -177,6 +178,7 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, const __grid_constant__ D
     const int g = h / (a.heads / a.groups);
     float4* S = (float4*)((float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + (size_t)rg * a.dv + col);
     const size_t step = (size_t)DELTA_RG * a.dv / 4;
+    if (!a.settled) pdl_wait();
     float4 s[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) s[j] = S[j * step];
@@ -757,7 +759,7 @@ extern "C" int braid_delta_rule(const float* q, long long q_stride, const float*
                                 const void* b, long long b_stride, int dtype, float* out, long long out_stride, void* state,
                                 long long state_stride, long long state_offset, const int* q_start, const int* q_len,
                                 const int* slot_ids, int rows, int n_seqs, int max_q_len, int heads, int groups, int dk, int dv,
-                                float* work, long long work_floats, void* stream) {
+                                float* work, long long work_floats, int settled, void* stream) {
     if (n_seqs <= 0 || rows <= 0 || max_q_len <= 0) return BRAID_OK;
     if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("delta_rule: %d heads do not divide into %d groups", heads, groups);
     if (dk <= 0 || dk > DELTA_MAX_DK || dv <= 0) BRAID_REFUSE("delta_rule: key size %d must be in (0, %d], value size %d positive", dk, DELTA_MAX_DK, dv);
@@ -767,7 +769,7 @@ extern "C" int braid_delta_rule(const float* q, long long q_stride, const float*
                 state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dk, dv,
                 (((uintptr_t)q | (uintptr_t)k) & 15) == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && dk % 4 == 0, ((uintptr_t)z & 15) == 0 && z_stride % 4 == 0 && dk % 4 == 0,
                 nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, (dv + DELTA_DVT - 1) / DELTA_DVT,
-                (max_q_len + DELTA_C - 1) / DELTA_C};
+                (max_q_len + DELTA_C - 1) / DELTA_C, settled};
     const long long spans = (a.tiles * DELTA_DVT + DELTA_OUT_COLS - 1) / DELTA_OUT_COLS;
     if (n_seqs > 65535 || a.tiles > 65535 || (work && a.max_chunks * spans > 65535)) BRAID_REFUSE("delta_rule: the step exceeds the grid limits");
     if (work) {
@@ -794,7 +796,8 @@ extern "C" int braid_delta_step(const float* q, long long q_stride, const float*
                                 const void* b, long long b_stride, int dtype, float* out, long long out_stride, void* state,
                                 long long state_stride, long long state_offset, const int* q_start, const int* q_len,
                                 const int* slot_ids, int n_seqs, int heads, int groups, int dk, int dv, const float* gate,
-                                long long gate_stride, const void* w, void* y, long long y_stride, float eps, void* stream) {
+                                long long gate_stride, const void* w, void* y, long long y_stride, float eps, int settled,
+                                void* stream) {
     if (n_seqs <= 0) return BRAID_OK;
     if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("delta_step: %d heads do not divide into %d groups", heads, groups);
     if ((dk != 64 && dk != 128) || dv <= 0 || dv % 64) BRAID_REFUSE("delta_step: built for keys of 64 or 128 and values in multiples of 64, not %d x %d", dk, dv);
@@ -807,6 +810,7 @@ extern "C" int braid_delta_step(const float* q, long long q_stride, const float*
     if (n_seqs > 65535 || dv / 64 > 65535) BRAID_REFUSE("delta_step: the step exceeds the grid limits");
     DeltaArgs a{q, q_stride, k, k_stride, v, v_stride, z, z_stride, bias, rate, b, b_stride, out, out_stride, (uint8_t*)state,
                 state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dk, dv};
+    a.settled = settled;
     const DeltaNorm m{gate, gate_stride, w, y, y_stride, eps};
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == BRAID_F32) return dk == 64 ? launch_delta_step<float, 64>(a, m, n_seqs, s) : launch_delta_step<float, 128>(a, m, n_seqs, s);

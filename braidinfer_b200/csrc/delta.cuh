@@ -21,6 +21,7 @@ struct DeltaArgs {
     float *w, *u, *qd, *kd, *p, *gc, *sc;
     __nv_bfloat16 *wp, *kp;                      // operands in three parts
     int tiles, max_chunks;                       // tiles of value columns
+    int settled;                                 // the state may be read before the wait (common.cuh)
 };
 
 // The place of chunk c of sequence seq among all chunks of the step: a sequence's chunks lie one after the other, and two

@@ -308,6 +308,7 @@ delta_chain_kernel(const __grid_constant__ DeltaArgs a) {
     const int n_all = a.q_len[seq];
     if (n_all <= 0) return;
     const int dk = a.dk, dv = a.dv, dvp = a.tiles * DLC_COLS, n_chunks = (n_all + C - 1) / C, tile = blockIdx.z * (DLC_COLS / 16) + cols, v0 = tile * 16 + lg;
+    // (the state before the wait, always: the rows' kernel triggers at its end, after a wait of its own, so everything before it is in memory)
     float* S_area = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * dk * dv;
     float S[KT][4];                                          // value columns v0 (+ 8), keys k0 + x * 8 + lq (+ 1)
 #pragma unroll

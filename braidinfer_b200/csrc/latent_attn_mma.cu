@@ -43,6 +43,7 @@ struct LatAttnArgs {
     float scale_log2;              // scale * log2(e)
     int* error_flag;
     const float* sinks;            // [heads] float32: a score a head that joins the denominator and has no value; or null
+    int settled;                   // keys from before the step may be read before the wait (common.cuh)
 };
 
 // The denominator of a finished row with its head's sink in it (m, l in units of log2), as the factor on the accumulators.
@@ -261,7 +262,7 @@ latent_attn_few_kernel(LatAttnArgs a) {
     __nv_bfloat16* Ks = Qs + FEW_ROWS * LDK;
     float* Sp = (float*)(Ks + 2 * BN * LDK);             // [2][4 warps][16][SP_LD]
     pdl_trigger();
-    // up to pdl_wait() only the step's tables and keys cached by earlier steps are read, which no kernel of this step writes
+    // up to pdl_wait() only the step's tables are read and, where those are in memory (`settled`), keys cached by earlier steps
     const int seq = blockIdx.y, split = blockIdx.z;
     const int pairs = a.q_len[seq] * a.heads;
     const int pair0 = blockIdx.x * FEW_ROWS;
@@ -295,7 +296,7 @@ latent_attn_few_kernel(LatAttnArgs a) {
             mt_cp_async16(dst + r * LDK + kc, src + (size_t)r * D + kc, 16);
         }
     };
-    auto cached = [&](int tile) { return tile <= my_hi && (tile + 1) * BN <= before; };
+    auto cached = [&](int tile) { return a.settled && tile <= my_hi && (tile + 1) * BN <= before; };
     const bool early0 = cached(my_lo), early1 = cached(my_lo + 1);
     if (early0) load_keys(my_lo, 0);
     if (early1) load_keys(my_lo + 1, 1);
@@ -530,7 +531,7 @@ extern "C" int braid_latent_attn_mma(const void* q, void* out, float* partial, c
                                      const int* q_start, const int* q_len, const int* kv_before, const int* token_seq,
                                      int rows, int row0, int n_seqs,
                                      int max_q_len, int heads, int table_cols, int num_pages, int window, int n_splits,
-                                     float scale, const float* sinks, int* error_flag, void* stream) {
+                                     float scale, const float* sinks, int settled, int* error_flag, void* stream) {
     if (rows <= 0 || n_seqs <= 0 || max_q_len <= 0) return BRAID_OK;
     if (!error_flag) BRAID_REFUSE("latent_attn_mma: error_flag is required");
     if (heads <= 0 || table_cols <= 0 || num_pages <= 0) BRAID_REFUSE("latent_attn_mma: heads=%d, table columns=%d, pages=%d", heads, table_cols, num_pages);
@@ -550,7 +551,7 @@ extern "C" int braid_latent_attn_mma(const void* q, void* out, float* partial, c
     }
     LatAttnArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, n_splits > 1 ? partial : nullptr, (const __nv_bfloat16*)cache,
                   page_table, q_start, q_len, kv_before, heads, table_cols, num_pages, window, n_splits, rows * heads, row0,
-                  scale * 1.4426950408889634f, error_flag, sinks};
+                  scale * 1.4426950408889634f, error_flag, sinks, settled};
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = few
         ? braid_launch(latent_attn_few_kernel, dim3((unsigned)tiles, n_seqs, n_splits), dim3(128), (size_t)SMEM_FEW, s, a)

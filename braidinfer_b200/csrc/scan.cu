@@ -32,6 +32,7 @@ struct ConvArgs {
     const int* q_start;
     const int* slot_ids;
     int rows, channels, taps, silu;
+    int settled;                 // the state may be read before the wait (common.cuh)
 };
 
 template <typename T>
@@ -164,8 +165,8 @@ conv_state_kernel(ConvArgs a, const int* __restrict__ q_len, int n_seqs) {
     }
 }
 
-// One token a sequence: a thread's VEC channels of one row, the state's rows asked for with the weights before the wait (no other kernel of a
-// step touches them) and moved on by the thread that read them, so that there is no second kernel.
+// One token a sequence: a thread's VEC channels of one row, the state's rows asked for with the weights before the wait (where that is safe:
+// `settled`) and moved on by the thread that read them, so that there is no second kernel.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(64)
 causal_conv_step_kernel(ConvArgs a, const int* __restrict__ q_len) {
@@ -177,14 +178,15 @@ causal_conv_step_kernel(ConvArgs a, const int* __restrict__ q_len) {
     float* st = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + c0;
     float in[TAPS][VEC], wl[VEC * TAPS], acc[VEC];
 #pragma unroll
-    for (int j = 0; j < TAPS - 1; ++j)
-#pragma unroll
-        for (int e = 0; e < VEC; e += 4) load_run<float, 4>(st + (size_t)j * a.channels + e, in[j] + e);
-#pragma unroll
     for (int u = 0; u < TAPS; ++u) load_run<T, VEC>((const T*)a.w + (size_t)c0 * TAPS + u * VEC, wl + u * VEC);
 #pragma unroll
     for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
     if (a.b) load_run<T, VEC>((const T*)a.b + c0, acc);
+    if (!a.settled) pdl_wait();
+#pragma unroll
+    for (int j = 0; j < TAPS - 1; ++j)
+#pragma unroll
+        for (int e = 0; e < VEC; e += 4) load_run<float, 4>(st + (size_t)j * a.channels + e, in[j] + e);
     pdl_wait();
     load_run<T, VEC>((const T*)a.x + (size_t)row * a.x_stride + c0, in[TAPS - 1]);
 #pragma unroll
@@ -203,13 +205,13 @@ causal_conv_step_kernel(ConvArgs a, const int* __restrict__ q_len) {
 extern "C" int braid_causal_conv(const void* x, long long x_stride, void* y, long long y_stride, const void* w, const void* b,
                                  int dtype, void* state, long long state_stride, long long state_offset,
                                  const int* token_seq, const int* q_start, const int* q_len, const int* slot_ids,
-                                 int rows, int n_seqs, int channels, int taps, int silu, int one_each, void* stream) {
+                                 int rows, int n_seqs, int channels, int taps, int silu, int one_each, int settled, void* stream) {
     if (rows <= 0 || n_seqs <= 0) return BRAID_OK;
     if (channels <= 0 || taps < 1) BRAID_REFUSE("causal_conv: channels=%d and taps=%d must be positive", channels, taps);
     if (!state || (state_offset & 3) || (state_stride & 3)) BRAID_REFUSE("causal_conv: the state area must be given, in multiples of 4 bytes");
     if (rows > 65535 * 16 || n_seqs > 65535) BRAID_REFUSE("causal_conv: the step exceeds the grid limits");
     ConvArgs a{x, x_stride, y, y_stride, w, b, (uint8_t*)state, state_stride, state_offset, token_seq, q_start, slot_ids,
-               rows, channels, taps, silu};
+               rows, channels, taps, silu, settled};
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = 256;
     dim3 g1((channels + threads - 1) / threads, rows), g2((channels + threads - 1) / threads, n_seqs);

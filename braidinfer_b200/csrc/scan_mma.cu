@@ -36,6 +36,7 @@ struct SsdArgs {
     const int *q_start, *q_len, *slot_ids;
     int heads, groups, dv;
     float q_scale;
+    int settled;                 // the state may be read before the wait (common.cuh)
 };
 
 // 16 bytes to shared memory, or zeros
@@ -80,6 +81,7 @@ ssd_chunk_kernel(const __grid_constant__ SsdArgs a) {
     const int grp = h / (a.heads / a.groups), cw = warp * 16;
     const float head_a = -expf(to_f32(a.a_log[h])), head_bias = to_f32(a.gate_bias[h]), skip = a.skip ? to_f32(a.skip[h]) : 0.f;
     float* S_area = (float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + j0 + cw + g;
+    if (!a.settled) pdl_wait();
     float S[KT][4];                                          // S^T: value columns cw + g (+ 8), keys x * 8 + q2 (+ 1)
 #pragma unroll
     for (int x = 0; x < KT; ++x)
@@ -363,7 +365,7 @@ extern "C" int braid_ssd_scan(const void* q, long long q_stride, const void* k, 
                               const void* gate, long long gate_stride, const void* gate_bias, const void* a_log, const void* skip,
                               float* out, long long out_stride, void* state, long long state_stride, long long state_offset,
                               const int* q_start, const int* q_len, const int* slot_ids, int n_seqs, int heads, int groups, int dk, int dv,
-                              float q_scale, void* stream) {
+                              float q_scale, int settled, void* stream) {
     if (n_seqs <= 0) return BRAID_OK;
     if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("ssd_scan: %d heads do not divide into %d groups", heads, groups);
     if ((dk != 64 && dk != 128) || dv <= 0 || dv % SSD_P) BRAID_REFUSE("ssd_scan: built for keys of 64 or 128 and values in multiples of 64, not %d x %d", dk, dv);
@@ -372,6 +374,6 @@ extern "C" int braid_ssd_scan(const void* q, long long q_stride, const void* k, 
     if (!gate_bias || !a_log || n_seqs > 65535 || dv / SSD_P > 65535) BRAID_REFUSE("ssd_scan: a bias and A_log are required, and the step must fit a launch");
     using B = const __nv_bfloat16*;
     SsdArgs a{(B)q, (B)k, (B)v, (B)gate, (B)gate_bias, (B)a_log, (B)skip, q_stride, k_stride, v_stride, gate_stride, out, out_stride,
-              (uint8_t*)state, state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dv, q_scale};
+              (uint8_t*)state, state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dv, q_scale, settled};
     return dk == 64 ? launch_ssd<64>(a, n_seqs, (cudaStream_t)stream) : launch_ssd<128>(a, n_seqs, (cudaStream_t)stream);
 }

@@ -3,7 +3,7 @@
 //
 // Such a step is a read and a write of the state and otherwise latency.  A CTA owns (head, sequence, COLS value columns); eight row groups
 // of threads take every eighth key row, four neighbouring columns a thread, so that a warp moves whole rows 16 bytes a lane.  The
-// state is asked for before the wait for the kernel's predecessor (no other kernel of a step touches it), all of it at once; what comes from
+// state is asked for before the wait for the kernel's predecessor where that is safe (`settled`, common.cuh), all of it at once; what comes from
 // the projections is one trip after it.  The walk over several tokens (linear_scan_kernel) stages eight tokens whatever there are, moves the
 // state four bytes a lane and is several times the code, which every SM fetches anew between two kernels.  Between the other kernels of a
 // decode step, walk / this, us: constant decays, 4 sequences of 8 heads of 128 x 256 14.5 / 3.2; a decay a head, 8 sequences of 32 heads of
@@ -31,6 +31,7 @@ struct ScanStepArgs {
     const void* w; void* y; long long y_stride;
     int gate_sigmoid;
     float eps, out_scale;
+    int settled;                               // the state may be read before the wait (common.cuh)
 };
 
 // four neighbouring numbers
@@ -63,6 +64,7 @@ scan_step_kernel(const __grid_constant__ ScanStepArgs a) {
     const int g = h / (a.heads / a.groups);
     float4* S = (float4*)((float*)(a.state + (size_t)a.slot_ids[seq] * a.state_stride + a.state_offset) + (size_t)h * DK * a.dv + (size_t)rg * a.dv + col);
     const size_t step = (size_t)STEP_RG * a.dv / 4;
+    if (!a.settled) pdl_wait();
     float4 s[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) s[j] = S[j * step];
@@ -159,7 +161,8 @@ extern "C" int braid_scan_step(const void* q, long long q_stride, const void* k,
                                float* out, long long out_stride, void* state, long long state_stride, long long state_offset,
                                const int* q_start, const int* q_len, const int* slot_ids, int dtype, int mode, int n_seqs, int heads,
                                int groups, int dk, int dv, float q_scale, float inv_tau, int act_silu, const void* z, long long z_stride,
-                               const void* w, void* y, long long y_stride, int gate_sigmoid, float eps, float out_scale, void* stream) {
+                               const void* w, void* y, long long y_stride, int gate_sigmoid, float eps, float out_scale, int settled,
+                               void* stream) {
     if (n_seqs <= 0) return BRAID_OK;
     if (heads <= 0 || groups <= 0 || heads % groups) BRAID_REFUSE("scan_step: %d heads do not divide into %d groups", heads, groups);
     if ((dk != 64 && dk != 128) || dv <= 0 || dv % 64) BRAID_REFUSE("scan_step: built for keys of 64 or 128 and values in multiples of 64, not %d x %d", dk, dv);
@@ -175,7 +178,7 @@ extern "C" int braid_scan_step(const void* q, long long q_stride, const void* k,
     if (n_seqs > 65535 || dv / 64 > 65535) BRAID_REFUSE("scan_step: the step exceeds the grid limits");
     ScanStepArgs a{q, k, v, q_stride, k_stride, v_stride, gate, gate_stride, gate_bias, a_log, skip, out, out_stride, (uint8_t*)state,
                    state_stride, state_offset, q_start, q_len, slot_ids, heads, groups, dv, act_silu, q_scale, inv_tau, z, z_stride, w, y,
-                   y_stride, gate_sigmoid, eps, out_scale};
+                   y_stride, gate_sigmoid, eps, out_scale, settled};
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == BRAID_F32) return dk == 64 ? launch_scan_step_cols<float, 64>(a, mode, n_seqs, s) : launch_scan_step_cols<float, 128>(a, mode, n_seqs, s);
     return dk == 64 ? launch_scan_step_cols<__nv_bfloat16, 64>(a, mode, n_seqs, s) : launch_scan_step_cols<__nv_bfloat16, 128>(a, mode, n_seqs, s);

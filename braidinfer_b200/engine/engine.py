@@ -220,6 +220,9 @@ class Engine:
                                pad_rows_to=token_tile(sum(n_new)) if short_prompt else 0, upload=False)
         ctx.kernels = self.kernels
         ctx.may_be_captured = shaped
+        # the step opens with a copy of its tables, or with their fetch and a graph's launch: both wait for all that runs, and every
+        # schedule entry has a state of its own
+        ctx.settled = True
         if shaped and ctx.page_tables:
             ctx.max_kv_len = max(t.shape[1] for t in ctx.page_tables) * PAGE_SIZE
         if short_prompt:

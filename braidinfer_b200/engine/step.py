@@ -44,6 +44,10 @@ class StepContext:
     # look at the shape and its bounds only (rows, max_q_len, max_kv_len), never at the host copies below.  Only the engine
     # knows that a step is none of these.
     may_be_captured: bool = True
+    # Whether everything that earlier steps wrote (states, cached rows) is in memory before the step's first kernel begins, and no
+    # kernel of the step reads a state that another of its kernels wrote: kernels then read those before the kernels ahead of
+    # them in the stream have ended (csrc/common.cuh).  Only who launches all of a step knows it.
+    settled: bool = False
     # host copies, for parts written in Python (tests' toy parts) and for launch shaping
     host_q_len: Tuple[int, ...] = ()
     host_kv_before: Tuple[int, ...] = ()

@@ -286,4 +286,4 @@ class LatentAttention(Mixer):
             n_splits = max(1, min(296 // ctas, tiles // 2, 32))
         K.attn_latent_mma(q_lat, o_lat, cache.storage, cache.page_table[seqs], ctx.q_start[seqs], ctx.q_len[seqs], ctx.kv_before[seqs],
                           ctx.token_seq[rows], n_seqs, max_q_len, self.rank, self.window, self.scale, n_splits=n_splits,
-                          sinks=self.sinks, row0=row0)
+                          sinks=self.sinks, row0=row0, settled=getattr(ctx, "settled", False))

@@ -142,3 +142,65 @@ def test_convolution(K, dtype, taps, channels, silu):
     check(y[:-1], torch.nn.functional.silu(want) if silu else want, 8 if dtype == BF else 20)
     got = state.view(torch.float32).view(S0.shape)
     assert torch.equal(got[SLOTS], inputs[:, 1:].float()) and torch.equal(got[[1, 2]], S0[[1, 2]])
+
+
+@pytest.mark.parametrize("what", ["channel", "head", "constant", "chunks of one decay a head", "delta", "delta, walked", "convolution"])
+def test_two_calls_on_one_state_with_nothing_between(K, what):
+    """The second call starts from what the first one leaves, whether or not the host waits between them."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    heads, dk, dv, n = 16, 128, 128, 8
+    chunks = what.startswith("chunks")
+    each = 20 if chunks else 1
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(n_seqs=n, max_q_len=each, q_start=i32([each * i for i in range(n)]), q_len=i32([each] * n), slot_ids=i32(list(range(n))),
+                                token_seq=i32([i // each for i in range(n * each)]), rows=n * each)
+    rows = n * each
+    q, k, v = (rnd(rows, heads * dk).to(BF) * 0.1 for _ in range(3))
+    z, bias, a_log, b = rnd(rows, heads * dk), rnd(heads * dk).to(BF), rnd(heads).to(BF), rnd(rows, heads).to(BF)
+    unit = lambda x: (x.float().view(rows, heads, dk) / x.float().view(rows, heads, dk).norm(dim=-1, keepdim=True)).flatten(1)
+    qu, ku, vf, taps = unit(q), unit(k), v.float(), rnd(heads * dk, 4).to(BF)
+    out, y = torch.empty(rows, heads * dv, device=DEV), torch.empty(rows, heads * dk, device=DEV, dtype=BF)
+    per = heads * dk * dv * 4 if what != "convolution" else 3 * heads * dk * 4
+
+    def call(state):
+        if what == "channel":
+            K.linear_scan(q, k, v, z, bias, out, state, 0, ctx, heads, heads, dk, dv, "channel")
+        elif what == "constant":
+            K.linear_scan(q, k, v, decay, None, out, state, 0, ctx, heads, heads, dk, dv, "constant")
+        elif what == "head" or chunks:
+            K.linear_scan(q, k, v, b, a_log, out, state, 0, ctx, heads, heads, dk, dv, "head", a_log=a_log)
+        elif what == "convolution":
+            K.causal_conv(q, y, taps, None, state, 0, ctx)
+        else:
+            K.delta_rule(qu, ku, vf, z, zb, rate, b, out, state, 0, ctx, heads, heads, dk, dv if what == "delta" else 112, False)
+
+    decay, zb, rate = torch.full((heads,), 0.9, device=DEV), bias.float(), torch.full((heads,), 0.5, device=DEV)
+    if what == "delta, walked":
+        vf, out = vf[:, :heads * 112], torch.empty(rows, heads * 112, device=DEV)
+        per = heads * dk * 112 * 4
+    start = rnd(n, per // 4).view(torch.uint8)
+    want = start.clone()
+    for _ in range(4):
+        call(want)
+        torch.cuda.synchronize()
+    want_out = out.clone()
+    for _ in range(5):
+        got = start.clone()
+        for _ in range(4):
+            call(got)
+        assert torch.equal(got, want) and torch.equal(out, want_out)
+
+
+def test_the_engine_says_that_its_steps_are_settled(K, monkeypatch):
+    from braidinfer_b200.engine.engine import Engine
+    from loduzen_tiny import LZ_CONFIGS
+    seen = []
+    e = Engine.from_random(LZ_CONFIGS["A"], max_tokens=256, verbose=False)
+    forward = e.model.forward
+    monkeypatch.setattr(e.model, "forward", lambda ctx, *a, **kw: seen.append(ctx.settled) or forward(ctx, *a, **kw))
+    s = e.open()
+    e.step([(s, [1, 2, 3])])
+    e.step([(s, [4])])
+    e.step([(s, [4])])
+    assert seen == [True] * len(seen) and len(seen) >= 2

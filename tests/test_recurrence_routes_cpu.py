@@ -39,15 +39,17 @@ def step(lens):
                                  q_len=i32(lens), slot_ids=i32(list(range(len(lens)))))
 
 
-def scan(K, mode, lens, heads=2, dk=128, dv=64, dtype=BF, v_cols=None, **how):
+def scan(K, mode, lens, heads=2, dk=128, dv=64, dtype=BF, v_cols=None, settled=False, **how):
     rows = sum(lens)
     vc = dv if v_cols is None else v_cols
     q, k, v = (torch.zeros(rows, n, dtype=dtype) for n in (heads * dk, heads * dk, heads * vc))
     gate = {"channel": torch.zeros(rows, heads * dk), "head": torch.zeros(rows, heads, dtype=dtype), "constant": torch.zeros(heads)}[mode]
     bias = torch.zeros(heads * dk if mode == "channel" else heads, dtype=dtype)
     state = torch.zeros(len(lens), heads * dk * dv * 4, dtype=torch.uint8)
-    K.linear_scan(q, k, v, gate, None if mode == "constant" else bias, torch.zeros(rows, heads * dv), state, 0, step(lens), heads, heads, dk, dv,
-                  mode, a_log=torch.zeros(heads, dtype=dtype) if mode == "head" else None, v_cols=v_cols, **how)
+    ctx = step(lens)
+    ctx.settled = settled
+    K.linear_scan(q, k, v, gate, None if mode == "constant" else bias, torch.zeros(rows, heads * dv), state, 0, ctx, heads, heads, dk, dv, mode,
+                  a_log=torch.zeros(heads, dtype=dtype) if mode == "head" else None, v_cols=v_cols, **how)
     return [n for n in K.entries.names() if not n.endswith("_floats")]
 
 
@@ -81,3 +83,23 @@ def test_norm_weights_that_start_anywhere(K, dtype, off):
     ctx.rows, ctx.n_tokens, ctx.token_seq = 3, 3, torch.arange(3, dtype=torch.int32)
     part.forward(torch.zeros(3, 64, dtype=dtype), torch.zeros(3, 64), ctx, None, torch.zeros(3, part.state_bytes(), dtype=torch.uint8))
     assert K.entries.names() == (["braid_scan_step"] if off % 4 == 0 else ["braid_scan_step", "braid_gated_norm"])
+
+
+# A kernel may read a state before the kernels ahead of it have ended only where the step says that nobody ahead writes it: two calls on one
+# state with nothing between them are anyone's right.
+@pytest.mark.parametrize("settled", [None, False, True])
+def test_states_are_read_early_only_in_steps_that_say_so(K, settled):
+    scan(K, "channel", [1, 1], settled=bool(settled))
+    scan(K, "head", [20], settled=bool(settled))
+    ctx = step([1, 1])
+    if settled is not None:
+        ctx.settled = settled
+    ctx.token_seq = torch.arange(2, dtype=torch.int32)
+    state = torch.zeros(2, 2 * 64 * 64 * 4, dtype=torch.uint8)
+    x = torch.zeros(2, 128)
+    K.causal_conv(x, torch.zeros(2, 128), torch.zeros(128, 4), None, state, 0, ctx)
+    for dk, dv in ((64, 64), (32, 64)):                              # the kernel of one token, the walk
+        K.delta_rule(torch.zeros(2, 2 * dk), torch.zeros(2, 2 * dk), torch.zeros(2, 2 * dv), torch.zeros(2, 2 * dk), torch.zeros(2 * dk), torch.ones(2),
+                     torch.zeros(2, 2), torch.zeros(2, 2 * dv), state, 0, ctx, 2, 2, dk, dv, False)
+    assert K.entries.names() == ["braid_scan_step", "braid_ssd_scan", "braid_causal_conv", "braid_delta_step", "braid_delta_rule"]
+    assert [args[-2] for _, args in K.entries.calls] == [int(bool(settled))] * 5          # (the stream comes last)
