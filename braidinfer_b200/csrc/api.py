@@ -1366,6 +1366,14 @@ class Kernels:
         return state.data_ptr(), state.stride(0), int(offset)
 
     @staticmethod
+    def _scratch(floats: int, device) -> Optional[torch.Tensor]:
+        """Scratch of a form that has another beside it, which does without; None where the device has no room for it."""
+        try:
+            return torch.empty(floats, dtype=torch.float32, device=device)
+        except torch.cuda.OutOfMemoryError:
+            return None
+
+    @staticmethod
     def _settled(ctx) -> int:
         """Whether a kernel may read its state before the kernels ahead of it in the stream have ended (`StepContext.settled`): not
         unless the step says so."""
@@ -1460,7 +1468,8 @@ class Kernels:
         S <- S + k u^T; out = S^T q, with g = exp(-rate softplus(z + bias)) and beta = sigmoid(b); S float32 [heads, dk, dv] at
         `state_offset` bytes of each slot.  q, k [rows, groups * dk], v, out [rows, heads * dv], z [rows, heads * dk], bias
         [heads * dk], rate [heads]: float32; b [rows, heads] in the run's type.  `chunked`: 64 tokens at a time instead of one
-        (the results differ by rounding only).  Steps of one token a sequence have a kernel of their own where `scan_step_fits`; there
+        (the results differ by rounding only), where the device has room for what that keeps (4 (dk dv + 64 dv + 257 dk + 4,096) bytes a head
+        and 64 tokens of the step).  Steps of one token a sequence have a kernel of their own where `scan_step_fits`; there
         `norm` may be (gate's logits float32 [rows, heads * dv], w [dv], y [rows, heads * dv], eps): instead of `out`, which may
         be None, y = o / rms(o) * w * sigmoid(gate) a head, as `delta_gated_norm` has it."""
         lib = self.part_library("delta")
@@ -1489,7 +1498,8 @@ class Kernels:
             return
         rows = out.shape[0]
         need = lib.braid_delta_work_floats(rows, ctx.n_seqs, heads, dk, dv) if chunked else 0
-        work = torch.empty(need, dtype=torch.float32, device=out.device) if need > 0 else None
+        work = self._scratch(need, out.device) if need > 0 else None
+        need = need if work is not None else 0
         self.launches += 3 if work is not None else 1
         self._check_lib(lib, lib.braid_delta_rule(
             q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), z.data_ptr(), z.stride(0),
@@ -1607,7 +1617,8 @@ class Kernels:
         w [dv], y [rows, heads * dv], eps, out_scale), all of the run's type: instead of `out`, which may be None,
         y = o / rms(o) * w * silu(gate) * out_scale a head, as `gated_norm` has it.
         bfloat16 rows of modes "channel" and "constant" run over chunks on the tensor cores where `scan_chunk_fits` and no `chunk`
-        is named, mode "head" where `ssd_pays`.  Else
+        is named, mode "head" where `ssd_pays`.  The former keeps dk dv + 64 dk + 4,096 + dk float32 numbers a head and 64 tokens of the step while it
+        runs (32,768 tokens of 16 heads of 128 x 256: 1.48 GB); without room for them the step goes on as if it did not fit.  Else
         a step whose longest sequence brings at least two chunks of `chunk` tokens (default: see SCAN_CHUNK; 0: never)
         walks its chunks side by side in three passes (see csrc/scan.cu); the results differ from the walk
         token by token by rounding only."""
@@ -1658,15 +1669,16 @@ class Kernels:
             return
         if chunk is None and mode in ("channel", "constant") and self.scan_chunk_fits(q, k, v, out, state, state_offset, ctx, dk, dv, mode):
             need = lib.braid_scan_chunk_work_floats(q.shape[0], ctx.n_seqs, heads, dk, dv)
-            work = torch.empty(need, dtype=torch.float32, device=out.device)
-            self.launches += 3
-            self._check_lib(lib, lib.braid_scan_chunk(
-                q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(),
-                gate.stride(0), _ptr(gate_bias), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
-                ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), q.shape[0], ctx.n_seqs, int(ctx.max_q_len),
-                heads, groups, dk, dv, float(q_scale), float(inv_tau), int(mode == "constant"), int(gate_is_decay), int(act_silu),
-                work.data_ptr(), need, self._stream()), "scan_chunk")
-            return
+            work = self._scratch(need, out.device)
+            if work is not None:
+                self.launches += 3
+                self._check_lib(lib, lib.braid_scan_chunk(
+                    q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), gate.data_ptr(),
+                    gate.stride(0), _ptr(gate_bias), out.data_ptr(), out.stride(0), *self._state_args(state, state_offset),
+                    ctx.q_start.data_ptr(), ctx.q_len.data_ptr(), ctx.slot_ids.data_ptr(), q.shape[0], ctx.n_seqs, int(ctx.max_q_len),
+                    heads, groups, dk, dv, float(q_scale), float(inv_tau), int(mode == "constant"), int(gate_is_decay), int(act_silu),
+                    work.data_ptr(), need, self._stream()), "scan_chunk")
+                return
         if chunk is None:
             chunk = SCAN_CHUNK if SCAN_CHUNK is not None else (128 if int(ctx.max_q_len) >= 1024 else 64)
         chunk = int(chunk)

@@ -103,3 +103,26 @@ def test_states_are_read_early_only_in_steps_that_say_so(K, settled):
                      torch.zeros(2, 2), torch.zeros(2, 2 * dv), state, 0, ctx, 2, 2, dk, dv, False)
     assert K.entries.names() == ["braid_scan_step", "braid_ssd_scan", "braid_causal_conv", "braid_delta_step", "braid_delta_rule"]
     assert [args[-2] for _, args in K.entries.calls] == [int(bool(settled))] * 5          # (the stream comes last)
+
+
+# The forms over chunks keep numbers of every chunk: without room for them the step is walked, as far as the device is concerned by the
+# same kernels as steps they do not take.
+def test_without_room_for_the_chunks_the_step_is_walked(K, monkeypatch):
+    empty = torch.empty
+
+    def full(*size, **how):
+        if size == (1 << 40,):
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **how)
+
+    monkeypatch.setattr(torch, "empty", full)
+    K.entries.braid_scan_chunk_work_floats = lambda *a: 1 << 40
+    K.entries.braid_delta_work_floats = lambda *a: 1 << 40
+    before = K.launches
+    assert scan(K, "channel", [300]) == ["braid_linear_scan"] and scan(K, "constant", [300], act_silu=True) == ["braid_linear_scan"] * 2
+    ctx, state = step([300]), torch.zeros(1, 2 * 64 * 64 * 4, dtype=torch.uint8)
+    K.delta_rule(torch.zeros(300, 128), torch.zeros(300, 128), torch.zeros(300, 128), torch.zeros(300, 128), torch.zeros(128), torch.ones(2),
+                 torch.zeros(300, 2), torch.zeros(300, 128), state, 0, ctx, 2, 2, 64, 64, True)
+    name, args = K.entries.calls[-1]
+    assert name == "braid_delta_rule" and args[-4:] == (None, 0, 0, 0)                # no scratch: token by token
+    assert K.launches - before == 3
