@@ -1592,7 +1592,7 @@ class Kernels:
         """Whether `linear_scan` in mode "channel" or "constant" takes the form over chunks on the tensor cores, which works decays out of
         their logits itself, once each."""
         return (SCAN_CHUNK is None and q.dtype == torch.bfloat16 and dk in (64, 128) and dv % 64 == 0
-                and int(ctx.max_q_len) >= self.SCAN_CHUNK_FROM[mode][dk == 128]
+                and self.SCAN_CHUNK_FROM[mode][dk == 128] <= int(ctx.max_q_len) <= 65535 // (dv // 64) * 64         # (a launch's CTAs)
                 and v.stride(0) % 8 == 0 and v.data_ptr() % 16 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 8 == 0
                 and (state.data_ptr() | int(state_offset) | state.stride(0)) % 16 == 0)
 
@@ -1758,8 +1758,8 @@ class Kernels:
     @staticmethod
     def f32_tc_pays(rows: int, m: int, k: int) -> bool:
         """Whether a float32 product of `rows` tokens runs on the tensor cores (csrc/gemm_f32_tc.cu): beyond the rows that the kernel of few
-        rows takes, wherever it was measured (64 x 128 with 17 tokens 10 us beside 12, the other sizes there)."""
-        return rows > 16 and m >= 64 and k >= 128
+        rows takes, wherever it was measured (64 x 128 with 17 tokens 10 us beside 12, the other sizes there), up to what a launch takes."""
+        return 16 < rows <= 65535 * 32 and m >= 64 and k >= 128
 
     def gemm_simt(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, residual: Optional[torch.Tensor] = None) -> None:
         n, k = x.shape
