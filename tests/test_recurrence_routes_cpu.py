@@ -129,7 +129,7 @@ def test_without_room_for_the_chunks_the_step_is_walked(K, monkeypatch):
 
 
 # steps whose chunks are more than a launch takes (keys of 64: where the walk, in chunks of 128, still runs)
-@pytest.mark.parametrize("longest, dv, fits", [(65535 * 64, 64, True), (65535 * 64 + 1, 64, False), (65535 * 16, 256, True), (65535 * 16 + 1, 256, False)])
+@pytest.mark.parametrize("longest, dv, fits", [(65535 * 64, 64, True), (65535 * 64 + 1, 64, False), (16383 * 64, 256, True), (16383 * 64 + 1, 256, False)])
 def test_steps_beyond_a_launch_go_on_to_the_walk(K, longest, dv, fits):
     x, out, state = torch.zeros(1, 2 * dv, dtype=BF), torch.zeros(1, 2 * dv), torch.zeros(1, 64, dtype=torch.uint8)
     ctx = types.SimpleNamespace(n_seqs=1, max_q_len=longest)
