@@ -107,6 +107,13 @@ class StepContext:
                 self.kernels.streamk_reduce(handle, tensor)
         return tensor
 
+    def ready_for(self, tensor: torch.Tensor, part) -> torch.Tensor:
+        """Complete `tensor` now, unless `part`, which reads it next, adds up the sum that is deferred on it."""
+        d = self.deferred.get(tensor.data_ptr())
+        if d is not None and not (part.accepts_deferred and (d[1] != "normed" or part.accepts_normed)):
+            self.resolve(tensor)
+        return tensor
+
     def drop_deferred(self) -> None:
         """Forget sums nobody will read (the step wants no logits)."""
         for handle, _ in self.deferred.values():

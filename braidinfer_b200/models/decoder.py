@@ -119,7 +119,5 @@ class DecoderModel:
             return None
         if self.streams is not None:
             return self.head.forward(self.streams.close(h, self.final_norm, ctx, ctx.want_rows, ctx.n_want))
-        if not self.final_norm.accepts_deferred:
-            ctx.resolve(h)
-        x = self.final_norm.forward(h, ctx, row_index=ctx.want_rows, rows=ctx.n_want)
+        x = self.final_norm.forward(ctx.ready_for(h, self.final_norm), ctx, row_index=ctx.want_rows, rows=ctx.n_want)
         return self.head.forward(x)

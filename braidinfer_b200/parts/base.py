@@ -24,8 +24,10 @@ class Part:
     graph_safe = True
 
     # A part that can finish a deferred sum inside its own kernel (see StepContext.deferred)
-    # says so here; every other part is handed tensors that are already complete.
+    # says so here; every other part is handed tensors that are already complete.  `accepts_normed`: also the normed result of a
+    # layer's own token input (kind "normed").
     accepts_deferred = False
+    accepts_normed = False
 
     # A mixer or feed-forward that sets this true takes `residual=None` and then returns its result alone
     # (float32) instead of residual + result: for blocks that norm a sublayer's result before they add it.

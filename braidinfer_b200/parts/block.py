@@ -47,8 +47,9 @@ class PreNormResidualBlock(Block):
 
     @staticmethod
     def _norm(norm, h, ctx, reader):
+        h = ctx.ready_for(h, norm)
         if not norm.accepts_deferred:
-            return norm.forward(ctx.resolve(h), ctx)
+            return norm.forward(h, ctx)
         # a norm that knows deferred sums may also leave its scale to a reader that takes row scales
         return norm.forward(h, ctx, reader_takes_row_scale=bool(reader.takes_row_scale()))
 

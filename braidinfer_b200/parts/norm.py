@@ -31,6 +31,7 @@ class RMSNorm(Norm):
     stored number instead of one a column; default False), gain (a constant factor on the result; default 1)."""
 
     accepts_deferred = True      # adds a deferred residual sum in the same kernel as the norm
+    accepts_normed = True
 
     def __init__(self, params, prefix, runtime) -> None:
         super().__init__(params, prefix, runtime)
