@@ -54,8 +54,9 @@ struct AttnSimpleArgs {
 // an item, every wpi-th block of keys each, and the first of them merges their maxima, denominators and sums in order.  Keys are
 // read 16 bytes at a time where a head's rows allow it (WIDE), values of four keys at a time, in the order of the keys.
 // DEEP: for steps whose CTAs do not fill the machine, which are a chain of trips to memory: a block's values (32 keys') and all 16-byte
-// loads of its keys are in flight together, whatever registers that takes.  The order of the sums is the same.  24 items of 200 keys of 64
-// numbers: 19.5 us with four of either in flight, 16.0 so.
+// loads of its keys are in flight together, whatever registers that takes.  The order of the sums is the same.  Heads of 64 in float32 / bfloat16, us
+// with four of either in flight and so: 3 tokens of 8 heads 200 keys 12.0 / 11.8 and 10.8 / 10.5, 2,000 keys 77 / 69 and 68 / 60.  Heads of up to
+// 64 only: with twice the values a lane it is slower everywhere (128: 17.2 / 15.7 and 29.3 / 26.0, 2,000 keys 123 / 108 and 214 / 185).
 template <typename T, int NI, bool WIDE, bool DEEP = false>
 __global__ void __launch_bounds__(ATTN_SIMPLE_WARPS * 32)
 attn_simple_kernel(AttnSimpleArgs a, int wpi) {
@@ -102,26 +103,7 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
             const int j = j0 + lane;
             float s = -INFINITY;
             const T *kbase = nullptr, *vrow = nullptr;
-            const int n_valid = min(32, end - j0);
-            if (j < end) {
-                const int block = j / a.page_size, off = j - block * a.page_size;
-                int page = (block < a.table_cols) ? table[block] : -1;
-                if (page < 0 || page >= a.num_pages) {      // never followed: flag it and read page 0 instead
-                    atomicExch(a.error_flag, 1);
-                    page = 0;
-                }
-                kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
-                vrow = kbase + (size_t)(a.nkh + val_h - kvh) * head_stride;
-            }
-            T vs[DEEP ? 32 : 1][NI];
-            if (DEEP)
-#pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, k);
-#pragma unroll
-                    for (int i = 0; i < NI; ++i) vs[DEEP ? k : 0][i] = (k < n_valid && lane + 32 * i < a.hd) ? vr[lane + 32 * i] : from_f32<T>(0.f);
-                }
-            if (j < end) {
+            auto score = [&]() {
                 float dot = 0.f;
                 if (WIDE) {
                     constexpr int VW = 16 / sizeof(T);
@@ -138,6 +120,28 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
                 s = dot * scale;
                 if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
                 if (a.bias_slope) s -= r1 * log1pf(r2 * (float)(pos - j));
+            };
+            if (j < end) {
+                const int block = j / a.page_size, off = j - block * a.page_size;
+                int page = (block < a.table_cols) ? table[block] : -1;
+                if (page < 0 || page >= a.num_pages) {      // never followed: flag it and read page 0 instead
+                    atomicExch(a.error_flag, 1);
+                    page = 0;
+                }
+                kbase = (const T*)a.cache + ((size_t)page * 2 * a.nkh + kvh) * head_stride + (size_t)off * a.hd;
+                vrow = kbase + (size_t)(a.nkh + val_h - kvh) * head_stride;
+                if constexpr (!DEEP) score();
+            }
+            T vs[DEEP ? 32 : 1][NI];                        // (DEEP)
+            if constexpr (DEEP) {
+                const int n_valid = min(32, end - j0);
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, k);
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) vs[k][i] = (k < n_valid && lane + 32 * i < a.hd) ? vr[lane + 32 * i] : from_f32<T>(0.f);
+                }
+                if (j < end) score();
             }
             const float cmax = warp_max(s);
             const float m_new = fmaxf(m, cmax);
@@ -150,30 +154,32 @@ attn_simple_kernel(AttnSimpleArgs a, int wpi) {
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < NI; ++i) acc[i] *= corr;
-            if (DEEP) {
+            const int n_valid = min(32, end - j0);
+            if constexpr (DEEP) {
 #pragma unroll
                 for (int k = 0; k < 32; ++k)
                     if (k < n_valid) {
                         const float pj = ps[k];
 #pragma unroll
-                        for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, to_f32(vs[DEEP ? k : 0][i]), acc[i]);
+                        for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, to_f32(vs[k][i]), acc[i]);
                     }
-            }
-            for (int jj = 0; jj < (DEEP ? 0 : n_valid); jj += 4) {
-                float v[4][NI];
+            } else {
+                for (int jj = 0; jj < n_valid; jj += 4) {
+                    float v[4][NI];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, jj + k);
+                    for (int k = 0; k < 4; ++k) {
+                        const T* vr = (const T*)__shfl_sync(0xffffffffu, (unsigned long long)vrow, jj + k);
 #pragma unroll
-                    for (int i = 0; i < NI; ++i) v[k][i] = (jj + k < n_valid && lane + 32 * i < a.hd) ? to_f32(vr[lane + 32 * i]) : 0.f;
+                        for (int i = 0; i < NI; ++i) v[k][i] = (jj + k < n_valid && lane + 32 * i < a.hd) ? to_f32(vr[lane + 32 * i]) : 0.f;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (jj + k < n_valid) {
+                            const float pj = ps[jj + k];
+#pragma unroll
+                            for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, v[k][i], acc[i]);
+                        }
                 }
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (jj + k < n_valid) {
-                        const float pj = ps[jj + k];
-#pragma unroll
-                        for (int i = 0; i < NI; ++i) acc[i] = fmaf(pj, v[k][i], acc[i]);
-                    }
             }
             __syncwarp();
         }
@@ -232,9 +238,8 @@ static void attn_simple_launch(const AttnSimpleArgs& a, cudaStream_t s) {
     const dim3 grid((unsigned)((items + per - 1) / per)), block(ATTN_SIMPLE_WARPS * 32);
     const size_t smem = (size_t)ATTN_SIMPLE_WARPS * (((a.hd + 3) & ~3) + 32 + 2) * sizeof(float);
     const bool wide = (a.hd * sizeof(T)) % 16 == 0 && ((uintptr_t)a.cache & 15) == 0;
-    if (wide && grid.x <= 148 && a.hd <= 128) {
-        if (a.hd <= 64) braid_launch(attn_simple_kernel<T, 2, true, true>, grid, block, smem, s, a, wpi);
-        else braid_launch(attn_simple_kernel<T, 4, true, true>, grid, block, smem, s, a, wpi);
+    if (wide && grid.x <= 148 && a.hd <= 64) {
+        braid_launch(attn_simple_kernel<T, 2, true, true>, grid, block, smem, s, a, wpi);
     } else if (a.hd <= 64) {
         if (wide) braid_launch(attn_simple_kernel<T, 2, true>, grid, block, smem, s, a, wpi);
         else braid_launch(attn_simple_kernel<T, 2, false>, grid, block, smem, s, a, wpi);
