@@ -5,8 +5,10 @@
 // The tensor cores cut off where float32 rounds, so an accumulator in tensor memory holds 64 numbers of k at a time (the five small
 // products first, then the first parts', four additions at the sum's own size) and is then added to the thread's float32 sums: measured
 // beside float64 (k 1024 / 2816 / 4096) it is 1.1e-7 / 1.5e-7 / 1.7e-7 of the result's size off where gemm_tile_kernel is 2.9e-7 to 5.7e-7 /
-// 4.8e-7 to 9.5e-7 / 5.7e-7 to 1.2e-6.  A result that is not finite is worked out again by float32 multiply-adds, so that infinities and numbers whose parts
-// overflow do what they do there.
+// 4.8e-7 to 9.5e-7 / 5.7e-7 to 1.2e-6.  Below 2^-110 an operand's parts would fall under bfloat16's smallest exponent and lose its low bits
+// (at 1e-37 all but 11), so operands are multiplied by 2^24 on their way: every float32 number is three parts then, and the results are 2^48
+// too large until the end.  A result that is not finite (there: from 2^80 on) is worked out again by float32 multiply-adds, so that infinities and
+// numbers whose parts or sums overflow do what they do there.
 //
 // A CTA of sixteen warps owns 128 weight rows x N tokens and walks k 64 at a time through two stages: while the tensor cores work on one, the
 // warps fetch the next block's float32 numbers, read the accumulator of the block before, and split the numbers into the swizzled
@@ -19,6 +21,7 @@
 #define F3_BK 64
 #define F3_BM 128
 #define F3_THREADS 512
+#define F3_UP 16777216.f                     // 2^24
 #define F3_ROWS (F3_THREADS / 16)            // rows of 16 float4 that the CTA takes at once
 
 struct GemmF32TcArgs {
@@ -33,20 +36,30 @@ template <int N> constexpr int f3_stage() { return 3 * (F3_BM + N) * F3_BK * 2; 
 template <int N> constexpr int f3_smem() { return 2 * f3_stage<N>() + 1024; }
 template <int N> constexpr uint32_t f3_cols() { return N <= 32 ? 64 : N <= 64 ? 128 : 256; }      // two accumulators, a power of two
 
+// F3_UP times two numbers
+__device__ __forceinline__ uint64_t f3_scaled(float a, float b) {
+    uint64_t v;
+    asm("{\n\t.reg .b64 x, up;\n\tmov.b64 x, {%1, %2};\n\tmov.b64 up, {%3, %3};\n\tmul.rn.f32x2 %0, x, up;\n\t}" : "=l"(v) : "f"(a), "f"(b), "f"(F3_UP));
+    return v;
+}
 // four numbers to their places in three operand tiles of `part` bytes: 128-byte rows, 16-byte runs swapped by the row's low bits
 __device__ __forceinline__ void f3_split(uint32_t tile, uint32_t part, int r, int c, float4 x) {
     const uint32_t at = tile + r * 128 + (((c >> 1) ^ (r & 7)) << 4) + (c & 1) * 8;
-    float v[4] = {x.x, x.y, x.z, x.w};
+    uint64_t v[2] = {f3_scaled(x.x, x.y), f3_scaled(x.z, x.w)};      // two numbers a register pair and instruction
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
         uint32_t w[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
+            float a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v[e]));
             // (the first two saturate: a number past the largest bfloat16 one is still a sum of finite parts)
-            if (p < 2) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w[e]) : "f"(v[2 * e + 1]), "f"(v[2 * e]));
-            else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[e]) : "f"(v[2 * e + 1]), "f"(v[2 * e]));
-            v[2 * e] -= __uint_as_float(w[e] << 16);
-            v[2 * e + 1] -= __uint_as_float(w[e] & 0xffff0000u);
+            if (p < 2) {
+                asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(w[e]) : "f"(b), "f"(a));
+                uint64_t part;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(part) : "r"(w[e] << 16), "r"(w[e] & 0xffff0000u));
+                asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(v[e]) : "l"(part));
+            } else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[e]) : "f"(b), "f"(a));
         }
         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + p * part), "r"(w[0]), "r"(w[1]) : "memory");
     }
@@ -156,7 +169,7 @@ gemm_f32_tc_kernel(const __grid_constant__ GemmF32TcArgs a) {
         for (int j = 0; j < COLS; ++j) {
             const int n = n0 + (warp >> 2) * COLS + j;
             if (n >= a.n_rows) break;
-            float v = acc[j];
+            float v = acc[j] * (1.f / F3_UP / F3_UP);
             if (!(fabsf(v) <= 3.402823466e38f)) {
                 v = 0.f;
                 for (int k = 0; k < a.k_in; ++k) v = fmaf(a.x[(size_t)n * a.ldx + k], a.w[(size_t)m * a.ldw + k], v);

@@ -49,6 +49,19 @@ def test_error_is_no_larger_than_that_of_float32_sums(K, monkeypatch):
         assert errors[0] <= errors[1]
 
 
+@pytest.mark.parametrize("ex, ew", [(-100, 0), (-112, 0), (0, -118), (-124, 3), (-124, 100), (-140, 0), (-60, -60), (60, 30), (100, -20), (60, 60)])
+def test_numbers_of_any_size(K, ex, ew):
+    """All of float32's bits count down to its smallest number, which the parts of an operand reach before the operand does."""
+    k = 512
+    x, w = rnd(40, k) * 2.0 ** (ex // 2) * 2.0 ** (ex - ex // 2), rnd(128, k, seed=1) * 2.0 ** ew
+    exact, out = x.double() @ w.double().T, torch.empty(40, 128, device=DEV)
+    K.gemm_simt(x, w, out)
+    # as in test_product, and one rounding where the result is smaller than 2^-126
+    most = (0.1 * k + 4) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 2.0 ** -149
+    assert ((out.double() - exact).abs() <= most).all()
+    K.check_device_errors()
+
+
 def test_numbers_that_are_not_finite(K, monkeypatch):
     x, w = rnd(100, 256), rnd(128, 256, seed=1)
     x[3, 5], x[7, 9], w[5, 9], x[60, 1] = float("inf"), float("nan"), float("-inf"), 3.4e38
