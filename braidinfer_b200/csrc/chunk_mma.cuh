@@ -17,6 +17,13 @@
 // is lost of the smallest is far below a sum's rounding, while a channel's decays over the sub-chunk multiply to 2^-100 or more; the
 // channels beyond are steep and multiplied up pair by pair.
 #define CHK_SPREAD 7.8886091e-31f          // 2^-100
+// Queries and keys that are decayed that far stay normal numbers, and hold three parts of bfloat16 (which ends at 2^-133), down to 2^-60 in
+// size because both are stored times CHK_UP; the scores' products lie between 2^-50 and 2^50 of their queries and keys, and fit up to CHK_LARGE.
+// Decays above one are taken as others while they multiply to CHK_GROWTH or less.  (Elsewhere an operand that has decayed below 2^-110 stands in
+// a sum beside ones that have not; what it loses is 2^-134 of the other factor.)
+#define CHK_UP 1.125899906842624e15f       // 2^50
+#define CHK_LARGE 274877906944.f           // 2^38
+#define CHK_GROWTH 1048576.f               // 2^20
 #define CHK_PPITCH (CHK_C + 8)
 
 __device__ __forceinline__ bool chk_not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
@@ -75,32 +82,34 @@ __device__ __forceinline__ uint4 chk_load8(const __nv_bfloat16* p, bool wide) {
 }
 
 // A channel's decays over a sub-chunk, by the thread that owns the two: `d` [16 rows of LD] holds the decays and gets the products from the
-// sub-chunk's start on; `k` is decayed to its end and, where asked for, `f` is k decayed from its start.  True: a steep channel.
+// sub-chunk's start on; `k` is decayed to its end and, where asked for, `f` is k decayed from its start, both times CHK_UP.  True: a steep
+// channel.
 template <int LD, bool FORWARD>
 __device__ __forceinline__ bool chk_decays(float* d, float* k, float* f, float* total, float* inv) {
-    float dec[CHK_SUB], prod = 1.f, after = 1.f;
+    float dec[CHK_SUB], prod = 1.f, after = CHK_UP;
 #pragma unroll
     for (int r = 0; r < CHK_SUB; ++r) dec[r] = d[r * LD];
 #pragma unroll
     for (int r = 0; r < CHK_SUB; ++r) {
         prod *= dec[r];
         d[r * LD] = prod;
-        if (FORWARD) f[r * LD] = k[r * LD] * prod;
+        if (FORWARD) f[r * LD] = k[r * LD] * (prod * CHK_UP);
     }
 #pragma unroll
     for (int r = CHK_SUB - 1; r >= 0; --r) {
         k[r * LD] *= after;
         after *= dec[r];
     }
-    const bool steep = !(prod >= CHK_SPREAD && prod <= 1.f / CHK_SPREAD);
+    const bool steep = !(prod >= CHK_SPREAD && prod <= CHK_GROWTH);
     *total = prod;
-    *inv = steep ? 0.f : 1.f / prod;
+    *inv = steep ? 0.f : (1.f / CHK_UP / CHK_UP) / prod;
     return steep;
 }
 
 // Products of a block of 16 rows (decayed from their sub-chunk's start) with the keys (decayed to their sub-chunk's end) of the same
 // sub-chunk J and the ones before it: acc[d] for sub-chunk J - d, TILES tiles of 8 keys from tile0 on, in mma.sync's layout; the products of
 // the first parts, and the small ones.  Between two sub-chunks lie the decays of those between; inside one, 1 / all of its decays.
+// Rows and keys are CHK_UP times theirs, the results are not.
 template <int DK, int LD, int TILES>
 __device__ __forceinline__ void chk_scores(const float* rows, const float* keys, const float* total, const float* inv, int J, int tile0,
                                            float (*acc)[TILES][2][4]) {
@@ -119,7 +128,7 @@ __device__ __forceinline__ void chk_scores(const float* rows, const float* keys,
             const float2 v = *reinterpret_cast<const float2*>(rows + (g + (e & 1) * 8) * LD + c + (e >> 1) * 8);
             chk_split2(v.x, v.y, a[0][e], a[1][e], a[2][e]);
         }
-        float2 f[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
+        float2 f[2] = {make_float2(1.f / CHK_UP, 1.f / CHK_UP), make_float2(1.f / CHK_UP, 1.f / CHK_UP)};
 #pragma unroll
         for (int d = 0; d < 4; ++d) {
             if (d > J) continue;
@@ -154,7 +163,7 @@ __device__ __forceinline__ void chk_scores(const float* rows, const float* keys,
 #pragma unroll
         for (int x = 0; x < TILES; ++x)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[d][x][0][e] += acc[d][x][1][e];
+            for (int e = 0; e < 4; ++e) acc[d][x][0][e] = (acc[d][x][0][e] + acc[d][x][1][e]) * (d == 0 ? 1.f : 1.f / CHK_UP);
 }
 
 // The steep channels' share of the blocks on the diagonal, pair by pair: for every sub-chunk J, `take(J, p, a)` after the sums of q_t k_s and

@@ -9,6 +9,8 @@
 // their accumulators, which are the operand of S^T W^T as U^T is of U^T K: the state never passes through shared memory, only the two
 // halves of S^T W^T meet there.  U and the states lie in memory as the lanes hold them, [16 value columns][16 tokens or keys][lane][8], which
 // is how the outputs' products want them too.
+// A token's numbers that are not finite may reach back inside its own block of 16 (zeros of the triangles times them), as they did in the sums on
+// the ordinary pipes; never to the tokens of earlier blocks, other heads or sequences.
 // Measured, 16 heads of 128 x 256, 1,777 + 1,244 tokens, us, beside float32 sums on the ordinary pipes: rows 171 / 272, chain 193 / 265,
 // outputs 94 / 142.  The chain is bound by mma.sync (768 a scheduler and chunk at 8.2 cycles are 6,300 of its 10,500 cycles), the rows by the
 // dependent products of the solve.
@@ -32,14 +34,14 @@ __global__ void __launch_bounds__(CHK_THREADS, 2)
 delta_rows_kernel(const __grid_constant__ DeltaArgs a) {
     constexpr int C = CHK_C, SUB = CHK_SUB, LD = DK + 8, NT = CHK_THREADS;
     extern __shared__ __align__(128) uint8_t dlc_bytes[];
-    float* sQ = (float*)dlc_bytes;                           // [C][LD]: decays, q decayed from its sub-chunk's start; then the solve's operands:
+    float* sQ = (float*)dlc_bytes;                           // [C][LD]: decays, q decayed from its sub-chunk's start (times CHK_UP); then the solve's operands:
     __nv_bfloat16* sA = (__nv_bfloat16*)dlc_bytes;           //   3 x [C][DLC_APITCH]: -beta_t A_ts
     __nv_bfloat16* sX = sA + 3 * C * DLC_APITCH;             //   3 x [C][DLC_TPITCH]: the inverses of the diagonal's blocks, side by side
     float* sL = (float*)(sX + 3 * C * DLC_TPITCH);           //   [C][17]: beta_t A_ts of the diagonal's blocks
-    float* sF = (float*)(dlc_bytes + dlc_first_bytes<DK>()); // [C][LD]: k decayed from its sub-chunk's start, then from the chunk's
-    float* sK = sF + C * LD;                                 // [C][LD]: k decayed to its sub-chunk's end
+    float* sF = (float*)(dlc_bytes + dlc_first_bytes<DK>()); // [C][LD]: k decayed from its sub-chunk's start (times CHK_UP), then from the chunk's
+    float* sK = sF + C * LD;                                 // [C][LD]: k decayed to its sub-chunk's end, times CHK_UP
     float* sT = sK + C * LD;                                 // [4][DK]: a sub-chunk's decays multiplied
-    float* sI = sT + 4 * DK;                                 // [4][DK]: 1 / that, 0 for a steep channel
+    float* sI = sT + 4 * DK;                                 // [4][DK]: 1 / (that CHK_UP^2), 0 for a steep channel
     float* sB = sI + 4 * DK;                                 // beta
     static_assert(CHK_STEEP_FLOATS(DK) * 4 <= dlc_first_bytes<DK>(), "the steep channels are staged where q was");
     const int h = blockIdx.x, seq = blockIdx.y, c = blockIdx.z, tid = threadIdx.x;
@@ -103,7 +105,7 @@ delta_rows_kernel(const __grid_constant__ DeltaArgs a) {
     for (int w = 0; w < N4; ++w) {
         float4* at = reinterpret_cast<float4*>(sQ + (row4 + w * STEP4) * LD + ch4);
         const float4 e = *at;
-        *at = make_float4(qx[w].x * e.x, qx[w].y * e.y, qx[w].z * e.z, qx[w].w * e.w);
+        *at = make_float4(qx[w].x * (e.x * CHK_UP), qx[w].y * (e.y * CHK_UP), qx[w].z * (e.z * CHK_UP), qx[w].w * (e.w * CHK_UP));
     }
     __syncthreads();
     // P's rows of 16 by the first four warps, A's by the others: rows with more sub-chunks share a scheduler with ones of fewer
@@ -132,6 +134,8 @@ delta_rows_kernel(const __grid_constant__ DeltaArgs a) {
                 else k[e] *= m[e];
             }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { x[e] *= 1.f / CHK_UP; f[e] *= 1.f / CHK_UP; k[e] *= 1.f / CHK_UP; }
         *reinterpret_cast<float4*>(gQ + idx) = make_float4(x[0], x[1], x[2], x[3]);
         *reinterpret_cast<float4*>(sF + t * LD + i) = make_float4(f[0], f[1], f[2], f[3]);
         chk_store_split4(gK + idx, C * DK, make_float4(k[0], k[1], k[2], k[3]));

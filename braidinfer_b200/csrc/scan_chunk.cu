@@ -13,7 +13,7 @@
 //
 // U and O are products on the tensor cores.  q, k and v as projected are bfloat16 numbers and exact there; what is float32 (decayed
 // q and k, P, S_0, anything that went through silu) goes in as the sum of three (chunk_mma.cuh).  A chunk with a number that is not finite
-// among its q, k, v, decays or its S_0 is walked token by token, so that it does what the walk does.
+// among its q, k, v, decays or its S_0, or with a q or k beyond CHK_LARGE, is walked token by token, so that it does what the walk does.
 //
 // The walk in two passes over chunks of 128 (scan.cu) is bound by shared-memory reads and shuffles: a state element costs a token five
 // instructions and a pass its own staging.  Measured beside it, with its kernel for the decays, L2 flushed, us: a decay a channel, 8 heads of
@@ -120,10 +120,10 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
     constexpr int C = CHK_C, SUB = CHK_SUB, LD = DK + 8, NT = CHK_THREADS;
     constexpr int PV = SILU ? 3 : 1;
     extern __shared__ __align__(16) float chk_sm[];
-    float* sQ = chk_sm;                                      // [C][LD]: decays; then q decayed from its sub-chunk's start
-    float* sK = sQ + C * LD;                                 // [C][LD]: k, then decayed to its sub-chunk's end
+    float* sQ = chk_sm;                                      // [C][LD]: decays; then q decayed from its sub-chunk's start, times CHK_UP
+    float* sK = sQ + C * LD;                                 // [C][LD]: k, then decayed to its sub-chunk's end, times CHK_UP
     float* sT = sK + C * LD;                                 // [4][DK]: a sub-chunk's decays multiplied
-    float* sI = sT + 4 * DK;                                 // [4][DK]: 1 / that, 0 for a steep channel
+    float* sI = sT + 4 * DK;                                 // [4][DK]: 1 / (that CHK_UP^2), 0 for a steep channel
     __nv_bfloat16* sV = (__nv_bfloat16*)(sI + 4 * DK);       // two buffers, or one of three parts
     static_assert(CHK_STEEP_FLOATS(DK) <= C * LD, "the steep channels are staged where q was");
     const int h = blockIdx.x, seq = blockIdx.y, c = blockIdx.z, tid = threadIdx.x;
@@ -177,7 +177,7 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
         }
         *at = make_float4(d[0], d[1], d[2], d[3]);
     }
-    auto widen = [&](uint4 x, float* y) {
+    auto widen = [&](uint4 x, float* y, float scale) {
         const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -187,14 +187,14 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             if (SILU) y[e] = silu_f32(y[e]);
-            bad |= chk_not_finite(y[e]);
+            bad |= !(fabsf(y[e] * scale) <= CHK_LARGE);
         }
     };
 #pragma unroll 1
     for (int t = row8; t < C; t += STEP8) {
         float* at = sK + t * LD + run;
         float y[8];
-        widen(*reinterpret_cast<const uint4*>(at), y);
+        widen(*reinterpret_cast<const uint4*>(at), y, 1.f);
         *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
         *reinterpret_cast<float4*>(at + 4) = make_float4(y[4], y[5], y[6], y[7]);
     }
@@ -210,11 +210,11 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
     for (int w = 0; w < C * DK / 8 / NT; ++w) {
         float* at = sQ + (row8 + w * STEP8) * LD + run;
         float y[8], e[8];
-        widen(qx[w], y);
+        widen(qx[w], y, a.q_scale);
         *reinterpret_cast<float4*>(e) = *reinterpret_cast<const float4*>(at);
         *reinterpret_cast<float4*>(e + 4) = *reinterpret_cast<const float4*>(at + 4);
 #pragma unroll
-        for (int x = 0; x < 8; ++x) y[x] *= a.q_scale * e[x];
+        for (int x = 0; x < 8; ++x) y[x] *= a.q_scale * (e[x] * CHK_UP);
         *reinterpret_cast<float4*>(at) = make_float4(y[0], y[1], y[2], y[3]);
         *reinterpret_cast<float4*>(at + 4) = make_float4(y[4], y[5], y[6], y[7]);
     }
@@ -232,6 +232,8 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
         for (int m = t / SUB - 1; m >= 0; --m)
 #pragma unroll
             for (int e = 0; e < 4; ++e) x[e] *= sT[m * DK + i + e];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] *= 1.f / CHK_UP;
         *reinterpret_cast<float4*>(gQ + idx) = make_float4(x[0], x[1], x[2], x[3]);
     }
     if (any_steep) {
@@ -262,7 +264,7 @@ scan_chunk_state_kernel(const __grid_constant__ ChunkArgs a) {
     const int m0 = warp % MT * 16, t0 = warp / MT * TILES;
     uint32_t ka[4][3][4];
     {
-        float tail[2] = {1.f, 1.f};
+        float tail[2] = {1.f / CHK_UP, 1.f / CHK_UP};
 #pragma unroll
         for (int ks = 3; ks >= 0; --ks) {
 #pragma unroll
