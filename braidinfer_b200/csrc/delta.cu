@@ -252,10 +252,11 @@ static int launch_delta_step(const DeltaArgs& a, const DeltaNorm& m, int n_seqs,
 
 // ------------------------------------------------------------------ inside every chunk
 #define DELTA_INTRA_THREADS 256
-template <int DKP> constexpr int delta_intra_smem() { return (3 * DELTA_C * (DKP + 4) + DELTA_C + 3 * DKP) * 4; }
+constexpr int DKP = DELTA_MAX_DK;        // these kernels hold keys of up to 256; ones of up to 128 have delta_chunk.cu's
+constexpr int delta_intra_smem() { return (3 * DELTA_C * (DKP + 4) + DELTA_C + 3 * DKP) * 4; }
 
-template <typename T, int DKP>
-__global__ void __launch_bounds__(DELTA_INTRA_THREADS, DKP <= 128 ? 2 : 1)
+template <typename T>
+__global__ void __launch_bounds__(DELTA_INTRA_THREADS, 1)
 delta_intra_kernel(DeltaArgs a) {
     constexpr int C = DELTA_C, SUB = DELTA_SUB, LD = DKP + 4, NT = DELTA_INTRA_THREADS;
     static_assert(DKP >= C, "A's rows fit where q's were");
@@ -444,11 +445,6 @@ delta_intra_kernel(DeltaArgs a) {
 }
 
 // ------------------------------------------------------------------ chunk after chunk
-__device__ __forceinline__ void delta_cp16(void* smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void delta_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void delta_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // N floats (a multiple of 4) that lie one after the other, by NT threads
 template <int N, int NT>
 __device__ __forceinline__ void delta_copy(float* dst, const float* src, int tid) {
@@ -464,13 +460,11 @@ __device__ __forceinline__ void delta_copy(float* dst, const float* src, int tid
 // bound by the reads of shared memory); the warps' partial tiles meet in shared memory, where the thread that owns four numbers
 // of U or of S adds them up.
 #define DELTA_STATE_THREADS 256
-#define DELTA_ALONE_SMEM (120 * 1024)
-template <int DKP> constexpr int delta_state_smem() {
+constexpr int delta_state_smem() {
     return (2 * DELTA_C * (DKP + 4) + (DKP + DELTA_C) * DELTA_DVT + 8 * DELTA_C * DELTA_DVT) * 4;
 }
 
-template <int DKP>
-__global__ void __launch_bounds__(DELTA_STATE_THREADS, DKP <= 128 ? 2 : 1)
+__global__ void __launch_bounds__(DELTA_STATE_THREADS, 1)
 delta_state_kernel(DeltaArgs a) {
     constexpr int C = DELTA_C, LD = DKP + 4, N = DELTA_DVT, NT = DELTA_STATE_THREADS;
     constexpr int RB = DKP / 64, KS = 8 / RB;             // row blocks of S, and slices of the tokens a row block
@@ -620,11 +614,10 @@ delta_state_kernel(DeltaArgs a) {
 // ------------------------------------------------------------------ outputs of every chunk
 // A CTA owns 64 tokens x 64 value columns of one (chunk, head); a lane's tile is 8 x 4.
 #define DELTA_OUT_THREADS 128
-template <int DKP> constexpr int delta_out_smem() {
+constexpr int delta_out_smem() {
     return (DELTA_C * (DKP + 4) + DKP * (DELTA_OUT_COLS + 4) + DELTA_C * (DELTA_C + 4) + DELTA_C * (DELTA_OUT_COLS + 4)) * 4;
 }
 
-template <int DKP>
 __global__ void __launch_bounds__(DELTA_OUT_THREADS)
 delta_out_kernel(DeltaArgs a) {
     constexpr int C = DELTA_C, LD = DKP + 4, LS = DELTA_OUT_COLS + 4, LP = C + 4, NT = DELTA_OUT_THREADS, N = DELTA_DVT;
@@ -718,31 +711,26 @@ extern "C" long long braid_delta_work_floats(int rows, int n_seqs, int heads, in
     return delta_blocks(rows, n_seqs, heads) * (3 * DELTA_C * (dkp + 4) + DELTA_C * dvp + DELTA_C * DELTA_C + dkp + dkp * dvp);
 }
 
-template <typename T, int DKP>
+template <typename T>
 static int launch_delta_chunks(const DeltaArgs& a, int n_seqs, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(delta_intra_kernel<T, DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_intra_smem<DKP>());
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_state_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         delta_state_smem<DKP>() > DELTA_ALONE_SMEM ? delta_state_smem<DKP>() : DELTA_ALONE_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_out_kernel<DKP>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_out_smem<DKP>());
+        cudaError_t e = cudaFuncSetAttribute(delta_intra_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_intra_smem());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_state_smem());
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_out_smem());
         if (e != cudaSuccess) { braid_set_error("delta_rule: cannot reserve shared memory: %s", cudaGetErrorString(e)); return (int)e; }
         configured = true;
     }
     const int spans = (a.tiles * DELTA_DVT + DELTA_OUT_COLS - 1) / DELTA_OUT_COLS;
-    braid_launch(delta_intra_kernel<T, DKP>, dim3(a.heads, n_seqs, a.max_chunks), dim3(DELTA_INTRA_THREADS), delta_intra_smem<DKP>(), s, a);
-    // where one CTA an SM covers the step, each asks for more than half of an SM's shared memory: launched while the kernel before
-    // drains, they would otherwise settle two and more on the SMs that are free first (8 heads of 128 x 256: 287 -> 220 us in all)
-    const bool alone = (long long)a.heads * n_seqs * a.tiles <= 148;
-    const int state_smem = alone && delta_state_smem<DKP>() < DELTA_ALONE_SMEM ? DELTA_ALONE_SMEM : delta_state_smem<DKP>();
-    braid_launch(delta_state_kernel<DKP>, dim3(a.heads, n_seqs, a.tiles), dim3(DELTA_STATE_THREADS), state_smem, s, a);
-    braid_launch(delta_out_kernel<DKP>, dim3(a.heads, n_seqs, a.max_chunks * spans), dim3(DELTA_OUT_THREADS), delta_out_smem<DKP>(), s, a);
+    braid_launch(delta_intra_kernel<T>, dim3(a.heads, n_seqs, a.max_chunks), dim3(DELTA_INTRA_THREADS), (size_t)delta_intra_smem(), s, a);
+    braid_launch(delta_state_kernel, dim3(a.heads, n_seqs, a.tiles), dim3(DELTA_STATE_THREADS), (size_t)delta_state_smem(), s, a);
+    braid_launch(delta_out_kernel, dim3(a.heads, n_seqs, a.max_chunks * spans), dim3(DELTA_OUT_THREADS), (size_t)delta_out_smem(), s, a);
     BRAID_LAUNCH_CHECK();
 }
 
 template <typename T>
 static int launch_delta(const DeltaArgs& a, int n_seqs, bool chunked, cudaStream_t s) {
-    if (chunked) return launch_delta_chunks<T, DELTA_MAX_DK>(a, n_seqs, s);
+    if (chunked) return launch_delta_chunks<T>(a, n_seqs, s);
     const int rg = a.dk <= 32 ? 4 : a.dk <= 64 ? 8 : 16;
     const int dvt = (DELTA_WALK_THREADS / rg) * DELTA_CV;
     const dim3 grid(a.heads, n_seqs, (a.dv + dvt - 1) / dvt), block(DELTA_WALK_THREADS);

@@ -36,6 +36,13 @@ __device__ __forceinline__ float delta_decay(float x, float rate) {
 }
 __device__ __forceinline__ float delta_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
+__device__ __forceinline__ void delta_cp16(uint32_t smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void delta_cp16(void* smem, const void* gmem) { delta_cp16((uint32_t)__cvta_generic_to_shared(smem), gmem); }
+__device__ __forceinline__ void delta_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void delta_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // The form over chunks for dk <= 128 (delta_chunk.cu): its scratch, and its launches.
 long long dlc_floats(long long blocks, int dk, int dv);
 int dlc_launch(const DeltaArgs& a, int dtype, int n_seqs, long long blocks, float* work, cudaStream_t s);

@@ -288,11 +288,6 @@ delta_rows_kernel(const __grid_constant__ DeltaArgs a) {
     pdl_trigger();
 }
 
-__device__ __forceinline__ void dlc_cp16(uint32_t smem, const void* gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void dlc_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void dlc_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // The byte offset of 16-byte run `c` of row `r` in a tile of rows of RUNS runs: runs are swapped within their group of eight by the row's
 // low bits, so that eight rows of one run lie in eight different banks' quads.
 template <int RUNS>
@@ -329,18 +324,18 @@ delta_chain_kernel(const __grid_constant__ DeltaArgs a) {
         const uint8_t *w = (const uint8_t*)(a.wp + blk * (3 * C * DK)), *k = (const uint8_t*)(a.kp + blk * (3 * C * DK));
         const uint32_t to = (c & 1) * BUF;
 #pragma unroll 4
-        for (int idx = tid; idx < 3 * C * DK / 8; idx += NT) dlc_cp16(sW + to + dlc_at<C / 8>(idx / (C / 8), idx % (C / 8)), w + idx * 16);
-        if (tid < DK / 4) dlc_cp16(chk_u32(sD + (c & 1) * DK + tid * 4), a.gc + blk * DK + tid * 4);
-        dlc_commit();
+        for (int idx = tid; idx < 3 * C * DK / 8; idx += NT) delta_cp16(sW + to + dlc_at<C / 8>(idx / (C / 8), idx % (C / 8)), w + idx * 16);
+        if (tid < DK / 4) delta_cp16(chk_u32(sD + (c & 1) * DK + tid * 4), a.gc + blk * DK + tid * 4);
+        delta_cp_commit();
 #pragma unroll 4
-        for (int idx = tid; idx < 3 * C * DK / 8; idx += NT) dlc_cp16(sK + to + dlc_at<DK / 8>(idx / (DK / 8), idx % (DK / 8)), k + idx * 16);
-        dlc_commit();
+        for (int idx = tid; idx < 3 * C * DK / 8; idx += NT) delta_cp16(sK + to + dlc_at<DK / 8>(idx / (DK / 8), idx % (DK / 8)), k + idx * 16);
+        delta_cp_commit();
     };
     ask(0);
     for (int c = 0; c < n_chunks; ++c) {
         const size_t blk = block0 + c * step;
         if (c + 1 < n_chunks) ask(c + 1);                    // (its buffers were read before the last barrier)
-        else { dlc_commit(); dlc_commit(); }
+        else { delta_cp_commit(); delta_cp_commit(); }
         const uint32_t w = sW + (c & 1) * BUF, k = sK + (c & 1) * BUF;
         float4* U = reinterpret_cast<float4*>(a.u + blk * (size_t)(C * dvp)) + (size_t)tile * (C * 4) + lane * 2;
         float u0[8][4];                                      // value columns v0 (+ 8), tokens x * 8 + lq (+ 1)
@@ -350,7 +345,7 @@ delta_chain_kernel(const __grid_constant__ DeltaArgs a) {
         float4* sc = reinterpret_cast<float4*>(a.sc + blk * (size_t)(DK * dvp)) + (size_t)tile * (DK * 4) + k0 * 4 + lane * 2;
 #pragma unroll
         for (int x = 0; x < KT; ++x) sc[(x >> 1) * 64 + (x & 1)] = make_float4(S[x][0], S[x][1], S[x][2], S[x][3]);
-        dlc_wait<3>();
+        delta_cp_wait<3>();
         __syncthreads();                                     // this chunk's W
         float u[8][2][4];                                    // this half of S^T W^T: the products of the first parts, and the small ones
 #pragma unroll
@@ -390,7 +385,7 @@ delta_chain_kernel(const __grid_constant__ DeltaArgs a) {
             for (int e = 0; e < 4; ++e) u[x][0][e] += u[x][1][e];
             mine[x * 32] = make_float4(u[x][0][0], u[x][0][1], u[x][0][2], u[x][0][3]);
         }
-        dlc_wait<2>();
+        delta_cp_wait<2>();
         __syncthreads();                                     // the other half, and this chunk's k
         uint32_t ua[4][3][4];
 #pragma unroll
@@ -442,7 +437,7 @@ delta_chain_kernel(const __grid_constant__ DeltaArgs a) {
         __syncthreads();                                     // W, k and the halves have been read
     }
     pdl_trigger();
-    dlc_wait<0>();
+    delta_cp_wait<0>();
 #pragma unroll
     for (int x = 0; x < KT; ++x)
 #pragma unroll

@@ -12,10 +12,11 @@
 //
 // A CTA of sixteen warps owns 128 weight rows x N tokens and walks k 64 at a time through two stages: while the tensor cores work on one, the
 // warps fetch the next block's float32 numbers, read the accumulator of the block before, and split the numbers into the swizzled
-// operand tiles of the other stage.  Bound by the splits and the barrier between two blocks (1.5 us a block of 64 where tcgen05.mma takes
-// 6 N cycles).  Measured beside gemm_tile_kernel (FFMA at 0.4 of its rate), L2 flushed, us: 480 tokens 1536 x 1024 33 / 75, 1024 x 1024
-// 31 / 45, 5632 x 1024 78 / 175, 1024 x 2816 72 / 108; 2,048 tokens 5632 x 1024 187 / 633, 4096 x 4096 533 / 1,836; 17 tokens 1536 x 1024
-// 31 / 43, 32768 x 1024 61 / 133, 200 x 516 21 / 27.  With 8 warps instead of 16 a CTA 2,048 tokens of 5632 x 1024 take 254 us.
+// operand tiles of the other stage.  Bound by the splits and the barrier between two blocks (2.0 us a block of 64 with N = 128, of which the
+// tensor cores work 12 N cycles, 0.8 us).  Measured beside gemm_tile_kernel (FFMA at 0.4 of its rate), L2 flushed, us: 480 tokens 1536 x 1024
+// 33 / 75, 1024 x 1024 32 / 45, 5632 x 1024 79 / 175, 1024 x 2816 69 / 108; 2,048 tokens 5632 x 1024 183 / 633, 4096 x 4096 512 / 1,836; 17 tokens
+// 1536 x 1024 30 / 43, 32768 x 1024 59 / 133, 200 x 516 21 / 27.  With 8 warps instead of 16 a CTA 2,048 tokens of 5632 x 1024 took 254 us where
+// 16 took 187.
 #include "tcgen05.cuh"
 
 #define F3_BK 64
