@@ -1376,7 +1376,7 @@ class Kernels:
     @staticmethod
     def _settled(ctx) -> int:
         """Whether a kernel may read its state before the kernels ahead of it in the stream have ended (`StepContext.settled`): not
-        unless the step says so."""
+        unless the step says so.  `linear_scan`, `delta_rule` and `causal_conv` may be called in a row on one state otherwise."""
         return int(getattr(ctx, "settled", False))
 
     def causal_conv(self, x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], state: torch.Tensor,
