@@ -135,3 +135,14 @@ def test_steps_beyond_a_launch_go_on_to_the_walk(K, longest, dv, fits):
     ctx = types.SimpleNamespace(n_seqs=1, max_q_len=longest)
     assert K.scan_chunk_fits(x, x, x, out, state, 0, ctx, 64, dv) is fits
     assert K.f32_tc_pays(65535 * 32, 64, 128) and not K.f32_tc_pays(65535 * 32 + 1, 64, 128)
+
+
+@pytest.mark.parametrize("settled", [None, False, True])
+def test_cached_keys_are_read_early_only_where_the_caller_says_so(K, monkeypatch, settled):
+    monkeypatch.setattr(K, "latent_attention_library", lambda rank, rot: K.entries, raising=False)
+    K._error_flag = torch.zeros(8, dtype=torch.int32)
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32)
+    K.attn_latent_mma(torch.zeros(1, 2, 80, dtype=BF), torch.zeros(1, 2, 64, dtype=BF), torch.zeros(3, 1, 1, 64, 80, dtype=BF), i32(0, 1)[None],
+                      i32(0), i32(1), i32(70), i32(0), 1, 1, 64, None, 0.1, **({} if settled is None else {"settled": settled}))
+    name, args = K.entries.calls[-1]
+    assert name == "braid_latent_attn_mma" and args[-3] == int(bool(settled))        # (then the error flag and the stream)
