@@ -149,8 +149,9 @@ latent_prep_kernel(LatentPrepArgs a) {
         if (p < half) {
             const int i0 = a.adjacent ? 2 * p : p, i1 = a.adjacent ? 2 * p + 1 : p + half;
             const float x0 = to_f32(in[i0]), x1 = to_f32(in[i1]);
-            out[i0] = from_f32<T>(x0 * cs - x1 * sn);
-            out[i1] = from_f32<T>(x1 * cs + x0 * sn);
+            // (which product of a turn is rounded first is said here, not left to the form: a cached key has the same bits whatever step wrote it)
+            out[i0] = from_f32<T>(fmaf(x0, cs, -(x1 * sn)));
+            out[i1] = from_f32<T>(fmaf(x1, cs, x0 * sn));
         } else {
             const int i = a.rot_dims + (p - half);
             out[i] = in[i];

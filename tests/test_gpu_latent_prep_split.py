@@ -40,3 +40,28 @@ def test_rows_by_themselves(dtype, heads, dim, rot, rank, rot_dims, adjacent):
     for a, b in zip(*out):
         assert ((a.double() - b.double()).abs() <= step * a.double().abs() + 2.0 ** -20).all()
     assert out[0][0].abs().max() > 0
+
+
+@pytest.mark.parametrize("rows", [13, 65, 300])
+@pytest.mark.parametrize("adjacent", [False, True])
+def test_a_turn_is_rounded_the_same_in_every_form(rows, adjacent):
+    """x0 cos - x1 sin and x1 cos + x0 sin, the product with the cosine unrounded."""
+    K = get_kernels(verbose=False)
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    heads, dim, rot, rank, ps = 4, 16, 64, 64, 64
+    cols, pages = heads * (dim + rot), -(-rows // ps)
+    proj = torch.randn(rows, cols + rank + rot, device=DEV, generator=g)
+    inv_freq, positions = torch.rand(rot // 2, device=DEV, generator=g), torch.arange(rows, dtype=torch.int32, device=DEV)
+    cache = torch.zeros(pages, 1, 1, ps, rank + rot, device=DEV)
+    q_lat = torch.zeros(rows, heads, rank + rot, device=DEV)
+    K.latent_prep(proj, cols, torch.ones(rank, device=DEV), inv_freq, positions, torch.zeros_like(positions),
+                  torch.arange(pages, dtype=torch.int32, device=DEV)[None], cache, q_lat, heads, dim, rot, rank, rot, ps, 1e-6, adjacent=adjacent)
+    angle = positions.float()[:, None] * inv_freq
+    sn, cs = angle.sin()[:, None], angle.cos()[:, None]
+    part = lambda x: (x[..., ::2], x[..., 1::2]) if adjacent else (x[..., :rot // 2], x[..., rot // 2:])
+    keys = cache.view(-1, rank + rot)[:rows, None, rank:]
+    for x, y in ((proj[:, :cols].view(rows, heads, -1)[:, :, dim:], q_lat[:, :, rank:]), (proj[:, None, cols + rank:], keys)):
+        (x0, x1), (y0, y1) = part(x), part(y)
+        # (float64 holds the product and, all but never rounded twice, the sum)
+        assert torch.equal(y0, (x0.double() * cs.double() - (x1 * sn).double()).float())
+        assert torch.equal(y1, (x1.double() * cs.double() + (x0 * sn).double()).float())
