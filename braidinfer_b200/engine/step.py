@@ -110,7 +110,7 @@ class StepContext:
     def ready_for(self, tensor: torch.Tensor, part) -> torch.Tensor:
         """Complete `tensor` now, unless `part`, which reads it next, adds up the sum that is deferred on it."""
         d = self.deferred.get(tensor.data_ptr())
-        if d is not None and not (part.accepts_deferred and (d[1] != "normed" or part.accepts_normed)):
+        if d is not None and not (part.accepts_deferred and (d[1] != "normed" or getattr(part, "accepts_normed", False))):
             self.resolve(tensor)
         return tensor
 
